@@ -155,6 +155,23 @@ def lib():
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The CPython extension over the same library (``csrc/bind.cpp``); raise if it is not built."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (the extension links against the libraries torch has loaded)
+        try:
+            from . import _native as ext
+        except ImportError as e:
+            raise RuntimeError("calibquant_b200/_native.so is missing or does not load: build it with "
+                               f"`python -m calibquant_b200.build` ({e})") from e
+        _native = ext
+    return _native
+
+
 def check(status: int, where: str):
     """Map a negative status to the exception type the reference raises for that failure:
     assertion-like argument/shape problems -> AssertionError/ValueError-compatible

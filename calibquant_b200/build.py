@@ -5,7 +5,8 @@
 replaces the reference's ``qjl/setup.py`` (four torch CUDAExtensions with no arch
 flags): one shared object, no torch headers, one architecture.  Every ``csrc/*.cu`` is
 compiled to an object file of its own (in parallel, rebuilt only when it or a header
-changed) and the objects are linked into ``libcalibquant_b200.so``.
+changed) and the objects are linked into ``libcalibquant_b200.so``.  The CPython extension ``_native.so``
+(``csrc/bind.cpp``: tensor checks, allocation and the C calls without Python in between) is compiled beside them.
 """
 
 from __future__ import annotations
@@ -21,6 +22,8 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libcalibquant_b200.so")
+BIND_SRC = os.path.join(CSRC, "bind.cpp")
+NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -57,7 +60,20 @@ def _stale(target: str, deps) -> bool:
 
 
 def needs_build() -> bool:
-    return _stale(LIB_PATH, sources() + _headers())
+    return _stale(LIB_PATH, sources() + _headers()) or _stale(NATIVE_PATH, [BIND_SRC] + _headers())
+
+
+def _bind_command():
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[f"-I{i}" for i in inc], BIND_SRC, "-o", NATIVE_PATH, f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda",
+            "-ltorch_cpu", "-ltorch_python", f"-L{PKG_DIR}", "-l:libcalibquant_b200.so", "-Wl,-rpath,$ORIGIN"]
 
 
 def build_library(force: bool = False, verbose: bool = False, extra=()) -> str:
@@ -85,6 +101,11 @@ def build_library(force: bool = False, verbose: bool = False, extra=()) -> str:
     if verbose:
         print(" ".join(cmd), flush=True)
     subprocess.run(cmd, check=True)
+    if force or _stale(NATIVE_PATH, [BIND_SRC] + hdrs):
+        cmd = _bind_command()
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.run(cmd, check=True)
     return LIB_PATH
 
 

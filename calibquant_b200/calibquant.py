@@ -13,7 +13,7 @@ import ctypes
 import torch
 
 from . import ops
-from ._lib import check, lib
+from ._lib import check, lib, native
 from .ops import _dtype_enum, _need_cuda, _ptr, _stream, _workspace
 
 DATA_TYPE = torch.float16
@@ -81,16 +81,7 @@ def quant(x, bits, per_channel=False, scale=1, post_scale=False):
 def quant_encode(x, bits, scale=1):
     """Fused ``quant`` + ``encode``: x [B,T,H,D] -> (enc uint8 [B,H,T,D*bits/8], scale, zero_point)
     without materialising the codes (replaces ``patch_internvl.py:292-339`` per tensor)."""
-    _need_cuda(x)
-    x = _prep(x)
-    B, T, H, D = x.shape
-    s, zp = quant_params(x, bits, scale)
-    enc = torch.empty((B, H, T, D * bits // 8), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        rc = lib().cq_calib_quantize(_ptr(x), B, T, H, D, _strides3(x), bits, _dtype_enum(x), _ptr(s), _ptr(zp),
-                                     0, None, _ptr(enc), _stream())
-    check(rc, "cq_calib_quantize")
-    return enc, s, zp
+    return native().quant_encode(x, bits, scale)
 
 
 def encode(X: torch.Tensor, bits=BITS_KV, datum_per_elem=int(8 / BITS_KV)):
@@ -152,48 +143,9 @@ def decode_attention(q, state, k_fp, v_fp, bits, sys_len, normalize=None, mask=N
     With ``t_fp_dev`` (int32 device scalar) the live number of full-precision tokens is read on the device and
     ``k_fp``/``v_fp`` are the whole pre-allocated buffers, so that a captured CUDA graph serves every step.
     Returns [B,Hq,1,D] in bfloat16 as the reference does."""
-    from ._lib import U8DecodeArgs
-    _need_cuda(q, k_fp, v_fp)
-    B, Hq, _, D = q.shape
-    Hkv, t_fp = k_fp.shape[1], k_fp.shape[2]
-    normalize = (bits <= 2) if normalize is None else normalize
-    enc_k, enc_v = state["enc_k"].contiguous(), state["enc_v"].contiguous()
-    t_vis = enc_k.shape[2]
-    params = [state[n] for n in ("scale_key", "zero_point_key", "scale_value", "zero_point_value")]
-    hs = params[0].numel() // (B * D)
-    if hs not in (Hq, Hkv) or any(p.numel() != B * hs * D or p.dtype != q.dtype for p in params):
-        raise ValueError("scale / zero point must hold one row of D values per query head or per KV head")
-    params = [p.contiguous() for p in params]
-    for t in (k_fp, v_fp):
-        if t_fp and (t.stride(3) != 1 or t.stride(2) != D):
-            raise ValueError("k_fp / v_fp token rows must be contiguous")
-    q3 = q.reshape(B, Hq, D).contiguous()
-    mask2 = None
-    if mask is not None:
-        mask2 = mask.reshape(B, -1).to(q.dtype).contiguous()
-        if mask2.shape[1] != t_vis + t_fp:
-            raise ValueError(f"mask must cover {t_vis + t_fp} keys, got {mask2.shape[1]}")
-    out = torch.empty((B, Hq, 1, D), dtype=torch.bfloat16, device=q.device)
-    a = U8DecodeArgs(batch=B, n_q_heads=Hq, n_kv_heads=Hkv, head_dim=D, t_vis=t_vis, t_fp=t_fp, t_sys=sys_len,
-                     bits=bits, dtype=_dtype_enum(q), calibrate=int(bool(normalize)), n_scale_heads=hs, reserved=0,
-                     q=q3.data_ptr(), enc_k=enc_k.data_ptr(), enc_v=enc_v.data_ptr(),
-                     scale_key=params[0].data_ptr(), zero_point_key=params[1].data_ptr(),
-                     scale_value=params[2].data_ptr(), zero_point_value=params[3].data_ptr(),
-                     k_fp=k_fp.data_ptr() if t_fp else None, v_fp=v_fp.data_ptr() if t_fp else None,
-                     fp_stride_b=k_fp.stride(0), fp_stride_h=k_fp.stride(1),
-                     mask=mask2.data_ptr() if mask2 is not None else None,
-                     mask_stride_b=mask2.stride(0) if mask2 is not None else 0, out=out.data_ptr(),
-                     t_fp_dev=t_fp_dev.data_ptr() if t_fp_dev is not None else None)
-    if k_fp.stride() != v_fp.stride():
-        raise ValueError("k_fp and v_fp must share strides")
-    nbytes = lib().cq_u8_decode_attn_workspace_bytes(ctypes.byref(a))
-    if nbytes == 0:
-        raise ValueError("cq_u8_decode_attn rejects this request (sizes, head counts or more than 51200 keys)")
-    ws = _workspace(nbytes + 256, q.device)
-    with torch.cuda.device(q.device):
-        rc = lib().cq_u8_decode_attn(ctypes.byref(a), ctypes.c_void_p(ws.data_ptr() + 256), nbytes, _stream())
-    check(rc, "cq_u8_decode_attn")
-    return out
+    return native().u8_decode_attention(q, state["enc_k"], state["enc_v"], state["scale_key"], state["zero_point_key"],
+                                        state["scale_value"], state["zero_point_value"], k_fp, v_fp, bits, sys_len,
+                                        normalize, mask, t_fp_dev)
 
 
 def decode_attention_unfused(q, state, k_fp, v_fp, bits, sys_len, normalize=None):

@@ -12,7 +12,7 @@ import ctypes
 import torch
 
 from . import _lib
-from ._lib import DecodeArgs, check, lib
+from ._lib import DecodeArgs, check, lib, native
 
 _DTYPES = {torch.float16: _lib.CQ_DTYPE_F16, torch.bfloat16: _lib.CQ_DTYPE_BF16}
 
@@ -56,29 +56,14 @@ class _OnDevice:
             torch.cuda.set_device(self.prev)
 
 
-_workspaces = {}
 _decode_ws_bytes = {}      # problem extents -> bytes, so a decode loop asks the library once
 
 
 def _workspace(nbytes: int, device, stream_handle=None) -> torch.Tensor:
     """Grow-only scratch buffer per (device, stream), zeroed when created: its first word is
     the sticky device status the decode kernels set when a bounded wait runs out."""
-    # A capture reuses the buffer an eager warm-up call created (a fixed address the replays can use).  A buffer
-    # that has to be created while a CUDA graph is being captured lives in that graph's memory pool: it is kept
-    # for captures only, eager calls on the same stream never see it.
     stream = torch.cuda.current_stream(device).cuda_stream if stream_handle is None else stream_handle
-    capturing = bool(torch.cuda.is_current_stream_capturing())
-    key = (device.index, stream, False)
-    buf = _workspaces.get(key)
-    if capturing and (buf is None or buf.numel() < nbytes):
-        key = (device.index, stream, True)
-        buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        new = torch.zeros(max(nbytes, 256), dtype=torch.uint8, device=device)
-        if buf is not None:
-            new[:4].copy_(buf[:4])      # a sticky status survives the regrowth
-        _workspaces[key] = buf = new
-    return buf
+    return native().workspace(nbytes, device.index, stream)
 
 
 def device_status(device=None) -> int:
@@ -87,9 +72,8 @@ def device_status(device=None) -> int:
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else device
     stream = torch.cuda.current_stream(device).cuda_stream
     status = 0
-    for capturing in (False, True):
-        buf = _workspaces.get((device.index, stream, capturing))
-        if buf is not None and status == 0:
+    for buf in native().workspaces_of(device.index, stream):
+        if status == 0:
             status = int(buf[:4].view(torch.int32).item())
     return status
 
@@ -99,20 +83,9 @@ def pack_last_dim(data: torch.Tensor, group_size: int, bits: int):
 
     Returns (code int32 [B,nh,R,L*bits/32], scale [B,nh,R,L/g], mn [B,nh,R,L/g]).
     """
-    _need_cuda(data)
     assert data.dim() == 4
-    B, nh, R, L = data.shape
-    assert L % group_size == 0
-    data = data.contiguous()
-    rows = B * nh * R
-    code = torch.empty((B, nh, R, L * bits // 32), dtype=torch.int32, device=data.device)
-    scale = torch.empty((B, nh, R, L // group_size), dtype=data.dtype, device=data.device)
-    mn = torch.empty_like(scale)
-    with torch.cuda.device(data.device):
-        rc = lib().cq_pack_last_dim(_ptr(data), rows, L, group_size, bits, _dtype_enum(data),
-                                    _ptr(code), _ptr(scale), _ptr(mn), _stream())
-    check(rc, "cq_pack_last_dim")
-    return code, scale, mn
+    assert data.shape[3] % group_size == 0
+    return native().pack_last_dim(data, group_size, bits)
 
 
 def pack_k_per_channel(k: torch.Tensor, group_size: int, bits: int):
@@ -121,21 +94,9 @@ def pack_k_per_channel(k: torch.Tensor, group_size: int, bits: int):
 
     Returns (code [B,H,D,T*bits/32], scale [B,H,D,T/g], mn [B,H,D,T/g]).
     """
-    _need_cuda(k)
     assert k.dim() == 4
-    B, H, T, D = k.shape
-    assert T % group_size == 0
-    if k.stride(3) != 1 or any(s % 8 for s in k.stride()[:3]) or k.data_ptr() % 16:
-        k = k.contiguous()
-    code = torch.empty((B, H, D, T * bits // 32), dtype=torch.int32, device=k.device)
-    scale = torch.empty((B, H, D, T // group_size), dtype=k.dtype, device=k.device)
-    mn = torch.empty_like(scale)
-    with torch.cuda.device(k.device):
-        rc = lib().cq_pack_k_per_channel(_ptr(k), B, H, T, D, k.stride(0), k.stride(1), k.stride(2),
-                                         group_size, bits, _dtype_enum(k),
-                                         _ptr(code), _ptr(scale), _ptr(mn), _stream())
-    check(rc, "cq_pack_k_per_channel")
-    return code, scale, mn
+    assert k.shape[2] % group_size == 0
+    return native().pack_k_per_channel(k, group_size, bits)
 
 
 def pack_v_per_token(v: torch.Tensor, group_size: int, bits: int):
@@ -144,20 +105,8 @@ def pack_v_per_token(v: torch.Tensor, group_size: int, bits: int):
 
     Returns (code [B,H,T,D*bits/32], scale [B,H,T,D/g], mn [B,H,T,D/g]).
     """
-    _need_cuda(v)
     assert v.dim() == 4
-    B, H, T, D = v.shape
-    if v.stride(3) != 1 or any(s % 8 for s in v.stride()[:3]) or v.data_ptr() % 16:
-        v = v.contiguous()
-    code = torch.empty((B, H, T, D * bits // 32), dtype=torch.int32, device=v.device)
-    scale = torch.empty((B, H, T, D // group_size), dtype=v.dtype, device=v.device)
-    mn = torch.empty_like(scale)
-    with torch.cuda.device(v.device):
-        rc = lib().cq_pack_v_per_token(_ptr(v), B, H, T, D, v.stride(0), v.stride(1), v.stride(2),
-                                       group_size, bits, _dtype_enum(v),
-                                       _ptr(code), _ptr(scale), _ptr(mn), _stream())
-    check(rc, "cq_pack_v_per_token")
-    return code, scale, mn
+    return native().pack_v_per_token(v, group_size, bits)
 
 
 def qbmm(group_size: int, fA: torch.Tensor, qB: torch.Tensor, scales: torch.Tensor,
@@ -167,23 +116,7 @@ def qbmm(group_size: int, fA: torch.Tensor, qB: torch.Tensor, scales: torch.Tens
     fA [B,Hq,1,K]; qB [B,Hkv,K,N*bits/32]; scales, zeros [B,Hkv,K,N/g].  Hkv may equal Hq
     (operands already expanded, as the reference passes them) or divide it (GQA).
     """
-    _need_cuda(fA, qB, scales, zeros)
-    assert fA.dim() == 4 and qB.dim() == 4
-    B, Hq, M, K = fA.shape
-    if M != 1:
-        raise ValueError("only M == 1 (one query row) is implemented")
-    Hkv = qB.shape[1]
-    N = qB.shape[-1] * (32 // bits)
-    fA, qB = fA.contiguous(), qB.contiguous()
-    scales, zeros = scales.contiguous(), zeros.contiguous()
-    out = torch.empty((B, Hq, 1, N), dtype=fA.dtype, device=fA.device)
-    nbytes = lib().cq_qbmm_workspace_bytes(B, Hq, K, N)
-    ws = _workspace(nbytes, fA.device)      # its first word is the status word device_status() reads
-    with torch.cuda.device(fA.device):
-        rc = lib().cq_qbmm(_ptr(fA), _ptr(qB), _ptr(scales), _ptr(zeros), _ptr(out), B, Hq, Hkv,
-                           K, N, group_size, bits, _dtype_enum(fA), _ptr(ws), ws.numel(), _stream())
-    check(rc, "cq_qbmm")
-    return out
+    return native().qbmm(group_size, fA, qB, scales, zeros, bits)
 
 
 def decode_attention(q, k_pack, v_pack, k_fp, v_fp, t_sys, bits, group_size=32,
@@ -201,6 +134,8 @@ def decode_attention(q, k_pack, v_pack, k_fp, v_fp, t_sys, bits, group_size=32,
     lands in ``out`` (a host tensor; page-locked memory is written by the kernel itself) and the call
     returns once it is there.
     """
+    if q.is_cuda and _profile is None:
+        return native().decode_attention(q, k_pack, v_pack, k_fp, v_fp, t_sys, bits, group_size, calibrate, mask, out, t_fp, t_fp_dev)
     host = not q.is_cuda
     dev = (k_fp if k_fp is not None else k_pack[0]).device
     _need_cuda(*(() if host else (q,)), k_fp, v_fp, mask, *(k_pack or ()), *(v_pack or ()))
@@ -329,22 +264,7 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out=Non
     q [B,T,Hq,D], k/v [B,T,Hkv,D] (any batch/token/head strides that are multiples of 8 elements,
     channels contiguous) -> o [B,T,Hq,D] in q.dtype.
     """
-    _need_cuda(q, k, v)
-    B, T, Hq, D = q.shape
-    Hkv = k.shape[2]
-
-    def ok(t):
-        return t.stride(3) == 1 and all(s % 8 == 0 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0
-
-    q, k, v = (t if ok(t) else t.contiguous() for t in (q, k, v))
-    if out is None:
-        out = torch.empty((B, T, Hq, D), dtype=q.dtype, device=q.device)
-    arr = lambda t: (ctypes.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
-    with torch.cuda.device(q.device):
-        rc = lib().cq_prefill_attn(_ptr(q), _ptr(k), _ptr(v), _ptr(out), B, T, Hq, Hkv, D,
-                                   arr(q), arr(k), arr(v), arr(out), _dtype_enum(q), _stream())
-    check(rc, "cq_prefill_attn")
-    return out
+    return native().prefill_attention(q, k, v, out)
 
 
 def prefill_rope_split(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache=None, v_cache=None,
@@ -356,47 +276,7 @@ def prefill_rope_split(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache=N
     the fp caches ``k_cache``/``v_cache`` [B,Hkv,capacity,D] are given, every token outside
     ``[vis_start, vis_start+vis_len)`` is also written there (rotated key, value), the tokens after the
     span following the ones before it."""
-    _need_cuda(qkv, cos, sin)
-    B, T = qkv.shape[0], qkv.shape[1]
-    D = cos.shape[-1]
-    per_tok = n_kv_heads * (n_rep + 2) * D
-    if qkv.dim() != 3 or qkv.shape[2] != per_tok:
-        raise ValueError(f"qkv must be [B,T,{per_tok}], got {tuple(qkv.shape)}")
-    if qkv.stride(2) != 1 or qkv.stride(0) % 8 or qkv.stride(1) % 8 or qkv.data_ptr() % 16:
-        qkv = qkv.contiguous()
-    if cos.dtype != qkv.dtype or sin.dtype != qkv.dtype:
-        raise TypeError("qkv and rotary tables must share one dtype")
-    cos, sin = cos.contiguous(), sin.contiguous()
-    pos = None
-    if position_ids is not None:
-        pos = position_ids.reshape(-1, T)
-        if pos.shape[0] == 1 and B > 1:
-            pos = pos.expand(B, T)
-        if pos.dtype != torch.int64 or pos.shape[0] != B:
-            raise ValueError("position_ids must be int64 [B,T]")
-        pos = pos.contiguous()
-    if (k_cache is None) != (v_cache is None):
-        raise ValueError("give both caches or neither")
-    cap = sb = sh = 0
-    if k_cache is not None:
-        for t in (k_cache, v_cache):
-            if t.dtype != qkv.dtype or t.stride(3) != 1 or t.stride(2) != D:
-                raise ValueError("caches must be [B,Hkv,capacity,D] of the data dtype with contiguous token rows")
-        if k_cache.stride() != v_cache.stride():
-            raise ValueError("k_cache and v_cache must share strides")
-        cap, sb, sh = k_cache.shape[2], k_cache.stride(0), k_cache.stride(1)
-        if T - vis_len > cap:
-            raise ValueError(f"{T - vis_len} full-precision tokens do not fit a cache of {cap}")
-    q = torch.empty((B, T, n_kv_heads * n_rep, D), dtype=qkv.dtype, device=qkv.device)
-    k = torch.empty((B, T, n_kv_heads, D), dtype=qkv.dtype, device=qkv.device)
-    with torch.cuda.device(qkv.device):
-        rc = lib().cq_prefill_rope_split(_ptr(qkv), qkv.stride(0), qkv.stride(1), _ptr(cos), _ptr(sin), cos.shape[0],
-                                         _ptr(pos), B, T, n_kv_heads, n_rep, D, _ptr(q), _ptr(k), _ptr(k_cache),
-                                         _ptr(v_cache), sb, sh, cap, int(vis_start), int(vis_len),
-                                         _dtype_enum(qkv), _stream())
-    check(rc, "cq_prefill_rope_split")
-    v = qkv.view(B, T, n_kv_heads, n_rep + 2, D)[:, :, :, n_rep + 1]
-    return q, k, v
+    return native().prefill_rope_split(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, vis_start, vis_len)
 
 
 def rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache,
@@ -407,39 +287,7 @@ def rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v
     ``k_cache``/``v_cache`` [B,Hkv,capacity,D] at token ``append_index`` -- or at ``t_fp_dev - 1`` when
     the live token count is the int32 device scalar ``t_fp_dev`` (which then already counts the new
     token).  Returns the rotated queries [B,Hq,1,D]."""
-    _need_cuda(qkv, cos, sin, position_ids, k_cache, v_cache)
-    B = qkv.shape[0]
-    D = cos.shape[-1]
-    qkv2 = qkv.reshape(B, -1)
-    if qkv2.stride(1) != 1:
-        qkv2 = qkv2.contiguous()
-    if qkv2.shape[1] != n_kv_heads * (n_rep + 2) * D:
-        raise ValueError(f"qkv rows must hold {n_kv_heads * (n_rep + 2) * D} elements, got {qkv2.shape[1]}")
-    if cos.dtype != qkv.dtype or sin.dtype != qkv.dtype or k_cache.dtype != qkv.dtype:
-        raise TypeError("qkv, rotary tables and caches must share one dtype")
-    cos, sin = cos.contiguous(), sin.contiguous()
-    pos = position_ids.reshape(-1)
-    if pos.dtype != torch.int64 or pos.numel() != B:
-        raise ValueError("position_ids must be int64 with one position per batch row")
-    pos = pos.contiguous()
-    for t in (k_cache, v_cache):
-        if t.stride(3) != 1 or t.stride(2) != D:
-            raise ValueError("cache token rows must be contiguous ([.., T, D] with stride D)")
-    if k_cache.stride() != v_cache.stride():
-        raise ValueError("k_cache and v_cache must share strides")
-    if (append_index is None) == (t_fp_dev is None):
-        raise ValueError("give exactly one of append_index and t_fp_dev")
-    if t_fp_dev is not None:
-        assert t_fp_dev.dtype == torch.int32 and t_fp_dev.is_cuda
-    q_out = torch.empty((B, n_kv_heads * n_rep, 1, D), dtype=qkv.dtype, device=qkv.device)
-    with torch.cuda.device(qkv.device):
-        rc = lib().cq_rope_split_append(_ptr(qkv2), qkv2.stride(0), _ptr(cos), _ptr(sin), cos.shape[0], _ptr(pos),
-                                        B, n_kv_heads, n_rep, D, _ptr(q_out), _ptr(k_cache), _ptr(v_cache),
-                                        k_cache.stride(0), k_cache.stride(1), k_cache.shape[2],
-                                        0 if append_index is None else int(append_index), _ptr(t_fp_dev),
-                                        _dtype_enum(qkv), _stream())
-    check(rc, "cq_rope_split_append")
-    return q_out
+    return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev)
 
 
 def add_rmsnorm(residual, delta, weight, eps, out=None, normalize=True):
