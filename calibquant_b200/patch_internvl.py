@@ -132,13 +132,17 @@ class _TextCache:
         self.length = length
         return self
 
-    def append(self, k, v):
-        n = k.shape[2]
+    def reserve(self, n):
+        """Room for ``n`` more tokens."""
         if self.length + n > self.k.shape[2]:
             grow = max(TEXT_CAPACITY_STEP, n)
             pad = torch.empty((*self.k.shape[:2], grow, self.k.shape[3]), dtype=self.k.dtype, device=self.k.device)
             self.k = torch.cat([self.k, pad], dim=2)
             self.v = torch.cat([self.v, pad.clone()], dim=2)
+
+    def append(self, k, v):
+        n = k.shape[2]
+        self.reserve(n)
         self.k[:, :, self.length:self.length + n] = k
         self.v[:, :, self.length:self.length + n] = v
         self.length += n
@@ -292,37 +296,47 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
         attn_output = self.wo(attn.reshape(bsz, q_len, -1))
         return attn_output, None, past_key_value
 
-    q, k, v = _split_qkv(self, hidden_states)
-    q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)          # [B,H,q,D] views
+    # ---- decode step -------------------------------------------------------------------------
     kv_seq_len = q_len
     if past_key_value is not None:
         kv_seq_len += past_key_value[0].shape[-2] + (self.image_token_num if LOW_BITS else 0)
-    cos, sin = self.rotary_emb(v, seq_len=kv_seq_len)
-    q, k = apply_rotary_pos_emb(q, k, cos, sin, position_ids)
-
-    # ---- decode step -------------------------------------------------------------------------
-    self._text_cache.append(k, v)
-    k_fp, v_fp = self._text_cache.views()
-    past_key_value = (k_fp, v_fp) if use_cache else None
+    tc = self._text_cache
+    cos, sin = self.rotary_emb(hidden_states, seq_len=kv_seq_len)
+    if self.head_dim == 128 and cos.dtype == sin.dtype == hidden_states.dtype == tc.k.dtype:
+        # one launch splits the projection, rotates q and k and appends k, v to the text cache (the torch ops
+        # below are ~15 launches, which took longer to issue than the whole step takes on the GPU)
+        n_rep = self.num_key_value_groups
+        tc.reserve(1)
+        pos = position_ids if position_ids.numel() == bsz else position_ids.expand(bsz, 1)
+        q = ops.rope_split_append(self.wqkv(hidden_states), cos, sin, pos,
+                                  self.wqkv.out_features // ((n_rep + 2) * self.head_dim), n_rep, tc.k, tc.v,
+                                  append_index=tc.length)
+        tc.length += 1
+    else:      # rotary tables of another type than the hidden states
+        q, k, v = _split_qkv(self, hidden_states)
+        q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)          # [B,H,q,D] views
+        q, k = apply_rotary_pos_emb(q, k, cos, sin, position_ids)
+        tc.append(k, v)
+    past_key_value = tc.views() if use_cache else None
     if attention_mask is not None and attention_mask.size() != (bsz, 1, q_len, kv_seq_len):
         raise ValueError(f"Attention mask should be of size {(bsz, 1, q_len, kv_seq_len)}, "
                          f"but is {attention_mask.size()}")
     t_sys = self.sprompt_len if LOW_BITS else 0
     if getattr(self, "_u8_state", None) is not None:
         from . import calibquant as _cq
+        k_fp, v_fp = past_key_value or tc.views()
         attn = _cq.decode_attention(q, self._u8_state, k_fp, v_fp, BITS_KV, t_sys, normalize=self.normalize,
                                     mask=attention_mask).to(q.dtype)             # bfloat16 out, as the reference
     else:
-        attn = ops.decode_attention(q, self.k_pack, self.v_pack, k_fp, v_fp, t_sys, BITS_KV,
+        attn = ops.decode_attention(q, self.k_pack, self.v_pack, tc.k, tc.v, t_sys, BITS_KV,
                                     group_size=GROUP_SIZE, calibrate=self.normalize and LOW_BITS,
-                                    mask=attention_mask)                         # [B,Hq,1,D]
+                                    mask=attention_mask, t_fp=tc.length)         # [B,Hq,1,D]
     local_heads = self.num_heads // _shard_world(self)
     if attn.size() != (bsz, local_heads, q_len, self.head_dim):
         raise ValueError(f"`attn_output` should be of size {(bsz, local_heads, q_len, self.head_dim)}, "
                          f"but is {attn.size()}")
-    attn = _gather_heads(self, attn.transpose(1, 2).reshape(bsz, q_len, -1))
-    attn_output = self.wo(attn.reshape(bsz, q_len, -1))
-    return attn_output, None, past_key_value
+    attn = _gather_heads(self, attn.view(bsz, q_len, -1))
+    return self.wo(attn), None, past_key_value
 
 
 def forward_internlm2_qjl(self, hidden_states: torch.Tensor,
