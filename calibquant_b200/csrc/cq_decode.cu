@@ -438,6 +438,7 @@ static int run_decode_bits(const cq_decode_args* a, const DecodeDims& dm, const 
 
 extern "C" size_t cq_decode_attn_workspace_bytes(const cq_decode_args* args) {
   if (cq::validate(args) != CQ_OK) return 0;
+  if (cq::cluster_path_eligible(args)) return 256;
   if (cq::mma_path_eligible(args)) return cq::mma_path_workspace_bytes(args);
   return cq::make_layout(cq::make_dims(args)).total;
 }
@@ -447,6 +448,10 @@ static int decode_attn_impl(const cq_decode_args* args, void* workspace, size_t 
   int rc = cq::validate(args);
   if (rc != CQ_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (cq::cluster_path_eligible(args)) {
+    if (!workspace || workspace_bytes < 256 || !cq::aligned16(workspace)) return CQ_ERR_WORKSPACE;
+    return cq::cluster_path_run(args, workspace, st, status_word);
+  }
   if (cq::mma_path_eligible(args)) {
     if (!workspace || workspace_bytes < cq::mma_path_workspace_bytes(args) || !cq::aligned16(workspace))
       return CQ_ERR_WORKSPACE;
@@ -474,13 +479,20 @@ extern "C" int cq_decode_attn_profile(const cq_decode_args* args, void* workspac
   int rc = cq::validate(args);
   if (rc != CQ_OK) return rc;
   if (!cq::mma_path_eligible(args)) return CQ_ERR_UNSUPPORTED;
-  if (!workspace || workspace_bytes < cq::mma_path_workspace_bytes(args) || !cq::aligned16(workspace))
+  const bool one_launch = cq::cluster_path_eligible(args);
+  if (!workspace || workspace_bytes < (one_launch ? 256 : cq::mma_path_workspace_bytes(args)) || !cq::aligned16(workspace))
     return CQ_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaEvent_t ev[5] = {};
   for (int i = 0; i < 5; ++i)
     if (cudaEventCreate(&ev[i]) != cudaSuccess) rc = CQ_ERR_LAUNCH;
-  if (rc == CQ_OK) rc = cq::mma_path_run(args, workspace, st, ev);
+  if (rc == CQ_OK && one_launch) {
+    cudaEventRecord(ev[0], st);
+    rc = cq::cluster_path_run(args, workspace, st);
+    for (int i = 1; i < 5; ++i) cudaEventRecord(ev[i], st);
+  } else if (rc == CQ_OK) {
+    rc = cq::mma_path_run(args, workspace, st, ev);
+  }
   if (rc == CQ_OK && cudaEventSynchronize(ev[4]) != cudaSuccess) rc = CQ_ERR_LAUNCH;
   for (int i = 0; i < 4 && rc == CQ_OK; ++i)
     if (cudaEventElapsedTime(&launch_ms[i], ev[i], ev[i + 1]) != cudaSuccess) rc = CQ_ERR_LAUNCH;

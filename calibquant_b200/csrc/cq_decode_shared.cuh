@@ -18,6 +18,9 @@ size_t mma_path_workspace_bytes(const cq_decode_args* args);
 int mma_path_run(const cq_decode_args* args, void* workspace, cudaStream_t stream, cudaEvent_t* events = nullptr,
                  int* status_word = nullptr);
 
+// The whole step in one launch (cq_decode_cluster.cu): spans whose logits fit the shared memory of a cluster.
+bool cluster_path_eligible(const cq_decode_args* args);
+int cluster_path_run(const cq_decode_args* args, void* workspace, cudaStream_t stream, int* status_word = nullptr);
 
 // The stand-alone quantized product (cq_qbmm) on the same kernels.  mma_qbmm_kind returns 0 when the
 // shapes or pointers are not ones the fast kernels take, 1 for the "q.K" use (K == 128) and 2 for the

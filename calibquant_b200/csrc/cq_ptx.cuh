@@ -41,6 +41,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
+// The same for N = 4, 8 or 16 bytes.
+template <int N>
+__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(N), "r"(src_bytes) : "memory");
+}
 // The mbarrier receives one arrival when all cp.async copies this thread has issued so far have completed; the
 // arrival is counted against the barrier's expected count (no increment of the pending count).
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {

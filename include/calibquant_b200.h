@@ -193,7 +193,8 @@ int cq_decode_attn(const cq_decode_args* args, void* workspace, size_t workspace
  * Per-launch device times of one step, for profiling (no reference counterpart: the reference has no
  * timers).  Runs the step exactly as cq_decode_attn does, with CUDA events recorded on `stream` between
  * its launches, waits for the last one and fills launch_ms[4] = {scores, attn.V, attn.V of the
- * full-precision tokens, combine} in milliseconds.  Only for requests the tensor-core kernels take
+ * full-precision tokens, combine} in milliseconds; where the step is a single launch (see cq_decode_attn) its time
+ * is launch_ms[0] and the others are what two event records in a row show.  Only for requests the tensor-core kernels take
  * (t_vis > 0, 16-byte aligned operands); CQ_ERR_UNSUPPORTED otherwise.  Synchronises.
  */
 int cq_decode_attn_profile(const cq_decode_args* args, void* workspace, size_t workspace_bytes,
