@@ -395,8 +395,8 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const size_t nbytes = cq_u8_decode_attn_workspace_bytes(&d);
   if (nbytes == 0)
     raise(PyExc_ValueError, "cq_u8_decode_attn rejects this request (sizes, head counts or more than 51200 keys)");
-  const Tensor ws = workspace((int64_t)nbytes + 256, q.get_device(), call.stream);
-  check(cq_u8_decode_attn(&d, (char*)ws.data_ptr() + 256, nbytes, call.stream), "cq_u8_decode_attn");
+  const Tensor ws = workspace((int64_t)nbytes, q.get_device(), call.stream);
+  check(cq_u8_decode_attn(&d, ws.data_ptr(), (size_t)ws.numel(), call.stream), "cq_u8_decode_attn");
   return wrap(out);
   CQ_END
 }

@@ -15,6 +15,8 @@
 
 #include "cq_common.cuh"
 #include "cq_ptx.cuh"
+#include "cq_u8_cluster.cuh"
+#include "cq_u8_format.cuh"
 
 namespace cq {
 namespace calib {
@@ -464,46 +466,7 @@ using namespace ptx;
 // byte 2 (or 3); the channel each k index stands for follows from that, and B is gathered to match.
 // A field at bit p of a half is the fp16 subnormal code * 2^(p-24); B carries 2^(4-p), so every
 // product weighs 2^-20.
-template <int BITS>
-struct LutMap {
-  // channel that k-block kb, lane column c, slot (0: a0.lo, 1: a0.hi, 2: a2.lo, 3: a2.hi) reads, and the
-  // bit position of its field inside the 16-bit half
-  static __device__ __forceinline__ void get(int kb, int c, int slot, int& chan, int& pos) {
-    if (BITS == 1) {             // word j = kb/2 (32 channels), bytes s, s+2 with s = kb%2
-      const int j = kb >> 1, s = kb & 1;
-      const int byte = s + 2 * (slot & 1);
-      pos = 2 * c + (slot >> 1);
-      chan = 32 * j + 8 * byte + (7 - pos);
-    } else if (BITS == 2) {      // word kb (16 channels): a0 from bytes 0,2, a2 from bytes 1,3; field c
-      const int byte = (slot >> 1) + 2 * (slot & 1);
-      pos = 2 * c;
-      chan = 16 * kb + 4 * byte + (3 - c);
-    } else {                     // words 2kb (a0) and 2kb+1 (a2), 8 channels each; nibble (c&1) of byte c>>1 (+2)
-      const int word = 2 * kb + (slot >> 1);
-      const int byte = (c >> 1) + 2 * (slot & 1);
-      pos = 0;                   // shifted down to bit 0 before masking
-      chan = 8 * word + 2 * byte + (1 - (c & 1));
-    }
-  }
-};
-
 constexpr int LS_TOK = 64;       // tokens per warp iteration (4 m-tiles)
-
-// Score type of the fused decode step: `fused_kernel(...) / sd - bias_k` is an fp16 tensor minus a tensor of
-// the data dtype, so torch keeps fp16 for fp16 data and promotes to fp32 for bf16 data.
-template <typename T> struct StepScore;
-template <> struct StepScore<__half> {
-  using type = __half;
-  static __device__ __forceinline__ float r(float v) { return rnd<__half>(v); }
-  static __device__ __forceinline__ __half make(float v) { return __float2half_rn(v); }
-  static __device__ __forceinline__ float load(__half v) { return __half2float(v); }
-};
-template <> struct StepScore<__nv_bfloat16> {
-  using type = float;
-  static __device__ __forceinline__ float r(float v) { return v; }
-  static __device__ __forceinline__ float make(float v) { return v; }
-  static __device__ __forceinline__ float load(float v) { return v; }
-};
 
 __device__ __forceinline__ void put_score(__half& dst, float v) { dst = __float2half_rn(v); }
 __device__ __forceinline__ void put_score(float& dst, float v) { dst = v; }
@@ -1306,7 +1269,7 @@ StepLayout step_layout(const cq_u8_decode_args* a) {
   StepLayout l{};
   const size_t rows = (size_t)a->batch * a->n_q_heads;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  size_t off = 0;
+  size_t off = 256;      // the first word is the sticky device status
   l.scores = off; off = up(off + rows * (size_t)a->t_vis * 4);
   l.a_vis = off;  off = up(off + rows * (size_t)a->t_vis * 2);
   l.a_fp = off;   off = up(off + rows * (size_t)a->t_fp * 2);
@@ -1338,7 +1301,7 @@ int step_check(const cq_u8_decode_args* a) {
 
 extern "C" size_t cq_u8_decode_attn_workspace_bytes(const cq_u8_decode_args* a) {
   if (step_check(a) != CQ_OK) return 0;
-  return step_layout(a).total;
+  return u8_cluster_eligible(a) ? 256 : step_layout(a).total;
 }
 
 template <typename T>
@@ -1404,8 +1367,10 @@ static int launch_step(const cq_u8_decode_args* a, char* ws, cudaStream_t st) {
 extern "C" int cq_u8_decode_attn(const cq_u8_decode_args* a, void* workspace, size_t workspace_bytes, void* stream) {
   const int rc = step_check(a);
   if (rc != CQ_OK) return rc;
-  if (!workspace || workspace_bytes < step_layout(a).total) return CQ_ERR_WORKSPACE;
+  const bool one_launch = u8_cluster_eligible(a);
+  if (!workspace || workspace_bytes < (one_launch ? 256 : step_layout(a).total)) return CQ_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (one_launch) return u8_cluster_run(a, workspace, st);
   if (a->dtype == CQ_DTYPE_F16) return launch_step<__half>(a, static_cast<char*>(workspace), st);
   return launch_step<__nv_bfloat16>(a, static_cast<char*>(workspace), st);
 }

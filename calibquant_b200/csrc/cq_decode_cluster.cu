@@ -21,6 +21,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "cq_cluster.cuh"
 #include "cq_decode_shared.cuh"
 #include "cq_decode_tile.cuh"
 
@@ -28,6 +29,8 @@ namespace cq {
 namespace mma {
 
 namespace cl {
+
+using namespace cluster;
 
 constexpr int NW = 8, THREADS = NW * 32;        // 16 warps per SM in two CTAs: 128 registers per thread
 constexpr int UNIT_TOK = 256, UNIT_G = 8;       // tokens / groups of a unit
@@ -53,38 +56,6 @@ struct Args {
   const void* mask;
 };
 
-// ---- cluster helpers -----------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t map_peer(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_peer(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_peer2(uint32_t addr, float a, float b) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
-}
-__device__ __forceinline__ void arrive_peer(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool wait_peers(uint64_t* bar, uint32_t max_tries) {      // phase 0, writes of the peers visible
-  for (uint32_t i = 0; i < max_tries; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)) : "memory");
-    if (ok) return true;
-    if (i > 64) __nanosleep(64);
-  }
-  return false;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
@@ -794,7 +765,7 @@ inline bool make_plan(const cq_decode_args* a, Plan* p) {
     if (S > n_units || (pairs * S <= sms && n_units > 8 * S)) continue;
     const int pitch = (n_units + S - 1) / S * UNIT_TOK + 8;
     const int64_t smem = 1024 + ring_bytes(a->bits) + (int64_t)n_rep * pitch * 2;
-    if (smem <= SMEM_TWO && pairs * S <= 2 * (int64_t)sms) { p->S = S; p->pitch = pitch; p->smem = (int)smem; return true; }
+    if (smem <= SMEM_TWO && pairs <= max_clusters(S)) { p->S = S; p->pitch = pitch; p->smem = (int)smem; return true; }
   }
   return false;
 }

@@ -179,7 +179,9 @@ typedef struct cq_decode_args {
 
 /*
  * Stream semantics: everything the call enqueues is ordered after the work already in `stream` and before
- * anything enqueued in it afterwards.  With full-precision tokens present, the tensor-core path runs their launch
+ * anything enqueued in it afterwards.  A step whose logits fit the shared memory of the clusters that are resident
+ * together (one cluster of up to 8 CTAs per KV head) is ONE launch.  Larger ones take three, and with full-precision
+ * tokens present the tensor-core path then runs their launch
  * on an internal side stream (one per host thread and device, created on first use) between two events recorded
  * in `stream` and in the side stream; under stream capture this records two parallel branches that join before the
  * last launch.  Make the first call on a device outside any capture.  The launches carry the
@@ -286,15 +288,16 @@ int cq_lut_out(const void* lut, const void* weights, const uint8_t* enc, void* o
                size_t workspace_bytes, void* stream);
 
 /*
- * cq_u8_decode_attn: one decode step of attention on this format, four launches (no reference entry point
- * of its own: it replaces the eager sequence patch_internvl.py:356-436 -- scores of the system and text
+ * cq_u8_decode_attn: one decode step of attention on this format, a single launch where the scores of a KV head
+ * fit the shared memory of a cluster, else four (no reference entry point of its own: it replaces the eager sequence patch_internvl.py:356-436 -- scores of the system and text
  * tokens, `fused_kernel(q * scale_key) / sqrt(D) - bias_k`, logit calibration :376-385, fp32 softmax,
  * `fused_kernel_wv(att) * scale_value - scale_value*zero_point_value*sum(att)`, the full-precision
  * products and the final cast to bfloat16 :436).
  *   q [B,Hq,D]; enc_k, enc_v uint8 [B,Hkv,t_vis,D*bits/8] (16-byte aligned);
  *   scale_*, zero_point_* [B,Hs,D] in the data dtype with Hs = n_scale_heads = Hq (as the reference keeps
  *   them, repeated per query head) or Hkv;  k_fp/v_fp as in cq_decode_args, tokens [sys | text];
- *   out [B,Hq,D] bfloat16 whatever the data dtype.  (t_vis + t_fp) * 4 bytes must fit 200 KB of shared
+ *   out [B,Hq,D] bfloat16 whatever the data dtype.  The first word of the workspace is a sticky status word as in
+ *   cq_decode_attn.  (t_vis + t_fp) * 4 bytes must fit 200 KB of shared
  *   memory (51 200 keys); larger requests return CQ_ERR_UNSUPPORTED.
  */
 typedef struct cq_u8_decode_args {
