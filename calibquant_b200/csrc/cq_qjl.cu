@@ -11,7 +11,7 @@
 // (token, block of 32 projections); the sign sums run over "bit set" terms only:
 // sum_p sgn_p x_p = 2 sum_{bit_p} x_p - sum_p x_p.  They serve unaligned buffers and sketch dims that are
 // not multiples of 128; otherwise quant_mma_kernel (persistent, projection resident in shared memory) and
-// score_mma_kernel (sign sums on the warp MMA, several groups per CTA) run.
+// score_rows_kernel (outlier projection and sign sums on the warp MMA, a group per warp) run.
 #include "cq_common.cuh"
 #include "cq_ptx.cuh"
 
@@ -200,172 +200,263 @@ score_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ 
   }
 }
 
-// The same estimate on the warp MMA (sketch dims multiples of 128).
-// One CTA walks GPC consecutive groups of one (batch, KV head); per group and chunk of 32 tokens:
-//   1. thread = projection p: the query-side terms x_p = (q S - q_out S)_p and (q_out S)_p per head, stored as
-//      fp16 pairs hi = fp16(x), lo = fp16(x - hi) in B-fragment order (the fp32 accumulator then holds the
-//      fp32-rounded sum).  With at most four query heads per KV head hi and lo share the eight MMA columns,
-//      otherwise two MMAs per step.
-//   2. eight warp tasks = (16-token tile) x (inlier | outlier sketch) x (half of the projections):
-//      A = the signs of 16 tokens x 16 projections as +-2^-24 (fp16 subnormal with the sign bit from the
-//      packed bit), so the MMA sums  sgn_p x_p  directly.
-//   3. thread = (token, head): norms, scale, store.
-// The B fragments and the partial sums are double-buffered: two CTA barriers per group; the sketch words
-// of the next group and the norms of this one are fetched before step 1.
-constexpr int GPC = 8;                  // groups per CTA
-constexpr int B_PITCH = 132;            // words per B-fragment column: lanes (g, c) of a fragment load hit 32 banks
+// The same estimate on the warp MMA (sketch dims that are multiples of 128), persistent: one CTA of 16 warps per SM keeps
+// the projection in shared memory as fp16 hi/lo rows (hi = fp16(x), lo = fp16(x - hi): fp32-exact sums), every warp works
+// off (group, 32 tokens) items by itself, without a CTA barrier.
+//
+// What bounded the earlier form: the query's outlier projection q_out S, which every group needs for its own 32 outlier
+// channels, as 32 x 256 x n_rep FMAs with an indexed load each (2650 cycles per group and SM, issue-bound), and two CTA
+// barriers per group.  Here it is a product with gathered rows: B = rows of S picked by ldmatrix (the row addresses ARE the
+// gather), A = the query's outlier channels; its accumulators (row = head, columns = projections 2c, 2c+1) are the layout
+// the sign product wants its B operand in, so nothing passes through shared memory.  Lanes g < 4 keep the fp16 value, lanes
+// g >= 4 the remainder of the same head (rows 4-7 of A repeat rows 0-3); with five to eight heads both are kept and the sign
+// product runs twice.
+//   * k-step b takes bits b and b + 16 of every sign word of a token: lane c needs only its words c and c + 4, and an operand
+//     register costs one shift and one LOP3.  The table's columns are in that order.
+//   * sum sgn (q S - q_out S) is summed as sum sgn (q S) - sum sgn (q_out S): the first operand is made once per KV head, the
+//     second serves both sketches.
+//   * The rows of an 8 x 8 matrix hit the bank group (channel mod 8): the 32 channels are dealt over the four matrices of a
+//     load by rank within their residue class (the order of the contraction is free).
+constexpr int SW = 16, STHREADS = SW * 32;
+constexpr int S_PITCH = MAX_SKETCH + 8;               // halves per projection row: channel d starts in bank group d % 8
+constexpr int S_TAB_BYTES = 2 * kHeadDim * S_PITCH * 2;
+constexpr int S_SIGN_BYTES = 2 * 32 * (MAX_SKETCH / 8);          // signs of 32 tokens, both sketches
+constexpr int S_QF_BYTES = (MAX_SKETCH / 16) * 32 * 8;           // fragments of q S: [k-step][lane] x (b0, b1)
+constexpr int S_SMEM = S_TAB_BYTES + SW * 2 * S_SIGN_BYTES + 2 * S_QF_BYTES + kMaxRep * kHeadDim * 2 + SW * 64;
+
+// projection at position 16 b + 8 half + 2 c + e of a table row: bit b + 16 e of word c + 4 half (256 projections), or
+// bit b + 8 half + 16 e of word c (128 projections)
+__device__ __forceinline__ int sign_proj(int pos, int sketch) {
+  const int b = pos >> 4, half = (pos >> 3) & 1, c = (pos >> 1) & 3, e = pos & 1;
+  return sketch == 256 ? 32 * (c + 4 * half) + b + 16 * e : 32 * c + b + 8 * half + 16 * e;
+}
 
 template <typename T, typename TP, int R>
-__global__ void __launch_bounds__(THREADS)
-score_mma_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ key_outlier_quant,
-                 const T* __restrict__ key_norm, const T* __restrict__ key_outlier_norm,
-                 const uint8_t* __restrict__ outlier_idx, const float* __restrict__ query_sketch,
-                 const T* __restrict__ query, const TP* __restrict__ proj_score, float* __restrict__ scores,
-                 int n_groups, int G, int n_rep, int sketch, int o_sketch, int oc) {
-  constexpr int NV = R / 4;                                  // fragment arrays per sketch: hi|lo in one, or hi and lo
-  __shared__ __align__(16) float qd_s[kHeadDim][R];          // query values [channel][head]
-  __shared__ __align__(16) __half b_s[2][2][NV][8][B_PITCH * 2];           // [buffer][in|out][hi|lo][column][projection]
-  __shared__ float part_s[2][2][32][2 * R + 1];              // [buffer][projection half][token][in heads | out heads]
-  __shared__ uint8_t otl_s[GPC][kHeadDim];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
-  const int64_t kbh = blockIdx.x;
-  const int n0 = blockIdx.y * GPC, n_here = min(GPC, n_groups - n0);
-  const int tok0 = blockIdx.z * 32;
-  const int n_tok = min(32, G - tok0);
-  const int64_t qrow0 = kbh * n_rep;
-  for (int i = tid; i < R * kHeadDim; i += THREADS) {
-    const int r = i >> 7, d = i & (kHeadDim - 1);
-    qd_s[d][r] = r < n_rep ? Elem<T>::to_f(query[(qrow0 + r) * kHeadDim + d]) : 0.f;
+__global__ void __launch_bounds__(STHREADS, 1)
+score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ key_outlier_quant,
+                  const T* __restrict__ key_norm, const T* __restrict__ key_outlier_norm,
+                  const uint8_t* __restrict__ outlier_idx, const float* __restrict__ query_sketch,
+                  const T* __restrict__ query, const TP* __restrict__ proj_score, float* __restrict__ scores,
+                  int n_kbh, int n_groups, int G, int n_rep, int sketch, int o_sketch, int oc) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __half* tab = reinterpret_cast<__half*>(smem);                                              // [hi|lo][channel][S_PITCH]
+  unsigned char* sign_s = smem + S_TAB_BYTES;                                                 // [warp][buffer][in|out][token][bytes]
+  uint2* qf_s = reinterpret_cast<uint2*>(sign_s + SW * 2 * S_SIGN_BYTES);                     // [value (R 8) | remainder][k-step][lane]
+  __half* q_s = reinterpret_cast<__half*>(qf_s + 2 * (MAX_SKETCH / 16) * 32);                 // [head][channel]
+  uint8_t* order_s = reinterpret_cast<uint8_t*>(q_s + kMaxRep * kHeadDim);                    // [warp][64]: channel per slot, free slots
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
+  // the projection, rows of channels, positions in sign order
+  for (int i = tid; i < kHeadDim * (sketch / 4); i += STHREADS) {
+    const int d = i / (sketch / 4), p = i % (sketch / 4) * 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float x = proj_f<TP>(proj_score[(int64_t)d * sketch + sign_proj(p + k, sketch)]);
+      const __half hi = __float2half_rn(x);
+      tab[d * S_PITCH + p + k] = hi;
+      tab[(kHeadDim + d) * S_PITCH + p + k] = __float2half_rn(x - __half2float(hi));
+    }
   }
-  for (int i = tid; i < n_here * oc; i += THREADS)
-    otl_s[i / oc][i % oc] = outlier_idx[(kbh * n_groups + n0) * oc + i] & (kHeadDim - 1);
-  // this thread's projection: the sketch of the whole query per head
-  const int p = tid;
-  float qs_reg[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) qs_reg[r] = (p < sketch && r < n_rep) ? query_sketch[(qrow0 + r) * sketch + p] : 0.f;
-  // this warp's MMA task and its sketch words
-  const int mt = warp & 1, io = (warp >> 1) & 1, kh = warp >> 2;
-  const int g = lane >> 2, c = lane & 3;
-  const int dim = io == 0 ? sketch : o_sketch;
-  const int n_ks = min(8, dim / 16 - kh * 8);                // k-steps of 16 projections in this half
-  const uint8_t* kbase = io == 0 ? key_quant : key_outlier_quant;
-  const int row_bytes = dim / 8;
-  const int t_lo = mt * 16 + g, t_hi = t_lo + 8;
-  auto load_words = [&](int gl, uint4& w_lo, uint4& w_hi) {
-    w_lo = make_uint4(0u, 0u, 0u, 0u); w_hi = make_uint4(0u, 0u, 0u, 0u);
-    if (n_ks <= 0 || gl >= n_here) return;
-    const int64_t tok = (kbh * n_groups + n0 + gl) * G + tok0;
-    if (t_lo < n_tok) w_lo = *reinterpret_cast<const uint4*>(kbase + (tok + t_lo) * row_bytes + kh * 16);
-    if (t_hi < n_tok) w_hi = *reinterpret_cast<const uint4*>(kbase + (tok + t_hi) * row_bytes + kh * 16);
-  };
-  uint4 cur_lo, cur_hi;
-  load_words(0, cur_lo, cur_hi);
-  // epilogue role: (token, head)
-  const int et = tid / R, er = tid % R;
-  const bool e_live = tid < 32 * R && et < n_tok && er < n_rep;
-  __syncthreads();
+  const int n_chunks = (G + 31) / 32, per_kbh = n_groups * n_chunks;
+  const int64_t n_items = (int64_t)n_kbh * per_kbh;
+  const int64_t it_first = blockIdx.x * n_items / gridDim.x, it_end = (blockIdx.x + 1) * n_items / gridDim.x;
+  const int rb = sketch / 8, orb = o_sketch / 8;
+  unsigned char* my_sign = sign_s + warp * 2 * S_SIGN_BYTES;
+  uint8_t* order = order_s + warp * 64;
+  const uint32_t tab_b = ptx::smem_u32(tab);
+  const float keep = R == 8 || g >= 4 ? 1.f : 0.f;      // R == 4: the lanes of the remainders
 
-  for (int gl = 0; gl < n_here; ++gl) {
-    const int buf = gl & 1;
-    const int64_t grp = kbh * n_groups + n0 + gl;
-    uint4 nxt_lo, nxt_hi;
-    load_words(gl + 1, nxt_lo, nxt_hi);
-    float norm_k = 0.f, norm_o = 0.f;
-    if (e_live) {
-      norm_k = Elem<T>::to_f(key_norm[grp * G + tok0 + et]);
-      norm_o = Elem<T>::to_f(key_outlier_norm[grp * G + tok0 + et]);
-    }
-    // ---- 1. query-side terms of projection p
-    if (p < sketch) {
-      float o[R];
+  for (int64_t seg = it_first; seg < it_end;) {       // runs of items of one (batch, KV head)
+    const int64_t kbh = seg / per_kbh;
+    const int64_t seg_end = min(it_end, (kbh + 1) * per_kbh);
+    const int64_t qrow0 = kbh * n_rep;
+    __syncthreads();
+    // q S of every head as B fragments: value in the lanes g < 4, remainder of the same head in g >= 4 (R == 8: both)
+    for (int i = tid; i < sketch * 2; i += STHREADS) {
+      const int b = i >> 5, l = i & 31, head = R == 4 ? (l >> 2) & 3 : l >> 2;
+      uint32_t v[2], rem[2];
 #pragma unroll
-      for (int r = 0; r < R; ++r) o[r] = 0.f;
-      for (int i = 0; i < oc; ++i) {
-        const int d = otl_s[gl][i];
-        const float pv = proj_f<TP>(proj_score[(int64_t)d * sketch + p]);
+      for (int half = 0; half < 2; ++half) {
+        float x[2];
 #pragma unroll
-        for (int r4 = 0; r4 < R; r4 += 4) {
-          const float4 qv = *reinterpret_cast<const float4*>(&qd_s[d][r4]);
-          o[r4] = fmaf(qv.x, pv, o[r4]); o[r4 + 1] = fmaf(qv.y, pv, o[r4 + 1]);
-          o[r4 + 2] = fmaf(qv.z, pv, o[r4 + 2]); o[r4 + 3] = fmaf(qv.w, pv, o[r4 + 3]);
-        }
+        for (int e = 0; e < 2; ++e)
+          x[e] = head < n_rep ? query_sketch[(qrow0 + head) * sketch + sign_proj(16 * b + 8 * half + 2 * (l & 3) + e, sketch)] : 0.f;
+        const __half2 h = __floats2half2_rn(x[0], x[1]);
+        const float2 f = __half22float2(h);
+        const __half2 lo = __floats2half2_rn(x[0] - f.x, x[1] - f.y);
+        v[half] = *reinterpret_cast<const uint32_t*>(&h);
+        rem[half] = *reinterpret_cast<const uint32_t*>(&lo);
       }
+      const bool low = R == 4 && l >= 16;
+      qf_s[i] = make_uint2(low ? rem[0] : v[0], low ? rem[1] : v[1]);
+      if (R == 8) qf_s[(MAX_SKETCH / 16) * 32 + i] = make_uint2(rem[0], rem[1]);
+    }
+    for (int i = tid; i < kMaxRep * kHeadDim; i += STHREADS) {
+      const int r = i >> 7, d = i & (kHeadDim - 1);
+      q_s[i] = __float2half_rn(r < n_rep ? Elem<T>::to_f(query[(qrow0 + r) * kHeadDim + d]) : 0.f);
+    }
+    __syncthreads();
+    // an item's sign words (contiguous: 32 tokens x sketch / 8 bytes each) through a double buffer of this warp
+    auto fetch = [&](int64_t item, int buf) {
+      if (item < seg_end) {
+        const int64_t loc = item - kbh * per_kbh, grp = kbh * n_groups + loc / n_chunks;
+        const int tok0 = (int)(loc % n_chunks) * 32, n_tok = min(32, G - tok0);
+        const uint8_t* a = key_quant + (grp * G + tok0) * rb;
+        const uint8_t* o = key_outlier_quant + (grp * G + tok0) * orb;
+        const uint32_t dst = ptx::smem_u32(my_sign + buf * S_SIGN_BYTES);
+        // rows of 32 bytes: the two 16-byte halves of every other four rows are exchanged, so that eight rows hit all banks
+        auto put = [&](uint32_t to, const uint8_t* from, int row_bytes) {
+          for (int i = lane; i < n_tok * row_bytes / 16; i += 32)
+            ptx::cp_async_zfill<16>(to + (uint32_t)((row_bytes == 32 ? i ^ ((i >> 3) & 1) : i) * 16), from + i * 16, 16);
+        };
+        put(dst, a, rb);
+        put(dst + S_SIGN_BYTES / 2, o, orb);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int64_t item = seg + warp;
+    fetch(item, 0);
+    for (int buf = 0; item < seg_end; item += SW, buf ^= 1) {
+      const int64_t loc = item - kbh * per_kbh, n = loc / n_chunks, grp = kbh * n_groups + n;
+      const int tok0 = (int)(loc % n_chunks) * 32, n_tok = min(32, G - tok0);
+      fetch(item + SW, buf ^ 1);
+      float nk[4], no[4];                             // norms of the lane's tokens g + 8 i
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
+      for (int i = 0; i < 4; ++i) {
+        const int64_t t = grp * G + tok0 + min(g + 8 * i, n_tok - 1);
+        nk[i] = Elem<T>::to_f(key_norm[t]);
+        no[i] = Elem<T>::to_f(key_outlier_norm[t]);
+      }
+      float acc[3][2][4];                             // [in: q S | in: q_out S | out: q_out S][m-tile][fragment]
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          if (which == 1 && p >= o_sketch) continue;
-          const float x = which == 0 ? qs_reg[r] - o[r] : o[r];
-          const __half hi = __float2half_rn(x);
-          const __half lo = __float2half_rn(x - __half2float(hi));
-          if constexpr (R == 4) {
-            b_s[buf][which][0][r][p] = hi;
-            b_s[buf][which][0][r + 4][p] = lo;
+      for (int i = 0; i < 24; ++i) (&acc[0][0][0])[i] = 0.f;
+      // u accumulates over blocks of 32 outlier channels; there is one block unless oc > 32
+      const int blocks = (oc + 31) / 32;
+      uint32_t qa[2][2], row[2];                      // A fragments and ldmatrix row of the block at hand
+      auto load_block = [&](int blk) {
+        const int i = blk * 32 + lane;
+        const bool have = i < oc;
+        const int d = have ? outlier_idx[grp * oc + i] & (kHeadDim - 1) : 0x80 | lane;      // bit 7: no channel
+        const uint32_t same = __match_any_sync(0xffffffffu, d & 7), lt = (1u << lane) - 1u;
+        const int rank = __popc(same & lt);
+        const bool over = rank >= 4;
+        const uint32_t taken = __reduce_or_sync(0xffffffffu, over ? 0u : 1u << (rank * 8 + (d & 7)));
+        const uint32_t ov = __ballot_sync(0xffffffffu, over);
+        if (!((taken >> lane) & 1u)) order[32 + __popc(~taken & lt)] = (uint8_t)lane;       // free slots in order
+        __syncwarp();
+        order[over ? order[32 + __popc(ov & lt)] : rank * 8 + (d & 7)] = (uint8_t)d;
+        __syncwarp();
+        const int head = R == 4 ? (g & 3) : g;
+        auto qv = [&](int slot) -> uint32_t {
+          const int ch = order[slot];
+          return ch & 0x80 ? 0u : (uint32_t)__half_as_ushort(q_s[head * kHeadDim + ch]);
+        };
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          qa[ks][0] = qv(16 * ks + 2 * c) | (qv(16 * ks + 2 * c + 1) << 16);
+          qa[ks][1] = qv(16 * ks + 2 * c + 8) | (qv(16 * ks + 2 * c + 9) << 16);
+          // matrices 0, 1 of a load: rows k 0-7 and 8-15 at positions 0-7; 2, 3: the same rows at positions 8-15
+          row[ks] = tab_b + (uint32_t)((order[16 * ks + (lane & 15)] & 0x7f) * S_PITCH * 2) + (uint32_t)(lane >> 4) * 16u;
+        }
+        __syncwarp();
+      };
+      if (blocks == 1) load_block(0);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      // sign words of the lane: rows g + 8 i, inverted, words c and c + 4 (128 projections: word c twice, eight bits apart).
+      // k-steps run from the top: the bits at hand are always 15 and 31
+      uint32_t x[2][4][2];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int bytes = s == 0 ? rb : orb;
+        const unsigned char* base = my_sign + buf * S_SIGN_BYTES + s * (S_SIGN_BYTES / 2);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = g + 8 * i, sw = bytes == 32 ? (r >> 2) & 1 : 0;
+          const uint32_t w = ~*reinterpret_cast<const uint32_t*>(base + r * bytes + (sw << 4) + 4 * c);
+          if (bytes == 32) {
+            x[s][i][0] = w;
+            x[s][i][1] = ~*reinterpret_cast<const uint32_t*>(base + r * bytes + ((1 ^ sw) << 4) + 4 * c);
           } else {
-            b_s[buf][which][0][r][p] = hi;
-            b_s[buf][which][NV - 1][r][p] = lo;
+            x[s][i][0] = sketch == 256 ? w : w << 8;
+            x[s][i][1] = w;
           }
         }
       }
-    }
-    __syncthreads();
-    // ---- 2. sign sums on the MMA
-    {
-      float acc[NV][4];
+      __syncwarp();      // the sign buffer may be refilled
+      const bool short_out = o_sketch < sketch;      // 128 of 256: only the first half of every k-step is in the outlier sketch
+#pragma unroll 2
+      for (int b = sketch / 16 - 1; b >= 0; --b) {
+        float u[2][4];                                // rows = heads, columns = the k-step's two halves
+        for (int blk = 0; blk < blocks; ++blk) {
+          if (blocks > 1) load_block(blk);
 #pragma unroll
-      for (int v = 0; v < NV; ++v) { acc[v][0] = acc[v][1] = acc[v][2] = acc[v][3] = 0.f; }
-      if (n_ks > 0) {
-        const uint32_t wl[4] = {cur_lo.x, cur_lo.y, cur_lo.z, cur_lo.w}, wh[4] = {cur_hi.x, cur_hi.y, cur_hi.z, cur_hi.w};
-        const uint32_t* bw[NV];
+          for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) bw[v] = reinterpret_cast<const uint32_t*>(&b_s[buf][io][v][g][0]);
+            for (int hl = 0; hl < 2; ++hl) {
+              uint32_t b0, b1, b2, b3;
+              ptx::ldmatrix_x4_trans(row[ks] + (uint32_t)(hl * kHeadDim * S_PITCH * 2 + 32 * b), b0, b1, b2, b3);
+              if (ks == 0 && hl == 0 && blk == 0) {
+                ptx::mma_f16_zero(u[0], qa[0][0], 0u, qa[0][1], 0u, b0, b1);
+                ptx::mma_f16_zero(u[1], qa[0][0], 0u, qa[0][1], 0u, b2, b3);
+              } else {
+                ptx::mma_f16(u[0], qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
+                ptx::mma_f16(u[1], qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
+              }
+            }
+        }
+        // q_out S as the B operand: fp16 value, or what it leaves over (R == 8: both)
+        uint32_t bv[2], bl[2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (j < n_ks) {
-            // inverted bits 2c, 2c+1 of the step's first byte and of its second byte give the sign bits of
-            // columns (2c, 2c+1) and (2c+8, 2c+9); the magnitude is one unit in the last place
-            const uint32_t zl = ~(wl[j >> 1] >> (16 * (j & 1) + 2 * c)) & 0x0303u;
-            const uint32_t zh = ~(wh[j >> 1] >> (16 * (j & 1) + 2 * c)) & 0x0303u;
-            const uint32_t a0 = (((zl << 15) | (zl << 30)) & 0x80008000u) | 0x00010001u;
-            const uint32_t a1 = (((zh << 15) | (zh << 30)) & 0x80008000u) | 0x00010001u;
-            const uint32_t a2 = (((zl << 7) | (zl << 22)) & 0x80008000u) | 0x00010001u;
-            const uint32_t a3 = (((zh << 7) | (zh << 22)) & 0x80008000u) | 0x00010001u;
-            const int pp = (kh * 8 + j) * 8 + c;                // pair of projections 2pp, 2pp+1
+        for (int half = 0; half < 2; ++half) {
+          const __half2 h = __floats2half2_rn(u[half][0], u[half][1]);
+          const float2 f = __half22float2(h);
+          const __half2 l = __floats2half2_rn(fmaf(-keep, f.x, u[half][0]), fmaf(-keep, f.y, u[half][1]));
+          bl[half] = *reinterpret_cast<const uint32_t*>(&l);
+          bv[half] = R == 4 ? bl[half] : *reinterpret_cast<const uint32_t*>(&h);
+        }
+        const uint2 qf = qf_s[b * 32 + lane];
+        const uint2 qr = R == 8 ? qf_s[(MAX_SKETCH / 16) * 32 + b * 32 + lane] : make_uint2(0u, 0u);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) ptx::mma_f16(acc[v], a0, a1, a2, a3, bw[v][pp], bw[v][pp + 4]);
+        for (int s = 0; s < 2; ++s) {
+          uint32_t a[4][2];                           // +-2^-24, negative where the bit is 0
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              a[i][e] = (x[s][i][e] & 0x80008000u) | 0x00010001u;
+              x[s][i][e] += x[s][i][e];
+            }
+          const uint32_t b1v = s == 1 && short_out ? 0u : bv[1], b1l = s == 1 && short_out ? 0u : bl[1];
+#pragma unroll
+          for (int mt = 0; mt < 2; ++mt) {
+            if (s == 0) ptx::mma_f16(acc[0][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], qf.x, qf.y);
+            ptx::mma_f16(acc[1 + s][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], bv[0], b1v);
+            if (R == 8) {
+              if (s == 0) ptx::mma_f16(acc[0][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], qr.x, qr.y);
+              ptx::mma_f16(acc[1 + s][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], bl[0], b1l);
+            }
           }
         }
       }
-      // acc[.][0..1] = (token g, columns 2c, 2c+1), acc[.][2..3] = (token g + 8, same columns)
-      constexpr float UNSCALE = 16777216.f;                    // the signs were +-2^-24
-      if constexpr (R == 4) {
-        // columns 0-3 hold the hi sums of heads 0-3, columns 4-7 the lo sums: lanes c and c+2 pair up
+      // columns 2c, 2c+1 = heads (R == 4: values in columns 0-3, remainders in 4-7)
+      const float scl = 1.2533141373155001f / (float)sketch * 16777216.f, scl_o = 1.2533141373155001f / (float)o_sketch * 16777216.f;
+      float norm_in[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[0][e] += __shfl_xor_sync(0xffffffffu, acc[0][e], 2);
-        if (c < 2) {
+      for (int i = 0; i < 4; ++i)      // the two norms are rounded separately, so the difference can dip below zero
+        norm_in[i] = scl * sqrtf(fmaxf(nk[i] * nk[i] - no[i] * no[i], 0.f));
+      float* dst = scores + (qrow0 + 2 * c) * ((int64_t)n_groups * G) + n * G + tok0 + g;
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            part_s[buf][kh][mt * 16 + g + 8 * (e >> 1)][io * R + 2 * c + (e & 1)] = acc[0][e] * UNSCALE;
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 2 * mt + (e >> 1);
+          float v = norm_in[i] * (acc[0][mt][e] - acc[1][mt][e]) + scl_o * no[i] * acc[2][mt][e];
+          if (R == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
+          if (2 * c + (e & 1) < n_rep && g + 8 * i < n_tok && (R == 8 || c < 2)) dst[(e & 1) * ((int64_t)n_groups * G) + 8 * i] = v;
         }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          part_s[buf][kh][mt * 16 + g + 8 * (e >> 1)][io * R + 2 * c + (e & 1)] = (acc[0][e] + acc[NV - 1][e]) * UNSCALE;
-      }
     }
-    __syncthreads();
-    // ---- 3. norms and scale
-    if (e_live) {
-      const float inner = part_s[buf][0][et][er] + part_s[buf][1][et][er];
-      const float outer = part_s[buf][0][et][R + er] + part_s[buf][1][et][R + er];
-      // |k_in|: the two norms are rounded separately, so the difference can dip below zero
-      const float norm_in = sqrtf(fmaxf(norm_k * norm_k - norm_o * norm_o, 0.f));
-      const float scl = 1.2533141373155001f / (float)sketch, scl_o = 1.2533141373155001f / (float)o_sketch;
-      scores[(qrow0 + er) * ((int64_t)n_groups * G) + (int64_t)(n0 + gl) * G + tok0 + et] =
-          scl * norm_in * inner + scl_o * norm_o * outer;
-    }
-    cur_lo = nxt_lo; cur_hi = nxt_hi;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    seg = seg_end;
   }
 }
 
@@ -619,15 +710,29 @@ extern "C" int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_out
     return CQ_ERR_UNSUPPORTED;
   if (n_groups > 65535) return CQ_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  dim3 grid((unsigned)(batch * n_kv_heads), (unsigned)n_groups, (unsigned)((group_size + 31) / 32));
-  // sketch rows that are whole 16-byte words: the tensor-core variant, several groups per CTA
+  // sketch rows that are whole 16-byte words: the persistent tensor-core kernel, one CTA per SM
   const bool use_mma = sketch_dim % 128 == 0 && outlier_sketch_dim % 128 == 0 && qjl::mma_ptrs_ok(key_quant, key_outlier_quant);
-  if (use_mma) grid.y = (unsigned)((n_groups + qjl::GPC - 1) / qjl::GPC);
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return CQ_ERR_LAUNCH;
+  const int64_t items = (int64_t)batch * n_kv_heads * n_groups * ((group_size + 31) / 32);
+  const unsigned grid_mma = (unsigned)((items + qjl::SW - 1) / qjl::SW < sms ? (items + qjl::SW - 1) / qjl::SW : sms);
+  const dim3 grid((unsigned)(batch * n_kv_heads), (unsigned)n_groups, (unsigned)((group_size + 31) / 32));
+#define CQ_QJL_ARGS(T, TP) key_quant, key_outlier_quant, static_cast<const T*>(key_norm), static_cast<const T*>(key_outlier_norm), \
+      outlier_indices, query_sketch, static_cast<const T*>(query), static_cast<const TP*>(proj_score), scores
 #define CQ_QJL_SCORE(T, TP, R)                                                                                 \
-  do { (use_mma ? qjl::score_mma_kernel<T, TP, R> : qjl::score_kernel<T, TP, R>)<<<grid, qjl::THREADS, 0, st>>>(key_quant, key_outlier_quant, \
-      static_cast<const T*>(key_norm), static_cast<const T*>(key_outlier_norm), outlier_indices, query_sketch,  \
-      static_cast<const T*>(query), static_cast<const TP*>(proj_score), scores, n_groups, group_size, n_rep,    \
-      sketch_dim, outlier_sketch_dim, outlier_count); } while (0)
+  do {                                                                                                         \
+    if (use_mma) {                                                                                             \
+      auto kern = qjl::score_rows_kernel<T, TP, R>;                                                            \
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, qjl::S_SMEM) != cudaSuccess) \
+        return CQ_ERR_LAUNCH;                                                                                  \
+      kern<<<grid_mma, qjl::STHREADS, qjl::S_SMEM, st>>>(CQ_QJL_ARGS(T, TP), batch * n_kv_heads, n_groups, group_size, n_rep, \
+                                                         sketch_dim, outlier_sketch_dim, outlier_count);       \
+    } else {                                                                                                   \
+      qjl::score_kernel<T, TP, R><<<grid, qjl::THREADS, 0, st>>>(CQ_QJL_ARGS(T, TP), n_groups, group_size, n_rep, sketch_dim, \
+                                                                 outlier_sketch_dim, outlier_count);           \
+    }                                                                                                          \
+  } while (0)
 #define CQ_QJL_SCORE_R(T, TP) do { if (n_rep <= 4) CQ_QJL_SCORE(T, TP, 4); else CQ_QJL_SCORE(T, TP, 8); } while (0)
   if (dtype == CQ_DTYPE_F16) {
     if (proj_dtype == CQ_DTYPE_F32) CQ_QJL_SCORE_R(__half, float); else CQ_QJL_SCORE_R(__half, __half);
@@ -636,5 +741,6 @@ extern "C" int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_out
   }
 #undef CQ_QJL_SCORE_R
 #undef CQ_QJL_SCORE
+#undef CQ_QJL_ARGS
   return cudaGetLastError() == cudaSuccess ? CQ_OK : CQ_ERR_LAUNCH;
 }
