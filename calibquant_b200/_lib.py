@@ -116,6 +116,9 @@ SIGNATURES = {
                                                  _c.c_int, _c.c_float, _c.c_int, _vp]),
     "cq_qjl_quant": (_c.c_int, [_vp, _vp, _vp, _c.c_int, _i64, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                 _c.c_int, _vp, _vp, _vp, _vp]),
+    "cq_qjl_build": (_c.c_int, [_vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_i64), _vp, _c.c_int, _c.c_int,
+                                _c.c_int, _c.c_int, _c.c_int, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "cq_qjl_status": (_c.c_int, []),
     "cq_qjl_gqa_score": (_c.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                     _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _vp, _vp]),
     "cq_decode_attn_workspace_bytes": (_sz, [_c.POINTER(DecodeArgs)]),

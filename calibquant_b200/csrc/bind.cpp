@@ -508,11 +508,84 @@ PyObject* py_prefill_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_END
 }
 
+// ---- QJL sign sketches -------------------------------------------------------------------------------------------------
+int proj_enum(const Tensor& proj, const Tensor& data) {
+  if (proj.scalar_type() == at::kFloat) return CQ_DTYPE_F32;
+  if (proj.scalar_type() == data.scalar_type()) return dtype_enum(data);
+  raise(PyExc_TypeError, "Unsupported data types for QJL: the projection must be float32 or match the keys");
+}
+
+// key_states [B,H,n,G,128], outlier_indices uint8 [B,H,n,oc], rand_prj [sketch,128], outlier_sketch_dim
+PyObject* py_qjl_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  CQ_BEGIN
+  want_args(n, 4, "qjl_quant");
+  for (int i = 0; i < 3; ++i) need_cuda(tensor(a[i]));
+  const Tensor k = contiguous(tensor(a[0])), idx = contiguous(tensor(a[1])), proj = contiguous(tensor(a[2]));
+  const int dt = dtype_enum(k), pdt = proj_enum(proj, k);
+  const int64_t B = k.size(0), H = k.size(1), N = k.size(2), G = k.size(3), D = k.size(4), s = proj.size(0), os = integer(a[3]);
+  if (idx.scalar_type() != at::kByte || idx.size(0) != B || idx.size(1) != H || idx.size(2) != N)
+    raise(PyExc_ValueError, "outlier_indices must be uint8 [B,H,n,outlier_count]");
+  Call call(k);
+  Tensor kq = empty({B, H, N, G, s / 8}, k, at::kByte), koq = empty({B, H, N, G, os / 8}, k, at::kByte), norms = empty({B, H, N, G}, k);
+  check(cq_qjl_quant(k.data_ptr(), (const uint8_t*)idx.data_ptr(), proj.data_ptr(), pdt, B * H * N, (int)G, (int)D, (int)s, (int)os,
+                     (int)idx.size(3), dt, (uint8_t*)kq.data_ptr(), (uint8_t*)koq.data_ptr(), norms.data_ptr(), call.stream), "cq_qjl_quant");
+  return wrap3(kq, koq, norms);
+  CQ_END
+}
+
+// keys [B,H,T,128] (strided), rand_prj [256,128], outlier_sketch_dim, outlier_count -> (idx, kq, koq, outlier norms, key norms)
+PyObject* py_qjl_build(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  CQ_BEGIN
+  want_args(n, 4, "qjl_build");
+  need_cuda(tensor(a[0])); need_cuda(tensor(a[1]));
+  const Tensor k = with_rows(tensor(a[0])), proj = contiguous(tensor(a[1]));
+  const int64_t B = k.size(0), H = k.size(1), N = k.size(2) / 32, os = integer(a[2]), oc = integer(a[3]), s = proj.size(0);
+  const int64_t st[3] = {k.stride(0), k.stride(1), k.stride(2)};
+  Call call(k);
+  Tensor idx = empty({B, H, N, oc}, k, at::kByte), kq = empty({B, H, N, 32, s / 8}, k, at::kByte);
+  Tensor koq = empty({B, H, N, 32, os / 8}, k, at::kByte), onorm = empty({B, H, N, 32}, k), knorm = empty({B, H, N, 32}, k);
+  check(cq_qjl_build(k.data_ptr(), (int)B, (int)H, (int)N, 32, (int)k.size(3), st, proj.data_ptr(), proj_enum(proj, k), (int)s, (int)os,
+                     (int)oc, dtype_enum(k), (uint8_t*)idx.data_ptr(), (uint8_t*)kq.data_ptr(), (uint8_t*)koq.data_ptr(),
+                     knorm.data_ptr(), onorm.data_ptr(), call.stream), "cq_qjl_build");
+  PyObject* tup = PyTuple_New(5);
+  if (!tup) throw PyRaised();
+  const Tensor all[5] = {idx, kq, koq, onorm, knorm};
+  for (int i = 0; i < 5; ++i) PyTuple_SET_ITEM(tup, i, wrap(all[i]));
+  return tup;
+  CQ_END
+}
+
+// key_quant, key_outlier_quant, key_norm, key_outlier_norm, outlier_indices, query_sketch | None, query [B,Hq,1,128], rand_prj
+PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  CQ_BEGIN
+  want_args(n, 8, "qjl_gqa_score");
+  for (int i = 0; i < 8; ++i)
+    if (a[i] != Py_None) need_cuda(tensor(a[i]));
+  const Tensor kq = contiguous(tensor(a[0])), koq = contiguous(tensor(a[1])), kn = contiguous(tensor(a[2])), on = contiguous(tensor(a[3]));
+  const Tensor idx = contiguous(tensor(a[4])), q = contiguous(tensor(a[6])), proj = contiguous(tensor(a[7]));
+  Tensor qs = opt_tensor(a[5]);
+  if (qs.defined()) qs = (qs.scalar_type() == at::kFloat ? qs : qs.to(at::kFloat)).contiguous();
+  const int64_t B = kq.size(0), Hkv = kq.size(1), N = kq.size(2), G = kq.size(3), Hq = q.size(1), D = q.size(-1);
+  const int dt = dtype_enum(q), pdt = proj_enum(proj, q);
+  if (kn.scalar_type() != q.scalar_type() || on.scalar_type() != q.scalar_type())
+    raise(PyExc_TypeError, "key norms must have the query dtype");
+  if (Hq % Hkv) raise(PyExc_ValueError, "query heads must be a multiple of key heads");
+  Call call(q);
+  Tensor scores = empty({B, Hq, N * G, 1}, q, at::kFloat);
+  check(cq_qjl_gqa_score((const uint8_t*)kq.data_ptr(), (const uint8_t*)koq.data_ptr(), kn.data_ptr(), on.data_ptr(),
+                         (const uint8_t*)idx.data_ptr(), qs.defined() ? (const float*)qs.data_ptr() : nullptr, q.data_ptr(),
+                         proj.data_ptr(), pdt, (int)B, (int)Hkv, (int)(Hq / Hkv), (int)N, (int)G, (int)D, (int)kq.size(4) * 8,
+                         (int)koq.size(4) * 8, (int)idx.size(3), dt, (float*)scores.data_ptr(), call.stream), "cq_qjl_gqa_score");
+  return wrap(scores);
+  CQ_END
+}
+
 #define CQ_FN(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     CQ_FN(workspace), CQ_FN(workspaces_of), CQ_FN(pack_last_dim), CQ_FN(pack_k_per_channel), CQ_FN(pack_v_per_token),
     CQ_FN(quant_encode), CQ_FN(qbmm), CQ_FN(decode_attention), CQ_FN(u8_decode_attention), CQ_FN(rope_split_append),
-    CQ_FN(prefill_rope_split), CQ_FN(prefill_attention), {nullptr, nullptr, 0, nullptr}};
+    CQ_FN(prefill_rope_split), CQ_FN(prefill_attention),
+    CQ_FN(qjl_quant), CQ_FN(qjl_build), CQ_FN(qjl_gqa_score), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Tensor-level entry points over libcalibquant_b200.so.", -1, methods};
 
 }  // namespace

@@ -70,7 +70,9 @@ class QJLSketch(torch.nn.Module):
             "query shape should match outlier indices and data quant shapes"
         assert data_quant.shape[:4] == norm_data.shape[:4], "data quant and its norm should have same shape"
         assert outlier_quant.shape[:4] == norm_outlier.shape[:4], "outlier quant and its norm should have same shape"
-        sketched_q = torch.matmul(query.to(self.proj_dir_score.dtype), self.proj_dir_score)
+        sketched_q = None      # formed by the score kernel, next to the projection it keeps in shared memory
+        if self.dim[1] % 128 or self.dim_outlier % 128 or (data_quant.data_ptr() | outlier_quant.data_ptr()) % 16:
+            sketched_q = torch.matmul(query.to(self.proj_dir_score.dtype), self.proj_dir_score)
         return qjl_kernel.qjl_gqa_score(data_quant, outlier_quant, norm_data, norm_outlier, outlier_indices,
                                         sketched_q, query, self.proj_dir_score)
 
@@ -98,13 +100,20 @@ class QJLKeyQuantizer:
         self.key_states_norm = None
         self.key_residual = None
 
-    def _sketch_groups(self, groups: torch.Tensor):
-        """groups [B,H,n,G,D] -> appends their sketches, outlier sets and norms."""
-        norms = groups.norm(dim=-2)
-        _, idx = norms.topk(self.outliers_count, dim=-1)
-        idx = idx.to(torch.uint8).contiguous()
-        kq, koq, onorm = self.qjl_sketch.quantize(groups.contiguous(), idx)
-        knorm = torch.norm(groups, dim=-1)
+    def _sketch(self, keys: torch.Tensor):
+        """keys [B,H,T,D], T a multiple of group_size -> appends their sketches, outlier sets and norms."""
+        proj = self.qjl_sketch.proj_dir_quant
+        if self.group_size == 32 and tuple(proj.shape) == (256, 128) and self.qjl_sketch.dim_outlier % 32 == 0 and \
+                proj.dtype in (torch.float32, keys.dtype):
+            idx, kq, koq, onorm, knorm = ops.qjl_build(keys, proj, self.qjl_sketch.dim_outlier, self.outliers_count)
+        else:
+            b, h, t, dim = keys.shape
+            groups = keys.reshape(b, h, t // self.group_size, self.group_size, dim)
+            norms = groups.norm(dim=-2)
+            _, idx = norms.topk(self.outliers_count, dim=-1)
+            idx = idx.to(torch.uint8).contiguous()
+            kq, koq, onorm = self.qjl_sketch.quantize(groups.contiguous(), idx)
+            knorm = torch.norm(groups, dim=-1)
         if self.key_states_quant is None:
             self.outlier_indices, self.key_states_quant, self.key_outliers_quant = idx, kq, koq
             self.key_outliers_norm, self.key_states_norm = onorm, knorm
@@ -117,16 +126,13 @@ class QJLKeyQuantizer:
 
     def build_sketch(self, key_states: torch.Tensor) -> None:
         """key_states [B,Hkv,T,D]: sketch the first T - T % buffer_size keys, keep the rest fp."""
-        b, h, _, dim = key_states.shape
         self.seq_len = key_states.shape[-2]
         residual_size = self.seq_len % self.buffer_size
         if residual_size > 0:
             self.key_residual = key_states[:, :, self.seq_len - residual_size:, :]
         if residual_size == self.seq_len:
             return None
-        num_groups = (self.seq_len - residual_size) // self.group_size
-        self._sketch_groups(key_states[:, :, :self.seq_len - residual_size, :].reshape(
-            (b, h, num_groups, self.group_size, dim)))
+        self._sketch(key_states[:, :, :self.seq_len - residual_size, :])
 
     def update_sketch(self, key_states: torch.Tensor) -> None:
         assert key_states.shape[-2] == 1, "appending more than one embedding in the stream!"
@@ -137,8 +143,7 @@ class QJLKeyQuantizer:
             self.key_residual = key_states
         if self.seq_len % self.buffer_size != 0:
             return None
-        b, h, _, dim = self.key_residual.shape
-        self._sketch_groups(self.key_residual.reshape((b, h, -1, self.group_size, dim)))
+        self._sketch(self.key_residual)
         self.key_residual = None
 
     def attention_score(self, query_states: torch.Tensor) -> torch.Tensor:

@@ -438,19 +438,34 @@ int cq_comm_allreduce_add_rmsnorm(const void* src, void* const* peer_buffers, in
  *   outlier_norms     [n_groups_total][group_size] in `dtype`: 2-norm of the outlier channels
  *   sketch_dim <= 256, sketch_dim and outlier_sketch_dim multiples of 32.
  *
+ * cq_qjl_build does the whole of QJLKeyQuantizer.build_sketch (qjl/qjl_utils.py:114-150) on strided keys: per group of 32
+ * keys the channel norms over the keys, the outlier_count channels of largest norm (as the data type holds the norms; the
+ * lower channel first where they are equal), both sketches and both norms.
+ *   keys              element (b,h,t,d) at keys[b*strides[0] + h*strides[1] + t*strides[2] + d], strides multiples of 8
+ *                     elements, 16-byte aligned; t < 32*n_groups
+ *   outlier_indices   uint8 [batch][heads][n_groups][outlier_count], largest norm first
+ *   key_norms, outlier_norms  [batch][heads][n_groups][32] in `dtype`; the sketches as above
+ *   group_size 32 and sketch_dim 256 only (CQ_ERR_UNSUPPORTED otherwise).
+ * cq_qjl_status: sticky device status of the sketching kernel, as cq_prefill_status.
+ *
  * cq_qjl_gqa_score replaces qjl/qjl_kernel.py:52-72 `qjl_gqa_score` -> `calc_gqa_score_kernel`
  * (qjl/csrc/qjl_gqa_score_kernel.cu:40-180), for any n_rep <= 8 (the reference's shared arrays hold 4):
  *   score[b,h,t] = sqrt(pi/2)/sketch_dim * |k_in| * sum_p sgn_p (qS - q_out S)_p
  *                + sqrt(pi/2)/outlier_sketch_dim * |k_out| * sum_{p<o} sgn'_p (q_out S)_p
  *   key_norm / key_outlier_norm [B,Hkv,n,G] in `dtype`; |k_in| = sqrt(max(|k|^2 - |k_out|^2, 0)) (the
  *   reference takes the square root of the unclamped difference); query_sketch fp32 [B,Hq,sketch_dim] =
- *   q @ proj_score; query [B,Hq,128]; proj_score [128][sketch_dim] (QJLSketch.proj_dir_score);
+ *   q @ proj_score, or NULL: the kernel forms it (sketch dims that are multiples of 128, 16-byte aligned operands); query [B,Hq,128]; proj_score [128][sketch_dim] (QJLSketch.proj_dir_score);
  *   scores fp32 [B,Hq,n*G].
  */
 int cq_qjl_quant(const void* keys, const uint8_t* outlier_indices, const void* proj, int proj_dtype,
                  int64_t n_groups_total, int group_size, int head_dim, int sketch_dim, int outlier_sketch_dim,
                  int outlier_count, int dtype, uint8_t* key_quant, uint8_t* key_outlier_quant,
                  void* outlier_norms, void* stream);
+int cq_qjl_build(const void* keys, int batch, int heads, int n_groups, int group_size, int head_dim, const int64_t* strides,
+                 const void* proj, int proj_dtype, int sketch_dim, int outlier_sketch_dim, int outlier_count, int dtype,
+                 uint8_t* outlier_indices, uint8_t* key_quant, uint8_t* key_outlier_quant, void* key_norms,
+                 void* outlier_norms, void* stream);
+int cq_qjl_status(void);
 int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_outlier_quant, const void* key_norm,
                      const void* key_outlier_norm, const uint8_t* outlier_indices, const float* query_sketch,
                      const void* query, const void* proj_score, int proj_dtype, int batch, int n_kv_heads,
