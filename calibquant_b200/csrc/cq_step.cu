@@ -158,67 +158,91 @@ swiglu_packed_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int64_t
 }
 
 // ---- prefill: split + rotary embedding of the whole prompt in one pass over the wqkv output ----------------
-// One thread owns the channel chunks [8c, 8c+8) and [64+8c, 64+8c+8) of one 128-channel row (a query head, the
-// key or the value of one KV head of one token): two 16-byte loads, the rotation of both chunks (they are each
-// other's rotate_half partners), 16-byte stores.  Queries go to q_out, keys to k_out (both [B,T,H,128], what
-// the prefill attention reads) and, for tokens outside the quantized span, to the full-precision cache together
-// with the values.  Values inside the span are not copied at all (the pack kernel reads them in place).
+// A warp owns one token and `heads_per` of its KV heads; eight lanes share a 128-channel row (a query head, the key or the
+// value of a KV head), lane c of them the channel chunks [8c, 8c+8) and [64+8c, 64+8c+8), which are each other's
+// rotate_half partners: two 16-byte loads, the rotation of both chunks, 16-byte stores.  Every row of a token takes the same
+// angles, so a lane loads its cosines and sines once and keeps them in registers; the loads of four passes (16 rows) are
+// issued together.  Queries go to q_out, keys to k_out (both [B,T,H,128], what the prefill attention reads) and, for tokens
+// outside the quantized span, to the full-precision cache together with the values.  Values inside the span are not
+// read (the pack kernel takes them in place).
+// HBM bound: 16 x 3392 tokens, 32 query and 8 KV heads, move 1.11 GB.  With a thread per chunk, which fetched the angles for
+// each row and read all values, that took 308 us; this takes 200 (5.5 TB/s).
 template <typename T>
 __global__ void __launch_bounds__(256)
 prefill_rope_split_kernel(const T* __restrict__ qkv, int64_t stride_b, int64_t stride_t, const T* __restrict__ cos_t,
                           const T* __restrict__ sin_t, int rope_len, const int64_t* __restrict__ position_ids,
                           int t_len, int n_kv_heads, int n_rep, T* __restrict__ q_out, T* __restrict__ k_out,
                           T* __restrict__ k_cache, T* __restrict__ v_cache, int64_t cache_stride_b,
-                          int64_t cache_stride_h, int capacity, int vis_start, int vis_len, int64_t total) {
-  const int slots = n_kv_heads * (n_rep + 2);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i & 7);
-    const int64_t row = i >> 3;                       // (b, t, slot)
-    const int slot_all = (int)(row % slots);
-    const int64_t bt = row / slots;
-    const int t = (int)(bt % t_len);
-    const int64_t b = bt / t_len;
-    const int hk = slot_all / (n_rep + 2), slot = slot_all % (n_rep + 2);
-    const T* src = qkv + b * stride_b + (int64_t)t * stride_t + (int64_t)slot_all * kHeadDim;
-    const int fp_idx = t < vis_start ? t : (t >= vis_start + vis_len ? t - vis_len : -1);   // row in the fp cache
-    const bool to_cache = fp_idx >= 0 && fp_idx < capacity && k_cache != nullptr;
-    const uint4 lo = *reinterpret_cast<const uint4*>(src + 8 * c), hi = *reinterpret_cast<const uint4*>(src + 64 + 8 * c);
-    if (slot == n_rep + 1) {                          // value: only the full-precision tokens are copied
-      if (to_cache) {
-        T* dst = v_cache + b * cache_stride_b + hk * cache_stride_h + (int64_t)fp_idx * kHeadDim;
-        *reinterpret_cast<uint4*>(dst + 8 * c) = lo;
-        *reinterpret_cast<uint4*>(dst + 64 + 8 * c) = hi;
-      }
-      continue;
-    }
-    int64_t pos = position_ids ? position_ids[b * t_len + t] : t;
-    pos = pos < 0 ? 0 : (pos >= rope_len ? rope_len - 1 : pos);
-    const T* cr = cos_t + pos * kHeadDim;
-    const T* sr = sin_t + pos * kHeadDim;
-    const uint4 c_lo = *reinterpret_cast<const uint4*>(cr + 8 * c), c_hi = *reinterpret_cast<const uint4*>(cr + 64 + 8 * c);
-    const uint4 s_lo = *reinterpret_cast<const uint4*>(sr + 8 * c), s_hi = *reinterpret_cast<const uint4*>(sr + 64 + 8 * c);
-    const T* x0 = reinterpret_cast<const T*>(&lo);  const T* x1 = reinterpret_cast<const T*>(&hi);
-    const T* cl = reinterpret_cast<const T*>(&c_lo); const T* chh = reinterpret_cast<const T*>(&c_hi);
-    const T* sl = reinterpret_cast<const T*>(&s_lo); const T* sh = reinterpret_cast<const T*>(&s_hi);
-    uint4 o_lo, o_hi;
-    T* ol = reinterpret_cast<T*>(&o_lo); T* oh = reinterpret_cast<T*>(&o_hi);
+                          int64_t cache_stride_h, int capacity, int vis_start, int vis_len, int64_t n_tokens, int heads_per) {
+  constexpr int U = 4;
+  const int64_t bt = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (bt >= n_tokens) return;
+  const int lane = threadIdx.x & 31, c = lane & 7;
+  const int64_t b = bt / t_len;
+  const int t = (int)(bt - b * t_len);
+  const int hk0 = blockIdx.y * heads_per, n_heads = min(heads_per, n_kv_heads - hk0);
+  const int fp_idx = t < vis_start ? t : (t >= vis_start + vis_len ? t - vis_len : -1);   // row in the fp cache
+  const bool to_cache = fp_idx >= 0 && fp_idx < capacity && k_cache != nullptr;
+  const T* src = qkv + b * stride_b + (int64_t)t * stride_t + (int64_t)hk0 * (n_rep + 2) * kHeadDim + 8 * c;
+  T* q_dst = q_out + (bt * n_kv_heads + hk0) * n_rep * kHeadDim + 8 * c;
+  T* k_dst = k_out + (bt * n_kv_heads + hk0) * kHeadDim + 8 * c;
+  const int64_t cache_row = b * cache_stride_b + hk0 * cache_stride_h + (int64_t)fp_idx * kHeadDim + 8 * c;
+
+  int64_t pos = position_ids ? position_ids[bt] : t;
+  pos = pos < 0 ? 0 : (pos >= rope_len ? rope_len - 1 : pos);
+  const T* cr = cos_t + pos * kHeadDim + 8 * c;
+  const T* sr = sin_t + pos * kHeadDim + 8 * c;
+  const uint4 c_lo = *reinterpret_cast<const uint4*>(cr), c_hi = *reinterpret_cast<const uint4*>(cr + 64);
+  const uint4 s_lo = *reinterpret_cast<const uint4*>(sr), s_hi = *reinterpret_cast<const uint4*>(sr + 64);
+  const T* cl = reinterpret_cast<const T*>(&c_lo); const T* chh = reinterpret_cast<const T*>(&c_hi);
+  const T* sl = reinterpret_cast<const T*>(&s_lo); const T* sh = reinterpret_cast<const T*>(&s_hi);
+
+  const int rows = n_heads * (n_rep + 1);             // rotated rows: the queries of a head, then its key
+  for (int r0 = lane >> 3; r0 < rows; r0 += 4 * U) {
+    uint4 lo[U], hi[U];
+    int hk[U], slot[U];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      // x*cos rounded, then + rotate_half(x)*sin with one more rounding (torch.addcmul on the rounded product)
-      const float a = Elem<T>::to_f(x0[e]), bb = Elem<T>::to_f(x1[e]);
-      const float p0 = rnd<T>(a * Elem<T>::to_f(cl[e])), p1 = rnd<T>(bb * Elem<T>::to_f(chh[e]));
-      ol[e] = Elem<T>::from_f(__fadd_rn(p0, __fmul_rn(-bb, Elem<T>::to_f(sl[e]))));
-      oh[e] = Elem<T>::from_f(__fadd_rn(p1, __fmul_rn(a, Elem<T>::to_f(sh[e]))));
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + 4 * u;
+      hk[u] = r / (n_rep + 1);
+      slot[u] = r - hk[u] * (n_rep + 1);
+      if (r < rows) {
+        const T* x = src + (int64_t)(hk[u] * (n_rep + 2) + slot[u]) * kHeadDim;
+        lo[u] = *reinterpret_cast<const uint4*>(x);
+        hi[u] = *reinterpret_cast<const uint4*>(x + 64);
+      }
     }
-    T* dst;
-    if (slot < n_rep) dst = q_out + ((b * t_len + t) * (int64_t)(n_kv_heads * n_rep) + (int64_t)hk * n_rep + slot) * kHeadDim;
-    else dst = k_out + ((b * t_len + t) * (int64_t)n_kv_heads + hk) * kHeadDim;
-    *reinterpret_cast<uint4*>(dst + 8 * c) = o_lo;
-    *reinterpret_cast<uint4*>(dst + 64 + 8 * c) = o_hi;
-    if (slot == n_rep && to_cache) {
-      T* kc = k_cache + b * cache_stride_b + hk * cache_stride_h + (int64_t)fp_idx * kHeadDim;
-      *reinterpret_cast<uint4*>(kc + 8 * c) = o_lo;
-      *reinterpret_cast<uint4*>(kc + 64 + 8 * c) = o_hi;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r0 + 4 * u >= rows) break;
+      const T* x0 = reinterpret_cast<const T*>(&lo[u]);  const T* x1 = reinterpret_cast<const T*>(&hi[u]);
+      uint4 o_lo, o_hi;
+      T* ol = reinterpret_cast<T*>(&o_lo); T* oh = reinterpret_cast<T*>(&o_hi);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        // x*cos rounded, then + rotate_half(x)*sin with one more rounding (torch.addcmul on the rounded product)
+        const float a = Elem<T>::to_f(x0[e]), bb = Elem<T>::to_f(x1[e]);
+        const float p0 = rnd<T>(a * Elem<T>::to_f(cl[e])), p1 = rnd<T>(bb * Elem<T>::to_f(chh[e]));
+        ol[e] = Elem<T>::from_f(__fadd_rn(p0, __fmul_rn(-bb, Elem<T>::to_f(sl[e]))));
+        oh[e] = Elem<T>::from_f(__fadd_rn(p1, __fmul_rn(a, Elem<T>::to_f(sh[e]))));
+      }
+      T* dst = slot[u] < n_rep ? q_dst + (int64_t)(hk[u] * n_rep + slot[u]) * kHeadDim : k_dst + (int64_t)hk[u] * kHeadDim;
+      *reinterpret_cast<uint4*>(dst) = o_lo;
+      *reinterpret_cast<uint4*>(dst + 64) = o_hi;
+      if (slot[u] == n_rep && to_cache) {
+        T* kc = k_cache + cache_row + hk[u] * cache_stride_h;
+        *reinterpret_cast<uint4*>(kc) = o_lo;
+        *reinterpret_cast<uint4*>(kc + 64) = o_hi;
+      }
+    }
+  }
+  if (to_cache) {
+    for (int h = lane >> 3; h < n_heads; h += 4) {
+      const T* x = src + (int64_t)(h * (n_rep + 2) + n_rep + 1) * kHeadDim;
+      const uint4 lo = *reinterpret_cast<const uint4*>(x), hi = *reinterpret_cast<const uint4*>(x + 64);
+      T* dst = v_cache + cache_row + h * cache_stride_h;
+      *reinterpret_cast<uint4*>(dst) = lo;
+      *reinterpret_cast<uint4*>(dst + 64) = hi;
     }
   }
 }
@@ -334,21 +358,26 @@ extern "C" int cq_prefill_rope_split(const void* qkv, int64_t qkv_stride_b, int6
   if (!step::aligned16(qkv) || !step::aligned16(cos_table) || !step::aligned16(sin_table) || !step::aligned16(q_out) ||
       !step::aligned16(k_out) || !step::aligned16(k_cache) || !step::aligned16(v_cache))
     return CQ_ERR_BAD_ARG;
-  const int64_t total = (int64_t)batch * t_len * n_kv_heads * (n_rep + 2) * 8;
-  const int64_t blocks = (total + 255) / 256;
-  const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
+  // A warp takes all heads of a token unless that leaves fewer than 16 warps per SM: then as few heads as fill the chip
+  const int64_t n_tokens = (int64_t)batch * t_len;
+  int parts = 1;
+  while (parts < n_kv_heads && parts < 32768 && n_tokens * parts < 148 * 16) parts *= 2;
+  parts = parts < n_kv_heads ? parts : n_kv_heads;
+  const int heads_per = (n_kv_heads + parts - 1) / parts;
+  if ((n_tokens + 7) / 8 > 0x7fffffff) return CQ_ERR_UNSUPPORTED;
+  const dim3 grid((unsigned)((n_tokens + 7) / 8), (unsigned)((n_kv_heads + heads_per - 1) / heads_per));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == CQ_DTYPE_F16)
     step::prefill_rope_split_kernel<__half><<<grid, 256, 0, st>>>(
         static_cast<const __half*>(qkv), qkv_stride_b, qkv_stride_t, static_cast<const __half*>(cos_table),
         static_cast<const __half*>(sin_table), rope_len, position_ids, t_len, n_kv_heads, n_rep,
         static_cast<__half*>(q_out), static_cast<__half*>(k_out), static_cast<__half*>(k_cache),
-        static_cast<__half*>(v_cache), cache_stride_b, cache_stride_h, capacity, vis_start, vis_len, total);
+        static_cast<__half*>(v_cache), cache_stride_b, cache_stride_h, capacity, vis_start, vis_len, n_tokens, heads_per);
   else
     step::prefill_rope_split_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
         static_cast<const __nv_bfloat16*>(qkv), qkv_stride_b, qkv_stride_t, static_cast<const __nv_bfloat16*>(cos_table),
         static_cast<const __nv_bfloat16*>(sin_table), rope_len, position_ids, t_len, n_kv_heads, n_rep,
         static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_out), static_cast<__nv_bfloat16*>(k_cache),
-        static_cast<__nv_bfloat16*>(v_cache), cache_stride_b, cache_stride_h, capacity, vis_start, vis_len, total);
+        static_cast<__nv_bfloat16*>(v_cache), cache_stride_b, cache_stride_h, capacity, vis_start, vis_len, n_tokens, heads_per);
   return cudaGetLastError() == cudaSuccess ? CQ_OK : CQ_ERR_LAUNCH;
 }
