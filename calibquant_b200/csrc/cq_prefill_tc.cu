@@ -1,12 +1,12 @@
 // Dense causal prefill attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA).
 //
-// One work item = 256 queries of one (batch, query head), as two 128-row tiles A and B that share the
-// K/V stream.  One CTA per SM; it starts with the item of its own block index and then takes over blocks of the
-// grid that have not been launched yet (cluster launch control), so tensor memory, barriers and the pipeline
-// are set up once per SM and the hardware's launch order and load balance are kept.  Roles:
+// One work item = 256 query rows as two 128-row tiles A and B that share the K/V stream: the same rows of two heads of a KV
+// head, or (odd number of heads per KV head) adjacent rows of one head.  One CTA per SM; it starts with the item of its own
+// block index and then takes over blocks of the grid that have not been launched yet (cluster launch control), so tensor
+// memory, barriers and the pipeline are set up once per SM and the hardware's launch order and load balance are kept.  Roles:
 //   warp 9 (one lane)  TMA producer: the item's Q tiles, then its 128-key K/V tiles through a two-stage ring
 //                        that runs on across items; asks for the next block when an item's loads are issued
-//   warp 8 (one lane)  MMA issuer:
+//   warp 8             MMA issuer (one elected lane):
 //        S_X = Q_X K^T   tcgen05.mma kind::f16, A = Q_X and B = K from shared memory (K-major), D in the
 //                        tile's 128 TMEM columns
 //        O_X += P_X V    A = P_X read from TENSOR MEMORY (16-bit pairs the softmax warps stored over the
@@ -25,14 +25,18 @@
 // TMEM columns: S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).  Operand tiles in shared
 // memory use the 128-byte swizzle: a [128 rows x 64 elements] TMA box lands directly in the
 // canonical UMMA layout (8-row atoms of 1024 bytes).
-// Measured on B200: one M128 N128 K16 product takes 85 cycles of the tensor pipe whether A comes from shared or
-// tensor memory (98 with the softmax warps' TMEM traffic beside it), so the 32 products of a key tile bound a
-// CTA at ~3100 cycles per key tile; the loop runs at ~3400.
+// Bound: the tensor pipe takes 64 cycles per M128 N128 K16 product (measured, from shared and from tensor memory alike), 2050
+// for the 32 products of a key tile; the 2 x 128 x 128 exponentials take 2048 cycles of the special-function unit.  What
+// is above that is the chain of one tile (S -> softmax -> P V -> next S) that the other tile does not cover.
+// 16 x 3392 tokens, 32 query / 8 KV heads, bfloat16: 1642 us (918 TFLOP/s, causal) with one lane running the issuer's loop and
+// spilling softmax warps; 1481 with the register split; 1384 (1090 TFLOP/s) with uniform issue.
 //
 // Every mbarrier wait is bounded; on a timeout the CTA records CQ_ERR_TIMEOUT in the status word,
 // skips its remaining waits, frees its TMEM and returns.
 #include <cuda.h>
 #include <stdlib.h>
+
+#include <type_traits>
 
 #include "cq_common.cuh"
 #include "cq_ptx.cuh"
@@ -48,7 +52,11 @@ constexpr int BM = 128, BN = 128;
 constexpr int PANEL_BYTES = 128 * 128;          // [128 rows][64 x 16-bit]
 constexpr int TILE_BYTES = 2 * PANEL_BYTES;     // [128 rows][128 x 16-bit]
 constexpr int SMEM_BYTES = TILE_BYTES * 7 + 1024;   // Q x2, K x2, V x2, output staging (+ alignment slack)
-constexpr int SOFTMAX_THREADS = 256, MMA_WARP = 8, TMA_WARP = 9, THREADS = SOFTMAX_THREADS + 64;
+constexpr int SOFTMAX_THREADS = 256, MMA_WARP = 8, TMA_WARP = 9, THREADS = SOFTMAX_THREADS + 128;
+// A row's 128 logits and 32 words of probabilities do not fit the 168 registers that 384 threads start with: the softmax
+// warpgroups take what the third one (producer, issuer, two idle warps) gives up.  256 x 200 + 128 x 96 = 63 488 of the
+// launch's 384 x 168 = 64 512.
+constexpr int SOFTMAX_REGS = 200, CONTROL_REGS = 96;
 constexpr uint32_t WAIT_TRIES = 1u << 22;
 constexpr long long WAIT_CYCLES = 1ll << 30;     // ~0.5 s: bound of the waits on the S / P hand-offs
 constexpr uint32_t TMEM_COLS = 512;
@@ -56,6 +64,7 @@ constexpr float RESCALE_LOG2 = 8.f;          // a row is rescaled when its maxim
 
 struct Params {
   int t_len, hq, hkv;
+  int pair;              // 1: the two tiles of an item are the same queries of two heads; 0: adjacent tiles of one head
   float scale_log2;
   uint32_t idesc_s, idesc_pv;
   int is_bf16;
@@ -130,6 +139,16 @@ __device__ __forceinline__ bool tile_all(int id, bool flag) {
 // barrier among the four softmax warps of one query tile
 __device__ __forceinline__ void tile_barrier(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
+// register split between warpgroups; every warp of a group runs it
+template <int N> __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+// 1 in one lane of a converged warp
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p;
+}
+
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -168,25 +187,25 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// One work item = 256 queries of one (batch, query head) = one block index of the grid (x: 256-query block,
-// longest rows first; y: query head; z: batch row).  A CTA starts with its own index and then takes over blocks
-// that have not been launched yet (cluster launch control).  Measured, the CTAs running at the same time keep
-// working on the query blocks and heads of a few KV heads, whose K/V tiles stay in L2, as with one CTA per block;
-// a static assignment of items sorted by length lost that and ran 6 % slower.
+// One work item = one block index of the grid (x: query rows, longest first; y: query head or pair of heads; z: batch
+// row).  A CTA starts with its own index and then takes over blocks that have not been launched yet (cluster launch
+// control).  Measured, the CTAs running at the same time keep working on the query blocks and heads of a few KV heads,
+// whose K/V tiles stay in L2, as with one CTA per block; a static assignment of items sorted by length lost that and ran
+// 6 % slower.
 struct Item {
-  int h, b, hk, q0, n_a, n_b, n_max;
+  int h, b, hk, q0, n_a, n_b, n_max;        // tile X = 0 (A), 1 (B): head h + X pair, queries q0 + X (1 - pair) BM ..
 };
 __device__ __forceinline__ Item decode_item(const Params& p, int bx, int by, int bz) {
   Item w;
   const int qt = (int)gridDim.x - 1 - bx;         // longest rows first
-  w.h = by;
+  w.h = by << p.pair;
   w.b = bz;
   w.hk = w.h / (p.hq / p.hkv);
-  w.q0 = qt * 2 * BM;
-  const int t_tiles = (p.t_len + BN - 1) / BN;
-  // key tiles of query tile X = 0 (A), 1 (B); B may lie wholly past the end
+  w.q0 = qt * (2 - p.pair) * BM;
+  const int t_tiles = (p.t_len + BN - 1) / BN, q1 = p.pair ? w.q0 : w.q0 + BM;
+  // key tiles of query tile A, B; B may lie wholly past the end
   w.n_a = min((w.q0 + BM + BN - 1) / BN, t_tiles);
-  w.n_b = w.q0 + BM < p.t_len ? min((w.q0 + 2 * BM + BN - 1) / BN, t_tiles) : 0;
+  w.n_b = q1 < p.t_len ? min((q1 + BM + BN - 1) / BN, t_tiles) : 0;
   w.n_max = max(w.n_a, w.n_b);
   return w;
 }
@@ -240,128 +259,187 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
 
-  if (warp == TMA_WARP) {
-    // ================= TMA producer (one lane) =================
-    if (lane == 0) {
-      bool ok = true;
-      uint32_t kv = 0;                          // K/V tiles this CTA has loaded so far
-      int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
-      for (uint32_t it = 0; ok; ++it) {         // items of this CTA
-        const Item w = decode_item(p, bx, by, bz);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          // Q_x of the previous item is read until its last S_x has completed
-          if (it > 0) ok = ok && mbar_wait_bounded(&bar_q_free[x], (it - 1) & 1, WAIT_TRIES);
-          if (!ok) break;
-          mbar_expect_tx(&bar_q[x], TILE_BYTES);
-          tma_load_4d(q_s + x * TILE_BYTES, &tm_q, 0, w.h, w.q0 + x * BM, w.b, &bar_q[x]);
-          tma_load_4d(q_s + x * TILE_BYTES + PANEL_BYTES, &tm_q, 64, w.h, w.q0 + x * BM, w.b, &bar_q[x]);
-        }
-        for (int j = 0; j < w.n_max && ok; ++j, ++kv) {
-          const uint32_t s = kv & 1;
-          if (kv >= 2) ok = mbar_wait_bounded(&bar_kv_free[s], ((kv - 2) >> 1) & 1, WAIT_TRIES);
-          if (!ok) break;
-          mbar_expect_tx(&bar_kv_full[s], 2 * TILE_BYTES);
-          tma_load_4d(k_s + s * TILE_BYTES, &tm_k, 0, w.hk, j * BN, w.b, &bar_kv_full[s]);
-          tma_load_4d(k_s + s * TILE_BYTES + PANEL_BYTES, &tm_k, 64, w.hk, j * BN, w.b, &bar_kv_full[s]);
-          tma_load_4d(v_s + s * TILE_BYTES, &tm_v, 0, w.hk, j * BN, w.b, &bar_kv_full[s]);
-          tma_load_4d(v_s + s * TILE_BYTES + PANEL_BYTES, &tm_v, 64, w.hk, j * BN, w.b, &bar_kv_full[s]);
-        }
-        if (!ok) break;
-        // All loads of this item are on their way (the other roles are about two key tiles behind): ask for the
-        // item's successor now, not earlier, so that a CTA does not sit on a block another CTA could start.
-        const uint32_t slot = it & 1;
-        if (it >= 2) ok = mbar_wait_bounded(&bar_clc_free[slot], ((it >> 1) - 1) & 1, WAIT_TRIES);
-        if (!ok) break;
-        mbar_expect_tx(&bar_clc_full[slot], 16);
-        clc_try_cancel(&clc_resp[slot], &bar_clc_full[slot]);
-        ok = mbar_wait_bounded(&bar_clc_full[slot], (it >> 1) & 1, WAIT_TRIES);
-        if (!ok || !clc_read(&clc_resp[slot], bx, by, bz)) break;
-      }
-      if (!ok) atomicExch(p.status, CQ_ERR_TIMEOUT);
-    }
-    __syncwarp();
-  } else if (warp == MMA_WARP) {
-    // ================= MMA issuer (one lane) =================
-    if (lane == 0) {
-      // descriptors of the operand tiles; a k-step only moves the start address (14-bit field of
-      // 16-byte units in the low word, which cannot carry: shared memory ends below 256 KB)
-      const uint64_t qd[2] = {smem_desc(smem_u32(q_s), 16, 1024), smem_desc(smem_u32(q_s + TILE_BYTES), 16, 1024)};
-      const uint64_t kd[2] = {smem_desc(smem_u32(k_s), 16, 1024), smem_desc(smem_u32(k_s + TILE_BYTES), 16, 1024)};
-      const uint64_t vd[2] = {smem_desc(smem_u32(v_s), PANEL_BYTES, 1024),
-                              smem_desc(smem_u32(v_s + TILE_BYTES), PANEL_BYTES, 1024)};
-      auto issue_s = [&](int x, uint32_t stage) {   // S_x = Q_x K^T on the K tile of that stage, known to be there
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {        // 16 channels per step; panel = ks/4, 32 B per step
-          const uint64_t off = (uint64_t)(((ks >> 2) * PANEL_BYTES + (ks & 3) * 32) >> 4);
-          umma(tmem + (uint32_t)x * 128u, qd[x] + off, kd[stage] + off, p.idesc_s, ks > 0);
-        }
-        umma_commit(&bar_s[x]);
-      };
-      bool ok = true;
-      uint32_t kv = 0, cnt[2] = {0, 0};           // K/V tiles, key tiles of A / B done so far
-      int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
-      for (uint32_t it = 0; ok; ++it) {
-        const Item w = decode_item(p, bx, by, bz);
-        const int n_x[2] = {w.n_a, w.n_b};
-        ok = mbar_wait_bounded(&bar_kv_full[kv & 1], (kv >> 1) & 1, WAIT_TRIES);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          ok = ok && mbar_wait_bounded(&bar_q[x], it & 1, WAIT_TRIES);
-          if (!ok) break;
-          tc_fence_after();
-          if (n_x[x] > 0) issue_s(x, kv & 1);
-          if (n_x[x] <= 1) umma_commit(&bar_q_free[x]);     // that was the item's last S_x (or it has none)
-        }
-        for (int j = 0; j < w.n_max && ok; ++j) {
-          const uint32_t s = (kv + j) & 1;
-          bool next_k_ready = false;
+  if (warp >= SOFTMAX_THREADS / 32) {
+    setmaxnreg_dec<CONTROL_REGS>();
+    if (warp == TMA_WARP) {
+      // ================= TMA producer (one lane) =================
+      if (lane == 0) {
+        bool ok = true;
+        uint32_t kv = 0;                          // K/V tiles this CTA has loaded so far
+        int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
+        for (uint32_t it = 0; ok; ++it) {         // items of this CTA
+          const Item w = decode_item(p, bx, by, bz);
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
-            if (j >= n_x[x]) continue;
-            // O_x += P_x(j) V(j), 16 keys = 8 TMEM columns per step; the first four steps start as soon as
-            // the probabilities of keys 0-63 are stored, while the softmax warps work on keys 64-127
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              ok = mbar_wait_cycles(&bar_p[x][hf], (cnt[x] + j) & 1, WAIT_CYCLES);
-              if (!ok) break;
-              tc_fence_after();
-#pragma unroll
-              for (int ks = 4 * hf; ks < 4 * hf + 4; ++ks)
-                umma_ts(tmem + 256u + (uint32_t)x * 128u, tmem + (uint32_t)x * 128u + (uint32_t)ks * 8u,
-                        vd[s] + (uint64_t)(ks * 2048 >> 4), p.idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-            }
+            // Q_x of the previous item is read until its last S_x has completed
+            if (it > 0) ok = ok && mbar_wait_bounded(&bar_q_free[x], (it - 1) & 1, WAIT_TRIES);
             if (!ok) break;
-            umma_commit(&bar_pv[x]);
-            // S_x(j+1) overwrites the columns P_x(j) lives in; the tensor pipe runs in issue order
-            if (j + 1 < n_x[x]) {
-              if (!next_k_ready) {
-                ok = mbar_wait_bounded(&bar_kv_full[s ^ 1], ((kv + j + 1) >> 1) & 1, WAIT_TRIES);
-                if (!ok) break;
-                tc_fence_after();
-                next_k_ready = true;
-              }
-              issue_s(x, s ^ 1);
-              if (j + 2 == n_x[x]) umma_commit(&bar_q_free[x]);   // the item's last S_x
-            }
+            mbar_expect_tx(&bar_q[x], TILE_BYTES);
+            const int hx = w.h + x * p.pair, qx0 = w.q0 + x * (1 - p.pair) * BM;
+            tma_load_4d(q_s + x * TILE_BYTES, &tm_q, 0, hx, qx0, w.b, &bar_q[x]);
+            tma_load_4d(q_s + x * TILE_BYTES + PANEL_BYTES, &tm_q, 64, hx, qx0, w.b, &bar_q[x]);
+          }
+          for (int j = 0; j < w.n_max && ok; ++j, ++kv) {
+            const uint32_t s = kv & 1;
+            if (kv >= 2) ok = mbar_wait_bounded(&bar_kv_free[s], ((kv - 2) >> 1) & 1, WAIT_TRIES);
+            if (!ok) break;
+            mbar_expect_tx(&bar_kv_full[s], 2 * TILE_BYTES);
+            tma_load_4d(k_s + s * TILE_BYTES, &tm_k, 0, w.hk, j * BN, w.b, &bar_kv_full[s]);
+            tma_load_4d(k_s + s * TILE_BYTES + PANEL_BYTES, &tm_k, 64, w.hk, j * BN, w.b, &bar_kv_full[s]);
+            tma_load_4d(v_s + s * TILE_BYTES, &tm_v, 0, w.hk, j * BN, w.b, &bar_kv_full[s]);
+            tma_load_4d(v_s + s * TILE_BYTES + PANEL_BYTES, &tm_v, 64, w.hk, j * BN, w.b, &bar_kv_full[s]);
           }
           if (!ok) break;
-          umma_commit(&bar_kv_free[s]);             // K(j), V(j) are free once everything issued so far has drained
+          // All loads of this item are on their way (the other roles are about two key tiles behind): ask for the
+          // item's successor now, not earlier, so that a CTA does not sit on a block another CTA could start.
+          const uint32_t slot = it & 1;
+          if (it >= 2) ok = mbar_wait_bounded(&bar_clc_free[slot], ((it >> 1) - 1) & 1, WAIT_TRIES);
+          if (!ok) break;
+          mbar_expect_tx(&bar_clc_full[slot], 16);
+          clc_try_cancel(&clc_resp[slot], &bar_clc_full[slot]);
+          ok = mbar_wait_bounded(&bar_clc_full[slot], (it >> 1) & 1, WAIT_TRIES);
+          if (!ok || !clc_read(&clc_resp[slot], bx, by, bz)) break;
+        }
+        if (!ok) atomicExch(p.status, CQ_ERR_TIMEOUT);
+      }
+      __syncwarp();
+    } else if (warp == MMA_WARP) {
+      // ================= MMA issuer =================
+      // The whole warp runs the loop and one elected lane issues: control flow and operands are uniform, so that a product costs
+      // the issuing lane a few instructions (one lane alone in the loop, with the stage as an index, could not keep the pipe fed)
+      const uint32_t lead = elect_one();
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint32_t q_b = smem_u32(q_s), k_b = smem_u32(k_s), v_b = smem_u32(v_s);
+      // descriptors of the operand tiles; a k-step only moves the start address (14-bit field of
+      // 16-byte units in the low word, which cannot carry: shared memory ends below 256 KB)
+      const uint64_t qd = smem_desc(q_b, 16, 1024), kd = smem_desc(k_b, 16, 1024), vd = smem_desc(v_b, PANEL_BYTES, 1024);
+      auto issue_s = [&](auto xc, auto sc) {        // S_x = Q_x K^T on the K tile of that stage, known to be there
+        constexpr int x = decltype(xc)::value, st = decltype(sc)::value;
+        if (lead) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) {          // 16 channels per step; panel = ks/4, 32 B per step
+            constexpr uint64_t tile = TILE_BYTES >> 4;
+            const uint64_t off = (uint64_t)(((ks >> 2) * PANEL_BYTES + (ks & 3) * 32) >> 4);
+            umma(tm + (uint32_t)x * 128u, qd + (x * tile + off), kd + (st * tile + off), p.idesc_s, ks > 0);
+          }
+          umma_commit(&bar_s[x]);
+        }
+      };
+      // O_x += P_x(j) V(j) of half the keys, 16 keys = 8 TMEM columns per step
+      auto issue_pv = [&](auto xc, auto sc, auto hc, bool acc) {
+        constexpr int x = decltype(xc)::value, st = decltype(sc)::value, hf = decltype(hc)::value;
+        if (lead) {
+#pragma unroll
+          for (int ks = 4 * hf; ks < 4 * hf + 4; ++ks)
+            umma_ts(tm + 256u + (uint32_t)x * 128u, tm + (uint32_t)x * 128u + (uint32_t)ks * 8u,
+                    vd + (uint64_t)((st * TILE_BYTES + ks * 2048) >> 4), p.idesc_pv, (ks > 0 || acc) ? 1u : 0u);
+        }
+      };
+      auto commit = [&](uint64_t* bar) { if (lead) umma_commit(bar); };
+      using C0 = std::integral_constant<int, 0>;
+      using C1 = std::integral_constant<int, 1>;
+      // every decision is the whole warp's, a timeout of one lane included
+      auto all = [](bool r) { return __all_sync(0xffffffffu, r) != 0; };
+      bool ok = true;
+      uint32_t kv = 0, cnt[2] = {0, 0};             // K/V tiles, key tiles of A / B done so far
+      int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
+      Item w = decode_item(p, bx, by, bz);
+      bool begun = false;                           // the item's S_A(0) has been issued behind the item before
+      for (uint32_t it = 0; ok; ++it) {
+        auto first_s = [&](auto xc) {
+          constexpr int x = decltype(xc)::value;
+          const int n = x == 0 ? w.n_a : w.n_b;
+          if (x == 0 && begun) return;
+          ok = ok && all(mbar_wait_bounded(&bar_q[x], it & 1, WAIT_TRIES));
+          if (!ok) return;
+          tc_fence_after();
+          if (n > 0) { if (kv & 1) issue_s(xc, C1{}); else issue_s(xc, C0{}); }
+          if (n <= 1) commit(&bar_q_free[x]);       // that was the item's last S_x (or it has none)
+        };
+        ok = all(mbar_wait_bounded(&bar_kv_full[kv & 1], (kv >> 1) & 1, WAIT_TRIES));
+        first_s(C0{});
+        first_s(C1{});
+        // the item's successor: 0 not asked yet, 1 known, 2 there is none
+        int next = 0;
+        Item w2 = w;
+        auto take_next = [&]() {
+          next = clc_read(&clc_resp[it & 1], bx, by, bz) ? 1 : 2;
+          __syncwarp();
+          if (lead) mbar_arrive(&bar_clc_free[it & 1]);
+          if (next == 1) w2 = decode_item(p, bx, by, bz);
+        };
+        begun = false;
+        bool next_k_ready = false;
+        // key tile j of query tile x, whose K/V tile is in stage st
+        auto step = [&](auto xc, auto sc, int j) {
+          constexpr int x = decltype(xc)::value, st = decltype(sc)::value;
+          using Other = std::integral_constant<int, st ^ 1>;
+          const int n = x == 0 ? w.n_a : w.n_b;
+          if (j >= n) return;
+          // the first four steps start as soon as the probabilities of keys 0-63 are stored, while the softmax warps work
+          // on keys 64-127
+          ok = all(mbar_wait_cycles(&bar_p[x][0], (cnt[x] + j) & 1, WAIT_CYCLES));
+          if (!ok) return;
+          tc_fence_after();
+          issue_pv(xc, sc, C0{}, j > 0);
+          ok = all(mbar_wait_cycles(&bar_p[x][1], (cnt[x] + j) & 1, WAIT_CYCLES));
+          if (!ok) return;
+          tc_fence_after();
+          issue_pv(xc, sc, C1{}, true);
+          commit(&bar_pv[x]);
+          // S_x(j+1) overwrites the columns P_x(j) lives in; the tensor pipe runs in issue order
+          if (j + 1 < n) {
+            if (!next_k_ready) {
+              ok = all(mbar_wait_bounded(&bar_kv_full[st ^ 1], ((kv + j + 1) >> 1) & 1, WAIT_TRIES));
+              if (!ok) return;
+              tc_fence_after();
+              next_k_ready = true;
+            }
+            issue_s(xc, Other{});
+            if (j + 2 == n) commit(&bar_q_free[x]);     // the item's last S_x
+          } else if (x == 0 && w.n_a == w.n_b) {
+            // A is through with the item, B still has P V of its last tile to come: the successor's S_A goes in between,
+            // as within an item, if its operands are there already (otherwise after B, where waiting holds up nothing).
+            // Tiles of unequal length would come into phase here and lose the overlap of softmax and products
+            if (all(mbar_try_wait(&bar_clc_full[it & 1], (it >> 1) & 1))) take_next();
+            if (next == 1 && all(mbar_try_wait(&bar_q[0], (it + 1) & 1)) && all(mbar_try_wait(&bar_kv_full[st ^ 1], ((kv + j + 1) >> 1) & 1))) {
+              tc_fence_after();
+              issue_s(C0{}, Other{});                   // n_a > 0 in every item
+              if (w2.n_a == 1) commit(&bar_q_free[0]);
+              begun = true;
+            }
+          }
+        };
+        for (int j = 0; j < w.n_max && ok; ++j) {
+          const uint32_t s = (kv + j) & 1;
+          next_k_ready = false;
+          if (s == 0) {
+            step(C0{}, C0{}, j);
+            if (ok) step(C1{}, C0{}, j);
+          } else {
+            step(C0{}, C1{}, j);
+            if (ok) step(C1{}, C1{}, j);
+          }
+          if (!ok) break;
+          commit(&bar_kv_free[s]);                  // K(j), V(j) are free once everything issued so far has drained
         }
         kv += (uint32_t)w.n_max;
         cnt[0] += (uint32_t)w.n_a;
         cnt[1] += (uint32_t)w.n_b;
         if (!ok) break;
-        ok = mbar_wait_bounded(&bar_clc_full[it & 1], (it >> 1) & 1, WAIT_TRIES);
-        if (!ok) break;
-        const bool more = clc_read(&clc_resp[it & 1], bx, by, bz);
-        mbar_arrive(&bar_clc_free[it & 1]);
-        if (!more) break;
+        if (next == 0) {
+          ok = all(mbar_wait_bounded(&bar_clc_full[it & 1], (it >> 1) & 1, WAIT_TRIES));
+          if (!ok) break;
+          take_next();
+        }
+        if (next == 2) break;
+        w = w2;
       }
-      if (!ok) atomicExch(p.status, CQ_ERR_TIMEOUT);
+      if (!ok && lead) atomicExch(p.status, CQ_ERR_TIMEOUT);
+      __syncwarp();
     }
-    __syncwarp();
   } else {
+    setmaxnreg_inc<SOFTMAX_REGS>();
     // ===== softmax: warps 0-3 tile A, 4-7 tile B; thread = one query row =====
     const int x = warp >> 2, quarter = warp & 3;
     const int r_in = quarter * 32 + lane;               // row inside the tile = TMEM lane
@@ -374,7 +452,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     for (uint32_t it = 0;; ++it) {
       const Item w = decode_item(p, bx, by, bz);
       const int n_x = x == 0 ? w.n_a : w.n_b;
-      const int qx0 = w.q0 + x * BM;
+      const int hx = w.h + x * p.pair, qx0 = w.q0 + x * (1 - p.pair) * BM;
       const int row = qx0 + r_in;
       float m_ref = -INFINITY, l_run = 0.f;             // reference maximum (log2 units), row sum
       for (int j = 0; j < n_x; ++j) {
@@ -473,8 +551,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tile_barrier(1 + x);
         if (quarter == 0 && lane == 0) {
           if (ok) {
-            tma_store_4d(&tm_o, o_s, 0, w.h, qx0, w.b);
-            tma_store_4d(&tm_o, o_s + PANEL_BYTES, 64, w.h, qx0, w.b);
+            tma_store_4d(&tm_o, o_s, 0, hx, qx0, w.b);
+            tma_store_4d(&tm_o, o_s + PANEL_BYTES, 64, hx, qx0, w.b);
             tma_store_commit_wait_read();
           } else {
             atomicExch(p.status, CQ_ERR_TIMEOUT);
@@ -561,12 +639,17 @@ int prefill_tc_run(const void* q, const void* k, const void* v, void* out, int b
   }
   Params p;
   p.t_len = t_len; p.hq = hq; p.hkv = hkv;
+  // Two heads of one KV head, same queries, share every K/V tile and have the same number of them, so that neither tile of an
+  // item waits for the other at its end.  Needs an even number of heads per KV head; a prompt of one tile gives twice the
+  // items (half of the chip would idle) with the heads apart
+  p.pair = (hq / hkv) % 2 == 0 && t_len > BM ? 1 : 0;
   p.scale_log2 = 1.4426950408889634f / sqrtf(128.f);
   p.idesc_s = make_idesc(is_bf16, 0, BM, BN);
   p.idesc_pv = make_idesc(is_bf16, 1, BM, BN);
   p.is_bf16 = is_bf16;
   p.status = status;
-  dim3 grid((unsigned)((t_len + 2 * BM - 1) / (2 * BM)), (unsigned)hq, (unsigned)batch);
+  const int rows = p.pair ? BM : 2 * BM;
+  dim3 grid((unsigned)((t_len + rows - 1) / rows), (unsigned)(p.pair ? hq / 2 : hq), (unsigned)batch);
   if (is_bf16) prefill_tc_kernel<true><<<grid, THREADS, SMEM_BYTES, st>>>(tq, tk, tv, to, p);
   else prefill_tc_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(tq, tk, tv, to, p);
   return check_launch();
