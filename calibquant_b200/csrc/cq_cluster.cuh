@@ -27,6 +27,7 @@ __device__ __forceinline__ void arrive_peer(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool wait_peers(uint64_t* bar, uint32_t max_tries) {      // phase 0, writes of the peers visible
+#pragma unroll 1
   for (uint32_t i = 0; i < max_tries; ++i) {
     uint32_t ok;
     asm volatile(
@@ -35,7 +36,6 @@ __device__ __forceinline__ bool wait_peers(uint64_t* bar, uint32_t max_tries) { 
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(smem_u32(bar)) : "memory");
     if (ok) return true;
-    if (i > 64) __nanosleep(64);
   }
   return false;
 }

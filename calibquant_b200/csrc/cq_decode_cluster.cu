@@ -242,8 +242,8 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   auto wait_full = [&](int k) {
     const int s = k % NS, turn = k / NS + 1;
     uint32_t tries = 0;
-    while (*reinterpret_cast<volatile int*>(&issued_s[s]) != turn && ++tries < WAIT_TRIES)
-      if (tries > 64) __nanosleep(64);
+#pragma unroll 1
+    while (*reinterpret_cast<volatile int*>(&issued_s[s]) != turn && ++tries < WAIT_TRIES) __nanosleep(32);
     __threadfence_block();
     const bool ok = tries < WAIT_TRIES && mbar_wait_bounded(&full_bar[s], (uint32_t)((k / NS) & 1), WAIT_TRIES);
     failed = !__all_sync(0xffffffffu, ok);

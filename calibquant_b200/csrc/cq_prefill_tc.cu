@@ -118,11 +118,12 @@ __device__ __forceinline__ bool clc_read(const void* resp, int& bx, int& by, int
 // A use counter in shared memory (monotonic, so a waiter may be any number of uses behind or ahead, which the
 // parity of an mbarrier phase cannot express): bounded wait until it has reached `target`.
 __device__ __forceinline__ bool wait_count(const uint32_t* ctr, uint32_t target, uint32_t max_tries) {
+#pragma unroll 1
   for (uint32_t i = 0; i < max_tries; ++i) {
     uint32_t v;
     asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(ctr)) : "memory");
     if (v >= target) return true;
-    if (i > 64) __nanosleep(64);
+    __nanosleep(32);
   }
   return false;
 }

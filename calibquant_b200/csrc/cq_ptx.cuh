@@ -64,12 +64,13 @@ __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Bounded wait: returns false when the phase did not complete within `max_tries` polls.
+// Bounded wait: returns false when the phase did not complete within `max_tries` polls (each of which suspends the thread
+// for a hardware-defined interval).  Nothing in the loop depends on its index: with a back-off after the first 64 polls the
+// compiler peeled those off, about 5 KB of instructions at every call (the prefill attention: 124 KB of code, now 58 KB).
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint32_t max_tries) {
-  for (uint32_t i = 0; i < max_tries; ++i) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < max_tries; ++i)
     if (mbar_try_wait(bar, parity)) return true;
-    if (i > 64) __nanosleep(64);
-  }
   return false;
 }
 
