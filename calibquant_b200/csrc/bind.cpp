@@ -224,6 +224,11 @@ PyObject* py_quant_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int dt = dtype_enum(x);
   Call call(x);
   Tensor s = empty({B, 1, H, D}, x), zp = empty({B, 1, H, D}, x), enc = empty({B, H, T, D * bits / 8}, x, at::kByte);
+  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && st[0] % 8 == 0 && st[1] % 8 == 0 && st[2] % 8 == 0) {
+    check(cq_calib_quant_encode(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, clip, dt, s.data_ptr(), zp.data_ptr(),
+                                (uint8_t*)enc.data_ptr(), call.stream), "cq_calib_quant_encode");
+    return wrap3(enc, s, zp);
+  }
   check(cq_calib_minmax(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, clip, dt, s.data_ptr(), zp.data_ptr(),
                         call.stream), "cq_calib_minmax");
   check(cq_calib_quantize(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, dt, s.data_ptr(), zp.data_ptr(), 0,

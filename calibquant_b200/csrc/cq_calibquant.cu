@@ -17,13 +17,10 @@
 #include "cq_ptx.cuh"
 #include "cq_u8_cluster.cuh"
 #include "cq_u8_format.cuh"
+#include "cq_u8_quant.cuh"
 
 namespace cq {
 namespace calib {
-
-template <typename T> struct Pk2;
-template <> struct Pk2<__half> { static __device__ __forceinline__ __half2 magic() { return __float2half2_rn(1024.f); } };
-template <> struct Pk2<__nv_bfloat16> { static __device__ __forceinline__ __nv_bfloat162 magic() { return __float2bfloat162_rn(128.f); } };
 
 constexpr int MM_SLICES = 8;   // token slices per (b,h) in the min/max kernel
 
@@ -50,9 +47,8 @@ minmax_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, int64_t
       mn = fminf(mn, mn_s[i][d]);
       mx = fmaxf(mx, mx_s[i][d]);
     }
-    const float x_min = rnd<T>(mn * clip), x_max = rnd<T>(mx * clip);
-    const float s = rnd<T>(__fdiv_rn(rnd<T>(x_max - x_min), (float)levels));
-    const float z = rnd<T>(__fdiv_rn(-x_min, s));
+    float s, z;
+    scale_zero<T>(mn, mx, clip, levels, s, z);
     scale[(int64_t)bh * kHeadDim + d] = Elem<T>::from_f(s);
     zp[(int64_t)bh * kHeadDim + d] = Elem<T>::from_f(z);
   }
@@ -64,12 +60,6 @@ minmax_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, int64_t
 // 16-bit min/max (exact).  The slices meet in the output arrays themselves, which hold the running
 // minimum (scale array) and maximum (zero-point array) as order-preserving 16-bit keys updated by
 // compare-and-swap; a last launch turns them into scale and zero point with the arithmetic of minmax_kernel.
-__device__ __forceinline__ unsigned short key16(unsigned short b) {
-  return (b & 0x8000u) ? (unsigned short)~b : (unsigned short)(b | 0x8000u);
-}
-__device__ __forceinline__ unsigned short unkey16(unsigned short k) {
-  return (k & 0x8000u) ? (unsigned short)(k & 0x7fffu) : (unsigned short)~k;
-}
 __global__ void minmax_init_kernel(unsigned short* __restrict__ mn_key, unsigned short* __restrict__ mx_key, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) { mn_key[i] = 0xffffu; mx_key[i] = 0u; }
@@ -160,9 +150,8 @@ __global__ void minmax_finish_kernel(T* __restrict__ scale, T* __restrict__ zp, 
   const unsigned short bl = unkey16(reinterpret_cast<const unsigned short*>(scale)[i]);
   const unsigned short bh = unkey16(reinterpret_cast<const unsigned short*>(zp)[i]);
   const float mn = Elem<T>::to_f(*reinterpret_cast<const T*>(&bl)), mx = Elem<T>::to_f(*reinterpret_cast<const T*>(&bh));
-  const float x_min = rnd<T>(mn * clip), x_max = rnd<T>(mx * clip);
-  const float s = rnd<T>(__fdiv_rn(rnd<T>(x_max - x_min), (float)levels));
-  const float z = rnd<T>(__fdiv_rn(-x_min, s));
+  float s, z;
+  scale_zero<T>(mn, mx, clip, levels, s, z);
   scale[i] = Elem<T>::from_f(s);
   zp[i] = Elem<T>::from_f(z);
 }
@@ -233,15 +222,6 @@ quantize_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, int64
 // per-element arithmetic.
 constexpr int QT_TOKENS = 2048;        // tokens per CTA
 
-template <typename T>
-__device__ __forceinline__ float ref_code(float x, float s, float z, int levels) {
-  const float y = rnd<T>(rnd<T>(__fdiv_rn(x, s)) + z);
-  return rintf(fminf(fmaxf(y, 0.f), (float)levels));
-}
-template <typename T> struct Finite16;
-template <> struct Finite16<__half> { static constexpr unsigned short MAXPOS = 0x7bffu; };
-template <> struct Finite16<__nv_bfloat16> { static constexpr unsigned short MAXPOS = 0x7f7fu; };
-
 template <typename T, int BITS>
 __global__ void __launch_bounds__(256)
 quantize_thr_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, int64_t st, int64_t sh,
@@ -259,27 +239,8 @@ quantize_thr_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
     const float z = Elem<T>::to_f(zp[(int64_t)bh * kHeadDim + tid]);
     bad = !(s > 0.f) || isinf(s) || isnan(z) || isinf(z);
     if (!bad) {
-      const unsigned short k_min = key16((unsigned short)(Finite16<T>::MAXPOS | 0x8000u)), k_max = key16(Finite16<T>::MAXPOS);
 #pragma unroll
-      for (int k = 0; k < LEVELS; ++k) {
-        unsigned lo = k_min, hi = k_max;
-        unsigned short theta;
-        const unsigned short b_lo = unkey16((unsigned short)lo), b_hi = unkey16((unsigned short)hi);
-        if (ref_code<T>(Elem<T>::to_f(*reinterpret_cast<const T*>(&b_lo)), s, z, LEVELS) > (float)k) {
-          theta = 0xfc00u;                              // every finite number exceeds level k: -inf
-          if (sizeof(T) == 2 && Finite16<T>::MAXPOS == 0x7f7fu) theta = 0xff80u;
-        } else if (ref_code<T>(Elem<T>::to_f(*reinterpret_cast<const T*>(&b_hi)), s, z, LEVELS) <= (float)k) {
-          theta = b_hi;                                 // only +inf exceeds the largest finite number
-        } else {
-          while (hi - lo > 1) {
-            const unsigned mid = (lo + hi) >> 1;
-            const unsigned short bm = unkey16((unsigned short)mid);
-            if (ref_code<T>(Elem<T>::to_f(*reinterpret_cast<const T*>(&bm)), s, z, LEVELS) <= (float)k) lo = mid; else hi = mid;
-          }
-          theta = unkey16((unsigned short)lo);
-        }
-        thr_s[k][tid] = *reinterpret_cast<const T*>(&theta);
-      }
+      for (int k = 0; k < LEVELS; ++k) thr_s[k][tid] = threshold<T>(s, z, k, LEVELS);
     }
   }
   const int any_bad = __syncthreads_or(bad);

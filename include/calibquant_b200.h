@@ -258,6 +258,13 @@ int cq_calib_minmax(const void* x, int batch, int t_len, int heads, int head_dim
                     int bits, float clip, int dtype, void* scale, void* zero_point, void* stream);
 
 /*
+ * cq_calib_quant_encode: cq_calib_minmax followed by cq_calib_quantize with enc_out, as one launch (a thread-block cluster per
+ * (batch, head)).  enc_out 4-byte aligned; the results are the same.
+ */
+int cq_calib_quant_encode(const void* x, int batch, int t_len, int heads, int head_dim, const int64_t* strides, int bits, float clip,
+                          int dtype, void* scale, void* zero_point, uint8_t* enc_out, void* stream);
+
+/*
  * cq_calib_quantize: the quantize / dequantize lines of calibquant.py:35-41 and, fused, the byte
  * packing of calibquant.py:114-137 `encode` (most significant field first).
  *   xq_out  (optional) : [B,T,H,D] contiguous, the codes as numbers of the data dtype
