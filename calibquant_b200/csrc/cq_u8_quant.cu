@@ -16,9 +16,10 @@ namespace calib {
 
 using namespace cluster;
 
-constexpr int QE_THREADS = 512, QE_LANES = QE_THREADS / 16, MAX_S = 8;
+constexpr int QE_THREADS = 512, QE_LANES = QE_THREADS / 16, MAX_S = 8, KEEP = 8;
 
-template <typename T, int BITS>
+// KEPT: the slice has at most KEEP rows per thread; they are loaded at once and stay in registers for the second use
+template <typename T, int BITS, bool KEPT>
 __global__ void __launch_bounds__(QE_THREADS, 2)
 quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, int64_t st, int64_t sh, float clip,
                     T* __restrict__ scale, T* __restrict__ zp, uint8_t* __restrict__ enc) {
@@ -34,23 +35,34 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
   const int t_begin = (int)((int64_t)t_len * rank / S), t_end = (int)((int64_t)t_len * (rank + 1) / S);      // not empty: S <= t_len
   const T* base = x + b * sb + h * sh + col * 8;
 
+  uint4 kept[KEPT ? KEEP : 1];
+  if (KEPT) {
+#pragma unroll
+    for (int u = 0; u < KEEP; ++u) kept[KEPT ? u : 0] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t_begin + tl + u * QE_LANES, t_end - 1) * st));
+  }
   // extremes of the slice; every thread starts from a row of it, so no neutral element is needed
   {
-    const uint4 first = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t_begin + tl, t_end - 1) * st));
+    const uint4 first = KEPT ? kept[0] : __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t_begin + tl, t_end - 1) * st));
     T2 mn[4], mx[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) mn[i] = mx[i] = reinterpret_cast<const T2*>(&first)[i];
+    auto take = [&](const uint4& v) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        mn[i] = __hmin2(mn[i], reinterpret_cast<const T2*>(&v)[i]);
+        mx[i] = __hmax2(mx[i], reinterpret_cast<const T2*>(&v)[i]);
+      }
+    };
+    if (KEPT) {
+#pragma unroll
+      for (int u = 0; u < KEEP; ++u) take(kept[KEPT ? u : 0]);
+    } else
     for (int t = t_begin + tl; t < t_end; t += U * QE_LANES) {
       uint4 v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t + u * QE_LANES, t_end - 1) * st));
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          mn[i] = __hmin2(mn[i], reinterpret_cast<const T2*>(&v[u])[i]);
-          mx[i] = __hmax2(mx[i], reinterpret_cast<const T2*>(&v[u])[i]);
-        }
+      for (int u = 0; u < U; ++u) take(v[u]);
     }
     // the two token lanes of a warp, then the warps
 #pragma unroll
@@ -121,8 +133,7 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
     float s[8], z[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) { s[i] = Elem<T>::to_f(sz_s[0][col * 8 + i]); z[i] = Elem<T>::to_f(sz_s[1][col * 8 + i]); }
-    for (int t = t_begin + tl; t < t_last; t += QE_LANES) {
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t, t_end - 1) * st));
+    auto encode = [&](int t, const uint4& raw) {
       const T* xv = reinterpret_cast<const T*>(&raw);
       uint32_t v = 0;
 #pragma unroll
@@ -131,6 +142,14 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
         v |= code << (8 * (i * BITS / 8) + 8 - BITS - (i * BITS) % 8);
       }
       store(t, v);
+    };
+    if (KEPT) {
+#pragma unroll
+      for (int u = 0; u < KEEP; ++u)
+        if (t_begin + u * QE_LANES < t_end) encode(t_begin + tl + u * QE_LANES, kept[KEPT ? u : 0]);
+    } else {
+      for (int t = t_begin + tl; t < t_last; t += QE_LANES)
+        encode(t, __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t, t_end - 1) * st)));
     }
     return;
   }
@@ -142,31 +161,38 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
 #pragma unroll
       for (int i = 0; i < 4; ++i) thr[k][i] = reinterpret_cast<const T2*>(&w)[i];
     }
-    for (int t0 = t_begin + tl; t0 < t_last; t0 += U * QE_LANES) {
-      uint4 v[U];
+    auto encode = [&](int t, const uint4& raw) {
+      const T2* xv = reinterpret_cast<const T2*>(&raw);
+      uint32_t r = 0;
+      if (BITS == 1) {
+        // channel i at bit 7 - i; pair p = channels (2p, 2p+1) -> bits 7-2p (low half), 22-2p (high half)
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t0 + u * QE_LANES, t_end - 1) * st));
+        for (int i = 0; i < 4; ++i) r |= __hgt2_mask(xv[i], thr[0][i]) & ((0x80u >> (2 * i)) | (0x400000u >> (2 * i)));
+        r = (r | (r >> 16)) & 0xffu;
+      } else {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const T2* xv = reinterpret_cast<const T2*>(&v[u]);
-        uint32_t r = 0;
-        if (BITS == 1) {
-          // channel i at bit 7 - i; pair p = channels (2p, 2p+1) -> bits 7-2p (low half), 22-2p (high half)
+        for (int i = 0; i < 4; ++i) {
+          T2 cnt = __hgt2(xv[i], thr[0][i]);             // the code as a number of the data type
 #pragma unroll
-          for (int i = 0; i < 4; ++i) r |= __hgt2_mask(xv[i], thr[0][i]) & ((0x80u >> (2 * i)) | (0x400000u >> (2 * i)));
-          r = (r | (r >> 16)) & 0xffu;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            T2 cnt = __hgt2(xv[i], thr[0][i]);             // the code as a number of the data type
-#pragma unroll
-            for (int k = 1; k < LEVELS; ++k) cnt = __hadd2(cnt, __hgt2(xv[i], thr[k][i]));
-            const T2 m = __hadd2(cnt, Pk2<T>::magic());    // 0..3 in the low mantissa bits
-            const uint32_t w = *reinterpret_cast<const uint32_t*>(&m) & 0x00030003u;
-            r |= (((w & 0xffffu) << 2) | (w >> 16)) << (8 * (i >> 1) + 4 - 4 * (i & 1));      // (code 2i, code 2i+1) as four bits
-          }
+          for (int k = 1; k < LEVELS; ++k) cnt = __hadd2(cnt, __hgt2(xv[i], thr[k][i]));
+          const T2 m = __hadd2(cnt, Pk2<T>::magic());    // 0..3 in the low mantissa bits
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(&m) & 0x00030003u;
+          r |= (((w & 0xffffu) << 2) | (w >> 16)) << (8 * (i >> 1) + 4 - 4 * (i & 1));      // (code 2i, code 2i+1) as four bits
         }
-        store(t0 + u * QE_LANES, r);
+      }
+      store(t, r);
+    };
+    if (KEPT) {
+#pragma unroll
+      for (int u = 0; u < KEEP; ++u)
+        if (t_begin + u * QE_LANES < t_end) encode(t_begin + tl + u * QE_LANES, kept[KEPT ? u : 0]);
+    } else {
+      for (int t0 = t_begin + tl; t0 < t_last; t0 += U * QE_LANES) {
+        uint4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t0 + u * QE_LANES, t_end - 1) * st));
+#pragma unroll
+        for (int u = 0; u < U; ++u) encode(t0 + u * QE_LANES, v[u]);
       }
     }
   }
@@ -188,7 +214,8 @@ static int launch_quant_encode(const void* x, int batch, int t_len, int heads, c
   attr[0].val.clusterDim.x = (unsigned)S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, quant_encode_kernel<T, BITS>, static_cast<const T*>(x), heads, t_len, strides[0], strides[1], strides[2], clip,
+  const bool fits = (t_len + S - 1) / S <= KEEP * QE_LANES;
+  if (cudaLaunchKernelEx(&cfg, fits ? quant_encode_kernel<T, BITS, true> : quant_encode_kernel<T, BITS, false>, static_cast<const T*>(x), heads, t_len, strides[0], strides[1], strides[2], clip,
                          static_cast<T*>(scale), static_cast<T*>(zp), enc) != cudaSuccess) {
     (void)cudaGetLastError();
     return CQ_ERR_LAUNCH;

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("bits,clip", [(1, 0.5), (2, 1), (4, 1)])
 @pytest.mark.parametrize("B,T,H,constant", [(1, 1, 1, False), (1, 127, 2, False), (2, 130, 8, True), (1, 259, 3, False), (1, 1283, 8, False),
-                                            (40, 96, 8, False)])
+                                            (1, 2050, 2, False), (40, 96, 8, False)])
 def test_quant_encode(dtype, bits, clip, B, T, H, constant):
     from calibquant_b200 import calibquant as cq
     g = torch.Generator().manual_seed(T + bits)
