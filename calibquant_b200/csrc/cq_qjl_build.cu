@@ -12,7 +12,7 @@
 // (norm, lower index first), write both A tiles in the 128-byte-swizzled K-major layout and read the accumulators back;
 // the 17th warp issues the products.  The two 128-projection halves of the accumulators are handed over separately, so that one
 // half is read while the other is being computed, and the statistics of the next tile lie under the products of this one.
-// 4 x 8 x 6688 bfloat16 keys, 32 outlier channels: 406 us for the six launches before, 104 us for this one.
+// 4 x 8 x 6688 bfloat16 keys, 32 outlier channels: 406 us for the six launches before, 80 us for this one.
 // Every wait is bounded; on a timeout the CTA writes the status word, frees its tensor memory and returns.
 #include <type_traits>
 
@@ -34,6 +34,7 @@ constexpr int A_PANEL = A_BYTES / 2, B_PANEL = B_BYTES / 2;
 constexpr int PART_BYTES = NW * kHeadDim * 4;             // per group: channel sums of the worker warps
 constexpr int SMEM = 2 * B_BYTES + 2 * A_BYTES + 4 * PART_BYTES + 4 * kHeadDim * 2 + 1024;
 constexpr uint32_t WAIT_TRIES = 1u << 22;
+constexpr int64_t NOWHERE = INT64_MIN;                      // a group past the end
 
 struct Args {
   int64_t n_groups_total;      // batch * heads * n_groups
@@ -74,6 +75,7 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
   __shared__ __align__(8) uint64_t bar_a, bar_d[2], bar_free[2];
   __shared__ uint32_t tmem_s;
   __shared__ uint32_t mask_s[4][4];
+  __shared__ int64_t base_s[2][4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t n_tiles = (a.n_groups_total + 3) / 4;
 
@@ -83,20 +85,32 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
     mbar_fence_init();
   }
   if (warp == NW) tmem_alloc(&tmem_s, 512);
-      // loader role: 16-byte piece ch of row r0 of each of the four groups
-      const int ch = tid & 15, r0 = tid >> 4;
-      uint4 v[4];
-      auto load = [&](int64_t tile) {
+      // where the four groups of a tile start (64-bit divisions: one thread per group, a tile ahead)
+  auto place = [&](int64_t tile, int slot) {
+    if (tid >= 4) return;
+    const int64_t grp = tile * 4 + tid;
+    int64_t at = NOWHERE;
+    if (grp < a.n_groups_total) {
+      const int64_t bh = grp / a.n_groups, n = grp - bh * a.n_groups, b = bh / a.heads;
+      at = b * a.stride_b + (bh - b * a.heads) * a.stride_h + n * G * a.stride_t;
+    }
+    base_s[slot][tid] = at;
+  };
+  // loader role: 16-byte piece ch of row r0 of each of the four groups
+  const int ch = tid & 15, r0 = tid >> 4;
+  uint4 v[4];
+  auto load = [&](int slot) {
 #pragma unroll
-        for (int gg = 0; gg < 4; ++gg) {
-          const int64_t grp = tile * 4 + gg;
-          const bool live = grp < a.n_groups_total;
-          const int64_t bh = live ? grp / a.n_groups : 0, n = live ? grp % a.n_groups : 0;
-          const T* src = keys + (bh / a.heads) * a.stride_b + (bh % a.heads) * a.stride_h + (n * G + r0) * a.stride_t + ch * 8;
-          v[gg] = live ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);
-        }
-      };
-  if (warp < NW) load(blockIdx.x);      // in flight while the table is built
+    for (int gg = 0; gg < 4; ++gg) {
+      const int64_t at = base_s[slot][gg];
+      v[gg] = make_uint4(0u, 0u, 0u, 0u);
+      if (at != NOWHERE) v[gg] = *reinterpret_cast<const uint4*>(keys + at + r0 * a.stride_t + ch * 8);
+    }
+  };
+  place(blockIdx.x, 0);
+  place((int64_t)blockIdx.x + gridDim.x, 1);
+  __syncthreads();
+  if (warp < NW) load(0);      // in flight while the table is built
   // S, rows of projections, as hi and lo in the swizzled K-major layout
   const bool wide = reinterpret_cast<uintptr_t>(proj) % 16 == 0;
 #pragma unroll 2
@@ -133,31 +147,34 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
   bool ok = true;
 
   if (warp == NW) {
-    // ================= products (one lane) =================
-    if (lane == 0) {
-      const uint64_t ad[2] = {smem_desc(smem_u32(a_s), 16, 1024), smem_desc(smem_u32(a_s + A_BYTES), 16, 1024)};
-      const uint64_t bd[2] = {smem_desc(smem_u32(b_s), 16, 1024), smem_desc(smem_u32(b_s + B_BYTES), 16, 1024)};
-      uint32_t i = 0;
-      for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++i) {
-        ok = mbar_wait_bounded(&bar_a, i & 1, WAIT_TRIES);
+    // ================= products =================
+    // the whole warp runs the loop and one elected lane issues, so that the operands are uniform
+    const uint32_t lead = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    auto all = [](bool r) { return __all_sync(0xffffffffu, r) != 0; };
+    const uint64_t ad = smem_desc(smem_u32(a_s), 16, 1024), bd = smem_desc(smem_u32(b_s), 16, 1024);
+    uint32_t i = 0;
+    for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++i) {
+      ok = all(mbar_wait_bounded(&bar_a, i & 1, WAIT_TRIES));
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (i > 0) ok = ok && mbar_wait_bounded(&bar_free[half], (i - 1) & 1, WAIT_TRIES);
-          if (!ok) break;
-          tc_fence_after();
+      for (int half = 0; half < 2; ++half) {
+        if (i > 0) ok = ok && all(mbar_wait_bounded(&bar_free[half], (i - 1) & 1, WAIT_TRIES));
+        if (!ok) break;
+        tc_fence_after();
+        if (lead) {
 #pragma unroll
           for (int src = 0; src < 2; ++src)
 #pragma unroll
             for (int hl = 0; hl < 2; ++hl)
 #pragma unroll
               for (int ks = 0; ks < 8; ++ks)      // 16 channels per step; 128 projections further down a panel for half 1
-                umma(tmem + (uint32_t)(src * 256 + half * 128), ad[src] + (uint64_t)(((ks >> 2) * A_PANEL + (ks & 3) * 32) >> 4),
-                     bd[hl] + (uint64_t)(((ks >> 2) * B_PANEL + half * 128 * 128 + (ks & 3) * 32) >> 4), a.idesc, (hl > 0 || ks > 0) ? 1u : 0u);
+                umma(tm + (uint32_t)(src * 256 + half * 128), ad + (uint64_t)((src * A_BYTES + (ks >> 2) * A_PANEL + (ks & 3) * 32) >> 4),
+                     bd + (uint64_t)((hl * B_BYTES + (ks >> 2) * B_PANEL + half * 128 * 128 + (ks & 3) * 32) >> 4), a.idesc, (hl > 0 || ks > 0) ? 1u : 0u);
           umma_commit(&bar_d[half]);
         }
       }
-      if (!ok) atomicExch(status, CQ_ERR_TIMEOUT);
     }
+    if (!ok && lead) atomicExch(status, CQ_ERR_TIMEOUT);
     __syncwarp();
   } else {
     // ================= workers =================
@@ -287,9 +304,10 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
       if (ok) ok = mbar_wait_bounded(&bar_d[half], phase, WAIT_TRIES);
       tc_fence_after();
       const uint32_t base = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(half * 128 + 32 * (warp >> 2));
-      // signs: in = all - out > 0, out > 0 (a zero of either sign gives 0).  Partial words, so that the bits do not form one
-      // chain; sixteen columns at a time, which is what the registers beside the next tile's keys hold
-      uint32_t in_w[4] = {0u, 0u, 0u, 0u}, out_w[4] = {0u, 0u, 0u, 0u};
+      // signs: in = all - out > 0, out > 0, each the sign bit of the opposite difference (which is +0 for equal numbers, and so 0
+      // for a zero of either sign), shifted into the word: one addition and one funnel shift a bit.  Eight columns to a chain;
+      // sixteen columns at a time, which is what the registers beside the next tile's keys hold
+      uint32_t in_w = 0u, out_w = 0u;
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         uint32_t all[16], o[16];
@@ -298,10 +316,16 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
         tmem_ld_wait();
         if (part == 1) { tc_fence_before(); mbar_arrive(&bar_free[half]); }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float x = __uint_as_float(o[i]);
-          in_w[i & 3] |= (__uint_as_float(all[i]) > x ? 1u : 0u) << (16 * part + i);      // all - out > 0: fp32 subtraction is sign-exact
-          out_w[i & 3] |= (x > 0.f ? 1u : 0u) << (16 * part + i);
+        for (int c8 = 0; c8 < 2; ++c8) {
+          uint32_t iw = 0u, ow = 0u;
+#pragma unroll
+          for (int i = 7; i >= 0; --i) {
+            const float x = __uint_as_float(o[8 * c8 + i]);
+            iw = __funnelshift_l(__float_as_uint(x - __uint_as_float(all[8 * c8 + i])), iw, 1);
+            ow = __funnelshift_l(__float_as_uint(0.f - x), ow, 1);
+          }
+          in_w |= iw << (16 * part + 8 * c8);
+          out_w |= ow << (16 * part + 8 * c8);
         }
       }
       const int row = 32 * (warp & 3) + lane;
@@ -309,9 +333,9 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
       if (ok && grp < a.n_groups_total) {
         const int64_t tok = tile * TILE + row;
         const int word = 4 * half + (warp >> 2);
-        *reinterpret_cast<uint32_t*>(key_quant + tok * (SKETCH / 8) + 4 * word) = (in_w[0] | in_w[1]) | (in_w[2] | in_w[3]);
+        *reinterpret_cast<uint32_t*>(key_quant + tok * (SKETCH / 8) + 4 * word) = in_w;
         if (32 * word < a.o_sketch)
-          *reinterpret_cast<uint32_t*>(key_outlier_quant + tok * (a.o_sketch / 8) + 4 * word) = (out_w[0] | out_w[1]) | (out_w[2] | out_w[3]);
+          *reinterpret_cast<uint32_t*>(key_outlier_quant + tok * (a.o_sketch / 8) + 4 * word) = out_w;
       }
     };
 
@@ -322,7 +346,8 @@ build_kernel(const Args a, const T* __restrict__ keys, const uint8_t* __restrict
       if (prev >= 0 && ok) ok = mbar_wait_bounded(&bar_d[1], (i - 1) & 1, WAIT_TRIES);      // the A tiles have been read
       stage();
       const int64_t next = tile + gridDim.x;
-      if (next < n_tiles) load(next);
+      if (next < n_tiles) load((i + 1) & 1);
+      place(next + gridDim.x, i & 1);      // read after the barriers of the statistics; this slot was last read before them
       if (prev >= 0) read_half(prev, 1, (i - 1) & 1);
       if (next < n_tiles) { statistics(next); take_masks(next); }
       read_half(tile, 0, i & 1);

@@ -359,7 +359,7 @@ extern "C" int cq_prefill_rope_split(const void* qkv, int64_t qkv_stride_b, int6
       !step::aligned16(k_out) || !step::aligned16(k_cache) || !step::aligned16(v_cache))
     return CQ_ERR_BAD_ARG;
   // A warp takes all heads of a token unless that gives the chip (16 warps per SM at a time) less than four rounds: then fewer heads,
-  // so that the last round is a small part (2 x 1401 tokens in rounds of 1.2: 17.8 us; of 4.7: SPLIT_US)
+  // so that the last round is a small part (2 x 1401 tokens in rounds of 1.2: 17.8 us; of 4.7: 17.2)
   const int64_t n_tokens = (int64_t)batch * t_len;
   int parts = 1;
   while (parts < n_kv_heads && parts < 32768 && n_tokens * parts < 4 * 148 * 16) parts *= 2;

