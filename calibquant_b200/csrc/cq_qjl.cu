@@ -212,23 +212,23 @@ score_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ 
 //
 // What bounded the earlier form: the query's outlier projection q_out S, which every group needs for its own 32 outlier
 // channels, as 32 x 256 x n_rep FMAs with an indexed load each (2650 cycles per group and SM, issue-bound), and two CTA
-// barriers per group.  Here it is a product with gathered rows: B = rows of S picked by ldmatrix (the row addresses ARE the
-// gather), A = the query's outlier channels; its accumulators (row = head, columns = projections 2c, 2c+1) are the layout
-// the sign product wants its B operand in, so nothing passes through shared memory.  Lanes g < 4 keep the fp16 value, lanes
-// g >= 4 the remainder of the same head (rows 4-7 of A repeat rows 0-3); with five to eight heads both are kept and the sign
-// product runs twice.
+// barriers per group.  Here it is a product with gathered rows: A = rows of S (transposed by ldmatrix; the row addresses ARE the
+// gather), B = the query's outlier channels, D = 16 projections x 8 columns, the heads.  q_out S and q S - q_out S are the
+// operands of the outlier and of the inlier sketch; a movmatrix turns each into the layout that the sign product wants its B
+// operand in, so nothing passes through shared memory.  Columns 0-3 keep the fp16 value, columns 4-7 the remainder of the same
+// head; with five to eight heads both are kept and the sign product runs twice.
 //   * k-step b takes bits b and b + 16 of every sign word of a token: lane c needs only its words c and c + 4, and an operand
 //     register costs one shift and one LOP3.  The table's columns are in that order.
-//   * sum sgn (q S - q_out S) is summed as sum sgn (q S) - sum sgn (q_out S): the first operand is made once per KV head, the
-//     second serves both sketches.
+//   * 8 products a k-step (n_rep <= 4).  With the gathered rows as B operand (no transposition, half of the 16 rows idle) and q S
+//     and q_out S against the inlier signs separately it was 14, and 153 us for 8 x 8 x 16384 keys; now 129.
 //   * The rows of an 8 x 8 matrix hit the bank group (channel mod 8): the 32 channels are dealt over the four matrices of a
 //     load by rank within their residue class (the order of the contraction is free).
 constexpr int SW = 16, STHREADS = SW * 32;
 constexpr int S_PITCH = MAX_SKETCH + 8;               // halves per projection row: channel d starts in bank group d % 8
 constexpr int S_TAB_BYTES = 2 * kHeadDim * S_PITCH * 2;
 constexpr int S_SIGN_BYTES = 2 * 32 * (MAX_SKETCH / 8);          // signs of 32 tokens, both sketches
-constexpr int S_QF_BYTES = (MAX_SKETCH / 16) * 32 * 8;           // fragments of q S: [k-step][lane] x (b0, b1)
-constexpr int S_SMEM = S_TAB_BYTES + SW * 2 * S_SIGN_BYTES + 2 * S_QF_BYTES + kMaxRep * kHeadDim * 2 + SW * 64;
+constexpr int S_QF_BYTES = (MAX_SKETCH / 16) * 32 * 16;          // q S as accumulators: [k-step][lane] x 4
+constexpr int S_SMEM = S_TAB_BYTES + SW * 2 * S_SIGN_BYTES + S_QF_BYTES + kMaxRep * kHeadDim * 2 + SW * 64;
 
 // projection at position 16 b + 8 half + 2 c + e of a table row: bit b + 16 e of word c + 4 half (256 projections), or
 // bit b + 8 half + 16 e of word c (128 projections)
@@ -237,7 +237,8 @@ __device__ __forceinline__ int sign_proj(int pos, int sketch) {
   return sketch == 256 ? 32 * (c + 4 * half) + b + 16 * e : 32 * c + b + 8 * half + 16 * e;
 }
 
-template <typename T, typename TP, int R>
+// ONE: at most 32 outlier channels and groups of at most 32 tokens: one block of channels, one item per group
+template <typename T, typename TP, int R, bool ONE>
 __global__ void __launch_bounds__(STHREADS, 1)
 score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ key_outlier_quant,
                   const T* __restrict__ key_norm, const T* __restrict__ key_outlier_norm,
@@ -247,8 +248,8 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
   extern __shared__ __align__(16) unsigned char smem[];
   __half* tab = reinterpret_cast<__half*>(smem);                                              // [hi|lo][channel][S_PITCH]
   unsigned char* sign_s = smem + S_TAB_BYTES;                                                 // [warp][buffer][in|out][token][bytes]
-  uint2* qf_s = reinterpret_cast<uint2*>(sign_s + SW * 2 * S_SIGN_BYTES);                     // [value (R 8) | remainder][k-step][lane]
-  __half* q_s = reinterpret_cast<__half*>(qf_s + 2 * (MAX_SKETCH / 16) * 32);                 // [head][channel]
+  float4* qf_s = reinterpret_cast<float4*>(sign_s + SW * 2 * S_SIGN_BYTES);                   // [k-step][lane]
+  __half* q_s = reinterpret_cast<__half*>(qf_s + (MAX_SKETCH / 16) * 32);                 // [head][channel]
   uint8_t* order_s = reinterpret_cast<uint8_t*>(q_s + kMaxRep * kHeadDim);                    // [warp][64]: channel per slot, free slots
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
   // the projection, rows of channels, positions in sign order: lane = eight adjacent positions, so that neighbouring lanes
@@ -272,14 +273,14 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
     *reinterpret_cast<uint4*>(tab + d * S_PITCH + pos) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(tab + (kHeadDim + d) * S_PITCH + pos) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
-  const int n_chunks = (G + 31) / 32, per_kbh = n_groups * n_chunks;
+  const int n_chunks = ONE ? 1 : (G + 31) / 32, per_kbh = n_groups * n_chunks;
   const int64_t n_items = (int64_t)n_kbh * per_kbh;
   const int64_t it_first = blockIdx.x * n_items / gridDim.x, it_end = (blockIdx.x + 1) * n_items / gridDim.x;
   const int rb = sketch / 8, orb = o_sketch / 8;
   unsigned char* my_sign = sign_s + warp * 2 * S_SIGN_BYTES;
   uint8_t* order = order_s + warp * 64;
   const uint32_t tab_b = ptx::smem_u32(tab);
-  const float keep = R == 8 || g >= 4 ? 1.f : 0.f;      // R == 4: the lanes of the remainders
+  const float keep = R == 8 || c >= 2 ? 1.f : 0.f;      // R == 4: the lanes (columns 4-7) of the remainders
 
   for (int64_t seg = it_first; seg < it_end;) {       // runs of items of one (batch, KV head)
     const int64_t kbh = seg / per_kbh;
@@ -291,54 +292,41 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
       q_s[i] = __float2half_rn(r < n_rep ? Elem<T>::to_f(query[(qrow0 + r) * kHeadDim + d]) : 0.f);
     }
     __syncthreads();
-    // q S of every head as B fragments: value in the lanes g < 4, remainder of the same head in g >= 4 (R == 8: both).  Not
-    // given: a product with the table, one k-step of positions per warp
-    auto fragment = [&](int i, float (&x)[2][2]) {
-      const bool low = R == 4 && (i & 31) >= 16;
-      uint32_t v[2], rem[2];
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const __half2 h = __floats2half2_rn(x[half][0], x[half][1]);
-        const float2 f = __half22float2(h);
-        const __half2 lo = __floats2half2_rn(x[half][0] - f.x, x[half][1] - f.y);
-        v[half] = *reinterpret_cast<const uint32_t*>(&h);
-        rem[half] = *reinterpret_cast<const uint32_t*>(&lo);
-      }
-      qf_s[i] = make_uint2(low ? rem[0] : v[0], low ? rem[1] : v[1]);
-      if (R == 8) qf_s[(MAX_SKETCH / 16) * 32 + i] = make_uint2(rem[0], rem[1]);
-    };
+    // q S as accumulators: rows = positions g, g + 8 of a k-step, columns 2c, 2c+1 = heads (R == 4: heads 0-3 twice).  Not given:
+    // a product with the table, one k-step of positions per warp
     if (query_sketch) {
       for (int i = tid; i < sketch * 2; i += STHREADS) {
-        const int b = i >> 5, l = i & 31, head = R == 4 ? (l >> 2) & 3 : l >> 2;
-        float x[2][2];
+        const int b = i >> 5, l = i & 31;
+        float x[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          x[k >> 1][k & 1] = head < n_rep ? query_sketch[(qrow0 + head) * sketch + sign_proj(16 * b + 8 * (k >> 1) + 2 * (l & 3) + (k & 1), sketch)] : 0.f;
-        fragment(i, x);
+        for (int k = 0; k < 4; ++k) {
+          const int head = (2 * (l & 3) + (k & 1)) & (R == 4 ? 3 : 7), pos = 16 * b + (l >> 2) + 8 * (k >> 1);
+          x[k] = head < n_rep ? query_sketch[(qrow0 + head) * sketch + sign_proj(pos, sketch)] : 0.f;
+        }
+        qf_s[i] = make_float4(x[0], x[1], x[2], x[3]);
       }
     } else if (warp < sketch / 16) {
-      float u[2][4] = {};
+      float u[4] = {};
       const __half* qh = q_s + (R == 4 ? (g & 3) : g) * kHeadDim + 2 * c;
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        const uint32_t a0 = *reinterpret_cast<const uint32_t*>(qh + 16 * ks), a2 = *reinterpret_cast<const uint32_t*>(qh + 16 * ks + 8);
+        const uint32_t q0 = *reinterpret_cast<const uint32_t*>(qh + 16 * ks), q1 = *reinterpret_cast<const uint32_t*>(qh + 16 * ks + 8);
 #pragma unroll
         for (int hl = 0; hl < 2; ++hl) {
           uint32_t b0, b1, b2, b3;
           ptx::ldmatrix_x4_trans(tab_b + (uint32_t)(((hl * kHeadDim + 16 * ks + (lane & 15)) * S_PITCH + 16 * warp) * 2 + (lane >> 4) * 16), b0, b1, b2, b3);
-          ptx::mma_f16(u[0], a0, 0u, a2, 0u, b0, b1);
-          ptx::mma_f16(u[1], a0, 0u, a2, 0u, b2, b3);
+          ptx::mma_f16(u, b0, b2, b1, b3, q0, q1);
         }
       }
-      float x[2][2] = {{u[0][0], u[0][1]}, {u[1][0], u[1][1]}};
-      fragment(warp * 32 + lane, x);
+      qf_s[warp * 32 + lane] = make_float4(u[0], u[1], u[2], u[3]);
     }
     __syncthreads();
     // an item's sign words (contiguous: 32 tokens x sketch / 8 bytes each) through a double buffer of this warp
     auto fetch = [&](int64_t item, int buf) {
       if (item < seg_end) {
-        const int64_t loc = item - kbh * per_kbh, grp = kbh * n_groups + loc / n_chunks;
-        const int tok0 = (int)(loc % n_chunks) * 32, n_tok = min(32, G - tok0);
+        const int loc = (int)(item - kbh * per_kbh), nn = ONE ? loc : loc / n_chunks, tok0 = ONE ? 0 : (loc - nn * n_chunks) * 32;
+        const int n_tok = min(32, G - tok0);
+        const int64_t grp = kbh * n_groups + nn;
         const uint8_t* a = key_quant + (grp * G + tok0) * rb;
         const uint8_t* o = key_outlier_quant + (grp * G + tok0) * orb;
         const uint32_t dst = ptx::smem_u32(my_sign + buf * S_SIGN_BYTES);
@@ -355,8 +343,9 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
     int64_t item = seg + warp;
     fetch(item, 0);
     for (int buf = 0; item < seg_end; item += SW, buf ^= 1) {
-      const int64_t loc = item - kbh * per_kbh, n = loc / n_chunks, grp = kbh * n_groups + n;
-      const int tok0 = (int)(loc % n_chunks) * 32, n_tok = min(32, G - tok0);
+      const int loc = (int)(item - kbh * per_kbh), n = ONE ? loc : loc / n_chunks, tok0 = ONE ? 0 : (loc - n * n_chunks) * 32;
+      const int n_tok = min(32, G - tok0);
+      const int64_t grp = kbh * n_groups + n;
       fetch(item + SW, buf ^ 1);
       float nk[4], no[4];                             // norms of the lane's tokens g + 8 i
 #pragma unroll
@@ -365,11 +354,11 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
         nk[i] = Elem<T>::to_f(key_norm[t]);
         no[i] = Elem<T>::to_f(key_outlier_norm[t]);
       }
-      float acc[3][2][4];                             // [in: q S | in: q_out S | out: q_out S][m-tile][fragment]
+      float acc[2][2][4];                             // [in | out][m-tile][fragment]
 #pragma unroll
-      for (int i = 0; i < 24; ++i) (&acc[0][0][0])[i] = 0.f;
+      for (int i = 0; i < 16; ++i) (&acc[0][0][0])[i] = 0.f;
       // u accumulates over blocks of 32 outlier channels; there is one block unless oc > 32
-      const int blocks = (oc + 31) / 32;
+      const int blocks = ONE ? 1 : (oc + 31) / 32;
       uint32_t qa[2][2], row[2];                      // A fragments and ldmatrix row of the block at hand
       auto load_block = [&](int blk) {
         const int i = blk * 32 + lane;
@@ -398,7 +387,7 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
         }
         __syncwarp();
       };
-      if (blocks == 1) load_block(0);
+      if (ONE || blocks == 1) load_block(0);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
       __syncwarp();
       // sign words of the lane: rows g + 8 i, inverted, words c and c + 4 (128 projections: word c twice, eight bits apart).
@@ -422,39 +411,40 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
         }
       }
       __syncwarp();      // the sign buffer may be refilled
+      const uint32_t two = 1u + (sketch > 0);         // not a constant: the shift becomes a multiplication, off the busy ALU pipe
       const bool short_out = o_sketch < sketch;      // 128 of 256: only the first half of every k-step is in the outlier sketch
 #pragma unroll 2
       for (int b = sketch / 16 - 1; b >= 0; --b) {
-        float u[2][4];                                // rows = heads, columns = the k-step's two halves
+        float u[2][4];                                // q_out S by the hi and the lo rows: rows = positions, columns = heads
         for (int blk = 0; blk < blocks; ++blk) {
-          if (blocks > 1) load_block(blk);
+          if (!ONE && blocks > 1) load_block(blk);
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
             for (int hl = 0; hl < 2; ++hl) {
               uint32_t b0, b1, b2, b3;
               ptx::ldmatrix_x4_trans(row[ks] + (uint32_t)(hl * kHeadDim * S_PITCH * 2 + 32 * b), b0, b1, b2, b3);
-              if (ks == 0 && hl == 0 && blk == 0) {
-                ptx::mma_f16_zero(u[0], qa[0][0], 0u, qa[0][1], 0u, b0, b1);
-                ptx::mma_f16_zero(u[1], qa[0][0], 0u, qa[0][1], 0u, b2, b3);
-              } else {
-                ptx::mma_f16(u[0], qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
-                ptx::mma_f16(u[1], qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
-              }
+              if (ks == 0 && blk == 0) ptx::mma_f16_zero(u[hl], b0, b2, b1, b3, qa[0][0], qa[0][1]);
+              else ptx::mma_f16(u[hl], b0, b2, b1, b3, qa[ks][0], qa[ks][1]);
             }
         }
-        // q_out S as the B operand: fp16 value, or what it leaves over (R == 8: both)
-        uint32_t bv[2], bl[2];
+        // the two operands: fp16 value, or what it leaves over (R == 8: both), as [position][head] -> B fragments
+        const float4 qs = qf_s[b * 32 + lane];
+        const float qv[4] = {qs.x, qs.y, qs.z, qs.w};
+        uint32_t bv[2][2], bl[2][2];                  // [in | out][positions 0-7 | 8-15]
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const __half2 h = __floats2half2_rn(u[half][0], u[half][1]);
-          const float2 f = __half22float2(h);
-          const __half2 l = __floats2half2_rn(fmaf(-keep, f.x, u[half][0]), fmaf(-keep, f.y, u[half][1]));
-          bl[half] = *reinterpret_cast<const uint32_t*>(&l);
-          bv[half] = R == 4 ? bl[half] : *reinterpret_cast<const uint32_t*>(&h);
+          const float o0 = u[0][2 * half] + u[1][2 * half], o1 = u[0][2 * half + 1] + u[1][2 * half + 1];
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const float x0 = s ? o0 : qv[2 * half] - o0, x1 = s ? o1 : qv[2 * half + 1] - o1;
+            const __half2 h = __floats2half2_rn(x0, x1);
+            const float2 f = __half22float2(h);
+            const __half2 l = __floats2half2_rn(fmaf(-keep, f.x, x0), fmaf(-keep, f.y, x1));
+            bl[s][half] = ptx::movmatrix_trans(*reinterpret_cast<const uint32_t*>(&l));
+            bv[s][half] = R == 4 ? bl[s][half] : ptx::movmatrix_trans(*reinterpret_cast<const uint32_t*>(&h));
+          }
         }
-        const uint2 qf = qf_s[b * 32 + lane];
-        const uint2 qr = R == 8 ? qf_s[(MAX_SKETCH / 16) * 32 + b * 32 + lane] : make_uint2(0u, 0u);
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           uint32_t a[4][2];                           // +-2^-24, negative where the bit is 0
@@ -463,17 +453,13 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               a[i][e] = (x[s][i][e] & 0x80008000u) | 0x00010001u;
-              x[s][i][e] += x[s][i][e];
+              asm("mad.lo.u32 %0, %0, %1, 0;" : "+r"(x[s][i][e]) : "r"(two));
             }
-          const uint32_t b1v = s == 1 && short_out ? 0u : bv[1], b1l = s == 1 && short_out ? 0u : bl[1];
+          const uint32_t b1v = s == 1 && short_out ? 0u : bv[s][1], b1l = s == 1 && short_out ? 0u : bl[s][1];
 #pragma unroll
           for (int mt = 0; mt < 2; ++mt) {
-            if (s == 0) ptx::mma_f16(acc[0][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], qf.x, qf.y);
-            ptx::mma_f16(acc[1 + s][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], bv[0], b1v);
-            if (R == 8) {
-              if (s == 0) ptx::mma_f16(acc[0][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], qr.x, qr.y);
-              ptx::mma_f16(acc[1 + s][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], bl[0], b1l);
-            }
+            ptx::mma_f16(acc[s][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], bv[s][0], b1v);
+            if (R == 8) ptx::mma_f16(acc[s][mt], a[2 * mt][0], a[2 * mt + 1][0], a[2 * mt][1], a[2 * mt + 1][1], bl[s][0], b1l);
           }
         }
       }
@@ -483,13 +469,13 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
 #pragma unroll
       for (int i = 0; i < 4; ++i)      // the two norms are rounded separately, so the difference can dip below zero
         norm_in[i] = scl * sqrtf(fmaxf(nk[i] * nk[i] - no[i] * no[i], 0.f));
-      float* dst = scores + (qrow0 + 2 * c) * ((int64_t)n_groups * G) + n * G + tok0 + g;
+      float* dst = scores + (qrow0 + 2 * c) * ((int64_t)n_groups * G) + (int64_t)n * G + tok0 + g;
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int i = 2 * mt + (e >> 1);
-          float v = norm_in[i] * (acc[0][mt][e] - acc[1][mt][e]) + scl_o * no[i] * acc[2][mt][e];
+          float v = norm_in[i] * acc[0][mt][e] + scl_o * no[i] * acc[1][mt][e];
           if (R == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
           if (2 * c + (e & 1) < n_rep && g + 8 * i < n_tok && (R == 8 || c < 2)) dst[(e & 1) * ((int64_t)n_groups * G) + 8 * i] = v;
         }
@@ -572,7 +558,7 @@ extern "C" int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_out
 #define CQ_QJL_SCORE(T, TP, R)                                                                                 \
   do {                                                                                                         \
     if (use_mma) {                                                                                             \
-      auto kern = qjl::score_rows_kernel<T, TP, R>;                                                            \
+      auto kern = group_size <= 32 && outlier_count <= 32 ? qjl::score_rows_kernel<T, TP, R, true> : qjl::score_rows_kernel<T, TP, R, false>;                                                            \
       if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, qjl::S_SMEM) != cudaSuccess) \
         return CQ_ERR_LAUNCH;                                                                                  \
       kern<<<grid_mma, qjl::STHREADS, qjl::S_SMEM, st>>>(CQ_QJL_ARGS(T, TP), batch * n_kv_heads, n_groups, group_size, n_rep, \
