@@ -70,7 +70,7 @@ class RotaryEmbedding(nn.Module):
             emb = torch.cat([torch.outer(t, inv)] * 2, dim=-1)
             cached = (emb.cos().to(x.dtype), emb.sin().to(x.dtype))
             self._cache[key] = cached
-        return cached[0][:seq_len], cached[1][:seq_len]
+        return cached[0].narrow(0, 0, seq_len), cached[1].narrow(0, 0, seq_len)
 
 
 class InternLM2Attention(nn.Module):

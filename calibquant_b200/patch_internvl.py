@@ -148,7 +148,7 @@ class _TextCache:
         self.length += n
 
     def views(self):
-        return self.k[:, :, :self.length], self.v[:, :, :self.length]
+        return self.k.narrow(2, 0, self.length), self.v.narrow(2, 0, self.length)
 
     # ---- static mode: the token count lives on the device, so that one captured CUDA graph can
     # ---- append a token and attend over the live part at every decode step
@@ -233,10 +233,12 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
     ``(K_fp, V_fp)`` tuple of system+text tokens and the quantized state lives on the module, as in
     the reference.
     """
-    self.sprompt_len = SPROMPT_LEN
-    self.image_token_num = _image_token_num()
-    self.normalize = BITS_KV <= 2
-    attention_mask = _pop_padding_mask(kwargs, attention_mask)
+    state = self.__dict__      # plain values: nn.Module.__setattr__ would look each of them up among parameters and modules
+    state["sprompt_len"] = SPROMPT_LEN
+    state["image_token_num"] = _image_token_num()
+    state["normalize"] = BITS_KV <= 2
+    if kwargs:
+        attention_mask = _pop_padding_mask(kwargs, attention_mask)
     bsz, q_len, _ = hidden_states.size()
 
     if q_len == 1 and getattr(self, "_static_decode", False):
@@ -305,12 +307,11 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
     if self.head_dim == 128 and cos.dtype == sin.dtype == hidden_states.dtype == tc.k.dtype:
         # one launch splits the projection, rotates q and k and appends k, v to the text cache (the torch ops
         # below are ~15 launches, which took longer to issue than the whole step takes on the GPU)
-        n_rep = self.num_key_value_groups
+        n_rep, wqkv = self.num_key_value_groups, self.wqkv
         tc.reserve(1)
         pos = position_ids if position_ids.numel() == bsz else position_ids.expand(bsz, 1)
-        q = ops.rope_split_append(self.wqkv(hidden_states), cos, sin, pos,
-                                  self.wqkv.out_features // ((n_rep + 2) * self.head_dim), n_rep, tc.k, tc.v,
-                                  append_index=tc.length)
+        q = ops.rope_split_append(wqkv(hidden_states), cos, sin, pos, wqkv.out_features // ((n_rep + 2) * self.head_dim), n_rep,
+                                  tc.k, tc.v, append_index=tc.length)
         tc.length += 1
     else:      # rotary tables of another type than the hidden states
         q, k, v = _split_qkv(self, hidden_states)
@@ -332,7 +333,7 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
                                     group_size=GROUP_SIZE, calibrate=self.normalize and LOW_BITS,
                                     mask=attention_mask, t_fp=tc.length)         # [B,Hq,1,D]
     local_heads = self.num_heads // _shard_world(self)
-    if attn.size() != (bsz, local_heads, q_len, self.head_dim):
+    if attn.shape != (bsz, local_heads, q_len, self.head_dim):
         raise ValueError(f"`attn_output` should be of size {(bsz, local_heads, q_len, self.head_dim)}, "
                          f"but is {attn.size()}")
     attn = _gather_heads(self, attn.view(bsz, q_len, -1))
