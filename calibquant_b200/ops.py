@@ -290,6 +290,17 @@ def rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v
     return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev)
 
 
+def qkv_rope_append(x, weight, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index):
+    """:func:`rope_split_append` of the projection ``x @ weight.T`` of up to four requests, x [B,1,K], in one launch that reads
+    the weight once (fp32 sums, rounded to the data type before the rotation)."""
+    return native().qkv_rope_append(x, weight, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index)
+
+
+def linear_small(x, weight):
+    """``x @ weight.T`` for up to four rows (x [.., K], weight [N, K], K a multiple of 8), fp32 sums."""
+    return native().linear_small(x, weight)
+
+
 def add_rmsnorm(residual, delta, weight, eps, out=None, normalize=True):
     """``residual += delta`` in place (skipped when ``delta`` is None), then RMSNorm of the rows of
     ``residual`` [..., hidden] scaled by ``weight``.  Returns the normalised tensor (None when

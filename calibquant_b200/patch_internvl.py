@@ -174,6 +174,24 @@ def _split_qkv(self, hidden_states):
     return q, qkv[..., -2, :], qkv[..., -1, :]
 
 
+def _small_weight(module, x, rows):
+    """The weight of a plain linear projection of few rows, for the launches that read it once; None where the module has to be
+    called (more rows, another module type, a bias, hooks, autograd or autocast at work, other dtypes or layouts)."""
+    if rows > 4 or type(module) is not torch.nn.Linear or torch.is_grad_enabled() or torch.is_autocast_enabled():
+        return None
+    d = module.__dict__
+    w = d["_parameters"].get("weight")      # absent where a parametrization computes it
+    if w is None or d["_parameters"]["bias"] is not None or d["_forward_hooks"] or d["_forward_pre_hooks"] or \
+            _GLOBAL_HOOKS[0] or _GLOBAL_HOOKS[1] or w.dtype is not x.dtype or w.dtype not in _HALF or not w.is_cuda or \
+            w.device != x.device or not w.is_contiguous() or w.shape[1] % 8 or w.data_ptr() % 16 or x.data_ptr() % 16 or not x.is_contiguous():
+        return None
+    return w
+
+
+_HALF = (torch.float16, torch.bfloat16)
+_GLOBAL_HOOKS = (torch.nn.modules.module._global_forward_hooks, torch.nn.modules.module._global_forward_pre_hooks)
+
+
 def _shard_world(self):
     shard = getattr(self, "_shard", None)
     return shard[1] if shard else 1
@@ -310,8 +328,12 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
         n_rep, wqkv = self.num_key_value_groups, self.wqkv
         tc.reserve(1)
         pos = position_ids if position_ids.numel() == bsz else position_ids.expand(bsz, 1)
-        q = ops.rope_split_append(wqkv(hidden_states), cos, sin, pos, wqkv.out_features // ((n_rep + 2) * self.head_dim), n_rep,
-                                  tc.k, tc.v, append_index=tc.length)
+        n_kv = wqkv.out_features // ((n_rep + 2) * self.head_dim)
+        w = _small_weight(wqkv, hidden_states, bsz)
+        if w is not None:      # a few requests: projection included
+            q = ops.qkv_rope_append(hidden_states, w, cos, sin, pos, n_kv, n_rep, tc.k, tc.v, tc.length)
+        else:
+            q = ops.rope_split_append(wqkv(hidden_states), cos, sin, pos, n_kv, n_rep, tc.k, tc.v, append_index=tc.length)
         tc.length += 1
     else:      # rotary tables of another type than the hidden states
         q, k, v = _split_qkv(self, hidden_states)
@@ -337,7 +359,9 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
         raise ValueError(f"`attn_output` should be of size {(bsz, local_heads, q_len, self.head_dim)}, "
                          f"but is {attn.size()}")
     attn = _gather_heads(self, attn.view(bsz, q_len, -1))
-    return self.wo(attn), None, past_key_value
+    wo = self.wo
+    w = _small_weight(wo, attn, bsz)
+    return wo(attn) if w is None else ops.linear_small(attn, w), None, past_key_value
 
 
 def forward_internlm2_qjl(self, hidden_states: torch.Tensor,
