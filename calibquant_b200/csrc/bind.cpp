@@ -110,6 +110,13 @@ Tensor empty(at::IntArrayRef size, const Tensor& like) { return at::empty(size, 
 Tensor empty(at::IntArrayRef size, const Tensor& like, at::ScalarType dt) { return at::empty(size, like.options().dtype(dt)); }
 
 PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
+PyObject* wrap2(Tensor a, Tensor b) {
+  PyObject* tup = PyTuple_New(2);
+  if (!tup) throw PyRaised();
+  PyTuple_SET_ITEM(tup, 0, wrap(std::move(a)));
+  PyTuple_SET_ITEM(tup, 1, wrap(std::move(b)));
+  return tup;
+}
 PyObject* wrap3(Tensor a, Tensor b, Tensor c) {
   PyObject* tup = PyTuple_New(3);
   if (!tup) throw PyRaised();
@@ -470,6 +477,28 @@ PyObject* py_qkv_rope_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_END
 }
 
+// x, weight -> whether the launches of few rows can take them (layouts, types, devices; the caller has counted the rows)
+PyObject* py_small_ok(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  CQ_BEGIN
+  want_args(n, 2, "small_ok");
+  const Tensor &x = tensor(a[0]), &w = tensor(a[1]);
+  const bool ok = w.is_cuda() && x.is_cuda() && w.device() == x.device() && w.scalar_type() == x.scalar_type() &&
+                  (x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16) && w.dim() == 2 && w.is_contiguous() && x.is_contiguous() &&
+                  x.size(-1) == w.size(1) && w.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0 &&
+                  reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0;
+  return PyBool_FromLong(ok);
+  CQ_END
+}
+
+// a, b, dim, length -> the first `length` of both along dim, as views
+PyObject* py_heads_of(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  CQ_BEGIN
+  want_args(n, 4, "heads_of");
+  const int64_t dim = integer(a[2]), len = integer(a[3]);
+  return wrap2(tensor(a[0]).narrow(dim, 0, len), tensor(a[1]).narrow(dim, 0, len));
+  CQ_END
+}
+
 // x [.., K] of up to four rows, weight [N, K] -> [.., N]
 PyObject* py_linear_small(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_BEGIN
@@ -633,7 +662,7 @@ PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define CQ_FN(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     CQ_FN(workspace), CQ_FN(workspaces_of), CQ_FN(pack_last_dim), CQ_FN(pack_k_per_channel), CQ_FN(pack_v_per_token),
-    CQ_FN(quant_encode), CQ_FN(qbmm), CQ_FN(decode_attention), CQ_FN(u8_decode_attention), CQ_FN(rope_split_append), CQ_FN(qkv_rope_append), CQ_FN(linear_small),
+    CQ_FN(quant_encode), CQ_FN(qbmm), CQ_FN(decode_attention), CQ_FN(u8_decode_attention), CQ_FN(rope_split_append), CQ_FN(qkv_rope_append), CQ_FN(linear_small), CQ_FN(small_ok), CQ_FN(heads_of),
     CQ_FN(prefill_rope_split), CQ_FN(prefill_attention),
     CQ_FN(qjl_quant), CQ_FN(qjl_build), CQ_FN(qjl_gqa_score), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Tensor-level entry points over libcalibquant_b200.so.", -1, methods};

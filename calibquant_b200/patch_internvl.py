@@ -28,6 +28,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import ops
+from ._lib import native
 from .qjl.matmul import cuda_quantized_bmm_dynamic
 from .qjl.new_pack import triton_quantize_and_pack_along_last_dim
 from .qjl.qjl_utils import QJLKeyQuantizer, repeat_kv_quant
@@ -148,7 +149,7 @@ class _TextCache:
         self.length += n
 
     def views(self):
-        return self.k.narrow(2, 0, self.length), self.v.narrow(2, 0, self.length)
+        return native().heads_of(self.k, self.v, 2, self.length)
 
     # ---- static mode: the token count lives on the device, so that one captured CUDA graph can
     # ---- append a token and attend over the live part at every decode step
@@ -182,13 +183,11 @@ def _small_weight(module, x, rows):
     d = module.__dict__
     w = d["_parameters"].get("weight")      # absent where a parametrization computes it
     if w is None or d["_parameters"]["bias"] is not None or d["_forward_hooks"] or d["_forward_pre_hooks"] or \
-            _GLOBAL_HOOKS[0] or _GLOBAL_HOOKS[1] or w.dtype is not x.dtype or w.dtype not in _HALF or not w.is_cuda or \
-            w.device != x.device or not w.is_contiguous() or w.shape[1] % 8 or w.data_ptr() % 16 or x.data_ptr() % 16 or not x.is_contiguous():
+            _GLOBAL_HOOKS[0] or _GLOBAL_HOOKS[1]:
         return None
-    return w
+    return w if native().small_ok(x, w) else None
 
 
-_HALF = (torch.float16, torch.bfloat16)
 _GLOBAL_HOOKS = (torch.nn.modules.module._global_forward_hooks, torch.nn.modules.module._global_forward_pre_hooks)
 
 
