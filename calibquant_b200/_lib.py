@@ -85,8 +85,6 @@ SIGNATURES = {
     "cq_calib_minmax": (_c.c_int, [_vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_i64), _c.c_int,
                                    _c.c_float, _c.c_int, _vp, _vp, _vp]),
     "cq_linear_small": (_c.c_int, [_vp, _vp, _vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _vp]),
-    "cq_qkv_rope_append": (_c.c_int, [_vp, _vp, _c.c_int, _vp, _vp, _c.c_int, _vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _vp, _vp, _vp,
-                                      _i64, _i64, _c.c_int, _c.c_int, _c.c_int, _vp]),
     "cq_calib_quant_encode": (_c.c_int, [_vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_i64), _c.c_int,
                                          _c.c_float, _c.c_int, _vp, _vp, _vp, _vp]),
     "cq_calib_quantize": (_c.c_int, [_vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_i64), _c.c_int,

@@ -414,12 +414,19 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ---- the launches around the attention -------------------------------------------------------------------------------
-// qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev
+// qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev [, weight: qkv is then the input of the
+// projection, x [B,1,K], and the matrix product is made here]
 PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_BEGIN
-  want_args(n, 10, "rope_split_append");
-  const Tensor &qkv_in = tensor(a[0]), &k_cache = tensor(a[6]), &v_cache = tensor(a[7]);
-  for (int i : {0, 1, 2, 3, 6, 7}) need_cuda(tensor(a[i]));
+  if (n != 11) want_args(n, 10, "rope_split_append");
+  Tensor qkv_in = tensor(a[0]);
+  if (n == 11) {
+    need_cuda(qkv_in);
+    need_cuda(tensor(a[10]));
+    qkv_in = at::mm(qkv_in.view({-1, qkv_in.size(-1)}), tensor(a[10]).t());
+  }
+  const Tensor &k_cache = tensor(a[6]), &v_cache = tensor(a[7]);
+  for (int i : {0, 1, 2, 3, 6, 7}) need_cuda(i == 0 ? qkv_in : tensor(a[i]));
   const Tensor cos = contiguous(tensor(a[1])), sin = contiguous(tensor(a[2])), pos = contiguous(tensor(a[3]));
   const int64_t hkv = integer(a[4]), n_rep = integer(a[5]), B = qkv_in.size(0), D = cos.size(-1);
   const int64_t per_row = qkv_in.numel() / std::max<int64_t>(B, 1);
@@ -446,33 +453,6 @@ PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
                              k_cache.stride(0), k_cache.stride(1), (int)k_cache.size(2),
                              a[8] == Py_None ? 0 : (int)integer(a[8]), live.defined() ? (const int32_t*)live.data_ptr() : nullptr,
                              dtype_enum(qkv), call.stream), "cq_rope_split_append");
-  return wrap(q);
-  CQ_END
-}
-
-// x [B,1,K], weight [Hkv*(n_rep+2)*D, K], cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index
-PyObject* py_qkv_rope_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  CQ_BEGIN
-  want_args(n, 10, "qkv_rope_append");
-  for (int i : {0, 1, 2, 3, 4, 7, 8}) need_cuda(tensor(a[i]));
-  const Tensor x = contiguous(tensor(a[0])), &w = tensor(a[1]), &k_cache = tensor(a[7]), &v_cache = tensor(a[8]);
-  const Tensor cos = contiguous(tensor(a[2])), sin = contiguous(tensor(a[3])), pos = contiguous(tensor(a[4]));
-  const int64_t hkv = integer(a[5]), n_rep = integer(a[6]), B = x.size(0), K = x.size(-1), D = cos.size(-1);
-  if (w.dim() != 2 || !w.is_contiguous() || w.size(0) != hkv * (n_rep + 2) * D || w.size(1) != K || x.numel() != B * K)
-    raise(PyExc_ValueError, "weight must be contiguous [n_kv_heads*(n_rep+2)*D, K] and x [B,1,K]");
-  for (const Tensor* t : {&w, &cos, &sin, &k_cache, &v_cache})
-    if (t->scalar_type() != x.scalar_type()) raise(PyExc_TypeError, "x, weight, rotary tables and caches must share one dtype");
-  if (pos.scalar_type() != at::kLong || pos.numel() != B)
-    raise(PyExc_ValueError, "position_ids must be int64 with one position per batch row");
-  for (const Tensor* t : {&k_cache, &v_cache})
-    if (t->stride(3) != 1 || t->stride(2) != D)
-      raise(PyExc_ValueError, "cache token rows must be contiguous ([.., T, D] with stride D)");
-  if (k_cache.strides() != v_cache.strides()) raise(PyExc_ValueError, "k_cache and v_cache must share strides");
-  Call call(x);
-  Tensor q = empty({B, hkv * n_rep, 1, D}, x);
-  check(cq_qkv_rope_append(x.data_ptr(), w.data_ptr(), (int)K, cos.data_ptr(), sin.data_ptr(), (int)cos.size(0), (const int64_t*)pos.data_ptr(),
-                           (int)B, (int)hkv, (int)n_rep, (int)D, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0),
-                           k_cache.stride(1), (int)k_cache.size(2), (int)integer(a[9]), dtype_enum(x), call.stream), "cq_qkv_rope_append");
   return wrap(q);
   CQ_END
 }
@@ -662,7 +642,7 @@ PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define CQ_FN(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     CQ_FN(workspace), CQ_FN(workspaces_of), CQ_FN(pack_last_dim), CQ_FN(pack_k_per_channel), CQ_FN(pack_v_per_token),
-    CQ_FN(quant_encode), CQ_FN(qbmm), CQ_FN(decode_attention), CQ_FN(u8_decode_attention), CQ_FN(rope_split_append), CQ_FN(qkv_rope_append), CQ_FN(linear_small), CQ_FN(small_ok), CQ_FN(heads_of),
+    CQ_FN(quant_encode), CQ_FN(qbmm), CQ_FN(decode_attention), CQ_FN(u8_decode_attention), CQ_FN(rope_split_append), CQ_FN(linear_small), CQ_FN(small_ok), CQ_FN(heads_of),
     CQ_FN(prefill_rope_split), CQ_FN(prefill_attention),
     CQ_FN(qjl_quant), CQ_FN(qjl_build), CQ_FN(qjl_gqa_score), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Tensor-level entry points over libcalibquant_b200.so.", -1, methods};

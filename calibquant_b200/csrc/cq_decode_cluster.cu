@@ -767,6 +767,20 @@ inline bool make_plan(const cq_decode_args* a, Plan* p) {
     const int64_t smem = 1024 + ring_bytes(a->bits) + (int64_t)n_rep * pitch * 2;
     if (smem <= SMEM_TWO && pairs <= max_clusters(S)) { p->S = S; p->pitch = pitch; p->smem = (int)smem; return true; }
   }
+  // More pairs than resident clusters: several rounds of the smallest cluster whose logits fit, where the last round is not mostly
+  // empty, or a CTA has enough units for it to matter less.  Against the separate launches (us): 64 x 8 x 4096 tokens, S = 1, 1.73
+  // rounds 79.5 / 88.1; 64 x 8 x 1024 x 6 heads 41.3 / 43.7; 32 x 8 x 8192, S = 2, 1.73 rounds 75.8 / 86.0; 24 x 8 x 6656,
+  // 1.30 rounds of 13 units 56.7 / 60.8; but 40 x 8 x 3328, 1.08 rounds 59.1 / 56.7; and at 4 bits 48 x 8 x 5120 112 / 106
+  if (a->bits > 2) return false;
+  for (int S = 1; S <= 4; S *= 2) {
+    const int units = (n_units + S - 1) / S, pitch = units * UNIT_TOK + 8;
+    const int64_t smem = 1024 + ring_bytes(a->bits) + (int64_t)n_rep * pitch * 2, fit = max_clusters(S);
+    if (S > n_units || smem > SMEM_TWO) continue;
+    const int64_t full = (pairs + fit - 1) / fit * fit;      // clusters the rounds have room for
+    if (pairs * 5 < full * 4 && (pairs * 64 < full * 41 || units < 12)) return false;
+    p->S = S; p->pitch = pitch; p->smem = (int)smem;
+    return true;
+  }
   return false;
 }
 

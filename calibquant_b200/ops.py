@@ -280,20 +280,17 @@ def prefill_rope_split(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache=N
 
 
 def rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache,
-                      append_index=None, t_fp_dev=None):
+                      append_index=None, t_fp_dev=None, weight=None):
     """One decode token per batch row: split the ``wqkv`` output ``qkv`` [B,1,Hkv*(n_rep+2)*D]
     (per KV head: n_rep query heads, key, value), rotate queries and key with the ``cos``/``sin``
     tables [S,D] at ``position_ids`` [B,1], and write the rotated key and the value into the fp caches
     ``k_cache``/``v_cache`` [B,Hkv,capacity,D] at token ``append_index`` -- or at ``t_fp_dev - 1`` when
     the live token count is the int32 device scalar ``t_fp_dev`` (which then already counts the new
-    token).  Returns the rotated queries [B,Hq,1,D]."""
+    token).  With ``weight`` [Hkv*(n_rep+2)*D, K], ``qkv`` is the input [B,1,K] of the projection.  Returns the rotated
+    queries [B,Hq,1,D]."""
+    if weight is not None:
+        return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev, weight)
     return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev)
-
-
-def qkv_rope_append(x, weight, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index):
-    """:func:`rope_split_append` of the projection ``x @ weight.T`` of up to four requests, x [B,1,K], in one launch that reads
-    the weight once (fp32 sums, rounded to the data type before the rotation)."""
-    return native().qkv_rope_append(x, weight, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index)
 
 
 def linear_small(x, weight):

@@ -175,10 +175,10 @@ def _split_qkv(self, hidden_states):
     return q, qkv[..., -2, :], qkv[..., -1, :]
 
 
-def _small_weight(module, x, rows):
-    """The weight of a plain linear projection of few rows, for the launches that read it once; None where the module has to be
-    called (more rows, another module type, a bias, hooks, autograd or autocast at work, other dtypes or layouts)."""
-    if rows > 4 or type(module) is not torch.nn.Linear or torch.is_grad_enabled() or torch.is_autocast_enabled():
+def _plain_weight(module, x):
+    """The weight of a plain linear projection, to be applied without going through the module; None where the module has to be
+    called (another type, a bias, hooks, autograd or autocast at work, other dtypes or layouts)."""
+    if type(module) is not torch.nn.Linear or torch.is_grad_enabled() or torch.is_autocast_enabled():
         return None
     d = module.__dict__
     w = d["_parameters"].get("weight")      # absent where a parametrization computes it
@@ -328,11 +328,9 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
         tc.reserve(1)
         pos = position_ids if position_ids.numel() == bsz else position_ids.expand(bsz, 1)
         n_kv = wqkv.out_features // ((n_rep + 2) * self.head_dim)
-        w = _small_weight(wqkv, hidden_states, bsz)
-        if w is not None:      # a few requests: projection included
-            q = ops.qkv_rope_append(hidden_states, w, cos, sin, pos, n_kv, n_rep, tc.k, tc.v, tc.length)
-        else:
-            q = ops.rope_split_append(wqkv(hidden_states), cos, sin, pos, n_kv, n_rep, tc.k, tc.v, append_index=tc.length)
+        w = _plain_weight(wqkv, hidden_states)
+        q = ops.rope_split_append(hidden_states if w is not None else wqkv(hidden_states), cos, sin, pos, n_kv, n_rep, tc.k, tc.v,
+                                  append_index=tc.length, weight=w)
         tc.length += 1
     else:      # rotary tables of another type than the hidden states
         q, k, v = _split_qkv(self, hidden_states)
@@ -359,7 +357,7 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
                          f"but is {attn.size()}")
     attn = _gather_heads(self, attn.view(bsz, q_len, -1))
     wo = self.wo
-    w = _small_weight(wo, attn, bsz)
+    w = _plain_weight(wo, attn) if bsz <= 4 else None
     return wo(attn) if w is None else ops.linear_small(attn, w), None, past_key_value
 
 

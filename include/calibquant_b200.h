@@ -365,16 +365,9 @@ int cq_rope_split_append(const void* qkv, int64_t qkv_stride_b, const void* cos_
                          int64_t cache_stride_h, int capacity, int append_index, const int32_t* t_fp_dev,
                          int dtype, void* stream);
 /*
- * cq_qkv_rope_append: cq_rope_split_append of x weight^T for up to four requests in one launch; x [batch, k] contiguous, weight
- * [n_kv_heads*(n_rep+2)*128, k] contiguous (rows as in the projection output above), k a multiple of 8, 16-byte aligned.  The sums
- * are fp32, rounded to the data type before the rotation.
- * cq_linear_small: out [rows, n] = x [rows, k] weight [n, k]^T for up to four rows, same alignment, fp32 sums.
- * More rows: CQ_ERR_UNSUPPORTED (a matrix product is the better tool).
+ * cq_linear_small: out [rows, n] = x [rows, k] weight [n, k]^T for up to four rows (more: CQ_ERR_UNSUPPORTED, a matrix product is
+ * the better tool); all contiguous and 16-byte aligned, k a multiple of 8; fp32 sums rounded once.
  */
-int cq_qkv_rope_append(const void* x, const void* weight, int k, const void* cos_table, const void* sin_table, int rope_len,
-                       const int64_t* position_ids, int batch, int n_kv_heads, int n_rep, int head_dim, void* q_out, void* k_cache,
-                       void* v_cache, int64_t cache_stride_b, int64_t cache_stride_h, int capacity, int append_index, int dtype,
-                       void* stream);
 int cq_linear_small(const void* x, const void* weight, void* out, int rows, int n, int k, int dtype, void* stream);
 /*
  * cq_prefill_rope_split is the same step for a whole prompt (patch_internvl.py:214-260 on q_len tokens,

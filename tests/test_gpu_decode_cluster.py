@@ -31,3 +31,15 @@ def test_single_launch_step_edges(ops, bits, B, hq, hkv, t_vis, t_txt, dtype, ma
     out, ref = _run_case(ops, B, hq, hkv, t_vis, t_txt, bits, dtype, seed=bits + t_vis + hq, with_mask=mask)
     assert rel_l2(out, ref) <= (1e-2 if dtype == torch.float16 else 3e-2), rel_l2(out, ref)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("B,hq,hkv,t_vis,t_txt,bits,dtype", [
+    (34, 16, 8, 4 * 256, 5, 1, torch.float16),         # one CTA per pair would leave the second round nearly empty: separate launches
+    (70, 32, 8, 2 * 256, 3, 2, torch.bfloat16),        # two rounds of one CTA per pair, the last one not full
+    (100, 6, 3, 256 + 96, 0, 1, torch.float16),        # just above one round, ragged span
+    (24, 64, 8, 24 * 256, 0, 1, torch.float16),        # eight heads: rounds of clusters of two
+])
+def test_more_pairs_than_resident_clusters(ops, B, hq, hkv, t_vis, t_txt, bits, dtype):
+    out, ref = _run_case(ops, B, hq, hkv, t_vis, t_txt, bits, dtype, seed=bits + t_vis + hq)
+    assert rel_l2(out, ref) <= (1e-2 if dtype == torch.float16 else 3e-2), rel_l2(out, ref)
+    assert ops.device_status() == 0
