@@ -65,6 +65,7 @@ constexpr float RESCALE_LOG2 = 8.f;          // a row is rescaled when its maxim
 struct Params {
   int t_len, hq, hkv;
   int pair;              // 1: the two tiles of an item are the same queries of two heads; 0: adjacent tiles of one head
+  int by_length;         // 1: block order (head, batch row, query rows), all longest rows first; 0: (query rows, head, batch row)
   float scale_log2;
   uint32_t idesc_s, idesc_pv;
   int is_bf16;
@@ -181,19 +182,19 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// One work item = one block index of the grid (x: query rows, longest first; y: query head or pair of heads; z: batch
-// row).  A CTA starts with its own index and then takes over blocks that have not been launched yet (cluster launch
-// control).  Measured, the CTAs running at the same time keep working on the query blocks and heads of a few KV heads,
-// whose K/V tiles stay in L2, as with one CTA per block; a static assignment of items sorted by length lost that and ran
-// 6 % slower.
+// One work item = one block index of the grid.  A CTA starts with its own index and then takes over blocks that have not been
+// launched yet (cluster launch control), in block order.  Where the keys and values do not fit L2 the query rows run fastest
+// (longest first): the CTAs running at the same time then work on the query blocks and heads of a few KV heads, whose K/V
+// tiles stay in L2, as with one CTA per block; items sorted by length lost that and ran 6 % slower at 16 x 3392 tokens.
+// Where they do fit, all longest items come first, so that the CTAs end together: 2 x 1401 tokens 51 -> 42 us, 1 x 3433 114 -> 94, 3 x 2500 173 -> 150, 2 x 6697 654 -> 624.
 struct Item {
   int h, b, hk, q0, n_a, n_b, n_max;        // tile X = 0 (A), 1 (B): head h + X pair, queries q0 + X (1 - pair) BM ..
 };
 __device__ __forceinline__ Item decode_item(const Params& p, int bx, int by, int bz) {
   Item w;
-  const int qt = (int)gridDim.x - 1 - bx;         // longest rows first
-  w.h = by << p.pair;
-  w.b = bz;
+  const int qt = p.by_length ? (int)gridDim.z - 1 - bz : (int)gridDim.x - 1 - bx;         // longest rows first
+  w.h = (p.by_length ? bx : by) << p.pair;
+  w.b = p.by_length ? by : bz;
   w.hk = w.h / (p.hq / p.hkv);
   w.q0 = qt * (2 - p.pair) * BM;
   const int t_tiles = (p.t_len + BN - 1) / BN, q1 = p.pair ? w.q0 : w.q0 + BM;
@@ -643,7 +644,9 @@ int prefill_tc_run(const void* q, const void* k, const void* v, void* out, int b
   p.is_bf16 = is_bf16;
   p.status = status;
   const int rows = p.pair ? BM : 2 * BM;
-  dim3 grid((unsigned)((t_len + rows - 1) / rows), (unsigned)(p.pair ? hq / 2 : hq), (unsigned)batch);
+  const unsigned tiles = (unsigned)((t_len + rows - 1) / rows), heads = (unsigned)(p.pair ? hq / 2 : hq);
+  p.by_length = (int64_t)batch * t_len * hkv * 2 * 128 * 2 <= (int64_t)64 << 20 && tiles <= 65535u ? 1 : 0;      // half of L2
+  const dim3 grid = p.by_length ? dim3(heads, (unsigned)batch, tiles) : dim3(tiles, heads, (unsigned)batch);
   if (is_bf16) prefill_tc_kernel<true><<<grid, THREADS, SMEM_BYTES, st>>>(tq, tk, tv, to, p);
   else prefill_tc_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(tq, tk, tv, to, p);
   return check_launch();
