@@ -184,6 +184,10 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   auto issue = [&](int k) {
     const int s = k % NS;
     unsigned char* base = smem + s * UB;
+    // told before the copies: what a waiting warp has to know is that the slot's barrier has entered this load's phase, which
+    // the release of the load before (seen by this thread) made sure of.  (A fence behind the copies cost ~800 cycles a load.)
+    __threadfence_block();
+    *reinterpret_cast<volatile int*>(&issued_s[s]) = k / NS + 1;
     if (RAGGED && k < n_u) {
       const int gr0 = (u0 + k) * UNIT_G;
       const int32_t* src = k_code + ((int64_t)pair * kHeadDim * n_groups + gr0) * BITS;
@@ -213,9 +217,6 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
       bulk_load_1d(base + CODE, v_scale + tok * 4, (uint32_t)(nt * 8), &full_bar[s]);
       bulk_load_1d(base + CODE + 2048, v_mn + tok * 4, (uint32_t)(nt * 8), &full_bar[s]);
     }
-    if (RAGGED) __syncwarp();
-    __threadfence_block();
-    *reinterpret_cast<volatile int*>(&issued_s[s]) = k / NS + 1;
   };
   // A warp is done with its share of load k; whoever completes the unit refills the slot.  There is no producer warp: a
   // ninth warp per CTA would cost every warp a quarter of its registers.
@@ -250,8 +251,11 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
     if (failed && lane == 0) atomicExch(status, CQ_ERR_TIMEOUT);
     return !failed;
   };
-  if (RAGGED ? warp == 0 : tid == 0)
-    for (int k = 0; k < min(NS, 2 * n_u); ++k) issue(k);
+  // the first loads of the slots, one by each warp (one after the other they took a thread 7000 of the 40 000 cycles that a CTA
+  // has for 16 x 8 x 3328 tokens)
+  static_assert(NS <= NW, "a warp per slot");
+  if (warp < min(NS, 2 * n_u) && (RAGGED || lane == 0)) issue(warp);
+  __syncwarp();
   // this CTA's share of the full-precision tokens (16-token tiles dealt out over the cluster), on its way into L2
   auto fp_range = [&](int& f0, int& f1) {
     const int t_fp = a.t_fp_dev ? min(*reinterpret_cast<const volatile int32_t*>(a.t_fp_dev), a.t_fp) : a.t_fp;
