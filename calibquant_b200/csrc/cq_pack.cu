@@ -8,6 +8,7 @@
 // word w of a row holds elements w*fpi .. w*fpi+fpi-1, element i in bits [i*b, (i+1)*b).
 #include "cq_common.cuh"
 #include <cstdlib>
+#include <type_traits>
 
 namespace cq {
 
@@ -92,7 +93,10 @@ __device__ __forceinline__ unsigned codes2(typename Pk<T>::T2 d2, const typename
 // 4-bit codes of two elements (low half -> bits [0,4), high half -> bits [16,20)) with the reference's rounding
 // points kept: d = x - mn rounded once to the data type, the quotient rounded to the data type, clamp and
 // round-half-even there; only the quotient itself runs in fp32 (see quotient()).
-template <typename T, bool PAIRED>
+// REFINE = false leaves the residual correction out: d * rcp is off by less than q 2^-23 (half an ulp each of the reciprocal and the
+// product), which stays below the distance of the exact quotient from every break point - more than 2^(e-22) (1 + 2^-11) for a
+// break point in [2^e, 2^(e+1)), see quotient() - as long as the reciprocal is a normal number.
+template <typename T, bool PAIRED, bool REFINE = true>
 __device__ __forceinline__ unsigned codes4_pair(typename Pk<T>::T2 x2, typename Pk<T>::T2 mn2, float s0, float r0,
                                                 float s1, float r1) {
   using T2 = typename Pk<T>::T2;
@@ -101,8 +105,8 @@ __device__ __forceinline__ unsigned codes4_pair(typename Pk<T>::T2 x2, typename 
   if (PAIRED) {          // measured: a gain where both elements share the scale, a loss where they do not
     quotient_pair(d.x, d.y, s0, s1, r0, r1, q0, q1);
   } else {
-    q0 = quotient(d.x, s0, r0);
-    q1 = quotient(d.y, s1, r1);
+    q0 = REFINE ? quotient(d.x, s0, r0) : d.x * r0;
+    q1 = REFINE ? quotient(d.y, s1, r1) : d.y * r1;
   }
   T2 y = Pk<T>::pair_rn(q0, q1);
   y = __hmin2(__hmax2(y, Pk<T>::bcast(0.f)), Pk<T>::bcast(15.f));   // the maximum drops the NaN of inf * 0 to 0
@@ -389,29 +393,41 @@ pack_k_per_channel_kernel(const T* __restrict__ k, int heads, int64_t T_len,
         words[0][0] = (ra & 0xffffu) | (rb << 16);
         words[1][0] = (ra >> 16) | (rb & 0xffff0000u);
       } else {
-        // codes of 16/BITS tokens collect in one register (first channel in the low half, second in the high
-        // half: one multiply-add per token), then the halves go to the two channels' words
+        // The compare masks are summed as plain integers: a mask is -l + 65536 (l - h) modulo 2^32 for the truth values l, h of
+        // its halves, so that the weighted sum over eight tokens is -A + 65536 (A - B) with the packed codes A, B of the two
+        // channels, which come apart at the end.  Six instructions a token and channel pair (a difference, three compares, a
+        // three-way sum, a multiply-add) instead of nine: the kernel was bound by issue at this width, 115 us for 8 x 8 x 32768
+        // keys against 99 at one bit, now 111.
         constexpr int TPA = 16 / BITS;
 #pragma unroll
         for (int t0 = 0; t0 < 32; t0 += TPA) {
           unsigned acc = 0;
 #pragma unroll
-          for (int j = 0; j < TPA; ++j) acc += codes2<T, BITS>(__hsub2(xv[t0 + j], mn2), thr) << (j * BITS);
-          words[0][t0 / FPI] |= (acc & 0xffffu) << ((t0 % FPI) * BITS);
-          words[1][t0 / FPI] |= (acc >> 16) << ((t0 % FPI) * BITS);
+          for (int j = 0; j < TPA; ++j) {
+            const T2 d = __hsub2(xv[t0 + j], mn2);                       // x - mn: one rounding, as the reference
+            acc += (__hgt2_mask(d, thr[0]) + __hgt2_mask(d, thr[1]) + __hgt2_mask(d, thr[2])) << (j * BITS);
+          }
+          const unsigned lo = (0u - acc) & 0xffffu, hi = (lo - ((acc + lo) >> 16)) & 0xffffu;
+          words[0][t0 / FPI] |= lo << ((t0 % FPI) * BITS);
+          words[1][t0 / FPI] |= hi << ((t0 % FPI) * BITS);
         }
       }
     } else {
       const float rcp[2] = {__frcp_rn(scale[0]), __frcp_rn(scale[1])};
+      auto encode = [&](auto refine) {
 #pragma unroll
-      for (int t0 = 0; t0 < 32; t0 += 4) {               // four tokens per register, as above
-        unsigned acc = 0;
+        for (int t0 = 0; t0 < 32; t0 += 4) {             // four tokens per register: first channel in the low half, second in the high half
+          unsigned acc = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc += codes4_pair<T, false>(xv[t0 + j], mn2, scale[0], rcp[0], scale[1], rcp[1]) << (j * BITS);
-        words[0][t0 / FPI] |= (acc & 0xffffu) << ((t0 % FPI) * BITS);
-        words[1][t0 / FPI] |= (acc >> 16) << ((t0 % FPI) * BITS);
-      }
+          for (int j = 0; j < 4; ++j)
+            acc += codes4_pair<T, false, decltype(refine)::value>(xv[t0 + j], mn2, scale[0], rcp[0], scale[1], rcp[1]) << (j * BITS);
+          words[0][t0 / FPI] |= (acc & 0xffffu) << ((t0 % FPI) * BITS);
+          words[1][t0 / FPI] |= (acc >> 16) << ((t0 % FPI) * BITS);
+        }
+      };
+      // the reciprocals of fp16 scales are normal numbers (an infinite scale gives 0 and code 0 either way)
+      if (std::is_same<T, __half>::value || (fminf(scale[0], scale[1]) > 1e-30f && fmaxf(scale[0], scale[1]) < 1e30f)) encode(std::false_type{});
+      else encode(std::true_type{});
     }
     const int gs = sub * (KT_TOKENS / 32) + gq;            // group inside the span
 #pragma unroll
