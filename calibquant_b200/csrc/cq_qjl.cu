@@ -366,8 +366,8 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
 #pragma unroll
         for (int v = 0; v < NV; ++v) (&acc[v][0][0][0])[i] = 0.f;
       }
-      // u accumulates over blocks of 32 outlier channels; there is one block unless oc > 32
-      const int blocks = ONE ? 1 : (oc + 31) / 32;
+      // u accumulates over blocks of 32 outlier channels; there is one block unless oc > 32 (an empty one where oc is 0)
+      const int blocks = ONE ? 1 : max(1, (oc + 31) / 32);
       uint32_t qa[2][2], row[2];                      // A fragments and ldmatrix row of the block at hand
       auto load_block = [&](int blk) {
         const int i = blk * 32 + lane;

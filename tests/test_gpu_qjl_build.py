@@ -1,5 +1,5 @@
 """The one-launch sketch of strided keys (tcgen05) against the torch ops and the CPU-oracle quantizer it stands for: tiles
-of four groups that end inside a (batch, head) run, a single group, outlier counts from none to all channels, short outlier
+of four groups that end inside a (batch, head) run, a single group, outlier counts from eight to all channels, short outlier
 sketches, both data types and projections of either type."""
 
 import pytest
