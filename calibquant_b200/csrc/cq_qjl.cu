@@ -12,6 +12,8 @@
 // sum_p sgn_p x_p = 2 sum_{bit_p} x_p - sum_p x_p.  They serve unaligned buffers, sketch dims that are not multiples of
 // 128 and, for the quantizer, other groups than 32 keys; otherwise the quantizer of cq_qjl_build.cu (tcgen05) and
 // score_rows_kernel (outlier projection and sign sums on the warp MMA, a group per warp) run.
+#include <type_traits>
+
 #include "cq_common.cuh"
 #include "cq_ptx.cuh"
 
@@ -251,6 +253,8 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
   float4* qf_s = reinterpret_cast<float4*>(sign_s + SW * 2 * S_SIGN_BYTES);                   // [k-step][lane]
   __half* q_s = reinterpret_cast<__half*>(qf_s + (MAX_SKETCH / 16) * 32);                 // [head][channel]
   uint8_t* order_s = reinterpret_cast<uint8_t*>(q_s + kMaxRep * kHeadDim);                    // [warp][64]: channel per slot, free slots
+  constexpr bool SCALED = std::is_same<T, __nv_bfloat16>::value;
+  __shared__ float2 scale_s[kMaxRep];                                                         // query rows: power of two, its inverse
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
   // the projection, rows of channels, positions in sign order: lane = eight adjacent positions, so that neighbouring lanes
   // read neighbouring projections and write neighbouring 16-byte pieces
@@ -287,9 +291,24 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
     const int64_t seg_end = min(it_end, (kbh + 1) * per_kbh);
     const int64_t qrow0 = kbh * n_rep;
     __syncthreads();
-    for (int i = tid; i < kMaxRep * kHeadDim; i += STHREADS) {
-      const int r = i >> 7, d = i & (kHeadDim - 1);
-      q_s[i] = __float2half_rn(r < n_rep ? Elem<T>::to_f(query[(qrow0 + r) * kHeadDim + d]) : 0.f);
+    // the queries as fp16 operands.  bfloat16 rows are scaled by a power of two that puts the largest element into [4, 8): their
+    // range is fp32's, and the sums with 128 channels stay within fp16's
+    if (warp < kMaxRep) {
+      float x[kHeadDim / 32], m = 0.f, up = 1.f, down = 1.f;
+#pragma unroll
+      for (int i = 0; i < kHeadDim / 32; ++i) {
+        x[i] = warp < n_rep ? Elem<T>::to_f(query[(qrow0 + warp) * kHeadDim + 32 * i + lane]) : 0.f;
+        m = fmaxf(m, fabsf(x[i]));
+      }
+      m = warp_max(m);
+      if (SCALED && m > 0.f && m < INFINITY) {
+        const uint32_t e = max(__float_as_uint(m) >> 23, 7u);      // biased exponent; numbers below 2^-120 are not worth more
+        up = __uint_as_float((127u + 127u + 2u - e) << 23);
+        down = __uint_as_float((e - 2u) << 23);
+      }
+#pragma unroll
+      for (int i = 0; i < kHeadDim / 32; ++i) q_s[warp * kHeadDim + 32 * i + lane] = __float2half_rn(x[i] * up);
+      if (SCALED && lane == 0) scale_s[warp] = make_float2(up, down);
     }
     __syncthreads();
     // q S as accumulators: rows = positions g, g + 8 of a k-step, columns 2c, 2c+1 = heads (R == 4: heads 0-3 twice).  Not given:
@@ -301,7 +320,7 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const int head = (2 * (l & 3) + (k & 1)) & (R == 4 ? 3 : 7), pos = 16 * b + (l >> 2) + 8 * (k >> 1);
-          x[k] = head < n_rep ? query_sketch[(qrow0 + head) * sketch + sign_proj(pos, sketch)] : 0.f;
+          x[k] = head < n_rep ? query_sketch[(qrow0 + head) * sketch + sign_proj(pos, sketch)] * (SCALED ? scale_s[head].x : 1.f) : 0.f;
         }
         qf_s[i] = make_float4(x[0], x[1], x[2], x[3]);
       }
@@ -494,6 +513,7 @@ score_rows_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restri
           const int i = 2 * mt + (e >> 1);
           float v = norm_in[i] * sum[0][mt][e] + scl_o * no[i] * sum[1][mt][e];
           if (R == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
+          if (SCALED) v *= scale_s[(2 * c + (e & 1)) & (R - 1)].y;
           if (2 * c + (e & 1) < n_rep && g + 8 * i < n_tok && (R == 8 || c < 2)) dst[(e & 1) * ((int64_t)n_groups * G) + 8 * i] = v;
         }
     }

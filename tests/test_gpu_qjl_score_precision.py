@@ -31,3 +31,26 @@ def test_sums_of_one_sign(rep):
         q[..., 64:] = 1.0
         exact = math.sqrt(math.pi / 2) / 256 * (q[0, :, 0].double() @ S.double()).sum(-1, keepdim=True)
         assert ((_one_group(q, S) - exact) / exact).abs().max() <= 3 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("given", [False, True])
+@pytest.mark.parametrize("rep,G,oc", [(4, 32, 32), (8, 32, 32), (3, 64, 40)])
+def test_bfloat16_queries_keep_their_range(rep, G, oc, given):
+    """Queries times a power of two give the scores times that power, bit for bit: beyond fp16's largest number (2^16) and
+    below its normal ones (2^-14) as well; rows of one call each have their own."""
+    from calibquant_b200 import ops
+    g = torch.Generator().manual_seed(rep)
+    n, S = 3, torch.randn(128, 256, generator=g)
+    q = torch.randn(1, 2 * rep, 1, 128, generator=g).bfloat16()
+    bits, obits = (torch.randint(0, 256, (1, 2, n, G, 32), generator=g, dtype=torch.uint8) for _ in range(2))
+    knorm, onorm = (torch.rand(1, 2, n, G, generator=g) + 3).bfloat16(), torch.rand(1, 2, n, G, generator=g).bfloat16()
+    idx = torch.stack([torch.randperm(128, generator=g)[:oc] for _ in range(2 * n)]).view(1, 2, n, oc).to(torch.uint8)
+    fixed = [t.cuda() for t in (bits, obits, knorm, onorm, idx)]
+
+    def scores(queries):
+        qs = (queries.double() @ S.double()).float().cuda() if given else None
+        return ops.qjl_gqa_score(*fixed, qs, queries.cuda(), S.cuda()).cpu()
+
+    base = scores(q)
+    factor = 2.0 ** torch.tensor([0., 20., -20., 60., -60., 3.]).repeat(2 * rep)[:2 * rep].view(1, -1, 1, 1)
+    assert torch.equal(scores((q.float() * factor).bfloat16()), base * factor)
