@@ -93,15 +93,24 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   }
   __syncthreads();
   cluster_arrive();
-  const int t_fp = a.t_fp_dev ? min(*reinterpret_cast<const volatile int32_t*>(a.t_fp_dev), a.t_fp) : a.t_fp;
-  const int n_t16 = (t_fp + 15) / 16, f0 = rank * n_t16 / S * 16, f1 = min(t_fp, (rank + 1) * n_t16 / S * 16), n_f = f1 - f0;
-  const int64_t fp_off = (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h + (int64_t)f0 * kHeadDim;
   const uint8_t* ek = enc_k + ((int64_t)pair * a.t_vis + tok0) * ROWB;
   const uint8_t* ev = enc_v + ((int64_t)pair * a.t_vis + tok0) * ROWB;
   for (int i = tid; i < n_tok * ROWB / 128; i += THREADS) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(ek + (int64_t)i * 128));
     asm volatile("prefetch.global.L2 [%0];" ::"l"(ev + (int64_t)i * 128));
   }
+  // this CTA's share of the full-precision tokens (16-token tiles dealt out over the cluster).  A launch before this one may
+  // still be advancing the live count: what is read here is good enough for a prefetch, and read again behind the wait
+  int t_fp, n_f, f0;
+  int64_t fp_off;
+  auto fp_range = [&]() {
+    t_fp = a.t_fp_dev ? min(*reinterpret_cast<const volatile int32_t*>(a.t_fp_dev), a.t_fp) : a.t_fp;
+    const int n_t16 = (t_fp + 15) / 16;
+    f0 = rank * n_t16 / S * 16;
+    n_f = min(t_fp, (rank + 1) * n_t16 / S * 16) - f0;
+    fp_off = (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h + (int64_t)f0 * kHeadDim;
+  };
+  fp_range();
   for (int i = tid; i < n_f * 4; i += THREADS)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(((i & 1) ? v_fp : k_fp) + fp_off + (int64_t)(i >> 1) * 64));
 
@@ -109,6 +118,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   float* fs = reinterpret_cast<float*>(smem + (size_t)a.n_rep * a.pitch * SB);   // full-precision scores [n_rep][fp_pitch]
   T* fpr = reinterpret_cast<T*>(fs);                                        // ... later their probabilities, [n_rep][2*fp_pitch]
   pdl_wait();
+  fp_range();
 
   // ---- query side: weights rnd(q * scale_key), bias_k = rnd(rnd(sum rnd(rnd(scale*zp) * q)) / sqrt(D))
   if (warp < a.n_rep) {
