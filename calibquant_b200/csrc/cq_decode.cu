@@ -517,9 +517,8 @@ static size_t host_stage_bytes(const cq_decode_args* a) {
   return align_up((size_t)a->batch * a->n_q_heads * kHeadDim * 2, 256);
 }
 // Page-locked query rows -> their device staging rows, 16 bytes per thread, read over the host link by the kernel
-// itself.  The score launch that follows is a programmatic dependent launch: it sets up its barriers and streams its
-// first key tiles while this copy runs, and touches the query only after it (griddepcontrol.wait); behind a
-// copy-engine transfer it could not start early.
+// itself.  The score launch that follows is a programmatic dependent launch: it starts and sets up its barriers while this
+// copy runs, and reads only after it (griddepcontrol.wait); behind a copy-engine transfer it could not start early.
 __global__ void stage_query_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int n) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -177,8 +177,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   __syncthreads();
   cluster_arrive();          // waited for before the first remote store: every peer's barriers exist then
 
-  // The ring holds the CTA's key units and then its value units, in order: load k goes to slot k % NS.  No launch of a
-  // decode step writes the packed operands, so these loads wait for nothing.
+  // The ring holds the CTA's key units and then its value units, in order: load k goes to slot k % NS.
   // Called by one thread, by a whole warp where RAGGED.
   const int n_groups = a.t_vis / kGroup;
   auto issue = [&](int k) {
@@ -251,10 +250,16 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
     if (failed && lane == 0) atomicExch(status, CQ_ERR_TIMEOUT);
     return !failed;
   };
+  // The query, the newest full-precision token and freshly packed operands come from the launches before this one: nothing is
+  // read before they have completed.  Steps that follow each other directly lose the overlap of the first loads with the tail
+  // of the step before: 1 x 8 x 256 tokens 11.1 us with the packed operands read ahead of the wait, 11.4 so; 4 x 8 x 5152
+  // 23.2, 24.0; 64 x 8 x 6656 164.5, 169.0.  (Requested into L2 ahead of the wait 16 x 8 x 3328 took 33.0: a bulk prefetch costs
+  // its thread as much as the load.)
+  pdl_wait();
   // the first loads of the slots, one by each warp (one after the other they took one thread 7000
   // cycles; 4 x 8 x 5152 masked tokens 24.0 -> 23.2 us, no difference where the ring's first units suffice for a while)
   static_assert(NS <= NW, "a warp per slot");
-  if (warp < min(NS, 2 * n_u) && (RAGGED || lane == 0)) issue(warp);
+  if (warp < min(NS, n_u) && (RAGGED || lane == 0)) issue(warp);
   __syncwarp();
   // this CTA's share of the full-precision tokens (16-token tiles dealt out over the cluster), on its way into L2
   auto fp_range = [&](int& f0, int& f1) {
@@ -275,7 +280,9 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
 
   const uint32_t ring = smem_u32(smem), lg = ring + ring_bytes(BITS);      // logits [n_rep][pitch] behind the ring
   const Lane<BITS> L(g);
-  pdl_wait();      // the query and the newest full-precision token come from the launches before
+  // value units of the first ring behind the key units, whose data is needed first: 16 x 8 x 3328 tokens 30.7 -> 28.7 us
+  if (warp >= n_u && warp < min(NS, 2 * n_u) && (RAGGED || lane == 0)) issue(warp);
+  __syncwarp();
 
   // ================= 1. scores =================
   {

@@ -152,7 +152,6 @@ k1_scores(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__ C
   const int n_pairs = dm.batch * dm.hkv;
   const int n_items = n_pairs * dm.n_ktiles;
 
-  pdl_launch_dependents();
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], LDG ? 32 : 1); mbar_init(&empty_bar[s], K1_WARPS); }
     mbar_fence_init();
@@ -164,6 +163,10 @@ k1_scores(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__ C
   const int it_first = (int)(((int64_t)blockIdx.x * n_items) / gridDim.x);
   const int it_end = (int)(((int64_t)(blockIdx.x + 1) * n_items) / gridDim.x);
 
+  // Nothing is read before the launches ahead of this one have completed: they may have packed the operands.  Only then is
+  // the attn.V launch let in, which requests its first packed values without waiting for this one.
+  pdl_wait();
+  pdl_launch_dependents();
   if (LDG && warp == K1_WARPS) {
     // ---- producer, all 32 lanes: 4-byte asynchronous copies of the tile's code words into the swizzled boxes
     constexpr int WPR = TILE_G * BITS;                 // words of a channel row inside a tile
@@ -231,10 +234,6 @@ k1_scores(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__ C
   }
   (void)word_in_group;
 
-  // The producer above streams only the packed keys, which no launch of a decode step writes, so it may run
-  // ahead of the kernel before this one in the stream; the query and the score buffer
-  // (still read by the previous step) are touched only after that kernel has completed.
-  pdl_wait();
   int cur_pair = -1;
   uint32_t qA[8], qB[8];
   bool failed = false;
@@ -660,8 +659,9 @@ k2_attn_v(const __grid_constant__ CUtensorMap tm_v,   // 2 and 4 bits: the value
   if (warp == K2_WARPS) {
     if (lane == 0) {
       fence_proxy_async_smem();
-      // the packed values do not depend on the score launch: the first ring of tiles is requested before
-      // waiting for it, the logit rows of those tiles after
+      // the packed values do not depend on the score launch, and what the launches before that one wrote is visible (it let
+      // this launch in behind its own wait): the first ring of tiles is requested before waiting for it, the logit rows of
+      // those tiles after
       auto load_values = [&](int k) {
         const int it = it_first + k, s = k % STAGES;
         const int pair = it / n_vt, vt = it % n_vt;
