@@ -14,6 +14,7 @@
 
 #include <map>
 #include <tuple>
+#include <vector>
 
 #include "../../include/calibquant_b200.h"
 
@@ -128,28 +129,50 @@ PyObject* wrap3(Tensor a, Tensor b, Tensor c) {
 
 // ---- scratch -------------------------------------------------------------------------------------------------------
 // Grow-only buffer per (device, stream), zeroed when created: its first word is the sticky device status the decode
-// kernels set when a bounded wait runs out.  A capture reuses the buffer an eager warm-up call created (a fixed address
-// the replays can use); a buffer that has to be created while a CUDA graph is being captured lives in that graph's
-// memory pool and is kept for captures only, eager calls on the same stream never see it.  Guarded by the GIL; the map
-// is never destroyed (at exit the CUDA context may be gone before it).
-using WsKey = std::tuple<int, cudaStream_t, bool>;
-std::map<WsKey, Tensor>& workspaces() { static auto* m = new std::map<WsKey, Tensor>(); return *m; }
+// kernels set when a bounded wait runs out.  Guarded by the GIL; the map is never destroyed (at exit the CUDA context may be
+// gone before it).
+//   * A capture takes the buffer an eager warm-up call created, if it is large enough, and the graph's replays go on using it
+//     for as long as the graph lives, which is not known here: such a buffer is never freed.  One that replaces it is at
+//     least twice its size, so that all the retired ones together are smaller than the one in use.
+//   * A buffer created during a capture lives in that graph's memory pool, like any intermediate of the graph: eager calls and
+//     other captures never see it, and the reference kept here ends with the next capture.
+struct Scratch {
+  Tensor buf;
+  unsigned long long capture = 0;      // the capture it was created in
+  bool in_graph = false;               // an eager buffer that a capture has used
+};
+using WsKey = std::tuple<int, cudaStream_t, bool>;      // device, stream, created during a capture
+std::map<WsKey, Scratch>& workspaces() { static auto* m = new std::map<WsKey, Scratch>(); return *m; }
+std::vector<Tensor>& retired() { static auto* v = new std::vector<Tensor>(); return *v; }
 
 Tensor workspace(int64_t nbytes, int device, cudaStream_t stream) {
-  auto& all = workspaces();
-  WsKey key(device, stream, false);
-  auto it = all.find(key);
-  if (it != all.end() && it->second.numel() >= nbytes) return it->second;
-  c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
-    key = WsKey(device, stream, true);
-    it = all.find(key);
-    if (it != all.end() && it->second.numel() >= nbytes) return it->second;
+  Scratch& eager = workspaces()[WsKey(device, stream, false)];
+  c10::cuda::OptionalCUDAGuard guard;
+  if (c10::cuda::current_device() != device) guard.set_index(static_cast<c10::DeviceIndex>(device));
+  const auto fresh = [&](int64_t n, const Tensor& before) {
+    Tensor buf = at::zeros({std::max<int64_t>(n, 256)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+    if (before.defined()) buf.narrow(0, 0, 4).copy_(before.narrow(0, 0, 4));      // a sticky status survives the regrowth
+    return buf;
+  };
+  const bool enough = eager.buf.defined() && eager.buf.numel() >= nbytes;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+    if (enough) return eager.buf;
+    Tensor buf = fresh(eager.in_graph ? std::max(nbytes, 2 * eager.buf.numel()) : nbytes, eager.buf);
+    if (eager.in_graph) retired().push_back(eager.buf);
+    eager = Scratch{buf, 0, false};
+    return buf;
   }
-  Tensor buf = at::zeros({std::max<int64_t>(nbytes, 256)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
-  if (it != all.end()) buf.narrow(0, 0, 4).copy_(it->second.narrow(0, 0, 4));      // a sticky status survives the regrowth
-  all[key] = buf;
-  return buf;
+  if (enough) {
+    eager.in_graph = true;
+    return eager.buf;
+  }
+  cudaStreamCaptureStatus status;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(c10::cuda::getCurrentCUDAStream(device).stream(), &status, &id));
+  Scratch& own = workspaces()[WsKey(device, stream, true)];
+  if (own.buf.defined() && own.capture == id && own.buf.numel() >= nbytes) return own.buf;
+  own = Scratch{fresh(nbytes, own.capture == id ? own.buf : Tensor()), id, true};
+  return own.buf;
 }
 
 PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -165,8 +188,8 @@ PyObject* py_workspaces_of(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyObject* list = PyList_New(0);
   for (const bool capturing : {false, true}) {
     auto it = workspaces().find(WsKey((int)integer(a[0]), reinterpret_cast<cudaStream_t>(integer(a[1])), capturing));
-    if (it == workspaces().end()) continue;
-    PyObject* t = wrap(it->second);
+    if (it == workspaces().end() || !it->second.buf.defined()) continue;
+    PyObject* t = wrap(it->second.buf);
     PyList_Append(list, t);
     Py_DECREF(t);
   }
