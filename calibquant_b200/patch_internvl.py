@@ -175,20 +175,24 @@ def _split_qkv(self, hidden_states):
     return q, qkv[..., -2, :], qkv[..., -1, :]
 
 
+_GLOBAL_HOOKS = (torch.nn.modules.module._global_forward_hooks, torch.nn.modules.module._global_forward_pre_hooks)
+_LINEAR_FORWARD = torch.nn.Linear.forward
+
+
 def _plain_weight(module, x):
     """The weight of a plain linear projection, to be applied without going through the module; None where the module has to be
-    called (another type, a bias, hooks, autograd or autocast at work, other dtypes or layouts)."""
+    called: another type, a bias, hooks, a ``forward`` put on the instance or the class (instrumentation, offloading), a weight
+    that is not a plain parameter (quantized or sharded subclasses, parametrizations), autograd or autocast at work, other
+    dtypes or layouts."""
     if type(module) is not torch.nn.Linear or torch.is_grad_enabled() or torch.is_autocast_enabled():
         return None
     d = module.__dict__
-    w = d["_parameters"].get("weight")      # absent where a parametrization computes it
-    if w is None or d["_parameters"]["bias"] is not None or d["_forward_hooks"] or d["_forward_pre_hooks"] or \
-            _GLOBAL_HOOKS[0] or _GLOBAL_HOOKS[1]:
+    params = d["_parameters"]
+    w = params.get("weight")
+    if type(w) is not torch.nn.Parameter or params.get("bias", w) is not None or d["_forward_hooks"] or d["_forward_pre_hooks"] or \
+            "forward" in d or torch.nn.Linear.forward is not _LINEAR_FORWARD or _GLOBAL_HOOKS[0] or _GLOBAL_HOOKS[1]:
         return None
     return w if native().small_ok(x, w) else None
-
-
-_GLOBAL_HOOKS = (torch.nn.modules.module._global_forward_hooks, torch.nn.modules.module._global_forward_pre_hooks)
 
 
 def _shard_world(self):
