@@ -8,7 +8,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAException.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -145,30 +145,34 @@ using WsKey = std::tuple<int, cudaStream_t, bool>;      // device, stream, creat
 std::map<WsKey, Scratch>& workspaces() { static auto* m = new std::map<WsKey, Scratch>(); return *m; }
 std::vector<Tensor>& retired() { static auto* v = new std::vector<Tensor>(); return *v; }
 
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();      // the default stream beside a capture
+  return status != cudaStreamCaptureStatusNone;
+}
+
 Tensor workspace(int64_t nbytes, int device, cudaStream_t stream) {
   Scratch& eager = workspaces()[WsKey(device, stream, false)];
-  c10::cuda::OptionalCUDAGuard guard;
-  if (c10::cuda::current_device() != device) guard.set_index(static_cast<c10::DeviceIndex>(device));
+  const bool enough = eager.buf.defined() && eager.buf.numel() >= nbytes, in_capture = capturing(stream);
+  if (enough) {
+    if (in_capture) eager.in_graph = true;
+    return eager.buf;
+  }
+  c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
   const auto fresh = [&](int64_t n, const Tensor& before) {
     Tensor buf = at::zeros({std::max<int64_t>(n, 256)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
     if (before.defined()) buf.narrow(0, 0, 4).copy_(before.narrow(0, 0, 4));      // a sticky status survives the regrowth
     return buf;
   };
-  const bool enough = eager.buf.defined() && eager.buf.numel() >= nbytes;
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
-    if (enough) return eager.buf;
+  if (!in_capture) {
     Tensor buf = fresh(eager.in_graph ? std::max(nbytes, 2 * eager.buf.numel()) : nbytes, eager.buf);
     if (eager.in_graph) retired().push_back(eager.buf);
     eager = Scratch{buf, 0, false};
     return buf;
   }
-  if (enough) {
-    eager.in_graph = true;
-    return eager.buf;
-  }
   cudaStreamCaptureStatus status;
   unsigned long long id = 0;
-  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(c10::cuda::getCurrentCUDAStream(device).stream(), &status, &id));
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id));
   Scratch& own = workspaces()[WsKey(device, stream, true)];
   if (own.buf.defined() && own.capture == id && own.buf.numel() >= nbytes) return own.buf;
   own = Scratch{fresh(nbytes, own.capture == id ? own.buf : Tensor()), id, true};
