@@ -99,6 +99,8 @@ SIGNATURES = {
     "cq_u8_decode_attn": (_c.c_int, [_c.POINTER(U8DecodeArgs), _vp, _sz, _vp]),
     "cq_rope_split_append": (_c.c_int, [_vp, _i64, _vp, _vp, _c.c_int, _vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                         _vp, _vp, _vp, _i64, _i64, _c.c_int, _c.c_int, _vp, _c.c_int, _vp]),
+    "cq_rope_split_append_strict": (_c.c_int, [_vp, _i64, _vp, _vp, _c.c_int, _vp, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
+                                        _vp, _vp, _vp, _i64, _i64, _c.c_int, _c.c_int, _vp, _c.c_int, _vp, _vp]),
     "cq_prefill_rope_split": (_c.c_int, [_vp, _i64, _i64, _vp, _vp, _c.c_int, _vp, _c.c_int, _c.c_int, _c.c_int,
                                          _c.c_int, _c.c_int, _vp, _vp, _vp, _vp, _i64, _i64, _c.c_int, _c.c_int,
                                          _c.c_int, _c.c_int, _vp]),

@@ -440,14 +440,49 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_END
 }
 
+// ---- refused positions ------------------------------------------------------------------------------------------------
+// A word of page-locked memory per (device, stream) that a launch sets when it refuses a position: as with any asynchronous
+// error, a later call on the stream raises.  None while a capture runs that no call on the stream has gone before.
+using FlagKey = std::pair<int, cudaStream_t>;
+struct Flag {
+  Tensor word;
+  int32_t* device = nullptr;
+};
+std::map<FlagKey, Flag>& refusals() { static auto* m = new std::map<FlagKey, Flag>(); return *m; }
+int32_t* refusal_flag(cudaStream_t stream, int device) {
+  Flag& f = refusals()[FlagKey(device, stream)];
+  if (!f.word.defined()) {
+    if (capturing(stream)) return nullptr;
+    Tensor word = at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    void* dev = nullptr;
+    C10_CUDA_CHECK(cudaHostGetDevicePointer(&dev, word.data_ptr(), 0));
+    f = Flag{word, static_cast<int32_t*>(dev)};
+  }
+  volatile int32_t* word = f.word.data_ptr<int32_t>();
+  if (*word != 0) {
+    *word = 0;
+    raise(PyExc_RuntimeError, "position_ids of an earlier decode step on this stream lie outside the rotary table");
+  }
+  return f.device;
+}
+// the word's value (0 where there is none); the caller has synchronised
+PyObject* py_refused(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  CQ_BEGIN
+  want_args(n, 2, "refused");      // device index, stream handle
+  auto it = refusals().find(FlagKey((int)integer(a[0]), reinterpret_cast<cudaStream_t>(integer(a[1]))));
+  if (it == refusals().end() || !it->second.word.defined()) return PyLong_FromLong(0);
+  return PyLong_FromLong(*static_cast<volatile int32_t*>(it->second.word.data_ptr<int32_t>()));
+  CQ_END
+}
+
 // ---- the launches around the attention -------------------------------------------------------------------------------
-// qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev [, weight: qkv is then the input of the
-// projection, x [B,1,K], and the matrix product is made here]
+// qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev, weight | None (given: qkv is the input
+// of the projection, x [B,1,K], and the matrix product is made here), strict: positions outside the table are refused
 PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_BEGIN
-  if (n != 11) want_args(n, 10, "rope_split_append");
+  want_args(n, 12, "rope_split_append");
   Tensor qkv_in = tensor(a[0]);
-  if (n == 11) {
+  if (a[10] != Py_None) {
     need_cuda(qkv_in);
     need_cuda(tensor(a[10]));
     qkv_in = at::mm(qkv_in.view({-1, qkv_in.size(-1)}), tensor(a[10]).t());
@@ -475,11 +510,20 @@ PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (live.defined()) check_counter(live);
   Call call(qkv);
   Tensor q = empty({B, hkv * n_rep, 1, D}, qkv);
-  check(cq_rope_split_append(qkv.data_ptr(), per_row, cos.data_ptr(), sin.data_ptr(), (int)cos.size(0), (const int64_t*)pos.data_ptr(),
-                             (int)B, (int)hkv, (int)n_rep, (int)D, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                             k_cache.stride(0), k_cache.stride(1), (int)k_cache.size(2),
-                             a[8] == Py_None ? 0 : (int)integer(a[8]), live.defined() ? (const int32_t*)live.data_ptr() : nullptr,
-                             dtype_enum(qkv), call.stream), "cq_rope_split_append");
+  const void* table[2] = {cos.data_ptr(), sin.data_ptr()};
+  const int at = a[8] == Py_None ? 0 : (int)integer(a[8]);
+  const int32_t* count = live.defined() ? (const int32_t*)live.data_ptr() : nullptr;
+  if (truth(a[11])) {
+    int32_t* refused = refusal_flag(call.stream, qkv.get_device());
+    check(cq_rope_split_append_strict(qkv.data_ptr(), per_row, table[0], table[1], (int)cos.size(0), (const int64_t*)pos.data_ptr(), (int)B,
+                                      (int)hkv, (int)n_rep, (int)D, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                                      k_cache.stride(0), k_cache.stride(1), (int)k_cache.size(2), at, count, dtype_enum(qkv), refused,
+                                      call.stream), "cq_rope_split_append_strict");
+  } else {
+    check(cq_rope_split_append(qkv.data_ptr(), per_row, table[0], table[1], (int)cos.size(0), (const int64_t*)pos.data_ptr(), (int)B,
+                               (int)hkv, (int)n_rep, (int)D, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0),
+                               k_cache.stride(1), (int)k_cache.size(2), at, count, dtype_enum(qkv), call.stream), "cq_rope_split_append");
+  }
   return wrap(q);
   CQ_END
 }
@@ -668,7 +712,7 @@ PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 #define CQ_FN(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    CQ_FN(workspace), CQ_FN(workspaces_of), CQ_FN(pack_last_dim), CQ_FN(pack_k_per_channel), CQ_FN(pack_v_per_token),
+    CQ_FN(workspace), CQ_FN(workspaces_of), CQ_FN(refused), CQ_FN(pack_last_dim), CQ_FN(pack_k_per_channel), CQ_FN(pack_v_per_token),
     CQ_FN(quant_encode), CQ_FN(qbmm), CQ_FN(decode_attention), CQ_FN(u8_decode_attention), CQ_FN(rope_split_append), CQ_FN(linear_small), CQ_FN(small_ok), CQ_FN(heads_of),
     CQ_FN(prefill_rope_split), CQ_FN(prefill_attention),
     CQ_FN(qjl_quant), CQ_FN(qjl_build), CQ_FN(qjl_gqa_score), {nullptr, nullptr, 0, nullptr}};

@@ -82,7 +82,7 @@ rope_split_append_kernel(const T* __restrict__ qkv, int64_t qkv_stride_b, const 
                          const T* __restrict__ sin_t, const int64_t* __restrict__ position_ids, int n_kv_heads,
                          int n_rep, T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache,
                          int64_t cache_stride_b, int64_t cache_stride_h, int capacity, int append_index,
-                         const int32_t* __restrict__ t_fp_dev, int rope_len) {
+                         const int32_t* __restrict__ t_fp_dev, int rope_len, int strict, volatile int* refused) {
   const int per_kv = n_rep + 2;
   const int b = blockIdx.x / (n_kv_heads * per_kv);
   const int rem = blockIdx.x % (n_kv_heads * per_kv);
@@ -104,6 +104,14 @@ rope_split_append_kernel(const T* __restrict__ qkv, int64_t qkv_stride_b, const 
     return;
   }
   int64_t pos = position_ids[b];
+  if (strict) {                                          // as torch indexes a table
+    if (pos < 0) pos += rope_len;
+    if (pos < 0 || pos >= rope_len) {
+      if (refused && d == 0) *refused = CQ_ERR_BAD_ARG;
+      dst[d] = dst[d + 64] = Elem<T>::from_f(__int_as_float(0x7fc00000));
+      return;
+    }
+  }
   pos = pos < 0 ? 0 : (pos >= rope_len ? rope_len - 1 : pos);
   const T* cr = cos_t + pos * kHeadDim;
   const T* sr = sin_t + pos * kHeadDim;
@@ -275,11 +283,10 @@ extern "C" int cq_add_rmsnorm(const void* delta, void* residual, const void* wei
   return cudaGetLastError() == cudaSuccess ? CQ_OK : CQ_ERR_LAUNCH;
 }
 
-extern "C" int cq_rope_split_append(const void* qkv, int64_t qkv_stride_b, const void* cos_table,
-                                    const void* sin_table, int rope_len, const int64_t* position_ids, int batch,
-                                    int n_kv_heads, int n_rep, int head_dim, void* q_out, void* k_cache,
-                                    void* v_cache, int64_t cache_stride_b, int64_t cache_stride_h, int capacity,
-                                    int append_index, const int32_t* t_fp_dev, int dtype, void* stream) {
+static int rope_split_append(const void* qkv, int64_t qkv_stride_b, const void* cos_table, const void* sin_table, int rope_len,
+                             const int64_t* position_ids, int batch, int n_kv_heads, int n_rep, int head_dim, void* q_out,
+                             void* k_cache, void* v_cache, int64_t cache_stride_b, int64_t cache_stride_h, int capacity,
+                             int append_index, const int32_t* t_fp_dev, int dtype, void* stream, int strict, int* refused) {
   if (batch == 0) return CQ_OK;
   if (!qkv || !cos_table || !sin_table || !position_ids || !q_out || !k_cache || !v_cache) return CQ_ERR_BAD_ARG;
   if (batch < 0 || n_kv_heads <= 0 || n_rep <= 0 || rope_len <= 0 || capacity <= 0) return CQ_ERR_BAD_ARG;
@@ -294,15 +301,33 @@ extern "C" int cq_rope_split_append(const void* qkv, int64_t qkv_stride_b, const
         static_cast<const __half*>(qkv), qkv_stride_b, static_cast<const __half*>(cos_table),
         static_cast<const __half*>(sin_table), position_ids, n_kv_heads, n_rep, static_cast<__half*>(q_out),
         static_cast<__half*>(k_cache), static_cast<__half*>(v_cache), cache_stride_b, cache_stride_h, capacity,
-        append_index, t_fp_dev, rope_len);
+        append_index, t_fp_dev, rope_len, strict, refused);
   else
     step::rope_split_append_kernel<__nv_bfloat16><<<(unsigned)blocks, 64, 0, st>>>(
         static_cast<const __nv_bfloat16*>(qkv), qkv_stride_b, static_cast<const __nv_bfloat16*>(cos_table),
         static_cast<const __nv_bfloat16*>(sin_table), position_ids, n_kv_heads, n_rep,
         static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache),
         static_cast<__nv_bfloat16*>(v_cache), cache_stride_b, cache_stride_h, capacity, append_index, t_fp_dev,
-        rope_len);
+        rope_len, strict, refused);
   return cudaGetLastError() == cudaSuccess ? CQ_OK : CQ_ERR_LAUNCH;
+}
+
+extern "C" int cq_rope_split_append(const void* qkv, int64_t qkv_stride_b, const void* cos_table,
+                                    const void* sin_table, int rope_len, const int64_t* position_ids, int batch,
+                                    int n_kv_heads, int n_rep, int head_dim, void* q_out, void* k_cache,
+                                    void* v_cache, int64_t cache_stride_b, int64_t cache_stride_h, int capacity,
+                                    int append_index, const int32_t* t_fp_dev, int dtype, void* stream) {
+  return rope_split_append(qkv, qkv_stride_b, cos_table, sin_table, rope_len, position_ids, batch, n_kv_heads, n_rep, head_dim, q_out, k_cache, v_cache,
+                           cache_stride_b, cache_stride_h, capacity, append_index, t_fp_dev, dtype, stream, 0, nullptr);
+}
+
+extern "C" int cq_rope_split_append_strict(const void* qkv, int64_t qkv_stride_b, const void* cos_table,
+                                           const void* sin_table, int rope_len, const int64_t* position_ids, int batch,
+                                           int n_kv_heads, int n_rep, int head_dim, void* q_out, void* k_cache,
+                                           void* v_cache, int64_t cache_stride_b, int64_t cache_stride_h, int capacity,
+                                           int append_index, const int32_t* t_fp_dev, int dtype, int32_t* refused, void* stream) {
+  return rope_split_append(qkv, qkv_stride_b, cos_table, sin_table, rope_len, position_ids, batch, n_kv_heads, n_rep, head_dim, q_out, k_cache, v_cache,
+                           cache_stride_b, cache_stride_h, capacity, append_index, t_fp_dev, dtype, stream, 1, refused);
 }
 
 extern "C" int cq_swiglu(const void* gate, const void* up, void* out, int64_t n, int dtype, void* stream) {

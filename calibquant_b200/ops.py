@@ -68,14 +68,16 @@ def _workspace(nbytes: int, device, stream_handle=None) -> torch.Tensor:
 
 def device_status(device=None) -> int:
     """Sticky status word of the current stream's decode workspace (0 = no device-side wait has
-    timed out since the workspace was created).  Synchronises the stream."""
+    timed out since the workspace was created), or that of refused positions (CQ_ERR_BAD_ARG until the next eager
+    step on the stream raises for them).  Synchronises the stream."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else device
-    stream = torch.cuda.current_stream(device).cuda_stream
+    stream = torch.cuda.current_stream(device)
     status = 0
-    for buf in native().workspaces_of(device.index, stream):
+    for buf in native().workspaces_of(device.index, stream.cuda_stream):
         if status == 0:
             status = int(buf[:4].view(torch.int32).item())
-    return status
+    stream.synchronize()
+    return status or native().refused(device.index, stream.cuda_stream)
 
 
 def pack_last_dim(data: torch.Tensor, group_size: int, bits: int):
@@ -288,9 +290,7 @@ def rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v
     the live token count is the int32 device scalar ``t_fp_dev`` (which then already counts the new
     token).  With ``weight`` [Hkv*(n_rep+2)*D, K], ``qkv`` is the input [B,1,K] of the projection.  Returns the rotated
     queries [B,Hq,1,D]."""
-    if weight is not None:
-        return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev, weight)
-    return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev)
+    return native().rope_split_append(qkv, cos, sin, position_ids, n_kv_heads, n_rep, k_cache, v_cache, append_index, t_fp_dev, weight, False)
 
 
 def linear_small(x, weight):

@@ -333,8 +333,8 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
         pos = position_ids if position_ids.numel() == bsz else position_ids.expand(bsz, 1)
         n_kv = wqkv.out_features // ((n_rep + 2) * self.head_dim)
         w = _plain_weight(wqkv, hidden_states)
-        q = ops.rope_split_append(hidden_states if w is not None else wqkv(hidden_states), cos, sin, pos, n_kv, n_rep, tc.k, tc.v,
-                                  append_index=tc.length, weight=w)
+        q = native().rope_split_append(hidden_states if w is not None else wqkv(hidden_states), cos, sin, pos, n_kv, n_rep, tc.k, tc.v,
+                                       tc.length, None, w, True)
         tc.length += 1
     else:      # rotary tables of another type than the hidden states
         q, k, v = _split_qkv(self, hidden_states)

@@ -365,6 +365,16 @@ int cq_rope_split_append(const void* qkv, int64_t qkv_stride_b, const void* cos_
                          int64_t cache_stride_h, int capacity, int append_index, const int32_t* t_fp_dev,
                          int dtype, void* stream);
 /*
+ * The same with positions as torch indexes a table (the patched forward's eager step): negative ones count from the end; a row
+ * whose position lies outside [-rope_len, rope_len) gets queries and a key that are not numbers, and *refused (device-visible
+ * memory, may be NULL) becomes CQ_ERR_BAD_ARG.
+ */
+int cq_rope_split_append_strict(const void* qkv, int64_t qkv_stride_b, const void* cos_table, const void* sin_table,
+                                int rope_len, const int64_t* position_ids, int batch, int n_kv_heads, int n_rep,
+                                int head_dim, void* q_out, void* k_cache, void* v_cache, int64_t cache_stride_b,
+                                int64_t cache_stride_h, int capacity, int append_index, const int32_t* t_fp_dev,
+                                int dtype, int32_t* refused, void* stream);
+/*
  * cq_linear_small: out [rows, n] = x [rows, k] weight [n, k]^T for up to four rows (more: CQ_ERR_UNSUPPORTED, a matrix product is
  * the better tool); all contiguous and 16-byte aligned, k a multiple of 8; fp32 sums rounded once.
  */
