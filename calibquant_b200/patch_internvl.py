@@ -331,6 +331,8 @@ def forward_internlm2_calibquant(self, hidden_states: torch.Tensor,
         n_rep, wqkv = self.num_key_value_groups, self.wqkv
         tc.reserve(1)
         pos = position_ids if position_ids.numel() == bsz else position_ids.expand(bsz, 1)
+        if pos.dtype is torch.int32 or not pos.is_cuda:      # torch indexes with these as well
+            pos = pos.to(device=hidden_states.device, dtype=torch.int64 if pos.dtype is torch.int32 else pos.dtype)
         n_kv = wqkv.out_features // ((n_rep + 2) * self.head_dim)
         w = _plain_weight(wqkv, hidden_states)
         q = native().rope_split_append(hidden_states if w is not None else wqkv(hidden_states), cos, sin, pos, n_kv, n_rep, tc.k, tc.v,

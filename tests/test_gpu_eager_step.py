@@ -92,3 +92,13 @@ def test_wrapped_projection_is_called(layer, name):
     out, _ = _step(layer, [T, T])
     assert calls == [T, 1]
     assert (out.float() - want.float()).norm() <= 1e-2 * want.float().norm()
+
+
+@pytest.mark.parametrize("dtype,device", [(torch.int32, "cuda"), (torch.int64, "cpu"), (torch.int32, "cpu")])
+def test_positions_of_other_types_and_on_the_host(layer, dtype, device):
+    want, _ = _step(layer, [T, T - 3])
+    with torch.no_grad():
+        x, past = _prompt(layer)
+        pos = torch.tensor([[T], [T - 3]], dtype=dtype, device=device)
+        out, _, _ = layer(x, position_ids=pos, past_key_value=past, use_cache=True)
+    assert torch.equal(out, want)
