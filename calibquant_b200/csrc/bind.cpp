@@ -81,6 +81,18 @@ bool truth(PyObject* o) {
 void need_cuda(const Tensor& t) {
   if (t.defined() && !t.is_cuda()) raise(PyExc_RuntimeError, "calibquant_b200 runs on CUDA tensors only (no CPU fallback)");
 }
+void want_dims(const Tensor& t, int64_t n, const char* what) {
+  if (t.dim() == n) return;
+  PyErr_Format(PyExc_ValueError, "%s must have %lld dimensions, got %lld", what, (long long)n, (long long)t.dim());
+  throw PyRaised();
+}
+// one query row per (batch row, head)
+void want_one_row(const Tensor& q, int64_t D) {
+  if (q.numel() == q.size(0) * q.size(1) * D) return;
+  PyErr_Format(PyExc_RuntimeError, "a decode step takes one query row per head, got %lld elements for %lld rows of %lld",
+               (long long)q.numel(), (long long)(q.size(0) * q.size(1)), (long long)D);
+  throw PyRaised();
+}
 int dtype_enum(const Tensor& t) {
   switch (t.scalar_type()) {
     case at::kHalf: return CQ_DTYPE_F16;
@@ -251,6 +263,7 @@ PyObject* py_quant_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_BEGIN
   want_args(n, 3, "quant_encode");      // x [B,T,H,D], bits, clip factor -> enc [B,H,T,D*bits/8], scale, zero point
   need_cuda(tensor(a[0]));
+  want_dims(tensor(a[0]), 4, "x");
   const Tensor x = with_rows(tensor(a[0]));
   const int64_t bits = integer(a[1]), B = x.size(0), T = x.size(1), H = x.size(2), D = x.size(3);
   const float clip = (float)real(a[2]);
@@ -333,6 +346,7 @@ PyObject* py_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   need_cuda(q_in); need_cuda(k_fp); need_cuda(v_fp); need_cuda(mask);
   if (!k_fp.defined() && !has_k) raise(PyExc_ValueError, "decode_attention needs packed or full-precision keys");
   const Tensor q = contiguous(q_in);
+  want_one_row(q, q.size(-1));
   cq_decode_args d = {};
   d.batch = (int32_t)q.size(0); d.n_q_heads = (int32_t)q.size(1); d.head_dim = (int32_t)q.size(-1);
   d.n_kv_heads = (int32_t)(k_fp.defined() ? k_fp.size(1) : kp[0].size(1));
@@ -387,6 +401,8 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor& q_in = tensor(a[0]);
   const Tensor &k_fp = tensor(a[7]), &v_fp = tensor(a[8]);
   need_cuda(q_in); need_cuda(k_fp); need_cuda(v_fp);
+  want_dims(q_in, 4, "q");
+  want_one_row(q_in, q_in.size(3));
   const Tensor q = contiguous(q_in);
   cq_u8_decode_args d = {};
   const int64_t B = q.size(0), Hq = q.size(1), D = q.size(3), Hkv = k_fp.size(1), t_fp = k_fp.size(2);
@@ -624,6 +640,7 @@ PyObject* py_prefill_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_BEGIN
   want_args(n, 4, "prefill_attention");      // q [B,T,Hq,D], k, v [B,T,Hkv,D], out | None
   for (int i = 0; i < 3; ++i) need_cuda(tensor(a[i]));
+  for (int i = 0; i < 3; ++i) want_dims(tensor(a[i]), 4, "q, k and v");
   const Tensor q = with_rows(tensor(a[0])), k = with_rows(tensor(a[1])), v = with_rows(tensor(a[2]));
   Tensor out = opt_tensor(a[3]);
   Call call(q);
@@ -650,6 +667,7 @@ PyObject* py_qjl_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
   CQ_BEGIN
   want_args(n, 4, "qjl_quant");
   for (int i = 0; i < 3; ++i) need_cuda(tensor(a[i]));
+  want_dims(tensor(a[0]), 5, "key_states");
   const Tensor k = contiguous(tensor(a[0])), idx = contiguous(tensor(a[1])), proj = contiguous(tensor(a[2]));
   const int dt = dtype_enum(k), pdt = proj_enum(proj, k);
   const int64_t B = k.size(0), H = k.size(1), N = k.size(2), G = k.size(3), D = k.size(4), s = proj.size(0), os = integer(a[3]);
@@ -691,6 +709,7 @@ PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
   want_args(n, 8, "qjl_gqa_score");
   for (int i = 0; i < 8; ++i)
     if (a[i] != Py_None) need_cuda(tensor(a[i]));
+  want_dims(tensor(a[0]), 5, "key_quant");
   const Tensor kq = contiguous(tensor(a[0])), koq = contiguous(tensor(a[1])), kn = contiguous(tensor(a[2])), on = contiguous(tensor(a[3]));
   const Tensor idx = contiguous(tensor(a[4])), q = contiguous(tensor(a[6])), proj = contiguous(tensor(a[7]));
   Tensor qs = opt_tensor(a[5]);
