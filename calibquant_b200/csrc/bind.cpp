@@ -521,6 +521,12 @@ PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (t->stride(3) != 1 || t->stride(2) != D)
       raise(PyExc_ValueError, "cache token rows must be contiguous ([.., T, D] with stride D)");
   if (k_cache.strides() != v_cache.strides()) raise(PyExc_ValueError, "k_cache and v_cache must share strides");
+  for (const Tensor* t : {&k_cache, &v_cache})
+    if (t->size(0) < B || t->size(1) < hkv || t->size(2) < k_cache.size(2)) {
+      PyErr_Format(PyExc_ValueError, "a cache of %lld rows and %lld heads does not hold %lld rows and %lld heads", (long long)t->size(0),
+                   (long long)t->size(1), (long long)B, (long long)hkv);
+      throw PyRaised();
+    }
   if ((a[8] == Py_None) == (a[9] == Py_None)) raise(PyExc_ValueError, "give exactly one of append_index and t_fp_dev");
   const Tensor live = opt_tensor(a[9]);
   if (live.defined()) check_counter(live);

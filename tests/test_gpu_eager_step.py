@@ -102,3 +102,22 @@ def test_positions_of_other_types_and_on_the_host(layer, dtype, device):
         pos = torch.tensor([[T], [T - 3]], dtype=dtype, device=device)
         out, _, _ = layer(x, position_ids=pos, past_key_value=past, use_cache=True)
     assert torch.equal(out, want)
+
+
+@torch.no_grad()
+def test_more_rows_than_the_cache_holds(layer):
+    x, past = _prompt(layer)
+    length = layer._text_cache.length
+    with pytest.raises(ValueError, match="does not hold"):
+        layer(torch.cat([x, x]), position_ids=torch.full((2 * B, 1), T, device="cuda"), past_key_value=past, use_cache=True)
+    assert layer._text_cache.length == length
+
+
+def test_append_to_a_smaller_cache():
+    from calibquant_b200 import ops
+    qkv, table = torch.zeros(2, 1, 12 * 128, device="cuda").half(), torch.zeros(2, 9, 128, device="cuda").half()
+    pos = torch.zeros(2, 1, dtype=torch.int64, device="cuda")
+    for shape in ((1, 2, 4, 128), (2, 1, 4, 128)):
+        cache = torch.zeros(2, *shape, device="cuda").half()
+        with pytest.raises(ValueError, match="does not hold"):
+            ops.rope_split_append(qkv, *table, pos, 2, 4, *cache, append_index=0)
