@@ -81,6 +81,11 @@ bool truth(PyObject* o) {
 void need_cuda(const Tensor& t) {
   if (t.defined() && !t.is_cuda()) raise(PyExc_RuntimeError, "calibquant_b200 runs on CUDA tensors only (no CPU fallback)");
 }
+// a number that is divided by (an integer division by zero would end the process)
+int64_t divisor(int64_t v, const char* what) {
+  if (v == 0) { PyErr_Format(PyExc_ZeroDivisionError, "%s is zero", what); throw PyRaised(); }
+  return v;
+}
 void want_dims(const Tensor& t, int64_t n, const char* what) {
   if (t.dim() == n) return;
   PyErr_Format(PyExc_ValueError, "%s must have %lld dimensions, got %lld", what, (long long)n, (long long)t.dim());
@@ -219,7 +224,7 @@ PyObject* py_pack_last_dim(PyObject*, PyObject* const* a, Py_ssize_t n) {
   want_args(n, 3, "pack_last_dim");      // data [B,nh,R,L], group_size, bits
   need_cuda(tensor(a[0]));
   const Tensor x = contiguous(tensor(a[0]));
-  const int64_t g = integer(a[1]), bits = integer(a[2]), B = x.size(0), nh = x.size(1), R = x.size(2), L = x.size(3);
+  const int64_t g = divisor(integer(a[1]), "group_size"), bits = integer(a[2]), B = x.size(0), nh = x.size(1), R = x.size(2), L = x.size(3);
   Call call(x);
   Tensor code = empty({B, nh, R, L * bits / 32}, x, at::kInt), scale = empty({B, nh, R, L / g}, x), mn = empty({B, nh, R, L / g}, x);
   check(cq_pack_last_dim(x.data_ptr(), B * nh * R, L, (int)g, (int)bits, dtype_enum(x), (int32_t*)code.data_ptr(),
@@ -233,7 +238,7 @@ PyObject* py_pack_k_per_channel(PyObject*, PyObject* const* a, Py_ssize_t n) {
   want_args(n, 3, "pack_k_per_channel");      // k [B,H,T,D], group_size, bits
   need_cuda(tensor(a[0]));
   const Tensor k = with_rows(tensor(a[0]));
-  const int64_t g = integer(a[1]), bits = integer(a[2]), B = k.size(0), H = k.size(1), T = k.size(2), D = k.size(3);
+  const int64_t g = divisor(integer(a[1]), "group_size"), bits = integer(a[2]), B = k.size(0), H = k.size(1), T = k.size(2), D = k.size(3);
   Call call(k);
   Tensor code = empty({B, H, D, T * bits / 32}, k, at::kInt), scale = empty({B, H, D, T / g}, k), mn = empty({B, H, D, T / g}, k);
   check(cq_pack_k_per_channel(k.data_ptr(), (int)B, (int)H, T, (int)D, k.stride(0), k.stride(1), k.stride(2), (int)g, (int)bits,
@@ -248,7 +253,7 @@ PyObject* py_pack_v_per_token(PyObject*, PyObject* const* a, Py_ssize_t n) {
   want_args(n, 3, "pack_v_per_token");      // v [B,H,T,D], group_size, bits
   need_cuda(tensor(a[0]));
   const Tensor v = with_rows(tensor(a[0]));
-  const int64_t g = integer(a[1]), bits = integer(a[2]), B = v.size(0), H = v.size(1), T = v.size(2), D = v.size(3);
+  const int64_t g = divisor(integer(a[1]), "group_size"), bits = integer(a[2]), B = v.size(0), H = v.size(1), T = v.size(2), D = v.size(3);
   Call call(v);
   Tensor code = empty({B, H, T, D * bits / 32}, v, at::kInt), scale = empty({B, H, T, D / g}, v), mn = empty({B, H, T, D / g}, v);
   check(cq_pack_v_per_token(v.data_ptr(), (int)B, (int)H, T, (int)D, v.stride(0), v.stride(1), v.stride(2), (int)g, (int)bits,
@@ -291,7 +296,7 @@ PyObject* py_qbmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 1; i < 5; ++i) need_cuda(tensor(a[i]));
   const Tensor fA = contiguous(tensor(a[1])), qB = contiguous(tensor(a[2])), s = contiguous(tensor(a[3])), z = contiguous(tensor(a[4]));
   if (fA.dim() != 4 || qB.dim() != 4) raise(PyExc_AssertionError, "fA and qB must have four dimensions");
-  const int64_t bits = integer(a[5]), B = fA.size(0), Hq = fA.size(1), K = fA.size(3), Hkv = qB.size(1);
+  const int64_t bits = divisor(integer(a[5]), "bits"), B = fA.size(0), Hq = fA.size(1), K = fA.size(3), Hkv = qB.size(1);
   if (fA.size(2) != 1) raise(PyExc_ValueError, "only M == 1 (one query row) is implemented");
   const int64_t N = qB.size(3) * (32 / bits);
   Call call(fA);
@@ -410,7 +415,7 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   need_cuda(enc_k); need_cuda(enc_v);
   d.bits = (int32_t)integer(a[9]);
   Tensor par[4];
-  const int64_t hs = tensor(a[3]).numel() / (B * D);
+  const int64_t hs = tensor(a[3]).numel() / divisor(B * D, "the number of query elements per head");
   for (int i = 0; i < 4; ++i) {
     const Tensor& p = tensor(a[3 + i]);
     if ((hs != Hq && hs != Hkv) || p.numel() != B * hs * D || p.scalar_type() != q.scalar_type())
@@ -724,7 +729,7 @@ PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int dt = dtype_enum(q), pdt = proj_enum(proj, q);
   if (kn.scalar_type() != q.scalar_type() || on.scalar_type() != q.scalar_type())
     raise(PyExc_TypeError, "key norms must have the query dtype");
-  if (Hq % Hkv) raise(PyExc_ValueError, "query heads must be a multiple of key heads");
+  if (Hq % divisor(Hkv, "the number of key heads")) raise(PyExc_ValueError, "query heads must be a multiple of key heads");
   Call call(q);
   Tensor scores = empty({B, Hq, N * G, 1}, q, at::kFloat);
   check(cq_qjl_gqa_score((const uint8_t*)kq.data_ptr(), (const uint8_t*)koq.data_ptr(), kn.data_ptr(), on.data_ptr(),

@@ -45,3 +45,19 @@ def test_other_numbers_of_dimensions():
     bits, norm = torch.zeros(1, 2, 2, 32, 32, 2, dtype=torch.uint8, device="cuda"), _half(1, 2, 2, 32)
     with pytest.raises(ValueError):
         ops.qjl_gqa_score(bits, bits, norm, norm, idx, None, _half(1, 8, 1, 128), proj.t().contiguous())
+
+
+def test_sizes_of_zero_raise():
+    """What Python refused as a division by zero must not end the process."""
+    from calibquant_b200 import calibquant as cq, ops
+    from calibquant_b200._lib import native
+    kp, vp = _packs()
+    fp, idx = _half(0, 2, 8, 128), torch.zeros(1, 0, 2, 8, dtype=torch.uint8, device="cuda")
+    bits, norm = torch.zeros(1, 0, 2, 32, 32, dtype=torch.uint8, device="cuda"), _half(1, 0, 2, 32)
+    calls = [lambda: ops.pack_v_per_token(_half(1, 2, 64, 128), 0, 2), lambda: ops.pack_k_per_channel(_half(1, 2, 64, 128), 0, 2),
+             lambda: ops.pack_last_dim(_half(1, 2, 64, 128), 0, 2), lambda: native().pack_last_dim(_half(1, 2, 64, 128), 0, 2),
+             lambda: ops.qbmm(32, _half(1, 8, 1, 64), *vp, 0), lambda: cq.decode_attention(_half(0, 8, 1, 128), _u8(), fp, fp, 2, 4),
+             lambda: ops.qjl_gqa_score(bits, bits, norm, norm, idx, None, _half(1, 8, 1, 128), torch.randn(128, 256, device="cuda"))]
+    for call in calls:
+        with pytest.raises(ZeroDivisionError):
+            call()
