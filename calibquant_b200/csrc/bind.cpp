@@ -115,6 +115,20 @@ bool rows_ok(const Tensor& t) {
 }
 Tensor with_rows(const Tensor& t) { return rows_ok(t) ? t : t.contiguous(); }
 
+// Other Python threads run while a call of the library is under way: a launch waits where the stream's queue is full, and what
+// it waits for may itself need the interpreter (a host function in the stream, another thread's launches).
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+// No Python object may be touched in `call`: its arguments are plain values and tensors' pointers.
+template <typename F>
+void launch(F&& call, const char* where) {
+  int rc;
+  { Unlocked u; rc = call(); }
+  check(rc, where);
+}
+
 struct Call {            // device and stream of one call
   c10::cuda::OptionalCUDAGuard guard;
   cudaStream_t stream;
@@ -227,8 +241,9 @@ PyObject* py_pack_last_dim(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t g = divisor(integer(a[1]), "group_size"), bits = integer(a[2]), B = x.size(0), nh = x.size(1), R = x.size(2), L = x.size(3);
   Call call(x);
   Tensor code = empty({B, nh, R, L * bits / 32}, x, at::kInt), scale = empty({B, nh, R, L / g}, x), mn = empty({B, nh, R, L / g}, x);
-  check(cq_pack_last_dim(x.data_ptr(), B * nh * R, L, (int)g, (int)bits, dtype_enum(x), (int32_t*)code.data_ptr(),
-                         scale.data_ptr(), mn.data_ptr(), call.stream), "cq_pack_last_dim");
+  const int dt = dtype_enum(x);
+  launch([&] { return cq_pack_last_dim(x.data_ptr(), B * nh * R, L, (int)g, (int)bits, dt, (int32_t*)code.data_ptr(),
+                         scale.data_ptr(), mn.data_ptr(), call.stream); }, "cq_pack_last_dim");
   return wrap3(code, scale, mn);
   CQ_END
 }
@@ -241,9 +256,9 @@ PyObject* py_pack_k_per_channel(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t g = divisor(integer(a[1]), "group_size"), bits = integer(a[2]), B = k.size(0), H = k.size(1), T = k.size(2), D = k.size(3);
   Call call(k);
   Tensor code = empty({B, H, D, T * bits / 32}, k, at::kInt), scale = empty({B, H, D, T / g}, k), mn = empty({B, H, D, T / g}, k);
-  check(cq_pack_k_per_channel(k.data_ptr(), (int)B, (int)H, T, (int)D, k.stride(0), k.stride(1), k.stride(2), (int)g, (int)bits,
-                              dtype_enum(k), (int32_t*)code.data_ptr(), scale.data_ptr(), mn.data_ptr(), call.stream),
-        "cq_pack_k_per_channel");
+  const int dt = dtype_enum(k);
+  launch([&] { return cq_pack_k_per_channel(k.data_ptr(), (int)B, (int)H, T, (int)D, k.stride(0), k.stride(1), k.stride(2), (int)g, (int)bits,
+                              dt, (int32_t*)code.data_ptr(), scale.data_ptr(), mn.data_ptr(), call.stream); }, "cq_pack_k_per_channel");
   return wrap3(code, scale, mn);
   CQ_END
 }
@@ -256,9 +271,9 @@ PyObject* py_pack_v_per_token(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t g = divisor(integer(a[1]), "group_size"), bits = integer(a[2]), B = v.size(0), H = v.size(1), T = v.size(2), D = v.size(3);
   Call call(v);
   Tensor code = empty({B, H, T, D * bits / 32}, v, at::kInt), scale = empty({B, H, T, D / g}, v), mn = empty({B, H, T, D / g}, v);
-  check(cq_pack_v_per_token(v.data_ptr(), (int)B, (int)H, T, (int)D, v.stride(0), v.stride(1), v.stride(2), (int)g, (int)bits,
-                            dtype_enum(v), (int32_t*)code.data_ptr(), scale.data_ptr(), mn.data_ptr(), call.stream),
-        "cq_pack_v_per_token");
+  const int dt = dtype_enum(v);
+  launch([&] { return cq_pack_v_per_token(v.data_ptr(), (int)B, (int)H, T, (int)D, v.stride(0), v.stride(1), v.stride(2), (int)g, (int)bits,
+                            dt, (int32_t*)code.data_ptr(), scale.data_ptr(), mn.data_ptr(), call.stream); }, "cq_pack_v_per_token");
   return wrap3(code, scale, mn);
   CQ_END
 }
@@ -277,14 +292,14 @@ PyObject* py_quant_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Call call(x);
   Tensor s = empty({B, 1, H, D}, x), zp = empty({B, 1, H, D}, x), enc = empty({B, H, T, D * bits / 8}, x, at::kByte);
   if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && st[0] % 8 == 0 && st[1] % 8 == 0 && st[2] % 8 == 0) {
-    check(cq_calib_quant_encode(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, clip, dt, s.data_ptr(), zp.data_ptr(),
-                                (uint8_t*)enc.data_ptr(), call.stream), "cq_calib_quant_encode");
+    launch([&] { return cq_calib_quant_encode(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, clip, dt, s.data_ptr(), zp.data_ptr(),
+                                (uint8_t*)enc.data_ptr(), call.stream); }, "cq_calib_quant_encode");
     return wrap3(enc, s, zp);
   }
-  check(cq_calib_minmax(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, clip, dt, s.data_ptr(), zp.data_ptr(),
-                        call.stream), "cq_calib_minmax");
-  check(cq_calib_quantize(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, dt, s.data_ptr(), zp.data_ptr(), 0,
-                          nullptr, (uint8_t*)enc.data_ptr(), call.stream), "cq_calib_quantize");
+  launch([&] { return cq_calib_minmax(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, clip, dt, s.data_ptr(), zp.data_ptr(),
+                        call.stream); }, "cq_calib_minmax");
+  launch([&] { return cq_calib_quantize(x.data_ptr(), (int)B, (int)T, (int)H, (int)D, st, (int)bits, dt, s.data_ptr(), zp.data_ptr(), 0,
+                          nullptr, (uint8_t*)enc.data_ptr(), call.stream); }, "cq_calib_quantize");
   return wrap3(enc, s, zp);
   CQ_END
 }
@@ -302,8 +317,9 @@ PyObject* py_qbmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Call call(fA);
   Tensor out = empty({B, Hq, 1, N}, fA);
   Tensor ws = workspace((int64_t)cq_qbmm_workspace_bytes((int)B, (int)Hq, K, N), fA.get_device(), call.stream);
-  check(cq_qbmm(fA.data_ptr(), (const int32_t*)qB.data_ptr(), s.data_ptr(), z.data_ptr(), out.data_ptr(), (int)B, (int)Hq, (int)Hkv,
-                K, N, (int)integer(a[0]), (int)bits, dtype_enum(fA), ws.data_ptr(), (size_t)ws.numel(), call.stream), "cq_qbmm");
+  const int group = (int)integer(a[0]), dt = dtype_enum(fA);
+  launch([&] { return cq_qbmm(fA.data_ptr(), (const int32_t*)qB.data_ptr(), s.data_ptr(), z.data_ptr(), out.data_ptr(), (int)B, (int)Hq, (int)Hkv,
+                K, N, group, (int)bits, dt, ws.data_ptr(), (size_t)ws.numel(), call.stream); }, "cq_qbmm");
   return wrap(out);
   CQ_END
 }
@@ -394,7 +410,7 @@ PyObject* py_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check(rc ? rc : CQ_ERR_WORKSPACE, "cq_decode_attn");
   }
   const Tensor ws = workspace((int64_t)nbytes, q.get_device(), call.stream);
-  check(cq_decode_attn(&d, ws.data_ptr(), (size_t)ws.numel(), call.stream), "cq_decode_attn");
+  launch([&] { return cq_decode_attn(&d, ws.data_ptr(), (size_t)ws.numel(), call.stream); }, "cq_decode_attn");
   return wrap(own_out ? out : out.reshape(q_in.sizes()));
   CQ_END
 }
@@ -456,7 +472,7 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (nbytes == 0)
     raise(PyExc_ValueError, "cq_u8_decode_attn rejects this request (sizes, head counts or more than 51200 keys)");
   const Tensor ws = workspace((int64_t)nbytes, q.get_device(), call.stream);
-  check(cq_u8_decode_attn(&d, ws.data_ptr(), (size_t)ws.numel(), call.stream), "cq_u8_decode_attn");
+  launch([&] { return cq_u8_decode_attn(&d, ws.data_ptr(), (size_t)ws.numel(), call.stream); }, "cq_u8_decode_attn");
   return wrap(out);
   CQ_END
 }
@@ -506,7 +522,9 @@ PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (a[10] != Py_None) {
     need_cuda(qkv_in);
     need_cuda(tensor(a[10]));
-    qkv_in = at::mm(qkv_in.view({-1, qkv_in.size(-1)}), tensor(a[10]).t());
+    const Tensor weight = tensor(a[10]);
+    Unlocked u;
+    qkv_in = at::mm(qkv_in.view({-1, qkv_in.size(-1)}), weight.t());
   }
   const Tensor &k_cache = tensor(a[6]), &v_cache = tensor(a[7]);
   for (int i : {0, 1, 2, 3, 6, 7}) need_cuda(i == 0 ? qkv_in : tensor(a[i]));
@@ -538,18 +556,18 @@ PyObject* py_rope_split_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Call call(qkv);
   Tensor q = empty({B, hkv * n_rep, 1, D}, qkv);
   const void* table[2] = {cos.data_ptr(), sin.data_ptr()};
-  const int at = a[8] == Py_None ? 0 : (int)integer(a[8]);
+  const int at = a[8] == Py_None ? 0 : (int)integer(a[8]), dt = dtype_enum(qkv);
   const int32_t* count = live.defined() ? (const int32_t*)live.data_ptr() : nullptr;
   if (truth(a[11])) {
     int32_t* refused = refusal_flag(call.stream, qkv.get_device());
-    check(cq_rope_split_append_strict(qkv.data_ptr(), per_row, table[0], table[1], (int)cos.size(0), (const int64_t*)pos.data_ptr(), (int)B,
+    launch([&] { return cq_rope_split_append_strict(qkv.data_ptr(), per_row, table[0], table[1], (int)cos.size(0), (const int64_t*)pos.data_ptr(), (int)B,
                                       (int)hkv, (int)n_rep, (int)D, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                                      k_cache.stride(0), k_cache.stride(1), (int)k_cache.size(2), at, count, dtype_enum(qkv), refused,
-                                      call.stream), "cq_rope_split_append_strict");
+                                      k_cache.stride(0), k_cache.stride(1), (int)k_cache.size(2), at, count, dt, refused,
+                                      call.stream); }, "cq_rope_split_append_strict");
   } else {
-    check(cq_rope_split_append(qkv.data_ptr(), per_row, table[0], table[1], (int)cos.size(0), (const int64_t*)pos.data_ptr(), (int)B,
+    launch([&] { return cq_rope_split_append(qkv.data_ptr(), per_row, table[0], table[1], (int)cos.size(0), (const int64_t*)pos.data_ptr(), (int)B,
                                (int)hkv, (int)n_rep, (int)D, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0),
-                               k_cache.stride(1), (int)k_cache.size(2), at, count, dtype_enum(qkv), call.stream), "cq_rope_split_append");
+                               k_cache.stride(1), (int)k_cache.size(2), at, count, dt, call.stream); }, "cq_rope_split_append");
   }
   return wrap(q);
   CQ_END
@@ -590,7 +608,8 @@ PyObject* py_linear_small(PyObject*, PyObject* const* a, Py_ssize_t n) {
   std::vector<int64_t> shape = x.sizes().vec();
   shape.back() = w.size(0);
   Tensor out = empty(shape, x);
-  check(cq_linear_small(x.data_ptr(), w.data_ptr(), out.data_ptr(), (int)rows, (int)w.size(0), (int)K, dtype_enum(x), call.stream), "cq_linear_small");
+  const int dt = dtype_enum(x);
+  launch([&] { return cq_linear_small(x.data_ptr(), w.data_ptr(), out.data_ptr(), (int)rows, (int)w.size(0), (int)K, dt, call.stream); }, "cq_linear_small");
   return wrap(out);
   CQ_END
 }
@@ -637,10 +656,11 @@ PyObject* py_prefill_rope_split(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   Call call(qkv);
   Tensor q = empty({B, T, hkv * n_rep, D}, qkv), k = empty({B, T, hkv, D}, qkv);
-  check(cq_prefill_rope_split(qkv.data_ptr(), qkv.stride(0), qkv.stride(1), cos.data_ptr(), sin.data_ptr(), (int)cos.size(0),
+  const int dt = dtype_enum(qkv);
+  launch([&] { return cq_prefill_rope_split(qkv.data_ptr(), qkv.stride(0), qkv.stride(1), cos.data_ptr(), sin.data_ptr(), (int)cos.size(0),
                               pos.defined() ? (const int64_t*)pos.data_ptr() : nullptr, (int)B, (int)T, (int)hkv, (int)n_rep, (int)D,
                               q.data_ptr(), k.data_ptr(), kc.defined() ? kc.data_ptr() : nullptr, vc.defined() ? vc.data_ptr() : nullptr,
-                              sb, sh, (int)cap, (int)vis_start, (int)vis_len, dtype_enum(qkv), call.stream), "cq_prefill_rope_split");
+                              sb, sh, (int)cap, (int)vis_start, (int)vis_len, dt, call.stream); }, "cq_prefill_rope_split");
   // the values stay where the projection put them: a strided view of [B,T,Hkv,n_rep+2,D]
   Tensor v = qkv.view({B, T, hkv, n_rep + 2, D}).select(3, n_rep + 1);
   return wrap3(q, k, v);
@@ -660,8 +680,9 @@ PyObject* py_prefill_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor* all[4] = {&q, &k, &v, &out};
   for (int i = 0; i < 4; ++i)
     for (int j = 0; j < 3; ++j) st[i][j] = all[i]->stride(j);
-  check(cq_prefill_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (int)q.size(0), (int)q.size(1), (int)q.size(2),
-                        (int)k.size(2), (int)q.size(3), st[0], st[1], st[2], st[3], dtype_enum(q), call.stream), "cq_prefill_attn");
+  const int dt = dtype_enum(q);
+  launch([&] { return cq_prefill_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (int)q.size(0), (int)q.size(1), (int)q.size(2),
+                        (int)k.size(2), (int)q.size(3), st[0], st[1], st[2], st[3], dt, call.stream); }, "cq_prefill_attn");
   return wrap(out);
   CQ_END
 }
@@ -686,8 +707,8 @@ PyObject* py_qjl_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
     raise(PyExc_ValueError, "outlier_indices must be uint8 [B,H,n,outlier_count]");
   Call call(k);
   Tensor kq = empty({B, H, N, G, s / 8}, k, at::kByte), koq = empty({B, H, N, G, os / 8}, k, at::kByte), norms = empty({B, H, N, G}, k);
-  check(cq_qjl_quant(k.data_ptr(), (const uint8_t*)idx.data_ptr(), proj.data_ptr(), pdt, B * H * N, (int)G, (int)D, (int)s, (int)os,
-                     (int)idx.size(3), dt, (uint8_t*)kq.data_ptr(), (uint8_t*)koq.data_ptr(), norms.data_ptr(), call.stream), "cq_qjl_quant");
+  launch([&] { return cq_qjl_quant(k.data_ptr(), (const uint8_t*)idx.data_ptr(), proj.data_ptr(), pdt, B * H * N, (int)G, (int)D, (int)s, (int)os,
+                     (int)idx.size(3), dt, (uint8_t*)kq.data_ptr(), (uint8_t*)koq.data_ptr(), norms.data_ptr(), call.stream); }, "cq_qjl_quant");
   return wrap3(kq, koq, norms);
   CQ_END
 }
@@ -703,9 +724,10 @@ PyObject* py_qjl_build(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Call call(k);
   Tensor idx = empty({B, H, N, oc}, k, at::kByte), kq = empty({B, H, N, 32, s / 8}, k, at::kByte);
   Tensor koq = empty({B, H, N, 32, os / 8}, k, at::kByte), onorm = empty({B, H, N, 32}, k), knorm = empty({B, H, N, 32}, k);
-  check(cq_qjl_build(k.data_ptr(), (int)B, (int)H, (int)N, 32, (int)k.size(3), st, proj.data_ptr(), proj_enum(proj, k), (int)s, (int)os,
-                     (int)oc, dtype_enum(k), (uint8_t*)idx.data_ptr(), (uint8_t*)kq.data_ptr(), (uint8_t*)koq.data_ptr(),
-                     knorm.data_ptr(), onorm.data_ptr(), call.stream), "cq_qjl_build");
+  const int dt = dtype_enum(k), pdt = proj_enum(proj, k);
+  launch([&] { return cq_qjl_build(k.data_ptr(), (int)B, (int)H, (int)N, 32, (int)k.size(3), st, proj.data_ptr(), pdt, (int)s, (int)os,
+                     (int)oc, dt, (uint8_t*)idx.data_ptr(), (uint8_t*)kq.data_ptr(), (uint8_t*)koq.data_ptr(),
+                     knorm.data_ptr(), onorm.data_ptr(), call.stream); }, "cq_qjl_build");
   PyObject* tup = PyTuple_New(5);
   if (!tup) throw PyRaised();
   const Tensor all[5] = {idx, kq, koq, onorm, knorm};
@@ -732,10 +754,10 @@ PyObject* py_qjl_gqa_score(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (Hq % divisor(Hkv, "the number of key heads")) raise(PyExc_ValueError, "query heads must be a multiple of key heads");
   Call call(q);
   Tensor scores = empty({B, Hq, N * G, 1}, q, at::kFloat);
-  check(cq_qjl_gqa_score((const uint8_t*)kq.data_ptr(), (const uint8_t*)koq.data_ptr(), kn.data_ptr(), on.data_ptr(),
+  launch([&] { return cq_qjl_gqa_score((const uint8_t*)kq.data_ptr(), (const uint8_t*)koq.data_ptr(), kn.data_ptr(), on.data_ptr(),
                          (const uint8_t*)idx.data_ptr(), qs.defined() ? (const float*)qs.data_ptr() : nullptr, q.data_ptr(),
                          proj.data_ptr(), pdt, (int)B, (int)Hkv, (int)(Hq / Hkv), (int)N, (int)G, (int)D, (int)kq.size(4) * 8,
-                         (int)koq.size(4) * 8, (int)idx.size(3), dt, (float*)scores.data_ptr(), call.stream), "cq_qjl_gqa_score");
+                         (int)koq.size(4) * 8, (int)idx.size(3), dt, (float*)scores.data_ptr(), call.stream); }, "cq_qjl_gqa_score");
   return wrap(scores);
   CQ_END
 }
