@@ -467,7 +467,10 @@ PyObject* py_u8_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (t_fp) { d.k_fp = k_fp.data_ptr(); d.v_fp = v_fp.data_ptr(); }
   d.fp_stride_b = k_fp.stride(0); d.fp_stride_h = k_fp.stride(1);
   d.out = out.data_ptr();
-  if (live.defined()) { check_counter(live); d.t_fp_dev = (const int32_t*)live.data_ptr(); }
+  if (live.defined()) {      // the low word of an int64 counter serves as well
+    if (live.scalar_type() != at::kLong || !live.is_cuda()) check_counter(live);
+    d.t_fp_dev = (const int32_t*)live.data_ptr();
+  }
   const size_t nbytes = cq_u8_decode_attn_workspace_bytes(&d);
   if (nbytes == 0)
     raise(PyExc_ValueError, "cq_u8_decode_attn rejects this request (sizes, head counts or more than 51200 keys)");

@@ -35,3 +35,11 @@ def test_step_sees_the_count_of_the_launch_before(fmt, B, t_vis):
     for i, out in enumerate(outs):      # e^-4 of the probability is left to the others
         newest = v_fp[:, :, 16 + i].repeat_interleave(rep, 1).float()
         assert (out[:, :, 0].float() - newest).norm() <= 0.1 * newest.norm()
+
+
+def test_uint8_step_takes_an_int64_count():
+    from calibquant_b200 import calibquant as cq
+    q, state, k_fp, v_fp = _step_inputs(2, 1, 8, 2, 8, 64, 24, torch.float16, seed=4)
+    args = q.cuda(), {n: t.cuda() for n, t in state.items()}, k_fp.cuda(), v_fp.cuda(), 2, 8
+    want, got = (cq.decode_attention(*args, t_fp_dev=torch.tensor([20], dtype=t, device="cuda")) for t in (torch.int32, torch.int64))
+    assert torch.equal(got, want)
