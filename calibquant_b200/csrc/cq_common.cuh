@@ -70,6 +70,13 @@ inline int check_launch() {
   return e == cudaSuccess ? CQ_OK : CQ_ERR_LAUNCH;
 }
 
+inline int sm_count() {      // of the current device
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
+  return v;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }

@@ -761,36 +761,62 @@ struct Plan { int S, pitch, smem; };
 constexpr int STATIC_SMEM = 9 * 1024;           // upper bound of the kernel's static shared memory
 constexpr int SMEM_TWO = 113 * 1024 - STATIC_SMEM;
 
-// The largest cluster with which the whole grid is resident at once, two CTAs per SM (one per SM, where the logits leave
-// no room for two, has half the warps and loses: 81 us against 71 at 8 x 8 x 32768 tokens).
-// A CTA spends ~16k cycles outside its loops (fill of the ring, exchanges, reductions), so grids of several rounds lose to
-// the separate launches of cq_decode_mma.cu: 16 x 8 KV heads x 3328 tokens at 1 bit take 40 / 24.8 / 33 / 55 us with
-// clusters of 1 / 2 / 4 / 8 (256 CTAs fit), 4 x 8 x 5120 tokens at 4 bits 50 / 28.8 / 23.8 / 17.8 us.
+// Estimates in microseconds, fitted to steps timed both ways and with every cluster size (7376 shapes: batch 1-64, 32 to 32768
+// visual and up to 1000 full-precision tokens, 1 to 8 query heads, all bit widths; they hold to about a tenth).
+struct Cost {
+  double unit, unit_ragged;      // a CTA's time per 256 visual tokens
+  double split, split_ragged;    // the separate launches', per 256 tokens of a KV head and SM
+};
+inline Cost cost_of(int bits) {
+  return bits == 1 ? Cost{1.15, 1.8, 1.1, 1.6} : bits == 2 ? Cost{1.5, 2.1, 1.27, 2.05} : Cost{1.95, 3.2, 1.53, 2.6};
+}
+
+// One launch, with which cluster, or the separate launches of cq_decode_mma.cu.
+//   * All clusters resident at once: whatever the estimates say, over the cluster sizes whose logits fit and whose CTAs all have
+//     a visual unit or 64 full-precision tokens.  (256 visual and 1000 text tokens in one CTA per KV head take 37 us, in
+//     clusters of eight 12.6, in separate launches 13.8; 20 x 8 x 5152 at 4 bits fit clusters of one only: 127 against 73.)
+//     A grid of at most a CTA per SM has half the warps: it stops paying at eight units a CTA, at 4 bits four (2 x 8 x 18432 tokens
+//     at 1 bit 30.9 us against 28.7; 2 x 8 x 9216 at 4 bits 20.5 against 15.2).  The estimate has to win by 4 %, so that ties stay
+//     where the step does not depend on its neighbours' tails.
+//   * More pairs than that, 1 and 2 bits, clusters of one or two with up to 16 units and three chunks a CTA: several rounds,
+//     where the last one is at least 0.85 full and there are at most four, or where the second of two is a quarter to a half
+//     full, when its CTAs have an SM each (294 shapes timed: 0.95 of the separate launches' time, 26 of them slower by more than
+//     3 %; 64 x 8 x 6656 at 2 bits and six heads 169 against 179; 80 x 8 x 3328, 2.16 rounds, would take 111 against 107).
 inline bool make_plan(const cq_decode_args* a, Plan* p) {
   const int n_rep = a->n_q_heads / a->n_kv_heads, n_units = (a->t_vis + UNIT_TOK - 1) / UNIT_TOK;
+  const int fp_chunks = (a->t_fp + FPC - 1) / FPC, most = n_units > (a->t_fp + 63) / 64 ? n_units : (a->t_fp + 63) / 64;
   const int64_t pairs = (int64_t)a->batch * a->n_kv_heads;
   const int sms = sm_count();
-  for (int S = MAX_CLUSTER; S >= 1; S /= 2) {
-    // clusters of eight that fill at most one CTA per SM: up to eight units each (2 x 8 x 18432 tokens: 30.9 us against
-    // 28.7 with the separate launches, which then have twice the warps)
-    if (S > n_units || (pairs * S <= sms && n_units > 8 * S)) continue;
-    const int pitch = (n_units + S - 1) / S * UNIT_TOK + 8;
+  const bool ragged = a->t_vis % UNIT_TOK != 0;
+  const Cost c = cost_of(a->bits);
+  const double heads = n_rep > 4 ? 1.2 : 1.0, load = (double)pairs * n_units / sms;
+  const auto units_of = [&](int S) { return (n_units + S - 1) / S; };
+  const auto chunks_of = [&](int S) { return (((a->t_fp + 15) / 16 + S - 1) / S + 7) / 8; };      // 16-token tiles are dealt out
+  const auto fits = [&](int S, Plan* q) {
+    const int pitch = units_of(S) * UNIT_TOK + 8;
     const int64_t smem = 1024 + ring_bytes(a->bits) + (int64_t)n_rep * pitch * 2;
-    if (smem <= SMEM_TWO && pairs <= max_clusters(S)) { p->S = S; p->pitch = pitch; p->smem = (int)smem; return true; }
-  }
-  // More pairs than resident clusters: several rounds of the smallest cluster whose logits fit, where the last round is not mostly
-  // empty, or a CTA has enough units for it to matter less.  Against the separate launches (us): 64 x 8 x 4096 tokens, S = 1, 1.73
-  // rounds 79.5 / 88.1; 64 x 8 x 1024 x 6 heads 41.3 / 43.7; 32 x 8 x 8192, S = 2, 1.73 rounds 75.8 / 86.0; 24 x 8 x 6656,
-  // 1.30 rounds of 13 units 56.7 / 60.8; but 40 x 8 x 3328, 1.08 rounds 59.1 / 56.7; and at 4 bits 48 x 8 x 5120 112 / 106
-  if (a->bits > 2) return false;
-  for (int S = 1; S <= 4; S *= 2) {
-    const int units = (n_units + S - 1) / S, pitch = units * UNIT_TOK + 8;
-    const int64_t smem = 1024 + ring_bytes(a->bits) + (int64_t)n_rep * pitch * 2, fit = max_clusters(S);
-    if (S > n_units || smem > SMEM_TWO) continue;
-    const int64_t full = (pairs + fit - 1) / fit * fit;      // clusters the rounds have room for
-    if (pairs * 5 < full * 4 && (pairs * 64 < full * 41 || units < 12)) return false;
-    p->S = S; p->pitch = pitch; p->smem = (int)smem;
+    if (smem > SMEM_TWO) return false;
+    q->S = S; q->pitch = pitch; q->smem = (int)smem;
     return true;
+  };
+  double best = 14.5 + (ragged ? 2.5 + c.split_ragged * heads * load : c.split * heads * load) + (a->t_fp ? 3.4 : 0.0) + 2.18 * pairs * fp_chunks / sms +
+                0.13 * pairs * n_rep / sms - (load < 4.0 ? 4.4 - 1.1 * load : 0.0);
+  bool resident = false, found = false;
+  Plan q;
+  for (int S = 1; S <= MAX_CLUSTER; S *= 2) {
+    if (S > most || !fits(S, &q) || pairs > max_clusters(S)) continue;
+    resident = true;
+    const bool two = pairs * S > sms;
+    if (!two && units_of(S) > (a->bits == 4 ? 4 : 8)) continue;
+    const double t = 7.0 + (two ? 1.55 : 1.0) * ((ragged ? c.unit_ragged : c.unit) * heads * units_of(S) + chunks_of(S) * (2.2 + 0.22 * n_rep));
+    if (t * 1.04 < best) { best = t * 1.04; *p = q; found = true; }
+  }
+  if (resident || a->bits > 2 || ragged) return found;
+  for (int S = 1; S <= 2; S *= 2) {
+    if (S > n_units || !fits(S, p)) continue;
+    const int64_t fit = max_clusters(S), rounds = (pairs + fit - 1) / fit;
+    return units_of(S) <= 16 && chunks_of(S) <= 3 &&
+           ((rounds <= 4 && pairs * 20 >= rounds * fit * 17) || (pairs * 4 >= fit * 5 && pairs * 2 <= fit * 3));
   }
   return false;
 }

@@ -184,13 +184,6 @@ inline bool make_v_map(CUtensorMap* tm_v, const void* code, uint64_t tokens) {
                   BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, 4 * BITS, 256);
 }
 
-inline int sm_count() {      // of the current device
-  int dev = 0, v = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
-  return v;
-}
-
 // Launch with the programmatic-stream-serialization attribute: the kernel may begin (up to its pdl_wait())
 // while the previous kernel of the stream drains.
 template <typename... KArgs, typename... Args>
