@@ -198,13 +198,19 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
   }
 }
 
+// The smallest cluster that puts two CTAs on every SM, as long as a CTA has 64 tokens (two rounds of its threads)
+static int cluster_of(int64_t bh, int t_len) {
+  const int sms = sm_count();
+  int S = 1;
+  while (S < MAX_S && bh * S < 2 * sms && t_len >= 128 * S) S *= 2;
+  return S;
+}
+
 template <typename T, int BITS>
 static int launch_quant_encode(const void* x, int batch, int t_len, int heads, const int64_t* strides, float clip, void* scale, void* zp,
                                uint8_t* enc, cudaStream_t st) {
-  // The smallest cluster that puts two CTAs on every SM, as long as a CTA has 64 tokens (two rounds of its threads)
   const int64_t bh = (int64_t)batch * heads;
-  int S = 1;
-  while (S < MAX_S && bh * S < 2 * 148 && t_len >= 128 * S) S *= 2;
+  const int S = cluster_of(bh, t_len);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(bh * S));
   cfg.blockDim = dim3(QE_THREADS);
@@ -236,6 +242,14 @@ extern "C" int cq_calib_quant_encode(const void* x, int batch, int t_len, int he
   if (!aligned16(x) || strides[0] % 8 || strides[1] % 8 || strides[2] % 8 || reinterpret_cast<uintptr_t>(enc_out) % 4) return CQ_ERR_BAD_ARG;
   if ((int64_t)batch * heads > 0x0fffffff) return CQ_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // Few (batch, head) pairs with long spans at 4 bits: a quotient per element, on clusters that fill less than the GPU.  The separate
+  // launches deal tokens over all SMs (1 x 16384, one head 43 us against 63; 2 x 16384 x 8 84 against 109; 2 x 3328 x 8, 416
+  // tokens a CTA, 37 against 29; 8 x 16384 x 8, two CTAs on every SM, 298 against 260)
+  const int64_t ctas = (int64_t)batch * heads * calib::cluster_of((int64_t)batch * heads, t_len);
+  if (bits == 4 && ctas < 2 * cq::sm_count() && t_len > 1024 * calib::cluster_of((int64_t)batch * heads, t_len)) {
+    const int rc = cq_calib_minmax(x, batch, t_len, heads, head_dim, strides, bits, clip, dtype, scale, zero_point, stream);
+    return rc ? rc : cq_calib_quantize(x, batch, t_len, heads, head_dim, strides, bits, dtype, scale, zero_point, 0, nullptr, enc_out, stream);
+  }
 #define CQ_QE(T, B) calib::launch_quant_encode<T, B>(x, batch, t_len, heads, strides, clip, scale, zero_point, enc_out, st)
   if (dtype == CQ_DTYPE_F16) return bits == 1 ? CQ_QE(__half, 1) : bits == 2 ? CQ_QE(__half, 2) : CQ_QE(__half, 4);
   return bits == 1 ? CQ_QE(__nv_bfloat16, 1) : bits == 2 ? CQ_QE(__nv_bfloat16, 2) : CQ_QE(__nv_bfloat16, 4);

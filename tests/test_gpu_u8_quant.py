@@ -30,3 +30,14 @@ def test_quant_encode(dtype, bits, clip, B, T, H, constant):
     assert T == 1 or constant or bool(good.all())
     mine = cqf.decode_bytes(enc.cpu(), bits).transpose(1, 2)
     assert torch.equal(mine[good].to(torch.int64), ref[good].to(torch.int64))
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 8300, 1), (2, 9001, 2), (1, 8192, 8)])
+def test_long_spans_of_few_heads_at_four_bits(B, T, H):
+    """Spans that the separate launches take: bytes, scales and zero points of the oracle."""
+    from calibquant_b200 import calibquant as cq
+    x = torch.randn(B, T, H, 128, generator=torch.Generator().manual_seed(T)).half()
+    codes, s, z = cqf.quant(x, 4, per_channel=True, post_scale=True)
+    enc, s_out, z_out = (t.cpu() for t in cq.quant_encode(x.cuda(), 4))
+    assert torch.equal(enc, cqf.encode(codes.transpose(1, 2), 4, 2))
+    assert torch.equal(s_out, s) and torch.equal(z_out, z)
