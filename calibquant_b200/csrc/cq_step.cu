@@ -196,19 +196,10 @@ prefill_rope_split_kernel(const T* __restrict__ qkv, int64_t stride_b, int64_t s
   T* k_dst = k_out + (bt * n_kv_heads + hk0) * kHeadDim + 8 * c;
   const int64_t cache_row = b * cache_stride_b + hk0 * cache_stride_h + (int64_t)fp_idx * kHeadDim + 8 * c;
 
-  int64_t pos = position_ids ? position_ids[bt] : t;
-  pos = pos < 0 ? 0 : (pos >= rope_len ? rope_len - 1 : pos);
-  const T* cr = cos_t + pos * kHeadDim + 8 * c;
-  const T* sr = sin_t + pos * kHeadDim + 8 * c;
-  const uint4 c_lo = *reinterpret_cast<const uint4*>(cr), c_hi = *reinterpret_cast<const uint4*>(cr + 64);
-  const uint4 s_lo = *reinterpret_cast<const uint4*>(sr), s_hi = *reinterpret_cast<const uint4*>(sr + 64);
-  const T* cl = reinterpret_cast<const T*>(&c_lo); const T* chh = reinterpret_cast<const T*>(&c_hi);
-  const T* sl = reinterpret_cast<const T*>(&s_lo); const T* sh = reinterpret_cast<const T*>(&s_hi);
-
   const int rows = n_heads * (n_rep + 1);             // rotated rows: the queries of a head, then its key
-  for (int r0 = lane >> 3; r0 < rows; r0 += 4 * U) {
-    uint4 lo[U], hi[U];
-    int hk[U], slot[U];
+  uint4 lo[U], hi[U];
+  int hk[U], slot[U];
+  auto load = [&](int r0) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int r = r0 + 4 * u;
@@ -220,6 +211,20 @@ prefill_rope_split_kernel(const T* __restrict__ qkv, int64_t stride_b, int64_t s
         hi[u] = *reinterpret_cast<const uint4*>(x + 64);
       }
     }
+  };
+  // the first rows are on their way while the position, and then its angles, are fetched
+  int64_t pos = position_ids ? position_ids[bt] : t;
+  load(lane >> 3);
+  pos = pos < 0 ? 0 : (pos >= rope_len ? rope_len - 1 : pos);
+  const T* cr = cos_t + pos * kHeadDim + 8 * c;
+  const T* sr = sin_t + pos * kHeadDim + 8 * c;
+  const uint4 c_lo = *reinterpret_cast<const uint4*>(cr), c_hi = *reinterpret_cast<const uint4*>(cr + 64);
+  const uint4 s_lo = *reinterpret_cast<const uint4*>(sr), s_hi = *reinterpret_cast<const uint4*>(sr + 64);
+  const T* cl = reinterpret_cast<const T*>(&c_lo); const T* chh = reinterpret_cast<const T*>(&c_hi);
+  const T* sl = reinterpret_cast<const T*>(&s_lo); const T* sh = reinterpret_cast<const T*>(&s_hi);
+
+  for (int r0 = lane >> 3; r0 < rows; r0 += 4 * U) {
+    if (r0 >= 4 * U) load(r0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (r0 + 4 * u >= rows) break;
@@ -387,7 +392,8 @@ extern "C" int cq_prefill_rope_split(const void* qkv, int64_t qkv_stride_b, int6
   // so that the last round is a small part (2 x 1401 tokens in rounds of 1.2: 17.8 us; of 4.7: 17.2)
   const int64_t n_tokens = (int64_t)batch * t_len;
   int parts = 1;
-  while (parts < n_kv_heads && parts < 32768 && n_tokens * parts < 4 * 148 * 16) parts *= 2;
+  const int64_t at_once = (int64_t)sm_count() * 16;
+  while (parts < n_kv_heads && parts < 32768 && n_tokens * parts < 4 * at_once) parts *= 2;
   parts = parts < n_kv_heads ? parts : n_kv_heads;
   const int heads_per = (n_kv_heads + parts - 1) / parts;
   if ((n_tokens + 7) / 8 > 0x7fffffff) return CQ_ERR_UNSUPPORTED;
