@@ -783,7 +783,9 @@ extern "C" int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_out
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return CQ_ERR_LAUNCH;
   const int64_t items = (int64_t)batch * n_kv_heads * n_groups * ((group_size + 31) / 32);
-  const unsigned grid_mma = (unsigned)((items + qjl::SW - 1) / qjl::SW < sms ? (items + qjl::SW - 1) / qjl::SW : sms);
+  // a CTA per 16 items, or per KV head where a head has fewer: a CTA goes from head to head behind barriers
+  const int64_t per_head = (int64_t)n_groups * ((group_size + 31) / 32), per_cta = per_head < qjl::SW ? per_head : qjl::SW;
+  const unsigned grid_mma = (unsigned)((items + per_cta - 1) / per_cta < sms ? (items + per_cta - 1) / per_cta : sms);
   const dim3 grid((unsigned)(batch * n_kv_heads), (unsigned)n_groups, (unsigned)((group_size + 31) / 32));
 #define CQ_QJL_ARGS(T, TP) key_quant, key_outlier_quant, static_cast<const T*>(key_norm), static_cast<const T*>(key_outlier_norm), \
       outlier_indices, query_sketch, static_cast<const T*>(query), static_cast<const TP*>(proj_score), scores
