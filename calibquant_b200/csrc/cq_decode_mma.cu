@@ -1317,7 +1317,10 @@ static int qbmm_run_t(int kind, const mma::Dims& d_in, const void* fA, const int
   float2* ml = reinterpret_cast<float2*>(ws + 256);
   const size_t rows = (size_t)d.batch * d.hq;
   float* partial = reinterpret_cast<float*>(ws + 256 + align_up(rows * (size_t)d.n_slots * sizeof(float2), 256));
-  auto launch_k2 = [&](auto k2, int smem2) -> int {
+  auto launch_k2 = [&](auto tile) -> int {      // its statics are the tile's own
+    constexpr int VT = decltype(tile)::value;
+    auto k2 = k2_attn_v<T, BITS, VT>;
+    const int smem2 = k2_smem_bytes(BITS, VT);
     static bool configured[64] = {};
     static int occ[64];
     static std::mutex mu;
@@ -1336,9 +1339,9 @@ static int qbmm_run_t(int kind, const mma::Dims& d_in, const void* fA, const int
   };
   int rc;
   if (d.chunk_tok == VT_LARGE)
-    rc = launch_k2(k2_attn_v<T, BITS, VT_LARGE>, k2_smem_bytes(BITS, VT_LARGE));
+    rc = launch_k2(std::integral_constant<int, VT_LARGE>{});
   else
-    rc = launch_k2(k2_attn_v<T, BITS, VT_SMALL>, k2_smem_bytes(BITS, VT_SMALL));
+    rc = launch_k2(std::integral_constant<int, VT_SMALL>{});
   if (rc != CQ_OK) return rc;
   if (d.n_slots >= 16)
     k3_combine<T, 4><<<d.batch * d.hq, kHeadDim * 4, 0, st>>>(d, partial, ml, static_cast<T*>(out));
