@@ -47,7 +47,6 @@ void want_args(Py_ssize_t got, Py_ssize_t want, const char* where) {
   if (got != want) { PyErr_Format(PyExc_TypeError, "%s takes %zd arguments, got %zd", where, want, got); throw PyRaised(); }
 }
 
-bool is_tensor(PyObject* o) { return THPVariable_Check(o); }
 const Tensor& tensor(PyObject* o) {
   if (!THPVariable_Check(o)) raise(PyExc_TypeError, "expected a torch.Tensor");
   return THPVariable_Unpack(o);

@@ -18,7 +18,8 @@ size_t mma_path_workspace_bytes(const cq_decode_args* args);
 int mma_path_run(const cq_decode_args* args, void* workspace, cudaStream_t stream, cudaEvent_t* events = nullptr,
                  int* status_word = nullptr);
 
-// The whole step in one launch (cq_decode_cluster.cu): spans whose logits fit the shared memory of a cluster.
+// The whole step in one launch (cq_decode_cluster.cu): spans whose logits fit the shared memory of a cluster, where that
+// is the faster form.
 bool cluster_path_eligible(const cq_decode_args* args);
 int cluster_path_run(const cq_decode_args* args, void* workspace, cudaStream_t stream, int* status_word = nullptr);
 

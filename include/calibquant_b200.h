@@ -179,8 +179,9 @@ typedef struct cq_decode_args {
 
 /*
  * Stream semantics: everything the call enqueues is ordered after the work already in `stream` and before
- * anything enqueued in it afterwards.  A step whose logits fit the shared memory of the clusters that are resident
- * together (one cluster of up to 8 CTAs per KV head) is ONE launch.  Larger ones take three, and with full-precision
+ * anything enqueued in it afterwards; it may directly follow the launch that packed its operands.  A step whose logits fit the
+ * shared memory of one cluster of up to 8 CTAs per KV head is ONE launch where that is the faster form (a rule on the sizes;
+ * cq_decode_attn_workspace_bytes is 256 then).  Others take three, and with full-precision
  * tokens present the tensor-core path then runs their launch
  * on an internal side stream (one per host thread and device, created on first use) between two events recorded
  * in `stream` and in the side stream; under stream capture this records two parallel branches that join before the
@@ -258,7 +259,7 @@ int cq_calib_minmax(const void* x, int batch, int t_len, int heads, int head_dim
                     int bits, float clip, int dtype, void* scale, void* zero_point, void* stream);
 
 /*
- * cq_calib_quant_encode: cq_calib_minmax followed by cq_calib_quantize with enc_out, as one launch (a thread-block cluster per
+ * cq_calib_quant_encode: cq_calib_minmax followed by cq_calib_quantize with enc_out, as one launch (long spans of few heads at 4 bits: the launches of both; a thread-block cluster per
  * (batch, head)).  enc_out 4-byte aligned; the results are the same.
  */
 int cq_calib_quant_encode(const void* x, int batch, int t_len, int heads, int head_dim, const int64_t* strides, int bits, float clip,
