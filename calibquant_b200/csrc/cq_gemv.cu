@@ -3,7 +3,8 @@
 // (3.8 TB/s) and 12 us of host time to issue, more than its share of the GPU; this takes 7.1 us.
 //   * A warp owns one row of W, its lanes 16-byte pieces in turn, four loads in flight; x comes from L1.  All warps of the sizes
 //     in use are resident at once: nothing is split along K, nothing is exchanged.
-// More than four rows: the multiplications begin to cost as much as the reading, and a matrix product takes over.
+// More than four rows: the multiplications begin to cost as much as the reading, and a matrix product takes over; at the tensor level also
+// for rows of more than 4096 elements (14336 -> 4096, one row: 31.8 us against 26.5), where a warp's chain of loads is the longer.
 // (The projection to queries, keys and values stays with the matrix product: a rounding of a query or key that falls the other
 // way moves the extreme logits, and with them the calibration of a whole row, by more than the data type's precision.)
 #include "cq_common.cuh"
