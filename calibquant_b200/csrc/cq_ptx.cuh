@@ -62,6 +62,25 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// The same with a hint that lets the hardware suspend the thread for up to 16 us a poll, and an end after about a second of
+// such polls.  For kernels whose roles wait for one another most of the time, so that the polls take fewer issue slots from the working
+// warps (QJL score estimate).
+__device__ __forceinline__ bool mbar_wait_suspended(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < (1u << 16); ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(16384u)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
 // Bounded wait for the hand-offs on a kernel's critical path: polls back to back (try_wait itself
 // suspends the thread for a hardware-defined interval, so this is not a hot spin) and gives up after
 // `max_cycles` of the SM clock.

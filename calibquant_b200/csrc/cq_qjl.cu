@@ -10,8 +10,9 @@
 // quant_kernel and score_kernel are CUDA-core kernels: one CTA per (group, chunk of 32 tokens); thread =
 // (token, block of 32 projections); the sign sums run over "bit set" terms only:
 // sum_p sgn_p x_p = 2 sum_{bit_p} x_p - sum_p x_p.  They serve unaligned buffers, sketch dims that are not multiples of
-// 128 and, for the quantizer, other groups than 32 keys; otherwise the quantizer of cq_qjl_build.cu (tcgen05) and
-// score_rows_kernel (outlier projection and sign sums on the warp MMA, a group per warp) run.
+// 128 and, for the quantizer, other groups than 32 keys; otherwise the tcgen05 kernels of cq_qjl_build.cu (quantizer) and
+// cq_qjl_score.cu (groups of 32 keys, 256 projections, up to four query heads per KV head), or score_rows_kernel (outlier
+// projection and sign sums on the warp MMA, a group per warp) run.
 #include <type_traits>
 
 #include "cq_common.cuh"
@@ -24,6 +25,11 @@ bool eligible(const void* keys, int group_size, int head_dim, int sketch, int o_
 int run(const void* keys, int batch, int heads, int n_groups, const int64_t* strides, const uint8_t* given, const void* proj, int proj_dtype,
         int o_sketch, int oc, int dtype, uint8_t* idx, uint8_t* kq, uint8_t* koq, void* knorm, void* onorm, cudaStream_t st);
 }  // namespace qjl_build
+namespace qjl_score {      // cq_qjl_score.cu: groups of 32 keys, 256 projections, up to four query heads per KV head
+bool eligible(const uint8_t* kq, const uint8_t* koq, int group_size, int sketch, int o_sketch, int n_rep);
+int run(const uint8_t* kq, const uint8_t* koq, const void* kn, const void* kon, const uint8_t* idx, const float* qs, const void* q,
+        const void* proj, int proj_dtype, int n_kbh, int n_rep, int n_groups, int o_sketch, int oc, int dtype, float* scores, cudaStream_t st);
+}  // namespace qjl_score
 namespace qjl {
 
 constexpr int WARPS = 8, THREADS = WARPS * 32;
@@ -208,7 +214,8 @@ score_kernel(const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ 
   }
 }
 
-// The same estimate on the warp MMA (sketch dims that are multiples of 128), persistent: one CTA of 16 warps per SM keeps
+// The same estimate on the warp MMA (sketch dims that are multiples of 128; other groups, sketches and head counts than those of
+// cq_qjl_score.cu), persistent: one CTA of 16 warps per SM keeps
 // the projection in shared memory as fp16 hi/lo rows (hi = fp16(x), lo = fp16(x - hi): fp32-exact sums), every warp works
 // off (group, 32 tokens) items by itself, without a CTA barrier.
 //
@@ -779,6 +786,10 @@ extern "C" int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_out
   // sketch rows that are whole 16-byte words: the persistent tensor-core kernel, one CTA per SM
   const bool use_mma = sketch_dim % 128 == 0 && outlier_sketch_dim % 128 == 0 && qjl::mma_ptrs_ok(key_quant, key_outlier_quant) && aligned16(proj_score);
   if (!query_sketch && !use_mma) return CQ_ERR_UNSUPPORTED;
+  // 8 x 8 x 16384 keys, four heads: 129 us on the warp MMA, 87 here; 1 x 8 x 512 15.1 and 10.2, 1 x 8 x 8192 16.2 and 15.9
+  if (use_mma && qjl_score::eligible(key_quant, key_outlier_quant, group_size, sketch_dim, outlier_sketch_dim, n_rep))
+    return qjl_score::run(key_quant, key_outlier_quant, key_norm, key_outlier_norm, outlier_indices, query_sketch, query, proj_score, proj_dtype,
+                          batch * n_kv_heads, n_rep, n_groups, outlier_sketch_dim, outlier_count, dtype, scores, st);
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return CQ_ERR_LAUNCH;

@@ -21,6 +21,9 @@
 #include "cq_tc.cuh"
 
 namespace cq {
+namespace qjl_score {      // cq_qjl_score.cu
+int status();
+}
 namespace qjl_build {
 
 using namespace ptx;
@@ -407,7 +410,7 @@ int run(const void* keys, int batch, int heads, int n_groups, const int64_t* str
 extern "C" int cq_qjl_status(void) {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, cq::qjl_build::g_status, sizeof(int)) != cudaSuccess) return CQ_ERR_LAUNCH;
-  return v;
+  return v != 0 ? v : cq::qjl_score::status();
 }
 
 extern "C" int cq_qjl_build(const void* keys, int batch, int heads, int n_groups, int group_size, int head_dim, const int64_t* strides,

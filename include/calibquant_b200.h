@@ -469,7 +469,7 @@ int cq_comm_allreduce_add_rmsnorm(const void* src, void* const* peer_buffers, in
  *   outlier_indices   uint8 [batch][heads][n_groups][outlier_count], largest norm first
  *   key_norms, outlier_norms  [batch][heads][n_groups][32] in `dtype`; the sketches as above
  *   group_size 32 and sketch_dim 256 only (CQ_ERR_UNSUPPORTED otherwise).
- * cq_qjl_status: sticky device status of the sketching kernel, as cq_prefill_status.
+ * cq_qjl_status: sticky device status of the tcgen05 sketching and score kernels, as cq_prefill_status.
  *
  * cq_qjl_gqa_score replaces qjl/qjl_kernel.py:52-72 `qjl_gqa_score` -> `calc_gqa_score_kernel`
  * (qjl/csrc/qjl_gqa_score_kernel.cu:40-180), for any n_rep <= 8 (the reference's shared arrays hold 4):
