@@ -256,6 +256,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   // 23.2, 24.0; 64 x 8 x 6656 164.5, 169.0.  (Requested into L2 ahead of the wait 16 x 8 x 3328 took 33.0: a bulk prefetch costs
   // its thread as much as the load.)
   pdl_wait();
+  const int t_live = a.t_fp_dev ? *reinterpret_cast<const volatile int32_t*>(a.t_fp_dev) : a.t_fp;      // on its way beside the loads below
   // the first loads of the slots, one by each warp (one after the other they took one thread 7000
   // cycles; 4 x 8 x 5152 masked tokens 24.0 -> 23.2 us, no difference where the ring's first units suffice for a while)
   static_assert(NS <= NW, "a warp per slot");
@@ -263,8 +264,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   __syncwarp();
   // this CTA's share of the full-precision tokens (16-token tiles dealt out over the cluster), on its way into L2
   auto fp_range = [&](int& f0, int& f1) {
-    const int t_fp = a.t_fp_dev ? min(*reinterpret_cast<const volatile int32_t*>(a.t_fp_dev), a.t_fp) : a.t_fp;
-    const int n_t16 = (t_fp + 15) / 16;
+    const int t_fp = min(t_live, a.t_fp), n_t16 = (t_fp + 15) / 16;
     f0 = rank * n_t16 / S * 16;
     f1 = min(t_fp, (rank + 1) * n_t16 / S * 16);
   };
@@ -460,32 +460,37 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   __syncthreads();
   if (tid < S) arrive_peer(map_peer(smem_u32(&stat_bar), tid));
 
-  // ---- full-precision tokens of this CTA, 128 at a time: scores as 16-token MMA tiles (K rows = A fragments straight
-  // from global memory), running maximum per head, probabilities rounded to the data type, P.V with warp w owning
-  // channels 16w .. 16w+15 (V words of two channels, paired over tokens by a byte permute)
-  float fo[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+  // ---- full-precision tokens of this CTA, 128 at a time: scores as 16-token MMA tiles, running maximum per head, probabilities
+  // rounded to the data type, P.V with warp w owning channels 32 (w / 2) .. + 31 of every other 64 tokens.  Keys and values come
+  // straight from global memory in pieces of 16 and 8 bytes: a lane's piece holds neighbouring channels, which the products take in
+  // the order they come.  (In the fragments' own 4-byte pieces the 80 loads of a thread, eight rows each, took 6900 cycles a chunk.)
+  float fo[4][4] = {};
   if (tid < kMaxRep) { fp_m[tid] = -INFINITY; fp_l[tid] = 0.f; }
   {
     int f0, f1;
     fp_range(f0, f1);
     const T* kf = k_fp + (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h;
-    const T* vf = v_fp + (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h + 16 * warp + 2 * g;
+    const T* vf = v_fp + (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h + 32 * (warp >> 1) + 4 * g;
     const T* mrow = a.mask ? static_cast<const T*>(a.mask) + (int64_t)b * a.mask_stride_b : nullptr;
     for (int t0 = f0; t0 < f1; t0 += FPC) {
       const int nt = min(FPC, f1 - t0);
       if (16 * warp < nt) {
         const int tt = 16 * warp;
-        const T* qrow = q + (row0 + (g < a.n_rep ? g : 0)) * kHeadDim + 2 * c;
-        const T* k_lo = kf + (int64_t)(t0 + min(tt + g, nt - 1)) * kHeadDim + 2 * c;       // rows past the end repeat
-        const T* k_hi = kf + (int64_t)(t0 + min(tt + g + 8, nt - 1)) * kHeadDim + 2 * c;   // the last token
+        const T* qrow = q + (row0 + (g < a.n_rep ? g : 0)) * kHeadDim + 8 * c;
+        const T* k_lo = kf + (int64_t)(t0 + min(tt + g, nt - 1)) * kHeadDim + 8 * c;       // rows past the end repeat
+        const T* k_hi = kf + (int64_t)(t0 + min(tt + g + 8, nt - 1)) * kHeadDim + 8 * c;   // the last token
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        uint4 lo[4], hi[4], qv[4];      // channels 32m + 8c .. + 7: four pairs, two k-steps
 #pragma unroll
-        for (int kt = 0; kt < 8; ++kt) {
-          const uint32_t a0 = *reinterpret_cast<const uint32_t*>(k_lo + kt * 16), a1 = *reinterpret_cast<const uint32_t*>(k_hi + kt * 16);
-          const uint32_t a2 = *reinterpret_cast<const uint32_t*>(k_lo + kt * 16 + 8), a3 = *reinterpret_cast<const uint32_t*>(k_hi + kt * 16 + 8);
-          const uint32_t b0 = g < a.n_rep ? *reinterpret_cast<const uint32_t*>(qrow + kt * 16) : 0u;
-          const uint32_t b1 = g < a.n_rep ? *reinterpret_cast<const uint32_t*>(qrow + kt * 16 + 8) : 0u;
-          mma_t<T>(acc, a0, a1, a2, a3, b0, b1);
+        for (int m = 0; m < 4; ++m) {
+          lo[m] = *reinterpret_cast<const uint4*>(k_lo + 32 * m);
+          hi[m] = *reinterpret_cast<const uint4*>(k_hi + 32 * m);
+          qv[m] = *reinterpret_cast<const uint4*>(qrow + 32 * m);      // columns past the last head repeat the first; they are not kept
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          mma_t<T>(acc, lo[m].x, hi[m].x, lo[m].y, hi[m].y, qv[m].x, qv[m].y);
+          mma_t<T>(acc, lo[m].z, hi[m].z, lo[m].w, hi[m].w, qv[m].z, qv[m].w);
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {       // acc[0..1] = (token tt+g, heads 2c, 2c+1), acc[2..3] = (token tt+g+8, same)
@@ -493,12 +498,14 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
           if (h < a.n_rep && t < nt) pf_s[h * PF_PITCH + t] = Elem<T>::from_f(__fdiv_rn(rnd<T>(acc[e]), 11.313708498984761f));
         }
       }
-      uint32_t v[FPC / 16][4];              // tokens 16k + 2c + {0, 1, 8, 9}, channels 16w + 2g (+1); on their way during the softmax
+      const int th = 64 * (warp & 1);
+      uint2 v[FPC / 32][4];                 // tokens th + 16k + 2c + {0, 1, 8, 9}, four channels; on their way during the softmax
 #pragma unroll
-      for (int k = 0; k < FPC / 16; ++k)
+      for (int k = 0; k < FPC / 32; ++k)
 #pragma unroll
         for (int r = 0; r < 4; ++r)         // past the end p is 0 and the value repeats the last token
-          v[k][r] = 16 * k < nt ? *reinterpret_cast<const uint32_t*>(vf + (int64_t)(t0 + min(16 * k + 2 * c + (r & 1) + 8 * (r >> 1), nt - 1)) * kHeadDim) : 0u;
+          v[k][r] = th + 16 * k < nt ? *reinterpret_cast<const uint2*>(vf + (int64_t)(t0 + min(th + 16 * k + 2 * c + (r & 1) + 8 * (r >> 1), nt - 1)) * kHeadDim)
+                                     : make_uint2(0u, 0u);
       __syncthreads();
       if (warp < a.n_rep) {                 // warp = head
         const int h = warp;
@@ -532,16 +539,17 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
       {
         const float alpha = g < a.n_rep ? fp_alpha[g] : 0.f;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) { fo[j][0] *= alpha; fo[j][1] *= alpha; }
-        const T* prow = pf_s + (g < a.n_rep ? g : 0) * PF_PITCH + 2 * c;
+        for (int j = 0; j < 4; ++j) { fo[j][0] *= alpha; fo[j][1] *= alpha; }
+        const T* prow = pf_s + (g < a.n_rep ? g : 0) * PF_PITCH + th + 2 * c;
 #pragma unroll
-        for (int k = 0; k < FPC / 16; ++k) {
-          if (16 * k >= nt) break;
-          uint32_t p0 = *reinterpret_cast<const uint32_t*>(prow + 16 * k), p1 = *reinterpret_cast<const uint32_t*>(prow + 16 * k + 8);
-          if (g >= a.n_rep) { p0 = 0u; p1 = 0u; }
-          // n-tile j: column n stands for channel 16w + 2n + j
-          mma_t<T>(fo[0], p0, 0u, p1, 0u, prmt(v[k][0], v[k][1], 0x5410), prmt(v[k][2], v[k][3], 0x5410));
-          mma_t<T>(fo[1], p0, 0u, p1, 0u, prmt(v[k][0], v[k][1], 0x7632), prmt(v[k][2], v[k][3], 0x7632));
+        for (int k = 0; k < FPC / 32; ++k) {
+          if (th + 16 * k >= nt) break;
+          const uint32_t p0 = *reinterpret_cast<const uint32_t*>(prow + 16 * k), p1 = *reinterpret_cast<const uint32_t*>(prow + 16 * k + 8);
+          // n-tile j: column n stands for channel 32 (w / 2) + 4n + j
+          mma_t<T>(fo[0], p0, 0u, p1, 0u, prmt(v[k][0].x, v[k][1].x, 0x5410), prmt(v[k][2].x, v[k][3].x, 0x5410));
+          mma_t<T>(fo[1], p0, 0u, p1, 0u, prmt(v[k][0].x, v[k][1].x, 0x7632), prmt(v[k][2].x, v[k][3].x, 0x7632));
+          mma_t<T>(fo[2], p0, 0u, p1, 0u, prmt(v[k][0].y, v[k][1].y, 0x5410), prmt(v[k][2].y, v[k][3].y, 0x5410));
+          mma_t<T>(fo[3], p0, 0u, p1, 0u, prmt(v[k][0].y, v[k][1].y, 0x7632), prmt(v[k][2].y, v[k][3].y, 0x7632));
         }
       }
       __syncthreads();       // the probabilities have been used
@@ -686,12 +694,13 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
     }
   }
   __syncthreads();            // the ring is idle: it holds the warps' sums from here on
-  float* fp_o = reinterpret_cast<float*>(smem) + NW * kMaxRep * RED_STRIDE;      // [head][channel]
+  float* fp_o = reinterpret_cast<float*>(smem) + NW * kMaxRep * RED_STRIDE;      // [token half][head][channel]
   {
     float* mine = reinterpret_cast<float*>(smem) + warp * kMaxRep * RED_STRIDE;
-    if (g < a.n_rep) {                       // fragment columns 2c, 2c+1 of n-tile j = channels 16w + 4c + j, + 2
-      float4* dst = reinterpret_cast<float4*>(fp_o + g * kHeadDim + 16 * warp + 4 * c);
-      *dst = make_float4(fo[0][0], fo[1][0], fo[0][1], fo[1][1]);
+    if (g < a.n_rep) {                       // fragment columns 2c, 2c+1 of n-tile j = channels 32 (w / 2) + 8c + j, + 4
+      float4* dst = reinterpret_cast<float4*>(fp_o + ((warp & 1) * kMaxRep + g) * kHeadDim + 32 * (warp >> 1) + 8 * c);
+      dst[0] = make_float4(fo[0][0], fo[1][0], fo[2][0], fo[3][0]);
+      dst[1] = make_float4(fo[0][1], fo[1][1], fo[2][1], fo[3][1]);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -728,7 +737,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
     // this CTA's visual and full-precision parts under one reference
     const float m_v = n_u > 0 ? __uint_as_float(cal_s[h][5]) : -INFINITY, m_f = fp_m[h], m = fmaxf(m_v, m_f);
     const float wv = m_v == -INFINITY ? 0.f : exp2f((m_v - m) * LOG2E), wf = m_f == -INFINITY ? 0.f : exp2f((m_f - m) * LOG2E);
-    o = o * wv + fp_o[e] * wf;
+    o = o * wv + (fp_o[e] + fp_o[kMaxRep * kHeadDim + e]) * wf;
     const int peer = e / slice;
     st_peer(map_peer(smem_u32(&recv_o[rank * slice + e % slice]), peer), o);
     if (d < S) st_peer2(map_peer(smem_u32(&recv_ml[rank][h]), d), m, l * wv + fp_l[h] * wf);

@@ -247,22 +247,37 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
     return p;
   });
 
-  // ---- full-precision scores of this CTA's tokens: rnd(rnd(q . k) / sqrt(D)) + mask
+  // ---- full-precision scores of this CTA's tokens: rnd(rnd(q . k) / sqrt(D)) + mask.  Keys (and values below) in pieces of 16 (8)
+  // bytes; a lane's piece holds neighbouring channels, which the products take in the order they come
+  const bool q_wide = reinterpret_cast<uintptr_t>(q) % 16 == 0;
   const int n_ft = (n_f + 15) / 16;
   const T* mrow = mask ? mask + (int64_t)b * a.mask_stride_b : nullptr;
   for (int ft = warp; ft < n_ft; ft += NW) {
-    const T* qrow = q + (row0 + (g < a.n_rep ? g : 0)) * kHeadDim + 2 * c;
-    const T* k_lo = k_fp + fp_off + (int64_t)min(16 * ft + g, n_f - 1) * kHeadDim + 2 * c;
-    const T* k_hi = k_fp + fp_off + (int64_t)min(16 * ft + g + 8, n_f - 1) * kHeadDim + 2 * c;
+    const T* qrow = q + (row0 + (g < a.n_rep ? g : 0)) * kHeadDim + 8 * c;
+    const T* k_lo = k_fp + fp_off + (int64_t)min(16 * ft + g, n_f - 1) * kHeadDim + 8 * c;
+    const T* k_hi = k_fp + fp_off + (int64_t)min(16 * ft + g + 8, n_f - 1) * kHeadDim + 8 * c;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    uint4 lo[4], hi[4], qv[4];      // channels 32m + 8c .. + 7: four pairs, two k-steps
 #pragma unroll
-    for (int kt = 0; kt < 8; ++kt) {
-      const uint32_t a0 = *reinterpret_cast<const uint32_t*>(k_lo + kt * 16), a1 = *reinterpret_cast<const uint32_t*>(k_hi + kt * 16);
-      const uint32_t a2 = *reinterpret_cast<const uint32_t*>(k_lo + kt * 16 + 8), a3 = *reinterpret_cast<const uint32_t*>(k_hi + kt * 16 + 8);
-      const uint32_t b0 = g < a.n_rep ? *reinterpret_cast<const uint32_t*>(qrow + kt * 16) : 0u;
-      const uint32_t b1 = g < a.n_rep ? *reinterpret_cast<const uint32_t*>(qrow + kt * 16 + 8) : 0u;
-      if constexpr (std::is_same<T, __nv_bfloat16>::value) mma_bf16(acc, a0, a1, a2, a3, b0, b1);
-      else mma_f16(acc, a0, a1, a2, a3, b0, b1);
+    for (int m = 0; m < 4; ++m) {
+      lo[m] = *reinterpret_cast<const uint4*>(k_lo + 32 * m);
+      hi[m] = *reinterpret_cast<const uint4*>(k_hi + 32 * m);
+      if (q_wide) {                 // columns past the last head repeat the first; they are not kept
+        qv[m] = *reinterpret_cast<const uint4*>(qrow + 32 * m);
+      } else {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(qrow + 32 * m);
+        qv[m] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        mma_bf16(acc, lo[m].x, hi[m].x, lo[m].y, hi[m].y, qv[m].x, qv[m].y);
+        mma_bf16(acc, lo[m].z, hi[m].z, lo[m].w, hi[m].w, qv[m].z, qv[m].w);
+      } else {
+        mma_f16(acc, lo[m].x, hi[m].x, lo[m].y, hi[m].y, qv[m].x, qv[m].y);
+        mma_f16(acc, lo[m].z, hi[m].z, lo[m].w, hi[m].w, qv[m].z, qv[m].w);
+      }
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -483,21 +498,20 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
       }
     }
   }
-  // full-precision segments: warp w owns channels 16w .. 16w+15; system and text keys are summed apart, as the reference
-  // adds their rounded products one after the other
-  float fo[2][2][4] = {};
+  // full-precision segments: warp w owns channels 32 (w / 2) .. + 31 of every other 16 tokens; system and text keys are summed
+  // apart, as the reference adds their rounded products one after the other
+  float fo[2][4][4] = {};
   {
-    const T* vf = v_fp + fp_off + 16 * warp + 2 * g;
+    const T* vf = v_fp + fp_off + 32 * (warp >> 1) + 4 * g;
     const T* prow = fpr + (size_t)(g < a.n_rep ? g : 0) * 2 * a.fp_pitch + 2 * c;
     const int n_sys = min(max(min(a.t_sys, t_fp) - f0, 0), n_f);
-#pragma unroll 4
-    for (int ft = 0; ft < n_ft; ++ft) {
-      uint32_t v[4];
+#pragma unroll 2
+    for (int ft = warp & 1; ft < n_ft; ft += 2) {
+      uint2 v[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r)
-        v[r] = *reinterpret_cast<const uint32_t*>(vf + (int64_t)min(16 * ft + 2 * c + (r & 1) + 8 * (r >> 1), n_f - 1) * kHeadDim);
-      uint32_t p[2] = {*reinterpret_cast<const uint32_t*>(prow + 16 * ft), *reinterpret_cast<const uint32_t*>(prow + 16 * ft + 8)};
-      if (g >= a.n_rep) p[0] = p[1] = 0u;
+        v[r] = *reinterpret_cast<const uint2*>(vf + (int64_t)min(16 * ft + 2 * c + (r & 1) + 8 * (r >> 1), n_f - 1) * kHeadDim);
+      const uint32_t p[2] = {*reinterpret_cast<const uint32_t*>(prow + 16 * ft), *reinterpret_cast<const uint32_t*>(prow + 16 * ft + 8)};
 #pragma unroll
       for (int seg = 0; seg < 2; ++seg) {
         if (seg == 0 ? 16 * ft >= n_sys : 16 * ft + 16 <= n_sys) continue;
@@ -508,15 +522,17 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
           const uint32_t keep = ((t < n_sys) == (seg == 0) ? 0xffffu : 0u) | ((t + 1 < n_sys) == (seg == 0) ? 0xffff0000u : 0u);
           ps[i] = p[i] & keep;
         }
-        // n-tile j: column n stands for channel 16w + 2n + j
-        mma_t<T>(fo[seg][0], ps[0], ps[1], prmt(v[0], v[1], 0x5410), prmt(v[2], v[3], 0x5410));
-        mma_t<T>(fo[seg][1], ps[0], ps[1], prmt(v[0], v[1], 0x7632), prmt(v[2], v[3], 0x7632));
+        // n-tile j: column n stands for channel 32 (w / 2) + 4n + j
+        mma_t<T>(fo[seg][0], ps[0], ps[1], prmt(v[0].x, v[1].x, 0x5410), prmt(v[2].x, v[3].x, 0x5410));
+        mma_t<T>(fo[seg][1], ps[0], ps[1], prmt(v[0].x, v[1].x, 0x7632), prmt(v[2].x, v[3].x, 0x7632));
+        mma_t<T>(fo[seg][2], ps[0], ps[1], prmt(v[0].y, v[1].y, 0x5410), prmt(v[2].y, v[3].y, 0x5410));
+        mma_t<T>(fo[seg][3], ps[0], ps[1], prmt(v[0].y, v[1].y, 0x7632), prmt(v[2].y, v[3].y, 0x7632));
       }
     }
   }
   __syncthreads();      // scores and probabilities have been used: their memory holds the warps' sums from here on
   float* red = reinterpret_cast<float*>(smem);                          // [warp][head][RED_STRIDE]
-  float* seg_s = red + NW * a.n_rep * RED_STRIDE;                       // [system | text][head][channel]
+  float* seg_s = red + NW * a.n_rep * RED_STRIDE;                       // [token parity][system | text][head][channel]
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     constexpr int NM = BITS == 1 ? 2 : 1;
@@ -542,8 +558,10 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   if (g < a.n_rep) {
 #pragma unroll
     for (int seg = 0; seg < 2; ++seg)
-      *reinterpret_cast<float4*>(seg_s + (seg * a.n_rep + g) * kHeadDim + 16 * warp + 4 * c) =
-          make_float4(fo[seg][0][0], fo[seg][1][0], fo[seg][0][1], fo[seg][1][1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)      // fragment columns 2c, 2c+1 of n-tile j = channels 32 (w / 2) + 8c + j, + 4
+        *reinterpret_cast<float4*>(seg_s + (((warp & 1) * 2 + seg) * a.n_rep + g) * kHeadDim + 32 * (warp >> 1) + 8 * c + 4 * i) =
+            make_float4(fo[seg][0][i], fo[seg][1][i], fo[seg][2][i], fo[seg][3][i]);
   }
   __syncthreads();
 
@@ -555,8 +573,8 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
 #pragma unroll
     for (int w = 0; w < NW; ++w) o += red[(w * a.n_rep + h) * RED_STRIDE + d];
     st_peer(map_peer(smem_u32(&recv_s[0][at]), peer), o);
-    st_peer(map_peer(smem_u32(&recv_s[1][at]), peer), seg_s[h * kHeadDim + d]);
-    st_peer(map_peer(smem_u32(&recv_s[2][at]), peer), seg_s[(a.n_rep + h) * kHeadDim + d]);
+    st_peer(map_peer(smem_u32(&recv_s[1][at]), peer), seg_s[h * kHeadDim + d] + seg_s[(2 * a.n_rep + h) * kHeadDim + d]);
+    st_peer(map_peer(smem_u32(&recv_s[2][at]), peer), seg_s[(a.n_rep + h) * kHeadDim + d] + seg_s[(3 * a.n_rep + h) * kHeadDim + d]);
     if (d < S) {
       float ps = 0.f;
 #pragma unroll
@@ -606,7 +624,7 @@ inline bool make_plan(const cq_u8_decode_args* a, Plan* p) {
     p->pitch = (n_items + S - 1) / S * ITEM + 8;
     p->fp_pitch = ((a->t_fp + 15) / 16 + S - 1) / S * 16 + 8;
     const size_t rows = (size_t)n_rep * ((size_t)p->pitch * sb + (size_t)p->fp_pitch * 4);
-    const size_t red = (size_t)(NW * n_rep * RED_STRIDE + 2 * n_rep * kHeadDim) * 4;
+    const size_t red = (size_t)(NW * n_rep * RED_STRIDE + 4 * n_rep * kHeadDim) * 4;
     const size_t smem = rows > red ? rows : red;
     if (smem <= 88 * 1024) { p->smem = (int)smem; return true; }
   }
