@@ -13,7 +13,9 @@
 //   4. partial sums scattered over the cluster by output slice, every CTA finishes its slice in the reference's order of
 //      roundings.
 // Codes are read straight from global memory (the lanes of a row share their 16-byte loads; the span is on its way into L2
-// since the first instruction).  Two CTAs of eight warps per SM.  Nothing waits for another cluster; waits are bounded.
+// since the first instruction).  Two CTAs of eight warps per SM.  What bounds it now is the instructions of a warp waiting for each
+// other: 14 000 and 9000 of 46 600 cycles in the loops of the two products, 9400 in the passes over the scores.  16 x 8 heads x 3328
+// bfloat16 keys, 1 bit: 32.8 -> 30.7 us; 3 x 8 x 418 at 4 bits 16.7 -> 13.1; 12 x 8 x 1479 fp16 24.6 -> 21.1.  Nothing waits for another cluster; waits are bounded.
 #include <mutex>
 #include <type_traits>
 
@@ -75,7 +77,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   __shared__ float bias_s[kMaxRep];
   __shared__ float red_s[NW][kMaxRep][2];
   __shared__ Pair peer_s[2][MAX_CLUSTER][kMaxRep];
-  __shared__ float m_s[kMaxRep], f_s[kMaxRep], psum_s[NW][kMaxRep];
+  __shared__ float m_s[kMaxRep], f_s[kMaxRep], e_s[kMaxRep], psum_s[NW][kMaxRep];
   __shared__ float recv_s[3][kMaxRep * kHeadDim + MAX_CLUSTER];      // codes, system, text: [source CTA][slice element]
   __shared__ float recv_p[MAX_CLUSTER][kMaxRep];
 
@@ -86,6 +88,9 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   const int i0 = rank * a.n_items / S, n_it = (rank + 1) * a.n_items / S - i0;
   const int tok0 = i0 * ITEM, n_tok = min(n_it * ITEM, a.t_vis - tok0);      // may be <= 0 without items
 
+  // on its way during the set-up; a launch before this one may still be advancing the live count, which is good enough for a
+  // prefetch and read again behind the wait
+  int live = a.t_fp_dev ? *reinterpret_cast<const volatile int32_t*>(a.t_fp_dev) : a.t_fp;
   pdl_launch_dependents();
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(&bar[i], S);
@@ -99,12 +104,11 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
     asm volatile("prefetch.global.L2 [%0];" ::"l"(ek + (int64_t)i * 128));
     asm volatile("prefetch.global.L2 [%0];" ::"l"(ev + (int64_t)i * 128));
   }
-  // this CTA's share of the full-precision tokens (16-token tiles dealt out over the cluster).  A launch before this one may
-  // still be advancing the live count: what is read here is good enough for a prefetch, and read again behind the wait
+  // this CTA's share of the full-precision tokens (16-token tiles dealt out over the cluster)
   int t_fp, n_f, f0;
   int64_t fp_off;
   auto fp_range = [&]() {
-    t_fp = a.t_fp_dev ? min(*reinterpret_cast<const volatile int32_t*>(a.t_fp_dev), a.t_fp) : a.t_fp;
+    t_fp = min(live, a.t_fp);
     const int n_t16 = (t_fp + 15) / 16;
     f0 = rank * n_t16 / S * 16;
     n_f = min(t_fp, (rank + 1) * n_t16 / S * 16) - f0;
@@ -118,7 +122,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   float* fs = reinterpret_cast<float*>(smem + (size_t)a.n_rep * a.pitch * SB);   // full-precision scores [n_rep][fp_pitch]
   T* fpr = reinterpret_cast<T*>(fs);                                        // ... later their probabilities, [n_rep][2*fp_pitch]
   pdl_wait();
-  fp_range();
+  if (a.t_fp_dev) live = *reinterpret_cast<const volatile int32_t*>(a.t_fp_dev);
 
   // ---- query side: weights rnd(q * scale_key), bias_k = rnd(rnd(sum rnd(rnd(scale*zp) * q)) / sqrt(D))
   if (warp < a.n_rep) {
@@ -137,6 +141,10 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
     if (lane == 0) bias_s[r] = rnd<T>(__fdiv_rn(rnd<T>(bs), 11.313708498984761f));
   }
   __syncthreads();
+  fp_range();
+
+  // this warp's share of the CTA's 16-token tiles, in both products
+  const int n_m16 = n_tok > 0 ? (n_tok + 15) / 16 : 0, m_first = warp * n_m16 / NW, m_last = (warp + 1) * n_m16 / NW;
 
   // ================= 1. visual scores =================
   // A register (two k values of one token) = one AND of the token's code word; B carries the weights in the channel order
@@ -161,55 +169,71 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
     const int sh4 = 4 * (c & 1) + 8 * (c >> 1);
     const float bias[2] = {2 * c < a.n_rep ? bias_s[2 * c] : 0.f, 2 * c + 1 < a.n_rep ? bias_s[2 * c + 1] : 0.f};
     float lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
-    constexpr int MT = BITS == 1 ? 4 : BITS == 2 ? 2 : 1;      // 16-token tiles whose loads are in flight together
-    for (int it = warp; it < n_it; it += NW) {
-#pragma unroll 1
-      for (int m0 = 0; m0 < 4; m0 += MT) {
-        uint32_t W[MT][2][WORDS];
+    // The warps take contiguous shares of the 16-token tiles (dealt out as items of 64 tokens, four rounds of eight warps were 3.25
+    // items' work), MT at a time, and request the words of the next ones before they work on those at hand.
+    constexpr int MT = BITS == 1 ? 2 : 1;
+    constexpr bool AHEAD = BITS < 4;              // at 4 bits there are no registers for it
+    struct Words { uint32_t w[MT][2][WORDS]; };
+    auto load = [&](Words& W, int m0) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            const int t = min(it * ITEM + 16 * (m0 + m) + g + 8 * hf, n_tok - 1);
-            const uint4* rp = reinterpret_cast<const uint4*>(ek + (int64_t)t * ROWB);
+        for (int hf = 0; hf < 2; ++hf) {
+          const int t = min(16 * (m0 + m) + g + 8 * hf, n_tok - 1);
+          const uint4* rp = reinterpret_cast<const uint4*>(ek + (int64_t)t * ROWB);
 #pragma unroll
-            for (int q4 = 0; q4 < WORDS / 4; ++q4) {
-              const uint4 v = rp[q4];
-              W[m][hf][4 * q4] = v.x; W[m][hf][4 * q4 + 1] = v.y; W[m][hf][4 * q4 + 2] = v.z; W[m][hf][4 * q4 + 3] = v.w;
-            }
+          for (int q4 = 0; q4 < WORDS / 4; ++q4) {
+            const uint4 v = rp[q4];
+            W.w[m][hf][4 * q4] = v.x; W.w[m][hf][4 * q4 + 1] = v.y; W.w[m][hf][4 * q4 + 2] = v.z; W.w[m][hf][4 * q4 + 3] = v.w;
           }
+        }
+    };
+    auto compute = [&](const Words& W, int m0) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int m = 0; m < MT; ++m) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};       // a tile past the share computes along, so that the chains of two interleave
 #pragma unroll
-          for (int kb = 0; kb < 8; ++kb) {
-            uint32_t a0, a1, a2, a3;
-            if (BITS == 1) {
-              const uint32_t x0 = W[m][0][kb >> 1] >> (8 * (kb & 1)), x1 = W[m][1][kb >> 1] >> (8 * (kb & 1));
-              a0 = x0 & m_a0; a1 = x1 & m_a0; a2 = x0 & m_a2; a3 = x1 & m_a2;
-            } else if (BITS == 2) {
-              const uint32_t x0 = W[m][0][kb], x1 = W[m][1][kb];
-              a0 = x0 & m_a0; a1 = x1 & m_a0; a2 = (x0 >> 8) & m_a0; a3 = (x1 >> 8) & m_a0;
-            } else {
-              a0 = (W[m][0][2 * kb] >> sh4) & m_a0; a1 = (W[m][1][2 * kb] >> sh4) & m_a0;
-              a2 = (W[m][0][2 * kb + 1] >> sh4) & m_a0; a3 = (W[m][1][2 * kb + 1] >> sh4) & m_a0;
-            }
-            mma_f16(acc, a0, a1, a2, a3, b0[kb], b1[kb]);
+        for (int kb = 0; kb < 8; ++kb) {
+          uint32_t a0, a1, a2, a3;
+          if (BITS == 1) {
+            const uint32_t x0 = W.w[m][0][kb >> 1] >> (8 * (kb & 1)), x1 = W.w[m][1][kb >> 1] >> (8 * (kb & 1));
+            a0 = x0 & m_a0; a1 = x1 & m_a0; a2 = x0 & m_a2; a3 = x1 & m_a2;
+          } else if (BITS == 2) {
+            const uint32_t x0 = W.w[m][0][kb], x1 = W.w[m][1][kb];
+            a0 = x0 & m_a0; a1 = x1 & m_a0; a2 = (x0 >> 8) & m_a0; a3 = (x1 >> 8) & m_a0;
+          } else {
+            a0 = (W.w[m][0][2 * kb] >> sh4) & m_a0; a1 = (W.w[m][1][2 * kb] >> sh4) & m_a0;
+            a2 = (W.w[m][0][2 * kb + 1] >> sh4) & m_a0; a3 = (W.w[m][1][2 * kb + 1] >> sh4) & m_a0;
           }
-          // acc[0..1] = (token g, heads 2c, 2c+1), acc[2..3] = (token g+8, same heads): fp16 product, / sqrt(D) (a product
-          // with the fp32 reciprocal: one score in 4000 lands on the neighbouring fp16 value), - bias_k in the score type
+          mma_f16(acc, a0, a1, a2, a3, b0[kb], b1[kb]);
+        }
+        // acc[0..1] = (token g, heads 2c, 2c+1), acc[2..3] = (token g+8, same heads): fp16 product, / sqrt(D) (a product
+        // with the fp32 reciprocal: one score in 4000 lands on the neighbouring fp16 value), - bias_k in the score type
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int r = 2 * c + (e & 1), t = it * ITEM + 16 * (m0 + m) + g + 8 * (e >> 1);
-            if (r < a.n_rep && t < n_tok) {
-              const float v = SS::r(rnd<__half>(rnd<__half>(acc[e] * 1048576.f) * 0.08838834764831845f) - bias[e & 1]);
-              reinterpret_cast<SO*>(sc_b)[r * a.pitch + t] = SS::make(v);
-              lo[e & 1] = fminf(lo[e & 1], v);
-              hi[e & 1] = fmaxf(hi[e & 1], v);
-            }
+        for (int e = 0; e < 4; ++e) {
+          const int r = 2 * c + (e & 1), t = 16 * (m0 + m) + g + 8 * (e >> 1);
+          if (r < a.n_rep && t < n_tok && m0 + m < m_last) {
+            const float v = SS::r(rnd<__half>(rnd<__half>(acc[e] * 1048576.f) * 0.08838834764831845f) - bias[e & 1]);
+            reinterpret_cast<SO*>(sc_b)[r * a.pitch + t] = SS::make(v);
+            lo[e & 1] = fminf(lo[e & 1], v);
+            hi[e & 1] = fmaxf(hi[e & 1], v);
           }
         }
       }
+    };
+    if (AHEAD) {
+      Words W0, W1;
+      if (m_first < m_last) load(W0, m_first);
+#pragma unroll 1
+      for (int m = m_first; m < m_last; m += 2 * MT) {
+        if (m + MT < m_last) load(W1, m + MT);
+        compute(W0, m);
+        if (m + 2 * MT < m_last) load(W0, m + 2 * MT);
+        if (m + MT < m_last) compute(W1, m + MT);
+      }
+    } else {
+#pragma unroll 1
+      for (int m = m_first; m < m_last; m += MT) { Words W; load(W, m); compute(W, m); }
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -317,71 +341,124 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   // off by 4.36e-3, with two roundings by 4.59e-3) and take a product with the reciprocal, which for numbers of 11 significant
   // bits rounds to the same fp16 number as the quotient.  Other rows round every operation; their quotient is that product
   // corrected by its residual (Markstein 1990), 1.2 us less than divisions at 16 x 8 heads x 3328 bfloat16 keys.
-  const bool packed = SB == 2 && a.calibrate && !mrow;
-  for (int h = 0; h < a.n_rep; ++h) {
-    float lo = INFINITY, hi = -INFINITY;
-    for (int p = 0; p < S; ++p) { lo = fminf(lo, peer_s[0][p][h].a); hi = fmaxf(hi, peer_s[0][p][h].b); }
-    const float span = SS::r(SS::r(hi + -3.f) - lo), denom = SS::r(SS::r(hi - lo) + 1e-8f), rden = 1.f / denom;
-    const __half2 lo2 = __float2half2_rn(lo), span2 = __float2half2_rn(span);
-    float m = -INFINITY;
-    for (int v = (tid + 256 - (h * n_vec & 255)) & 255; v < n_vec; v += THREADS) {
-      float x[8];
-      load8(h, v, x);
-      if (packed) {
+  // Without a mask the calibration is monotonous, so the largest calibrated score is that of one of the extremes, and known before
+  // the pass that calibrates, which then sums the exponentials as well; in fp32 rows it leaves them in place of the scores, and the
+  // later pass multiplies them.  (Calibration, sum and probabilities as three passes, two of them with exponentials, took 11 300
+  // cycles of 50 200 at 16 x 8 heads x 3328 keys; now 9400.)
+  const bool early = !mrow;
+  struct Calib { float lo, hi, span, denom, rden; };
+  auto calib_of = [&](int h) {
+    Calib k{INFINITY, -INFINITY, 0.f, 0.f, 0.f};
+    for (int p = 0; p < S; ++p) { k.lo = fminf(k.lo, peer_s[0][p][h].a); k.hi = fmaxf(k.hi, peer_s[0][p][h].b); }
+    k.span = SS::r(SS::r(k.hi + -3.f) - k.lo);
+    k.denom = SS::r(SS::r(k.hi - k.lo) + 1e-8f);
+    k.rden = 1.f / k.denom;
+    return k;
+  };
+  auto calibrated = [&](float x, const Calib& k) {
+    const float d = SS::r(x - k.lo), n = d * k.rden;
+    return SS::r(SS::r(SS::r(fmaf(fmaf(-n, k.denom, d), k.rden, n)) * k.span) + k.lo);
+  };
+  auto calibrated2 = [&](float x, float y, const Calib& k) {      // two of an fp16 row without a mask
+    const __half2 lo2 = __float2half2_rn(k.lo);
+    const float2 d = __half22float2(__hsub2(__floats2half2_rn(x, y), lo2));
+    return __half22float2(__hfma2(__floats2half2_rn(d.x * k.rden, d.y * k.rden), __float2half2_rn(k.span), lo2));
+  };
+  auto store8 = [&](int h, int v, const float (&x)[8]) {
+    unsigned char* p = sc_b + (size_t)(h * a.pitch + 8 * v) * SB;
+    if constexpr (SB == 2) {
+      uint4 w;
+      __half2* h2 = reinterpret_cast<__half2*>(&w);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h2[j] = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
+      *reinterpret_cast<uint4*>(p) = w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) reinterpret_cast<float4*>(p)[j] = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+    }
+  };
+  if (early) {
+    if (warp < a.n_rep) {
+      const Calib k = calib_of(warp);
+      float m = k.hi;
+      if (a.calibrate) {
+        const float2 y = SB == 2 ? calibrated2(k.lo, k.hi, k) : make_float2(calibrated(k.lo, k), calibrated(k.hi, k));
+        m = fmaxf(y.x, y.y);
+      }
+      for (int t = lane; t < n_f; t += 32) m = fmaxf(m, fs[warp * a.fp_pitch + t]);
+      m = warp_max(m);
+      if (lane == 0) m_s[warp] = m;
+    }
+    __syncthreads();
+    for (int h = 0; h < a.n_rep; ++h) {
+      const Calib k = calib_of(h);
+      const float m = m_s[h], ml = m == -INFINITY ? 0.f : m * LOG2E;
+      float l = 0.f;
+      for (int v = (tid + 256 - (h * n_vec & 255)) & 255; v < n_vec; v += THREADS) {
+        float x[8];
+        load8(h, v, x);
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
-          const float2 d = __half22float2(__hsub2(__floats2half2_rn(x[j], x[j + 1]), lo2));
-          const float2 y = __half22float2(__hfma2(__floats2half2_rn(d.x * rden, d.y * rden), span2, lo2));
-          x[j] = y.x; x[j + 1] = y.y;
+          if (a.calibrate) {
+            const float2 y = SB == 2 ? calibrated2(x[j], x[j + 1], k) : make_float2(calibrated(x[j], k), calibrated(x[j + 1], k));
+            x[j] = y.x; x[j + 1] = y.y;
+          }
+#pragma unroll
+          for (int i = j; i < j + 2; ++i) {
+            if (8 * v + i >= n_tok) x[i] = -INFINITY;
+            const float e = ex2(fmaf(x[i], LOG2E, -ml));
+            l += e;
+            if (SB == 4) x[i] = e;
+          }
         }
+        store8(h, v, x);
       }
+      for (int t = tid; t < n_f; t += THREADS) l += ex2(fmaf(fs[h * a.fp_pitch + t], LOG2E, -ml));
+      l = warp_sum(l);
+      if (lane == 0) red_s[warp][h][1] = l;
+    }
+  } else {
+    for (int h = 0; h < a.n_rep; ++h) {
+      const Calib k = calib_of(h);
+      float m = -INFINITY;
+      for (int v = (tid + 256 - (h * n_vec & 255)) & 255; v < n_vec; v += THREADS) {
+        float x[8];
+        load8(h, v, x);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int t = 8 * v + j;
-        if (a.calibrate && !packed) {
-          const float d = SS::r(x[j] - lo), n = d * rden;
-          x[j] = SS::r(SS::r(SS::r(fmaf(fmaf(-n, denom, d), rden, n)) * span) + lo);
+        for (int j = 0; j < 8; ++j) {
+          const int t = 8 * v + j;
+          if (a.calibrate) x[j] = calibrated(x[j], k);
+          if (t < n_tok) x[j] = SS::r(x[j] + Elem<T>::to_f(mrow[a.t_sys + tok0 + t]));
+          else x[j] = -INFINITY;
+          m = fmaxf(m, x[j]);
         }
-        if (mrow && t < n_tok) x[j] = SS::r(x[j] + Elem<T>::to_f(mrow[a.t_sys + tok0 + t]));
-        if (t >= n_tok) x[j] = -INFINITY;
-        m = fmaxf(m, x[j]);
+        store8(h, v, x);
       }
-      unsigned char* p = sc_b + (size_t)(h * a.pitch + 8 * v) * SB;
-      if constexpr (SB == 2) {
-        uint4 w;
-        __half2* h2 = reinterpret_cast<__half2*>(&w);
+      for (int t = tid; t < n_f; t += THREADS) m = fmaxf(m, fs[h * a.fp_pitch + t]);
+      m = warp_max(m);
+      if (lane == 0) red_s[warp][h][0] = m;
+    }
+    __syncthreads();
+    if (tid < a.n_rep) {
+      float m = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) h2[j] = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
-        *reinterpret_cast<uint4*>(p) = w;
-      } else {
+      for (int w = 0; w < NW; ++w) m = fmaxf(m, red_s[w][tid][0]);
+      m_s[tid] = m;
+    }
+    __syncthreads();
+    for (int h = 0; h < a.n_rep; ++h) {
+      const float m = m_s[h], ml = m == -INFINITY ? 0.f : m * LOG2E;
+      float l = 0.f;
+      for (int v = (tid + 256 - (h * n_vec & 255)) & 255; v < n_vec; v += THREADS) {
+        float x[8];
+        load8(h, v, x);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) reinterpret_cast<float4*>(p)[j] = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+        for (int j = 0; j < 8; ++j) l += ex2(fmaf(x[j], LOG2E, -ml));
       }
+      for (int t = tid; t < n_f; t += THREADS) l += ex2(fmaf(fs[h * a.fp_pitch + t], LOG2E, -ml));
+      l = warp_sum(l);
+      if (lane == 0) red_s[warp][h][1] = l;
     }
-    for (int t = tid; t < n_f; t += THREADS) m = fmaxf(m, fs[h * a.fp_pitch + t]);
-    m = warp_max(m);
-    if (lane == 0) red_s[warp][h][0] = m;
-  }
-  __syncthreads();
-  if (tid < a.n_rep) {
-    float m = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) m = fmaxf(m, red_s[w][tid][0]);
-    m_s[tid] = m;
-  }
-  __syncthreads();
-  for (int h = 0; h < a.n_rep; ++h) {
-    const float m = m_s[h], ml = m == -INFINITY ? 0.f : m * LOG2E;
-    float l = 0.f;
-    for (int v = (tid + 256 - (h * n_vec & 255)) & 255; v < n_vec; v += THREADS) {
-      float x[8];
-      load8(h, v, x);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) l += ex2(fmaf(x[j], LOG2E, -ml));
-    }
-    for (int t = tid; t < n_f; t += THREADS) l += ex2(fmaf(fs[h * a.fp_pitch + t], LOG2E, -ml));
-    l = warp_sum(l);
-    if (lane == 0) red_s[warp][h][1] = l;
   }
   __syncthreads();
   push(1, [&](int h) {
@@ -398,6 +475,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
       const Pair v = peer_s[1][p][tid];
       if (v.a != -INFINITY) l += v.b * exp2f((v.a - m) * LOG2E);
     }
+    e_s[tid] = exp2f((m_s[tid] - m) * LOG2E) / l;      // what turns this CTA's exponentials into probabilities
     m_s[tid] = m;
     f_s[tid] = 1.f / l;
   }
@@ -406,7 +484,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
   // ================= 3. probabilities, attn.V =================
   // in place: the 8 tokens of a vector become 16 bytes of fp16 at the vector's first byte
   for (int h = 0; h < a.n_rep; ++h) {
-    const float ml = m_s[h] * LOG2E, inv = f_s[h];
+    const float ml = m_s[h] * LOG2E, inv = f_s[h], scale = e_s[h];
     float ps = 0.f;
     for (int v = (tid + 256 - (h * n_vec & 255)) & 255; v < n_vec; v += THREADS) {
       float x[8];
@@ -415,7 +493,8 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
       __half2* h2 = reinterpret_cast<__half2*>(&w);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float p0 = rnd<T>(ex2(fmaf(x[2 * j], LOG2E, -ml)) * inv), p1 = rnd<T>(ex2(fmaf(x[2 * j + 1], LOG2E, -ml)) * inv);
+        const float p0 = rnd<T>(SB == 4 && early ? x[2 * j] * scale : ex2(fmaf(x[2 * j], LOG2E, -ml)) * inv);
+        const float p1 = rnd<T>(SB == 4 && early ? x[2 * j + 1] * scale : ex2(fmaf(x[2 * j + 1], LOG2E, -ml)) * inv);
         ps += p0 + p1;
         h2[j] = __floats2half2_rn(p0, p1);
       }
@@ -453,49 +532,51 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
       m1[i] = (FIELD << (p0 + BITS)) * 0x00010001u;
     }
     const unsigned char* prow = sc_b + (size_t)((g < a.n_rep ? g : 0) * a.pitch) * SB;
-    for (int it = warp; it < n_it; it += NW) {
-#pragma unroll(BITS == 4 ? 1 : 2)
-      for (int kq = 0; kq < 4; ++kq) {
-        const int tk = it * ITEM + 16 * kq;
-        if (tk >= n_tok) break;
-        uint32_t p0 = *reinterpret_cast<const uint32_t*>(prow + (size_t)tk * SB + 4 * c);
-        uint32_t p1 = *reinterpret_cast<const uint32_t*>(prow + (size_t)(tk + 8) * SB + 4 * c);
-        if (g >= a.n_rep) { p0 = 0u; p1 = 0u; }
-        const uint8_t* r[4];
+    struct Words { uint32_t w[4][WORDS]; };       // rows of tokens 2c, 2c+1, 2c+8, 2c+9 (4 bits: the lane's word pairs)
+    auto load = [&](Words& W, int m) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)      // tokens past the end have p = 0
-          r[i] = ev + (int64_t)min(tk + 2 * c + (i & 1) + 8 * (i >> 1), n_tok - 1) * ROWB;
+      for (int i = 0; i < 4; ++i) {               // tokens past the end have p = 0
+        const uint8_t* r = ev + (int64_t)min(16 * m + 2 * c + (i & 1) + 8 * (i >> 1), n_tok - 1) * ROWB;
         if (BITS == 4) {
-          uint2 w[4][4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int qd = 0; qd < 4; ++qd) w[i][qd] = *reinterpret_cast<const uint2*>(r[i] + 16 * qd + 8 * (g >> 2));
 #pragma unroll
           for (int qd = 0; qd < 4; ++qd) {
-            const uint32_t xa = prmt(w[0][qd].x, w[1][qd].x, sel), ya = prmt(w[2][qd].x, w[3][qd].x, sel);
-            mma_f16(acc[2 * qd], xa & m0[0], xa & m1[0], ya & m0[0], ya & m1[0], p0, p1);
-            const uint32_t xb = prmt(w[0][qd].y, w[1][qd].y, sel), yb = prmt(w[2][qd].y, w[3][qd].y, sel);
-            mma_f16(acc[2 * qd + 1], xb & m0[0], xb & m1[0], yb & m0[0], yb & m1[0], p0, p1);
+            const uint2 v = *reinterpret_cast<const uint2*>(r + 16 * qd + 8 * (g >> 2));
+            W.w[i][2 * qd] = v.x; W.w[i][2 * qd + 1] = v.y;
           }
         } else {
-          uint32_t w[4][WORDS];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int q4 = 0; q4 < WORDS / 4; ++q4) {
-              const uint4 v = reinterpret_cast<const uint4*>(r[i])[q4];
-              w[i][4 * q4] = v.x; w[i][4 * q4 + 1] = v.y; w[i][4 * q4 + 2] = v.z; w[i][4 * q4 + 3] = v.w;
-            }
-#pragma unroll
-          for (int wd = 0; wd < WORDS; ++wd) {
-            const uint32_t x = prmt(w[0][wd], w[1][wd], sel), y = prmt(w[2][wd], w[3][wd], sel);
-#pragma unroll
-            for (int i = 0; i < NM; ++i)
-              mma_f16(acc[(wd * NM + i) & 7], x & m0[i], x & m1[i], y & m0[i], y & m1[i], p0, p1);
+          for (int q4 = 0; q4 < WORDS / 4; ++q4) {
+            const uint4 v = reinterpret_cast<const uint4*>(r)[q4];
+            W.w[i][4 * q4] = v.x; W.w[i][4 * q4 + 1] = v.y; W.w[i][4 * q4 + 2] = v.z; W.w[i][4 * q4 + 3] = v.w;
           }
         }
       }
+    };
+    auto compute = [&](const Words& W, int m) {   // columns past the last head take the first one's; they are not kept
+      const uint32_t p0 = *reinterpret_cast<const uint32_t*>(prow + (size_t)(16 * m) * SB + 4 * c);
+      const uint32_t p1 = *reinterpret_cast<const uint32_t*>(prow + (size_t)(16 * m + 8) * SB + 4 * c);
+      constexpr int NWD = 8 / NM;                 // words a row: m-tiles NM wd .. NM wd + NM - 1
+#pragma unroll
+      for (int wd = 0; wd < NWD; ++wd) {
+        const uint32_t x = prmt(W.w[0][wd], W.w[1][wd], sel), y = prmt(W.w[2][wd], W.w[3][wd], sel);
+#pragma unroll
+        for (int i = 0; i < NM; ++i)
+          mma_f16(acc[wd * NM + i], x & m0[i], x & m1[i], y & m0[i], y & m1[i], p0, p1);
+      }
+    };
+    if (BITS == 1) {                              // the next tile's words are requested ahead; more bits leave no registers for it
+      Words W0, W1;
+      if (m_first < m_last) load(W0, m_first);
+#pragma unroll 1
+      for (int m = m_first; m < m_last; m += 2) {
+        if (m + 1 < m_last) load(W1, m + 1);
+        compute(W0, m);
+        if (m + 2 < m_last) load(W0, m + 2);
+        if (m + 1 < m_last) compute(W1, m + 1);
+      }
+    } else {
+#pragma unroll(BITS == 4 ? 1 : 2)
+      for (int m = m_first; m < m_last; ++m) { Words W; load(W, m); compute(W, m); }
     }
   }
   // full-precision segments: warp w owns channels 32 (w / 2) .. + 31 of every other 16 tokens; system and text keys are summed

@@ -31,3 +31,17 @@ def test_u8_single_launch_edges(bits, dtype, B, hq, hkv, t_vis, t_txt, sys_len):
     assert torch.equal(torch.isfinite(ref.float()), torch.isfinite(out.cpu().float()))
     assert rel_l2(torch.where(ok, out.cpu().float(), 0.), torch.where(ok, ref.float(), 0.)) <= 1e-2
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("q_scale,fp_scale", [(0.02, 1.0), (1.0, 4.0), (1.0, 0.05)])
+def test_u8_maximum_from_the_extremes(dtype, q_scale, fp_scale):
+    """Scores within 3 of each other, which the calibration turns around; full-precision scores of some CTAs far above the visual
+    ones, so that a CTA's maximum is not the cluster's; far below.  bfloat16 probabilities (2^-9) set the bar."""
+    from calibquant_b200 import calibquant as cq, ops
+    q, state, k_fp, v_fp = _step_inputs(1, 2, 8, 2, 5, 1111, 60, dtype, seed=7)
+    q, k_fp = q * q_scale, k_fp * fp_scale
+    ref = cqf.decode_attention(q, state, k_fp, v_fp, 1, 5)
+    out = cq.decode_attention(q.cuda(), {n: t.cuda() for n, t in state.items()}, k_fp.cuda(), v_fp.cuda(), 1, 5)
+    assert rel_l2(out.cpu(), ref) <= 1e-2
+    assert ops.device_status() == 0
