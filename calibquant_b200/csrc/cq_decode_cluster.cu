@@ -351,9 +351,16 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
       for (int ch = sub * CHUNKS / share; ch < (sub + 1) * CHUNKS / share; ++ch) {
         transpose_bytes<ROW>(base, ch, lane >> 2, c);
         __syncwarp();
+        // Below 4 bits the first products have a zero addend in place of cleared accumulators: 64 x 8 x 6656 at 2 bits 158.1 ->
+        // 156.2 us, 16 x 8 x 3328 at 1 bit 24.4 -> 23.9 (at 4 bits 9.8 -> 10.0 for 5 x 8 x 256, nothing elsewhere).
         float acc[GU][2][4];
+        if (BITS == 4)
 #pragma unroll
-        for (int i = 0; i < GU * 8; ++i) (&acc[0][0][0])[i] = 0.f;
+          for (int i = 0; i < GU * 8; ++i) (&acc[0][0][0])[i] = 0.f;
+        auto mma = [](float (&d)[4], bool first, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+          if (BITS < 4 && first) mma_f16_zero(d, a0, a1, a2, a3, b0, b1);
+          else mma_f16(d, a0, a1, a2, a3, b0, b1);
+        };
 #pragma unroll
         for (int kt = 0; kt < 8; ++kt) {
           const uint32_t ca = cell<ROW>(base, cell_row(kt, L.j, c), ch);
@@ -376,13 +383,13 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
             }
             if (BITS == 1) {
               const uint32_t lo = W[x], hi = W[x] >> 8;
-              mma_f16(acc[x][0], lo & L.m0[0], lo & L.m1[0], hi & L.m0[0], hi & L.m1[0], b0, b1);
-              mma_f16(acc[x][1], lo & L.m0[L.NM - 1], lo & L.m1[L.NM - 1], hi & L.m0[L.NM - 1], hi & L.m1[L.NM - 1], b0, b1);
+              mma(acc[x][0], kt == 0, lo & L.m0[0], lo & L.m1[0], hi & L.m0[0], hi & L.m1[0], b0, b1);
+              mma(acc[x][1], kt == 0, lo & L.m0[L.NM - 1], lo & L.m1[L.NM - 1], hi & L.m0[L.NM - 1], hi & L.m1[L.NM - 1], b0, b1);
             } else {
 #pragma unroll
               for (int i = 0; i < 2; ++i) {
                 const uint32_t lo = W[(BITS == 4 ? 0 : 2 * x) + i], hi = lo >> 8;
-                mma_f16(acc[x][i], lo & L.m0[0], lo & L.m1[0], hi & L.m0[0], hi & L.m1[0], b0, b1);
+                mma(acc[x][i], kt == 0, lo & L.m0[0], lo & L.m1[0], hi & L.m0[0], hi & L.m1[0], b0, b1);
               }
             }
           }
@@ -621,7 +628,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   {
     const uint32_t zoff = (uint32_t)(g < 4 ? g : 0) * 4u;
     const uint32_t z_and = g < 4 ? 0xffffffffu : 0u, z_or = g == 4 ? 0x3c003c00u : 0u;
-    const uint32_t lgh = lg + (uint32_t)((g < a.n_rep ? g : 0) * a.pitch * 2);
+    const uint32_t lgh = lg + (uint32_t)((g < a.n_rep ? g : 0) * a.pitch * 2);      // columns past the last head are not kept
     const uint32_t odd = (lane >> 3) & 1;      // pairs of odd k-steps are swapped (see transpose_bytes)
     const uint32_t sel_lo = odd ? 0x1054u : 0x5410u, sel_hi = odd ? 0x3276u : 0x7632u;
     for (int it = warp; it < n_u * V_SHARE && !failed; it += NW) {
@@ -648,11 +655,10 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
         __syncwarp();
 #pragma unroll
         for (int kq = 0; kq < VI / 16; ++kq) {
-          if (kq * 16 >= nt) break;
+          if ((BITS == 4 || kq % 2 == 0) && kq * 16 >= nt) break;      // live tokens come in groups of 32 (at 4 bits 24.2 -> 24.4 us, 4 x 8 x 5152)
           const int t0 = kq * 16 + 2 * c;                              // first token of the lane's first pair, in the item
           uint32_t pp0 = lds32(lgh + (uint32_t)(u * UNIT_TOK + tq + t0) * 2u), pp1 = lds32(lgh + (uint32_t)(u * UNIT_TOK + tq + t0 + 8) * 2u);
           if (kq & 1) { pp0 = prmt(pp0, pp0, 0x1032); pp1 = prmt(pp1, pp1, 0x1032); }
-          if (g >= a.n_rep) { pp0 = 0u; pp1 = 0u; }
           const uint4 s0 = lds128(vs_b + (uint32_t)t0 * 8u), s1 = lds128(vs_b + (uint32_t)(t0 + 8) * 8u);
           const uint32_t z0 = lds32(vm_b + (uint32_t)t0 * 8u + zoff), z1 = lds32(vm_b + (uint32_t)(t0 + 8) * 8u + zoff);
           const uint32_t bA[4] = {hmul2_u32(pp0, s0.x), hmul2_u32(pp0, s0.y), hmul2_u32(pp0, s0.z), hmul2_u32(pp0, s0.w)};
