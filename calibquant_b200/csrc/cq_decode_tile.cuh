@@ -6,8 +6,6 @@
 #include <cuda.h>
 #include <string.h>
 
-#include <utility>
-
 #include "cq_common.cuh"
 #include "cq_ptx.cuh"
 
@@ -182,24 +180,6 @@ inline bool make_v_map(CUtensorMap* tm_v, const void* code, uint64_t tokens) {
   if (BITS == 1) { memset(tm_v, 0, sizeof(*tm_v)); return true; }
   return make_map(tm_v, code, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, 4 * BITS, tokens,
                   BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, 4 * BITS, 256);
-}
-
-// Launch with the programmatic-stream-serialization attribute: the kernel may begin (up to its pdl_wait())
-// while the previous kernel of the stream drains.
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
 }  // namespace mma

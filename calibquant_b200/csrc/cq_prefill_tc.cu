@@ -248,6 +248,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     stage_done = 0;
     mbar_fence_init();
   }
+  // The launch before this one may still run up to here.  The wait comes before the tensor memory is taken: a kernel that
+  // this one waits for must not have to wait for it.
+  pdl_wait();
   if (warp == MMA_WARP) tmem_alloc(&tmem_base_s, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
@@ -647,8 +650,10 @@ int prefill_tc_run(const void* q, const void* k, const void* v, void* out, int b
   const unsigned tiles = (unsigned)((t_len + rows - 1) / rows), heads = (unsigned)(p.pair ? hq / 2 : hq);
   p.by_length = (int64_t)batch * t_len * hkv * 2 * 128 * 2 <= (int64_t)64 << 20 && tiles <= 65535u ? 1 : 0;      // half of L2
   const dim3 grid = p.by_length ? dim3(heads, (unsigned)batch, tiles) : dim3(tiles, heads, (unsigned)batch);
-  if (is_bf16) prefill_tc_kernel<true><<<grid, THREADS, SMEM_BYTES, st>>>(tq, tk, tv, to, p);
-  else prefill_tc_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(tq, tk, tv, to, p);
+  if (launch_pdl(is_bf16 ? prefill_tc_kernel<true> : prefill_tc_kernel<false>, grid, dim3(THREADS), SMEM_BYTES, st, tq, tk, tv, to, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return CQ_ERR_LAUNCH;
+  }
   return check_launch();
 }
 

@@ -212,6 +212,13 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
 // pdl_launch_dependents() lets the next kernel in the stream start early once every CTA has called it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The same for a kernel that reads through the read-only path: such loads may be moved over a wait that they do not
+// depend on, so the pointer that they start from comes out of the wait.
+template <typename P>
+__device__ __forceinline__ const P* pdl_wait_for(const P* p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+  return p;
+}
 
 }  // namespace ptx
 }  // namespace cq
