@@ -71,6 +71,11 @@ inline int check_launch() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CQ_OK : CQ_ERR_LAUNCH;
 }
+inline int launched(cudaError_t e) {      // what launch_pdl gave
+  if (e == cudaSuccess) return check_launch();
+  (void)cudaGetLastError();
+  return CQ_ERR_LAUNCH;
+}
 
 inline int sm_count() {      // of the current device
   int dev = 0, v = 0;

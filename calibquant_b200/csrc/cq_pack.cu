@@ -7,6 +7,7 @@
 //   code  = rint_half_even(clamp(y, 0, 2^b - 1))
 // word w of a row holds elements w*fpi .. w*fpi+fpi-1, element i in bits [i*b, (i+1)*b).
 #include "cq_common.cuh"
+#include "cq_ptx.cuh"
 #include <cstdlib>
 #include <type_traits>
 
@@ -219,6 +220,7 @@ pack_last_dim_group_kernel(const T* __restrict__ data, int64_t n_groups, int32_t
   using T2 = typename Pk<T>::T2;
   constexpr int LEVELS = (1 << BITS) - 1;
   const int64_t grp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  data = ptx::pdl_wait_for(data);            // every thread, before the first access (see pack_k_per_channel_kernel)
   if (grp >= n_groups) return;
   uint4 raw[4];
   const uint4* src = reinterpret_cast<const uint4*>(data) + grp * 4;
@@ -228,7 +230,7 @@ pack_last_dim_group_kernel(const T* __restrict__ data, int64_t n_groups, int32_t
                                          t * view.stride_t + (grp & 3) * 32);
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) raw[k] = __ldg(src + k);
+  for (int k = 0; k < 4; ++k) raw[k] = ptx::ld_global16(src + k);
   const T2* xv = reinterpret_cast<const T2*>(raw);              // 16 pairs
   T2 mn2 = xv[0], mx2 = xv[0];
 #pragma unroll
@@ -321,6 +323,10 @@ pack_k_per_channel_kernel(const T* __restrict__ k, int heads, int64_t T_len,
   T (*scale_s)[SP] = reinterpret_cast<T (*)[SP]>(pack_smem + TILES_BYTES + kHeadDim * CP * 4);
   T (*mn_s)[SP] = scale_s + kHeadDim;
 
+  // The launch before this one may still drain: it wrote k, and may read what is written here.  Keys and values, back to back:
+  // 1 x 8 x 256 tokens 5.4 -> 4.7 us, 2 x 1280 8.6 -> 7.9, 4 x 3328 13.6 -> 13.0.  Neither kernel lets the next launch come up
+  // before its own CTAs have left: early CTAs then crowd on the SMs that are free at that moment (2 x 1280 10.5).
+  k = ptx::pdl_wait_for(k);
   const int bh = blockIdx.y;
   const int b = bh / heads, h = bh % heads;
   const int64_t span0 = (int64_t)blockIdx.x * SPAN;
@@ -474,12 +480,13 @@ int launch_pack_last_dim(const void* data, int64_t rows, int64_t L, int bits, in
     const int64_t n_groups = n_chunks / 4;
     const int64_t gblocks = (n_groups + 255) / 256;
     if (gblocks > 0x7fffffffLL) return CQ_ERR_UNSUPPORTED;
+    cudaError_t e;
     switch (bits) {
-      case 1: pack_last_dim_group_kernel<T, 1><<<(unsigned)gblocks, 256, 0, st>>>(d, n_groups, code, s, m); break;
-      case 2: pack_last_dim_group_kernel<T, 2><<<(unsigned)gblocks, 256, 0, st>>>(d, n_groups, code, s, m); break;
-      default: pack_last_dim_group_kernel<T, 4><<<(unsigned)gblocks, 256, 0, st>>>(d, n_groups, code, s, m); break;
+      case 1: e = launch_pdl(pack_last_dim_group_kernel<T, 1>, dim3((unsigned)gblocks), dim3(256), 0, st, d, n_groups, code, s, m, RowView{}); break;
+      case 2: e = launch_pdl(pack_last_dim_group_kernel<T, 2>, dim3((unsigned)gblocks), dim3(256), 0, st, d, n_groups, code, s, m, RowView{}); break;
+      default: e = launch_pdl(pack_last_dim_group_kernel<T, 4>, dim3((unsigned)gblocks), dim3(256), 0, st, d, n_groups, code, s, m, RowView{}); break;
     }
-    return check_launch();
+    return launched(e);
   }
   switch (bits) {
     case 1: pack_last_dim_kernel<T, 1><<<(unsigned)blocks, 256, 0, st>>>(d, n_chunks, code, s, m); break;
@@ -508,11 +515,11 @@ int launch_pack_k(const void* k, int batch, int heads, int64_t T_len, int64_t sb
   T* s = static_cast<T*>(scale);
   T* m = static_cast<T*>(mn);
   switch (bits) {
-    case 1: pack_k_per_channel_kernel<T, 1><<<grid, 256, smem, st>>>(d, heads, T_len, sb, sh, st_, code, s, m); break;
-    case 2: pack_k_per_channel_kernel<T, 2><<<grid, 256, smem, st>>>(d, heads, T_len, sb, sh, st_, code, s, m); break;
-    default: pack_k_per_channel_kernel<T, 4><<<grid, 256, smem, st>>>(d, heads, T_len, sb, sh, st_, code, s, m); break;
+    case 1: e = launch_pdl(pack_k_per_channel_kernel<T, 1>, grid, dim3(256), smem, st, d, heads, T_len, sb, sh, st_, code, s, m); break;
+    case 2: e = launch_pdl(pack_k_per_channel_kernel<T, 2>, grid, dim3(256), smem, st, d, heads, T_len, sb, sh, st_, code, s, m); break;
+    default: e = launch_pdl(pack_k_per_channel_kernel<T, 4>, grid, dim3(256), smem, st, d, heads, T_len, sb, sh, st_, code, s, m); break;
   }
-  return check_launch();
+  return launched(e);
 }
 
 }  // namespace cq
@@ -549,9 +556,10 @@ extern "C" int cq_pack_v_per_token(const void* v, int batch, int heads, int64_t 
   const int64_t n_groups = (int64_t)batch * heads * T * 4;
   const int64_t gblocks = (n_groups + 255) / 256;
   if (gblocks > 0x7fffffffLL) return CQ_ERR_UNSUPPORTED;
+  cudaError_t e;
 #define CQ_LAUNCH_V(TYPE, B)                                                                              \
-  cq::pack_last_dim_group_kernel<TYPE, B><<<(unsigned)gblocks, 256, 0, st>>>(                              \
-      static_cast<const TYPE*>(v), n_groups, code, static_cast<TYPE*>(scale), static_cast<TYPE*>(mn), view)
+  e = cq::launch_pdl(cq::pack_last_dim_group_kernel<TYPE, B>, dim3((unsigned)gblocks), dim3(256), 0, st,    \
+                     static_cast<const TYPE*>(v), n_groups, code, static_cast<TYPE*>(scale), static_cast<TYPE*>(mn), view)
   if (dtype == CQ_DTYPE_F16) {
     if (bits == 1) CQ_LAUNCH_V(__half, 1); else if (bits == 2) CQ_LAUNCH_V(__half, 2); else CQ_LAUNCH_V(__half, 4);
   } else {
@@ -559,7 +567,7 @@ extern "C" int cq_pack_v_per_token(const void* v, int batch, int heads, int64_t 
     else CQ_LAUNCH_V(__nv_bfloat16, 4);
   }
 #undef CQ_LAUNCH_V
-  return cq::check_launch();
+  return cq::launched(e);
 }
 
 extern "C" int cq_pack_k_per_channel(const void* k, int batch, int heads, int64_t T, int D,

@@ -650,11 +650,7 @@ int prefill_tc_run(const void* q, const void* k, const void* v, void* out, int b
   const unsigned tiles = (unsigned)((t_len + rows - 1) / rows), heads = (unsigned)(p.pair ? hq / 2 : hq);
   p.by_length = (int64_t)batch * t_len * hkv * 2 * 128 * 2 <= (int64_t)64 << 20 && tiles <= 65535u ? 1 : 0;      // half of L2
   const dim3 grid = p.by_length ? dim3(heads, (unsigned)batch, tiles) : dim3(tiles, heads, (unsigned)batch);
-  if (launch_pdl(is_bf16 ? prefill_tc_kernel<true> : prefill_tc_kernel<false>, grid, dim3(THREADS), SMEM_BYTES, st, tq, tk, tv, to, p) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return CQ_ERR_LAUNCH;
-  }
-  return check_launch();
+  return launched(launch_pdl(is_bf16 ? prefill_tc_kernel<true> : prefill_tc_kernel<false>, grid, dim3(THREADS), SMEM_BYTES, st, tq, tk, tv, to, p));
 }
 
 }  // namespace cq

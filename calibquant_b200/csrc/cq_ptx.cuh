@@ -212,12 +212,18 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
 // pdl_launch_dependents() lets the next kernel in the stream start early once every CTA has called it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// The same for a kernel that reads through the read-only path: such loads may be moved over a wait that they do not
-// depend on, so the pointer that they start from comes out of the wait.
+// The same for a kernel whose loads are not volatile: they could be moved over a wait that they do not depend on, so the
+// pointer that they start from comes out of the wait.  What an overlapping launch wrote is not read through the read-only path
+// (ld.global.nc, __ldg, or a plain load from a __restrict__ pointer to const): ld_global16.
 template <typename P>
 __device__ __forceinline__ const P* pdl_wait_for(const P* p) {
   asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
   return p;
+}
+__device__ __forceinline__ uint4 ld_global16(const void* p) {
+  uint4 v;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 
 }  // namespace ptx

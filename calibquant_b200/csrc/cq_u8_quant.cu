@@ -45,11 +45,11 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
   uint4 kept[KEPT ? KEEP : 1];
   if (KEPT) {
 #pragma unroll
-    for (int u = 0; u < KEEP; ++u) kept[KEPT ? u : 0] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t_begin + tl + u * QE_LANES, t_end - 1) * st));
+    for (int u = 0; u < KEEP; ++u) kept[KEPT ? u : 0] = ptx::ld_global16(base + (int64_t)min(t_begin + tl + u * QE_LANES, t_end - 1) * st);
   }
   // extremes of the slice; every thread starts from a row of it, so no neutral element is needed
   {
-    const uint4 first = KEPT ? kept[0] : __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t_begin + tl, t_end - 1) * st));
+    const uint4 first = KEPT ? kept[0] : ptx::ld_global16(base + (int64_t)min(t_begin + tl, t_end - 1) * st);
     T2 mn[4], mx[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) mn[i] = mx[i] = reinterpret_cast<const T2*>(&first)[i];
@@ -67,7 +67,7 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
     for (int t = t_begin + tl; t < t_end; t += U * QE_LANES) {
       uint4 v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t + u * QE_LANES, t_end - 1) * st));
+      for (int u = 0; u < U; ++u) v[u] = ptx::ld_global16(base + (int64_t)min(t + u * QE_LANES, t_end - 1) * st);
 #pragma unroll
       for (int u = 0; u < U; ++u) take(v[u]);
     }
@@ -156,7 +156,7 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
         if (t_begin + u * QE_LANES < t_end) encode(t_begin + tl + u * QE_LANES, kept[KEPT ? u : 0]);
     } else {
       for (int t = t_begin + tl; t < t_last; t += QE_LANES)
-        encode(t, __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t, t_end - 1) * st)));
+        encode(t, ptx::ld_global16(base + (int64_t)min(t, t_end - 1) * st));
     }
     return;
   }
@@ -197,7 +197,7 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
       for (int t0 = t_begin + tl; t0 < t_last; t0 += U * QE_LANES) {
         uint4 v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)min(t0 + u * QE_LANES, t_end - 1) * st));
+        for (int u = 0; u < U; ++u) v[u] = ptx::ld_global16(base + (int64_t)min(t0 + u * QE_LANES, t_end - 1) * st);
 #pragma unroll
         for (int u = 0; u < U; ++u) encode(t0 + u * QE_LANES, v[u]);
       }
