@@ -1,5 +1,5 @@
-"""QJL score estimate on the 5th-generation tensor cores: edges of its tiles (16 groups), units (4 groups) and heads, against 64-bit
-arithmetic of the oracle's formula."""
+"""QJL score estimate on the 5th-generation tensor cores, against 64-bit arithmetic of the oracle's formula: calls of one unit (4
+groups) a CTA with every form of the operands, and calls of several tiles (4 to 16 groups) a CTA."""
 
 import math
 
@@ -49,6 +49,43 @@ def test_against_64_bits(n, rep, oc, so, given, dtype, pdtype):
     assert rel_l2(got, ref) <= 1e-5
     for head in range(2 * rep):
         assert rel_l2(got[:, head], ref[:, head]) <= 2e-5
+    assert lib().cq_qjl_status() == 0
+
+
+@pytest.mark.parametrize("kbh,n,rep,so,given", [
+    (64, 70, 4, 256, False),       # a ragged last tile
+    (64, 40, 3, 128, True),
+    (40, 99, 4, 256, False),       # heads change within a CTA
+    (160, 18, 4, 256, True),
+    (16, 257, 1, 128, False),
+    (37, 131, 2, 256, False),
+    (1200, 4, 4, 256, False),      # a head a unit: more tiles a CTA than the ring of totals has slots
+    (1300, 3, 3, 128, True),
+])
+def test_many_tiles_a_cta(kbh, n, rep, so, given):
+    """Every barrier in its later phases, both operand buffers, the ring of totals, changes of the head within a CTA.  More than four
+    units a CTA make at least two tiles, whatever their size (four units at most).  Another query for every head; bounds as
+    above."""
+    from calibquant_b200 import ops
+    from calibquant_b200._lib import lib
+    assert kbh * -(-n // 4) > 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(kbh)
+    rand = lambda *shape: torch.rand(*shape, generator=g, device="cuda")
+    S = torch.randn(128, 256, generator=g, device="cuda")
+    q = (torch.randn(1, kbh * rep, 1, 128, generator=g, device="cuda") * (1 + 5 * rand(1, kbh * rep, 1, 1))).half()
+    bits, obits = (torch.randint(0, 256, (1, kbh, n, 32, w // 8), generator=g, dtype=torch.uint8, device="cuda") for w in (256, so))
+    onorm = (rand(1, kbh, n, 32) * 4).half()
+    knorm = (onorm.float() + rand(1, kbh, n, 32) * 6).half()
+    idx = rand(1, kbh, n, 128).topk(32, -1)[1].to(torch.uint8)
+    qs = (q.float().view(-1, 128) @ S).view(1, kbh * rep, 1, 256) if given else None
+    args = (bits, obits, knorm, onorm, idx, qs, q, S)
+    got = ops.qjl_gqa_score(*args).cpu()
+    for _ in range(3):
+        assert torch.equal(ops.qjl_gqa_score(*args).cpu(), got)
+    ref = _exact(*[None if t is None else t.cpu() for t in args])
+    assert rel_l2(got, ref) <= 1e-5
+    err, size = (got.double() - ref).view(kbh, rep, n, 32).norm(dim=-1), ref.view(kbh, rep, n, 32).norm(dim=-1)
+    assert float((err / size).max()) <= 4e-5          # group by group
     assert lib().cq_qjl_status() == 0
 
 
