@@ -79,6 +79,31 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
   lo = h2_bits(__floats2half2_rn(a - f.x, b - f.y));
 }
 
+// A channel named more than once counts as often.  The products have it once; what the further mentions add to a key's scores is
+// summed here in fp32 (none of the quantizers names a channel twice; as a factor of the fp16 query, three mentions of an element
+// lost its last bits).  A call, so that it takes no registers from the kernel.
+template <typename T, typename TP>
+__device__ __noinline__ void further_mentions(const uint8_t* idx, int oc, const uint8_t* sign_in, const uint8_t* sign_out, int o_sketch, float nk,
+                                              float no, const T* query, int n_rep, const TP* proj, float* scores, int64_t row_len) {
+  const float norm_in = 1.2533141373155001f / (float)SKETCH * sqrtf(fmaxf(nk * nk - no * no, 0.f)), norm_out = 1.2533141373155001f / (float)o_sketch * no;
+  uint64_t seen_lo = 0, seen_hi = 0;
+  for (int i = 0; i < oc; ++i) {
+    const int d = idx[i] & (kHeadDim - 1);
+    const uint64_t bit = 1ull << (d & 63);
+    const bool again = ((d < 64 ? seen_lo : seen_hi) & bit) != 0;
+    if (d < 64) seen_lo |= bit; else seen_hi |= bit;
+    if (!again) continue;
+    float in = 0.f, out = 0.f;                       // signs times the channel's projections
+    for (int p = 0; p < SKETCH; ++p) {
+      const float x = proj_f<TP>(proj[(int64_t)d * SKETCH + p]);
+      in += (sign_in[p >> 3] >> (p & 7)) & 1 ? x : -x;
+      if (p < o_sketch) out += (sign_out[p >> 3] >> (p & 7)) & 1 ? x : -x;
+    }
+    for (int h = 0; h < n_rep; ++h)
+      scores[h * row_len] += Elem<T>::to_f(query[(int64_t)h * kHeadDim + d]) * (norm_out * out - norm_in * in);
+  }
+}
+
 template <typename T, typename TP>
 __global__ void __launch_bounds__(THREADS, 1)
 score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t* __restrict__ key_outlier_quant,
@@ -97,7 +122,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
   __shared__ float tot_in_s[8][MAX_TG][R], tot_out_s[8][MAX_TG][R];            // sums of q_out S
   __shared__ float tot_q_s[8][R], down_s[8][R], up_s[8][R];                    // sums of q S; powers of two of the queries' scaling
   __shared__ float smax_s[N_WARPS];
-  __shared__ uint8_t count_s[N_QUERY][kHeadDim];
+  __shared__ int again_s;                                                      // does a group of the CTA name a channel more than once?
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile0 = (int)((int64_t)blockIdx.x * a.n_tiles / gridDim.x), tile1 = (int)((int64_t)(blockIdx.x + 1) * a.n_tiles / gridDim.x);
   // A tile: number within the CTA, KV head, first group within the head.  (Divided out anew at every use, the positions were half
@@ -120,6 +145,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
   const int n_tiles = tile1 - tile0;
 
   if (tid == 0) {
+    again_s = 0;
     mbar_init(&bar_q, N_QUERY);
     mbar_init(&bar_out, 1);
     mbar_init(&bar_out_free, N_SKETCH);
@@ -311,20 +337,20 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
         } else if (wq == 0 && qc == 0) {
           tot_q_s[slot][qh] = tot_q_s[(slot + 7) & 7][qh]; down_s[slot][qh] = down_s[(slot + 7) & 7][qh];
         }
-        uint8_t channel[PER];
-#pragma unroll
-        for (int j = 0; j < PER; ++j) channel[j] = ch_ahead[j];
-        fetch_channels(after(t));
-#pragma unroll
+        int missing = 0;                       // mentions less channels
+#pragma unroll 1
         for (int j = 0; j < PER; ++j) {
           const int gi = wq + N_QUERY * j, n = t.first + gi;
           if (gi >= a.tg) break;
+          uint32_t ch = ch_ahead[0];
+#pragma unroll
+          for (int i = 1; i < PER; ++i) ch = i == j ? ch_ahead[i] : ch;
           const uint8_t* idx = outlier_idx + ((int64_t)t.kbh * a.n_groups + n) * a.oc;
           uint32_t mask[4] = {0u, 0u, 0u, 0u};
           if (n < a.n_groups) {
             for (int i0 = 0; i0 < a.oc; i0 += 32) {
               const bool have = i0 + lane < a.oc;
-              const int d = i0 == 0 ? channel[j] & (kHeadDim - 1) : have ? idx[i0 + lane] & (kHeadDim - 1) : 0;
+              const int d = i0 == 0 ? ch & (kHeadDim - 1) : have ? idx[i0 + lane] & (kHeadDim - 1) : 0;
 #pragma unroll
               for (int m = 0; m < 4; ++m) mask[m] |= __reduce_or_sync(0xffffffffu, have && (d >> 5) == m ? 1u << (d & 31) : 0u);
             }
@@ -336,28 +362,15 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
             const uint32_t m = (i < 4 ? lo8 : hi8) >> (2 * (i & 3));
             w[i] = qw[i] & (((m & 1u) ? 0x0000ffffu : 0u) | ((m & 2u) ? 0xffff0000u : 0u));
           }
-          if (n < a.n_groups && __popc(mask[0]) + __popc(mask[1]) + __popc(mask[2]) + __popc(mask[3]) != a.oc) {
-            // a channel named more than once counts as often
-            uint8_t* cnt = count_s[wq];
-            reinterpret_cast<uint32_t*>(cnt)[lane] = 0u;
-            __syncwarp();
-            if (lane == 0)
-              for (int i = 0; i < a.oc; ++i) ++cnt[idx[i] & (kHeadDim - 1)];
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint8_t* c = cnt + (i >> 2) * 64 + qc * 8 + (i & 3) * 2;
-              const float2 f = h2_floats(w[i]);
-              w[i] = h2_bits(__floats2half2_rn(f.x * (float)c[0], f.y * (float)c[1]));
-            }
-            __syncwarp();
-          }
+          if (n < a.n_groups) missing += a.oc - (__popc(mask[0]) + __popc(mask[1]) + __popc(mask[2]) + __popc(mask[3]));
           put_row(gi * R + qh, w);
           const float ti = dot(w, sum_in_s), to = a.o_sketch == SKETCH ? ti : dot(w, sum_out_s);
           if (qc == 0) { tot_in_s[slot][gi][qh] = ti; tot_out_s[slot][gi][qh] = to; }
         }
         fence_proxy_async_smem();
+        if (missing != 0) again_s = 1;         // (tested group by group it cost 8 x 8 x 16384 keys 2.4 us)
         arrive(&bar_q);
+        fetch_channels(after(t));
       };
 
       Tile t = first_tile();
@@ -518,6 +531,15 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
         }
         t = next;
       }
+      // every further mention of a channel, once the products' scores are written (within the loop it cost every call 6 %)
+      if (again_s)
+        for (Tile t = first_tile(); t.i < n_tiles && ok; t = after(t))
+          for (int n = t.first + quad; n < min(t.first + a.tg, a.n_groups); n += UNIT_G) {
+            const int64_t group = (int64_t)t.kbh * a.n_groups + n, key = group * G + lane;
+            further_mentions<T, TP>(outlier_idx + group * a.oc, a.oc, key_quant + key * (SKETCH / 8), key_outlier_quant + key * (a.o_sketch / 8), a.o_sketch,
+                                    Elem<T>::to_f(key_norm[key]), Elem<T>::to_f(key_outlier_norm[key]), query + (int64_t)t.kbh * a.n_rep * kHeadDim,
+                                    a.n_rep, proj, scores + (int64_t)t.kbh * a.n_rep * row_len + n * G + lane, row_len);
+          }
     }
     if (!ok && lane == 0) atomicExch(status, CQ_ERR_TIMEOUT);
   }

@@ -102,3 +102,35 @@ def test_other_heads_keep_their_scores():
     q[0, 2, 0, 7] = float("inf")
     got = ops.qjl_gqa_score(*args, None, q.cuda(), S.cuda())
     assert torch.equal(got[:, [0, 1, 3]], base[:, [0, 1, 3]]) and not torch.isfinite(got[:, 2]).any()
+
+
+def _one(dtype, S, q, seed=3, n=9, oc=32, onorm_is=None, knorm_is=None, given=None):
+    """(arguments, exact scores) of one KV head's queries q over n groups."""
+    g = torch.Generator().manual_seed(seed)
+    bits, obits = (torch.randint(0, 256, (1, 1, n, 32, 32), generator=g, dtype=torch.uint8) for _ in range(2))
+    onorm = torch.rand(1, 1, n, 32, generator=g).to(dtype) if onorm_is is None else torch.full((1, 1, n, 32), onorm_is, dtype=dtype)
+    knorm = (torch.rand(1, 1, n, 32, generator=g) + 3).to(dtype) if knorm_is is None else torch.full((1, 1, n, 32), knorm_is, dtype=dtype)
+    idx = torch.stack([torch.randperm(128, generator=g)[:oc] for _ in range(n)]).view(1, 1, n, oc).to(torch.uint8)
+    return [bits, obits, knorm, onorm, idx, given, q.to(dtype), S]
+
+
+def _error(args):
+    from calibquant_b200 import ops
+    got = ops.qjl_gqa_score(*[None if t is None else t.cuda() for t in args]).cpu()
+    return rel_l2(got, _exact(*args))
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -10])
+@pytest.mark.parametrize("given", [False, True])
+def test_channels_named_many_times(scale, given):
+    """Three and more mentions of an fp16 element have more bits than fp16, and with a small projection more than its range.  The
+    projection is fp16, so that only sums round."""
+    g = torch.Generator().manual_seed(11)
+    S, q = (torch.randn(128, 256, generator=g) * scale).half().float(), torch.randn(1, 4, 1, 128, generator=g)
+    args = _one(torch.half, S, q, given=None if not given else (q.half().float() @ S))
+    idx = args[4]
+    idx[:, :, 0, 1:3] = idx[:, :, 0, :1]
+    idx[:, :, 4, 5:12] = idx[:, :, 4, :1]
+    idx[:, :, 5] = idx[:, :, 5, :1]             # one channel, 32 times
+    idx[:, :, 8, 20:] = idx[:, :, 8, :12]       # twelve channels twice
+    assert _error(args) <= 1e-5
