@@ -302,8 +302,8 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
       auto build_queries = [&](const Tile& t) {
         const int slot = t.i & 7;
         if (t.fresh) {
-          // scaled so that the elements and their sums with 128 channels stay below 2^15: fp16 operands keep what they can of the
-          // remainders
+          // scaled so that the elements, their sums with 128 channels and a given q S stay below 2^15: fp16 operands keep what they
+          // can of the remainders
           const T* src = query + ((int64_t)t.kbh * a.n_rep + qh) * kHeadDim + qc * 8;
           float x[16], m = 0.f, up = 1.f, down = 1.f;
 #pragma unroll
@@ -313,8 +313,22 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
           }
 #pragma unroll
           for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-          const float bound = fmaxf(128.f * smax, 1.f) * m;
-          if (m > 0.f && bound < INFINITY) {
+          float tq = 0.f, sketch_max = 0.f;      // of a given q S
+          if (query_sketch) {
+            if (qh < a.n_rep)
+              for (int p = qc; p < SKETCH; p += 8) {
+                const float v = query_sketch[((int64_t)t.kbh * a.n_rep + qh) * SKETCH + p];
+                tq += v;
+                sketch_max = fmaxf(sketch_max, fabsf(v));
+              }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+              tq += __shfl_xor_sync(0xffffffffu, tq, o);
+              sketch_max = fmaxf(sketch_max, __shfl_xor_sync(0xffffffffu, sketch_max, o));
+            }
+          }
+          const float bound = fmaxf(fmaxf(128.f * smax, 1.f) * m, sketch_max);
+          if (bound > 0.f && bound < INFINITY) {
             const int e = (int)(__float_as_uint(bound) >> 23) - 127;       // bound < 2^(e+1)
             const int s = max(-126, min(126, 14 - e));
             up = __uint_as_float((uint32_t)(127 + s) << 23);
@@ -324,14 +338,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
           for (int i = 0; i < 8; ++i) qw[i] = h2_bits(__floats2half2_rn(x[2 * i] * up, x[2 * i + 1] * up));
           if (wq == 0) {
             put_row(a.tg * R + qh, qw);
-            float tq = dot(qw, sum_in_s);
-            if (query_sketch) {
-              tq = 0.f;
-              if (qh < a.n_rep)
-                for (int p = qc; p < SKETCH; p += 8) tq += query_sketch[((int64_t)t.kbh * a.n_rep + qh) * SKETCH + p] * up;
-#pragma unroll
-              for (int o = 1; o < 8; o <<= 1) tq += __shfl_xor_sync(0xffffffffu, tq, o);
-            }
+            tq = query_sketch ? tq * up : dot(qw, sum_in_s);
             if (qc == 0) { tot_q_s[slot][qh] = tq; down_s[slot][qh] = down; up_s[slot][qh] = up; }
           }
         } else if (wq == 0 && qc == 0) {

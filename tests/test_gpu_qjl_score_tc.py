@@ -134,3 +134,17 @@ def test_channels_named_many_times(scale, given):
     idx[:, :, 5] = idx[:, :, 5, :1]             # one channel, 32 times
     idx[:, :, 8, 20:] = idx[:, :, 8, :12]       # twelve channels twice
     assert _error(args) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.half, torch.bfloat16])
+def test_given_sketch_of_another_size(dtype):
+    """The sketch of the query is an argument of its own: larger than the query and the projection let expect, and of a zero query."""
+    g = torch.Generator().manual_seed(12)
+    S, q = torch.randn(128, 256, generator=g), torch.randn(1, 4, 1, 128, generator=g)
+    q[:, 1] = 0
+    given = torch.randn(1, 4, 1, 256, generator=g) * torch.tensor([3e4, 10., 3e4, 1.]).view(1, 4, 1, 1)
+    args = _one(dtype, S, q, given=given)
+    for head in range(4):
+        one = args[:5] + [given[:, head:head + 1], args[6][:, head:head + 1], S]
+        assert _error(one) <= 1e-5
+    assert _error(args) <= 1e-5
