@@ -327,10 +327,13 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
               sketch_max = fmaxf(sketch_max, __shfl_xor_sync(0xffffffffu, sketch_max, o));
             }
           }
-          const float bound = fmaxf(fmaxf(128.f * smax, 1.f) * m, sketch_max);
+          // (in units of a power of two near the largest element: 128 channels of bfloat16 numbers can leave fp32's range)
+          const int em = m > 0.f ? max(-126, min(126, (int)(__float_as_uint(m) >> 23) - 127)) : 0;
+          const float unit = __uint_as_float((uint32_t)(127 - em) << 23);
+          const float bound = fmaxf(fmaxf(128.f * smax, 1.f) * (m * unit), sketch_max * unit);
           if (bound > 0.f && bound < INFINITY) {
             const int e = (int)(__float_as_uint(bound) >> 23) - 127;       // bound < 2^(e+1)
-            const int s = max(-126, min(126, 14 - e));
+            const int s = max(-126, min(126, 14 - e - em));
             up = __uint_as_float((uint32_t)(127 + s) << 23);
             down = __uint_as_float((uint32_t)(127 - s) << 23);
           }

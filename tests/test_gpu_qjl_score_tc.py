@@ -148,3 +148,11 @@ def test_given_sketch_of_another_size(dtype):
         one = args[:5] + [given[:, head:head + 1], args[6][:, head:head + 1], S]
         assert _error(one) <= 1e-5
     assert _error(args) <= 1e-5
+
+
+def test_bfloat16_queries_near_the_end_of_the_range():
+    """128 channels of such numbers are past fp32's range, their scores with small keys are not."""
+    g = torch.Generator().manual_seed(13)
+    S, q = torch.randn(128, 256, generator=g), torch.randn(1, 4, 1, 128, generator=g) * 1e37
+    assert _error(_one(torch.bfloat16, S, q, onorm_is=2.0 ** -9, knorm_is=2.0 ** -8)) <= 1e-5
+    assert _error(_one(torch.bfloat16, S, q * 1e-70, onorm_is=1., knorm_is=2.)) <= 1e-5
