@@ -219,12 +219,12 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
 #pragma unroll
           for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-            for (int hl = 0; hl < 2; ++hl)
+            for (int hl = 1; hl >= 0; --hl)      // the tensor core truncates as it adds: first what is small
 #pragma unroll
               for (int ks = 0; ks < 8; ++ks)
                 umma(tm + T_OUT + (uint32_t)mt * T_OUT_TILE,
                      td + (uint64_t)((hl * TAB_BYTES + (ks >> 2) * TAB_PANEL + mt * 128 * 128 + (ks & 3) * 32) >> 4),
-                     qd + (uint64_t)(((ks >> 2) * Q_PANEL + (ks & 3) * 32) >> 4), idesc, (hl > 0 || ks > 0) ? 1u : 0u);
+                     qd + (uint64_t)(((ks >> 2) * Q_PANEL + (ks & 3) * 32) >> 4), idesc, (hl == 0 || ks > 0) ? 1u : 0u);
           umma_commit(&bar_out);
         }
         __syncwarp();

@@ -156,3 +156,15 @@ def test_bfloat16_queries_near_the_end_of_the_range():
     S, q = torch.randn(128, 256, generator=g), torch.randn(1, 4, 1, 128, generator=g) * 1e37
     assert _error(_one(torch.bfloat16, S, q, onorm_is=2.0 ** -9, knorm_is=2.0 ** -8)) <= 1e-5
     assert _error(_one(torch.bfloat16, S, q * 1e-70, onorm_is=1., knorm_is=2.)) <= 1e-5
+
+
+@pytest.mark.parametrize("given", [False, True])
+def test_inlier_part_of_a_query_in_the_outlier_channels(given):
+    """Outlier norms of zero: what counts is q S - q_out S, 1/170 of either.  Eight additions of the hi rows' products lose 2^-24 of them
+    each in the mean: 8 x 170 x 2^-24 (where the lo rows' follow, sixteen)."""
+    g = torch.Generator().manual_seed(14)
+    S, q = torch.randn(128, 256, generator=g), torch.randn(1, 4, 1, 128, generator=g)
+    q[..., :32] *= 300
+    args = _one(torch.half, S, q, onorm_is=0., knorm_is=3., given=None if not given else (q.half().double() @ S.double()).float())
+    args[4][...] = torch.arange(32, dtype=torch.uint8)
+    assert _error(args) <= 8.2e-5
