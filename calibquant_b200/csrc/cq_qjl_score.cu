@@ -156,6 +156,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
   if (warp == W_ISSUE) tmem_alloc(&tmem_s, 512);
   // S^T, rows of projections, as hi and lo in the swizzled K-major layout; lanes take neighbouring projections
   float smax = 0.f;
+  float* const part_s = reinterpret_cast<float*>(x_s);      // sums over 32 projections: [projection / 32][channel]; until the first sketches
 #pragma unroll 2
   for (int i = tid; i < SKETCH * 16; i += THREADS) {
     const int p = i & 255, pc = i >> 8;
@@ -164,35 +165,34 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
     for (int j = 0; j < 8; ++j) { x[j] = proj_f<TP>(proj[(int64_t)(pc * 8 + j) * SKETCH + p]); smax = fmaxf(smax, fabsf(x[j])); }
     uint32_t hi[4], lo[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) split2(x[2 * j], x[2 * j + 1], hi[j], lo[j]);
+    for (int j = 0; j < 4; ++j) {
+      split2(x[2 * j], x[2 * j + 1], hi[j], lo[j]);
+      // The sums are of the numbers that the products take: against sums of S itself, the rounding of small elements counted
+      // twice where the bit is set (elements of 1e-3: scores off by 2.5e-5, so by 1.7e-5)
+      const float2 h = h2_floats(hi[j]), l = h2_floats(lo[j]);
+      x[2 * j] = h.x + l.x;
+      x[2 * j + 1] = h.y + l.y;
+    }
+    // over the warp's 32 projections, channels dealt out over the lanes as the sums get fewer
+#pragma unroll
+    for (int n = 4, o = 16; n >= 1; n /= 2, o /= 2)
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        const bool up = lane & o;
+        const float other = __shfl_xor_sync(0xffffffffu, up ? x[j] : x[j + n], o);
+        x[j] = (up ? x[j + n] : x[j]) + other;
+      }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+    if ((lane & 3) == 0) part_s[(p >> 5) * kHeadDim + pc * 8 + (lane >> 2)] = x[0];
     unsigned char* dst = tab_s + (pc >> 3) * TAB_PANEL + p * 128 + (((pc & 7) ^ (p & 7)) << 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(dst + TAB_BYTES) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
   smax = warp_max(smax);
   if (lane == 0) smax_s[warp] = smax;
-  {                                                          // channel sums, the rows of a warp in flight together
-    constexpr int ROWS = (kHeadDim + N_WARPS - 1) / N_WARPS;
-    float sum[ROWS], sum_o[ROWS];
-#pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-      sum[i] = sum_o[i] = 0.f;
-#pragma unroll
-      for (int j = 0; j < SKETCH / 32; ++j) {
-        const int d = min(warp + N_WARPS * i, kHeadDim - 1);
-        const float x = proj_f<TP>(proj[(int64_t)d * SKETCH + 32 * j + lane]);
-        sum[i] += x;
-        if (32 * j < a.o_sketch) sum_o[i] += x;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-      const float si = warp_sum(sum[i]), so = warp_sum(sum_o[i]);
-      if (lane == 0 && warp + N_WARPS * i < kHeadDim) { sum_in_s[warp + N_WARPS * i] = si; sum_out_s[warp + N_WARPS * i] = so; }
-    }
-  }
-  // rows of no query, columns of no sketch
-  for (int i = tid; i < (Q_BYTES + 2 * X_BYTES) / 16; i += THREADS) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0u, 0u, 0u, 0u);
+  // rows of no query
+  for (int i = tid; i < Q_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0u, 0u, 0u, 0u);
   fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -267,6 +267,19 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
       // ================= masked queries =================
       const int wq = warp - W_QUERY;
       for (int w = 0; w < N_WARPS; ++w) smax = fmaxf(smax, smax_s[w]);
+      {
+        const int d = tid - W_QUERY * 32;
+        float sum = 0.f, sum_o = 0.f;
+#pragma unroll
+        for (int i = 0; i < SKETCH / 32; ++i) {
+          const float x = part_s[i * kHeadDim + d];
+          sum += x;
+          if (32 * i < a.o_sketch) sum_o += x;
+        }
+        sum_in_s[d] = sum;
+        sum_out_s[d] = sum_o;
+        asm volatile("bar.sync 1, %0;" ::"n"(N_QUERY * 32) : "memory");
+      }
       // ---- queries with their group's outlier channels: a warp takes every fourth group, a lane head lane / 8, channels
       // 8 (lane % 8) .. + 7 and + 64
       uint32_t qw[8];                       // the lane's sixteen channels, scaled by a power of two

@@ -168,3 +168,10 @@ def test_inlier_part_of_a_query_in_the_outlier_channels(given):
     args = _one(torch.half, S, q, onorm_is=0., knorm_is=3., given=None if not given else (q.half().double() @ S.double()).float())
     args[4][...] = torch.arange(32, dtype=torch.uint8)
     assert _error(args) <= 8.2e-5
+
+
+def test_small_projection():
+    """Elements of 1e-3 are kept to 2^-25, 1.7e-5 of them in the mean; a sum of theirs is off by as much."""
+    g = torch.Generator().manual_seed(15)
+    S, q = torch.randn(128, 256, generator=g) * 1e-3, torch.randn(1, 4, 1, 128, generator=g)
+    assert _error(_one(torch.half, S, q, n=60)) <= 2.1e-5
