@@ -598,7 +598,8 @@ int run(const uint8_t* kq, const uint8_t* koq, const void* kn, const void* kon, 
   Args a;
   a.n_kbh = n_kbh; a.n_groups = n_groups; a.n_rep = n_rep; a.o_sketch = o_sketch; a.oc = oc;
   // groups per tile: the first product costs a tile about as much as two thirds of a unit, whatever its width; smaller tiles where
-  // they fill the SMs better
+  // they fill the SMs better or
+  // hold the same groups (1 x 4 groups: 11.2 us with a tile of 16, 10.0 with one of 4; on the warp MMA 10.8)
   a.n_tiles = 0;
   double best = 1e30;
   for (int tg = MAX_TG; tg >= UNIT_G; tg /= 2) {
@@ -607,7 +608,7 @@ int run(const uint8_t* kq, const uint8_t* koq, const void* kn, const void* kon, 
     if (tiles > 0x7fffffff) continue;
     const int units = tg < n_groups ? tg / UNIT_G : (n_groups + UNIT_G - 1) / UNIT_G;
     const double cost = (double)((tiles + sms - 1) / sms) * (units + 0.7);
-    if (cost < best) { best = cost; a.tg = tg; a.tiles_per_kbh = per; a.n_tiles = (int)tiles; }
+    if (cost <= best) { best = cost; a.tg = tg; a.tiles_per_kbh = per; a.n_tiles = (int)tiles; }
   }
   if (a.n_tiles == 0) return CQ_ERR_UNSUPPORTED;
   a.idesc_q = make_idesc(0, 0, 128, a.tg * R);
