@@ -18,7 +18,7 @@
 // Six roles of warps (below) hand these steps on through mbarriers.  What bounds it now: a tcgen05.mma of 128 rows takes ~70 cycles of
 // the pipe however few columns it has, 32 of them a unit and 32 a tile: 2600 of the 2900 cycles that a unit takes.  8 x 8 x 16384 keys,
 // 32 query heads: 129 -> 87 us; 1 x 8 x 512 keys 15.1 -> 10.2 us; error against 64-bit sums 4.6e-6 -> 7e-7 (the product truncates less
-// often than the warp MMA).  Every wait is bounded; on a timeout the CTA writes the status word, frees its tensor memory and returns.
+// often than the warp MMA).  Every wait is bounded; on a timeout the CTA writes the status word and NaN for its scores, frees its tensor memory and returns.
 #include <type_traits>
 
 #include "cq_common.cuh"
@@ -81,11 +81,13 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
 
 // A channel named more than once counts as often.  The products have it once; what the further mentions add to a key's scores is
 // summed here in fp32 (none of the quantizers names a channel twice; as a factor of the fp16 query, three mentions of an element
-// lost its last bits).  A call, so that it takes no registers from the kernel.
+// lost its last bits).  With oc < 0 they become NaN.  A call, so that it takes no registers from the kernel.
 template <typename T, typename TP>
 __device__ __noinline__ void further_mentions(const uint8_t* idx, int oc, const uint8_t* sign_in, const uint8_t* sign_out, int o_sketch, float nk,
                                               float no, const T* query, int n_rep, const TP* proj, float* scores, int64_t row_len) {
   const float norm_in = 1.2533141373155001f / (float)SKETCH * sqrtf(fmaxf(nk * nk - no * no, 0.f)), norm_out = 1.2533141373155001f / (float)o_sketch * no;
+  if (oc < 0)
+    for (int h = 0; h < n_rep; ++h) scores[h * row_len] = __int_as_float(0x7fc00000);
   uint64_t seen_lo = 0, seen_hi = 0;
   for (int i = 0; i < oc; ++i) {
     const int d = idx[i] & (kHeadDim - 1);
@@ -554,12 +556,15 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
         }
         t = next;
       }
-      // every further mention of a channel, once the products' scores are written (within the loop it cost every call 6 %)
+      // every further mention of a channel, once the products' scores are written (within the loop it cost every call 6 %); NaN where a
+      // wait ran out, so that no score of the CTA stays what it was in memory
+      if (!ok) again_s = 1;
+      __syncwarp();
       if (again_s)
-        for (Tile t = first_tile(); t.i < n_tiles && ok; t = after(t))
+        for (Tile t = first_tile(); t.i < n_tiles; t = after(t))
           for (int n = t.first + quad; n < min(t.first + a.tg, a.n_groups); n += UNIT_G) {
             const int64_t group = (int64_t)t.kbh * a.n_groups + n, key = group * G + lane;
-            further_mentions<T, TP>(outlier_idx + group * a.oc, a.oc, key_quant + key * (SKETCH / 8), key_outlier_quant + key * (a.o_sketch / 8), a.o_sketch,
+            further_mentions<T, TP>(outlier_idx + group * a.oc, ok ? a.oc : -1, key_quant + key * (SKETCH / 8), key_outlier_quant + key * (a.o_sketch / 8), a.o_sketch,
                                     Elem<T>::to_f(key_norm[key]), Elem<T>::to_f(key_outlier_norm[key]), query + (int64_t)t.kbh * a.n_rep * kHeadDim,
                                     a.n_rep, proj, scores + (int64_t)t.kbh * a.n_rep * row_len + n * G + lane, row_len);
           }

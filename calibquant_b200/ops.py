@@ -68,8 +68,9 @@ def _workspace(nbytes: int, device, stream_handle=None) -> torch.Tensor:
 
 def device_status(device=None) -> int:
     """Sticky status word of the current stream's decode workspace (0 = no device-side wait has
-    timed out since the workspace was created), or that of refused positions (CQ_ERR_BAD_ARG until the next eager
-    step on the stream raises for them).  Synchronises the stream."""
+    timed out since the workspace was created), or that of the QJL sketch and score kernels of the device (whose scores are NaN where
+    a wait ran out), or that of refused positions (CQ_ERR_BAD_ARG until the next eager step on the stream raises for them).
+    Synchronises the stream."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else device
     stream = torch.cuda.current_stream(device)
     status = 0
@@ -77,6 +78,9 @@ def device_status(device=None) -> int:
         if status == 0:
             status = int(buf[:4].view(torch.int32).item())
     stream.synchronize()
+    if status == 0:
+        with _OnDevice(device):
+            status = lib().cq_qjl_status()
     return status or native().refused(device.index, stream.cuda_stream)
 
 

@@ -175,3 +175,15 @@ def test_small_projection():
     g = torch.Generator().manual_seed(15)
     S, q = torch.randn(128, 256, generator=g) * 1e-3, torch.randn(1, 4, 1, 128, generator=g)
     assert _error(_one(torch.half, S, q, n=60)) <= 2.1e-5
+
+
+def test_device_status_covers_the_scores(monkeypatch):
+    """No wait is made to run out: the library's answer is replaced on the host."""
+    from calibquant_b200 import _lib, ops
+
+    class TimedOut:
+        cq_qjl_status = staticmethod(lambda: _lib.CQ_ERR_TIMEOUT)
+
+    assert ops.device_status() == 0
+    monkeypatch.setattr(ops, "lib", TimedOut)
+    assert ops.device_status() == _lib.CQ_ERR_TIMEOUT
