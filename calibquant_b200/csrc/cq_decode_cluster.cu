@@ -138,9 +138,9 @@ template <typename T, int BITS, bool SPLIT, bool RAGGED>
 __global__ void __launch_bounds__(THREADS, 2)
 step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__ CUtensorMap tm_ks,
             const __grid_constant__ CUtensorMap tm_kmn, const __grid_constant__ CUtensorMap tm_v, const Args a,
-            const T* q, const int32_t* __restrict__ v_code, const T* __restrict__ v_scale, const T* __restrict__ v_mn,
+            const T* q, const int32_t* v_code, const T* v_scale, const T* v_mn,   // inputs: written by an overlapping launch, no read-only loads
             const T* k_fp, const T* v_fp, T* __restrict__ out, int* __restrict__ status,
-            const int32_t* __restrict__ k_code, const T* __restrict__ k_scale, const T* __restrict__ k_mn) {
+            const int32_t* k_code, const T* k_scale, const T* k_mn) {
   using T2 = typename D16<T>::T2;
   constexpr int NS = n_slots(BITS), UB = unit_bytes(BITS), CODE = 4096 * BITS;
   constexpr int GU = 4 / BITS, CHUNKS = UNIT_G / GU;       // groups per 16-byte chunk of a channel row, chunks of a key unit

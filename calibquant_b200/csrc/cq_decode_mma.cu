@@ -101,7 +101,7 @@ struct Dims {
 // Number of full-precision tokens this launch works on: the by-value extent, or, when the caller keeps
 // the count on the device (a decode step replayed from a CUDA graph), that count clamped to it.
 __device__ __forceinline__ int live_t_fp(const Dims& dm) {
-  return dm.t_fp_dev ? min(__ldg(dm.t_fp_dev), dm.t_fp) : dm.t_fp;
+  return dm.t_fp_dev ? min(*reinterpret_cast<const volatile int32_t*>(dm.t_fp_dev), dm.t_fp) : dm.t_fp;
 }
 
 // =================================================================================================
@@ -126,10 +126,9 @@ __device__ __forceinline__ int live_t_fp(const Dims& dm) {
 template <typename T, int BITS, bool SPLIT, bool LDG = false>
 __global__ void __launch_bounds__(K1_THREADS, k1_min_ctas(BITS))
 k1_scores(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__ CUtensorMap tm_ks,
-          const __grid_constant__ CUtensorMap tm_kmn, Dims dm, const T* __restrict__ q,
+          const __grid_constant__ CUtensorMap tm_kmn, Dims dm, const T* q,   // inputs: written by an overlapping launch, no read-only loads
           T* __restrict__ scores, float2* __restrict__ tile_mm, int* __restrict__ status,
-          const int32_t* __restrict__ code_g = nullptr, const T* __restrict__ ks_g = nullptr,
-          const T* __restrict__ kmn_g = nullptr) {
+          const int32_t* code_g = nullptr, const T* ks_g = nullptr, const T* kmn_g = nullptr) {
   using T2 = typename D16<T>::T2;
   constexpr int STAGES = k1_stages(BITS);
   constexpr int STAGE_BYTES = k1_stage_bytes(BITS);
@@ -468,7 +467,7 @@ k1_scores(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__ C
 // Writes the (max, sum, acc[128]) partials of the fp slots that k3 merges.
 template <typename T>
 __global__ void __launch_bounds__(THREADS)
-k2_fp_tokens(Dims dm, const T* __restrict__ q, const T* __restrict__ k_fp, const T* __restrict__ v_fp,
+k2_fp_tokens(Dims dm, const T* q, const T* k_fp, const T* v_fp,   // written by an overlapping launch: no read-only loads
              float* __restrict__ partial, float2* __restrict__ ml) {
   constexpr int PF_PITCH = 128 + 8;         // probability row pitch (elements): rows land on different banks
   constexpr int VROW = kHeadDim * 2 + 16;   // staged V row pitch in bytes, for conflict-free ldmatrix
@@ -494,8 +493,8 @@ k2_fp_tokens(Dims dm, const T* __restrict__ q, const T* __restrict__ k_fp, const
       uint32_t bq[8][2];
 #pragma unroll
       for (int kt = 0; kt < 8; ++kt) {
-        bq[kt][0] = g < dm.n_rep ? __ldg(reinterpret_cast<const uint32_t*>(qrow + kt * 16)) : 0u;
-        bq[kt][1] = g < dm.n_rep ? __ldg(reinterpret_cast<const uint32_t*>(qrow + kt * 16 + 8)) : 0u;
+        bq[kt][0] = g < dm.n_rep ? *reinterpret_cast<const uint32_t*>(qrow + kt * 16) : 0u;
+        bq[kt][1] = g < dm.n_rep ? *reinterpret_cast<const uint32_t*>(qrow + kt * 16 + 8) : 0u;
       }
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
@@ -506,10 +505,10 @@ k2_fp_tokens(Dims dm, const T* __restrict__ q, const T* __restrict__ k_fp, const
         uint32_t a[8][4];
 #pragma unroll
         for (int kt = 0; kt < 8; ++kt) {
-          a[kt][0] = __ldg(reinterpret_cast<const uint32_t*>(k_lo + kt * 16));
-          a[kt][1] = __ldg(reinterpret_cast<const uint32_t*>(k_hi + kt * 16));
-          a[kt][2] = __ldg(reinterpret_cast<const uint32_t*>(k_lo + kt * 16 + 8));
-          a[kt][3] = __ldg(reinterpret_cast<const uint32_t*>(k_hi + kt * 16 + 8));
+          a[kt][0] = *reinterpret_cast<const uint32_t*>(k_lo + kt * 16);
+          a[kt][1] = *reinterpret_cast<const uint32_t*>(k_hi + kt * 16);
+          a[kt][2] = *reinterpret_cast<const uint32_t*>(k_lo + kt * 16 + 8);
+          a[kt][3] = *reinterpret_cast<const uint32_t*>(k_hi + kt * 16 + 8);
         }
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -570,7 +569,7 @@ k2_fp_tokens(Dims dm, const T* __restrict__ q, const T* __restrict__ k_fp, const
       for (int i = tid; i < FP_SUB * 16; i += THREADS) {
         const int t = i >> 4, cidx = i & 15;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (ts + t < nt) v = __ldg(reinterpret_cast<const uint4*>(vf + (int64_t)(ts + t) * kHeadDim) + cidx);
+        if (ts + t < nt) v = reinterpret_cast<const uint4*>(vf + (int64_t)(ts + t) * kHeadDim)[cidx];
         *reinterpret_cast<uint4*>(smem + t * VROW + cidx * 16) = v;
       }
       __syncthreads();
@@ -617,8 +616,7 @@ template <typename T, int BITS, int VT>
 __global__ void __launch_bounds__(K2_THREADS, 2)
 k2_attn_v(const __grid_constant__ CUtensorMap tm_v,   // 2 and 4 bits: the value codes as [tokens][row words], swizzled boxes
           Dims dm, const T* scores, const float2* tile_mm,   // written by the launch before: no read-only loads
-          const int32_t* __restrict__ v_code, const T* __restrict__ v_scale,
-          const T* __restrict__ v_mn,
+          const int32_t* v_code, const T* v_scale, const T* v_mn,
           float* __restrict__ partial, float2* __restrict__ ml, int* __restrict__ status) {
   using T2 = typename D16<T>::T2;
   constexpr int STAGES = k2_stages(BITS, VT);
