@@ -3,8 +3,8 @@
 // What bounded the step as four launches (scores, softmax of a whole row per CTA, attn.V, finish): 107 us at 16 x 3328
 // tokens, 1 bit, of which 28 us were softmax CTAs that walked the full-precision keys one warp per key and 22 us were
 // finish CTAs that walked the full-precision values one row after the other; the scores went through memory as fp32.
-// Here a CTA owns a share of the visual tokens (items of 64) and of the full-precision tokens (tiles of 16), keeps its
-// scores in shared memory and does both products of both spans on the warp MMA:
+// Here a CTA owns a share of the visual tokens (items of 64, dealt out over its warps in 16-token tiles) and of the full-precision
+// tokens (tiles of 16), keeps its scores in shared memory and does both products of both spans on the warp MMA:
 //   1. visual scores, extremes -> every peer (remote stores), full-precision scores while they travel;
 //   2. calibration and mask, local maximum and sum of exponentials -> every peer: the global sum has to be known before
 //      a probability is rounded, because the reference rounds the normalised ones and multiplies their sum with the zero
@@ -14,8 +14,12 @@
 //      roundings.
 // Codes are read straight from global memory (the lanes of a row share their 16-byte loads; the span is on its way into L2
 // since the first instruction).  Two CTAs of eight warps per SM.  What bounds it now is the instructions of a warp waiting for each
-// other: 14 000 and 9000 of 46 600 cycles in the loops of the two products, 9400 in the passes over the scores.  16 x 8 heads x 3328
-// bfloat16 keys, 1 bit: 32.8 -> 30.7 us; 3 x 8 x 418 at 4 bits 16.7 -> 13.1; 12 x 8 x 1479 fp16 24.6 -> 21.1.  Nothing waits for another cluster; waits are bounded.
+// other: 14 000 and 9000 of 46 600 cycles in the loops of the two products, 9400 in the two passes over the scores.  16 x 8 heads x
+// 3328 bfloat16 keys, 1 bit, with the maximum from the extremes, shares of 16-token tiles, the next words ahead and two chains of
+// products together: 32.8 -> 30.7 us; 3 x 8 x 418 at 4 bits 16.7 -> 13.1; 12 x 8 x 1479 fp16 24.6 -> 21.1.  Nothing waits for another
+// cluster; waits are bounded.
+// The sums of the full-precision scores run over the channels in the order of the loads, so a score may round to the other of two
+// neighbouring numbers than in another order; against 64 bits the step is as near either way.
 #include <mutex>
 #include <type_traits>
 
@@ -33,7 +37,7 @@ using namespace ptx;
 using namespace cluster;
 
 constexpr int NW = 8, THREADS = NW * 32;
-constexpr int ITEM = 64;                        // visual tokens a warp takes at a time
+constexpr int ITEM = 64;                        // visual tokens by which the span is dealt out over the cluster
 constexpr int MAX_CLUSTER = 8;
 constexpr uint32_t WAIT_TRIES = 1u << 22;
 constexpr float LOG2E = 1.4426950408889634f;
@@ -172,7 +176,6 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
     // The warps take contiguous shares of the 16-token tiles (dealt out as items of 64 tokens, four rounds of eight warps were 3.25
     // items' work), MT at a time, and request the words of the next ones before they work on those at hand.
     constexpr int MT = BITS == 1 ? 2 : 1;
-    constexpr bool AHEAD = BITS < 4;              // at 4 bits there are no registers for it
     struct Words { uint32_t w[MT][2][WORDS]; };
     auto load = [&](Words& W, int m0) {
 #pragma unroll
@@ -221,7 +224,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
         }
       }
     };
-    if (AHEAD) {
+    if (BITS == 1) {
       Words W0, W1;
       if (m_first < m_last) load(W0, m_first);
 #pragma unroll 1
@@ -231,7 +234,17 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
         if (m + 2 * MT < m_last) load(W0, m + 2 * MT);
         if (m + MT < m_last) compute(W1, m + MT);
       }
-    } else {
+    } else if (BITS == 2) {      // one body and moves: 8 x 8 x 2000 tokens 17.3 -> 16.8 us, 16 x 8 x 3328 33.6 -> 32.4
+      Words W;
+      if (m_first < m_last) load(W, m_first);
+#pragma unroll 1
+      for (int m = m_first; m < m_last; m += MT) {
+        Words next;
+        load(next, min(m + MT, m_last - 1));
+        compute(W, m);
+        W = next;
+      }
+    } else {                     // no registers for words ahead
 #pragma unroll 1
       for (int m = m_first; m < m_last; m += MT) { Words W; load(W, m); compute(W, m); }
     }
@@ -575,7 +588,7 @@ u8_step_kernel(const Args a, const T* q, const uint8_t* enc_k, const uint8_t* en
         if (m + 1 < m_last) compute(W1, m + 1);
       }
     } else {
-#pragma unroll(BITS == 4 ? 1 : 2)
+#pragma unroll 1                                  // two bodies at 2 bits: 8 x 8 x 2000 tokens 18.2 us, one 17.3
       for (int m = m_first; m < m_last; ++m) { Words W; load(W, m); compute(W, m); }
     }
   }
