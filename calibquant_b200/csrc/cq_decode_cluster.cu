@@ -252,9 +252,9 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   };
   // The query, the newest full-precision token and freshly packed operands come from the launches before this one: nothing is
   // read before they have completed.  Steps that follow each other directly lose the overlap of the first loads with the tail
-  // of the step before: 1 x 8 x 256 tokens 11.1 us with the packed operands read ahead of the wait, 11.4 so; 4 x 8 x 5152
-  // 23.2, 24.0; 64 x 8 x 6656 164.5, 169.0.  (Requested into L2 ahead of the wait 16 x 8 x 3328 took 33.0: a bulk prefetch costs
-  // its thread as much as the load.)
+  // of the step before (timed before the wider pieces below: 1 x 8 x 256 tokens 11.1 us with the packed operands read ahead of the
+  // wait, 11.4 so; 4 x 8 x 5152 23.2, 24.0; 64 x 8 x 6656 164.5, 169.0; with them 10.9, 24.4 and 160.6).  (Requested into L2 ahead of
+  // the wait 16 x 8 x 3328 took 33.0: a bulk prefetch costs its thread as much as the load.)
   pdl_wait();
   const int t_live = a.t_fp_dev ? *reinterpret_cast<const volatile int32_t*>(a.t_fp_dev) : a.t_fp;      // on its way beside the loads below
   // the first loads of the slots, one by each warp (one after the other they took one thread 7000
@@ -471,13 +471,17 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
   // rounded to the data type, P.V with warp w owning channels 32 (w / 2) .. + 31 of every other 64 tokens.  Keys and values come
   // straight from global memory in pieces of 16 and 8 bytes: a lane's piece holds neighbouring channels, which the products take in
   // the order they come.  (In the fragments' own 4-byte pieces the 80 loads of a thread, eight rows each, took 6900 cycles a chunk.)
-  float fo[4][4] = {};
+  // At 4 bits values come in 4-byte pieces, channels 16 w .. + 15 of all tokens: half the sums to keep through attn.V, where that
+  // width has no registers left (with other kernels between the steps 2 x 8 x 5120 tokens 19.35 us with 8-byte pieces, 18.9 so;
+  // 4 x 8 x 5120 masked 20.2, 19.7).  Ragged spans keep the wide ones (4 x 8 x 5152 masked, one step after the other, 24.3 against 24.7).
+  constexpr int VW = BITS == 4 && !RAGGED ? 1 : 2;
+  float fo[2 * VW][4] = {};
   if (tid < kMaxRep) { fp_m[tid] = -INFINITY; fp_l[tid] = 0.f; }
   {
     int f0, f1;
     fp_range(f0, f1);
     const T* kf = k_fp + (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h;
-    const T* vf = v_fp + (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h + 32 * (warp >> 1) + 4 * g;
+    const T* vf = v_fp + (int64_t)b * a.fp_stride_b + (int64_t)hk * a.fp_stride_h + (VW == 2 ? 32 * (warp >> 1) + 4 * g : 16 * warp + 2 * g);
     const T* mrow = a.mask ? static_cast<const T*>(a.mask) + (int64_t)b * a.mask_stride_b : nullptr;
     for (int t0 = f0; t0 < f1; t0 += FPC) {
       const int nt = min(FPC, f1 - t0);
@@ -505,14 +509,16 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
           if (h < a.n_rep && t < nt) pf_s[h * PF_PITCH + t] = Elem<T>::from_f(__fdiv_rn(rnd<T>(acc[e]), 11.313708498984761f));
         }
       }
-      const int th = 64 * (warp & 1);
-      uint2 v[FPC / 32][4];                 // tokens th + 16k + 2c + {0, 1, 8, 9}, four channels; on their way during the softmax
+      using Piece = typename std::conditional<VW == 2, uint2, uint32_t>::type;
+      constexpr int NK = FPC / (16 * VW);
+      const int th = VW == 2 ? 64 * (warp & 1) : 0;
+      Piece v[NK][4];                       // tokens th + 16k + 2c + {0, 1, 8, 9}, 2 VW channels; on their way during the softmax
 #pragma unroll
-      for (int k = 0; k < FPC / 32; ++k)
+      for (int k = 0; k < NK; ++k)
 #pragma unroll
         for (int r = 0; r < 4; ++r)         // past the end p is 0 and the value repeats the last token
-          v[k][r] = th + 16 * k < nt ? *reinterpret_cast<const uint2*>(vf + (int64_t)(t0 + min(th + 16 * k + 2 * c + (r & 1) + 8 * (r >> 1), nt - 1)) * kHeadDim)
-                                     : make_uint2(0u, 0u);
+          v[k][r] = th + 16 * k < nt ? *reinterpret_cast<const Piece*>(vf + (int64_t)(t0 + min(th + 16 * k + 2 * c + (r & 1) + 8 * (r >> 1), nt - 1)) * kHeadDim)
+                                     : Piece{};
       __syncthreads();
       if (warp < a.n_rep) {                 // warp = head
         const int h = warp;
@@ -546,17 +552,19 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
       {
         const float alpha = g < a.n_rep ? fp_alpha[g] : 0.f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { fo[j][0] *= alpha; fo[j][1] *= alpha; }
+        for (int j = 0; j < 2 * VW; ++j) { fo[j][0] *= alpha; fo[j][1] *= alpha; }
         const T* prow = pf_s + (g < a.n_rep ? g : 0) * PF_PITCH + th + 2 * c;
 #pragma unroll
-        for (int k = 0; k < FPC / 32; ++k) {
+        for (int k = 0; k < NK; ++k) {
           if (th + 16 * k >= nt) break;
           const uint32_t p0 = *reinterpret_cast<const uint32_t*>(prow + 16 * k), p1 = *reinterpret_cast<const uint32_t*>(prow + 16 * k + 8);
-          // n-tile j: column n stands for channel 32 (w / 2) + 4n + j
-          mma_t<T>(fo[0], p0, 0u, p1, 0u, prmt(v[k][0].x, v[k][1].x, 0x5410), prmt(v[k][2].x, v[k][3].x, 0x5410));
-          mma_t<T>(fo[1], p0, 0u, p1, 0u, prmt(v[k][0].x, v[k][1].x, 0x7632), prmt(v[k][2].x, v[k][3].x, 0x7632));
-          mma_t<T>(fo[2], p0, 0u, p1, 0u, prmt(v[k][0].y, v[k][1].y, 0x5410), prmt(v[k][2].y, v[k][3].y, 0x5410));
-          mma_t<T>(fo[3], p0, 0u, p1, 0u, prmt(v[k][0].y, v[k][1].y, 0x7632), prmt(v[k][2].y, v[k][3].y, 0x7632));
+          // n-tile j: column n stands for channel 32 (w / 2) + 4n + j (4 bits: 16w + 2n + j)
+#pragma unroll
+          for (int i = 0; i < VW; ++i) {
+            auto word = [&](int r) { return reinterpret_cast<const uint32_t*>(&v[k][r])[i]; };
+            mma_t<T>(fo[2 * i], p0, 0u, p1, 0u, prmt(word(0), word(1), 0x5410), prmt(word(2), word(3), 0x5410));
+            mma_t<T>(fo[2 * i + 1], p0, 0u, p1, 0u, prmt(word(0), word(1), 0x7632), prmt(word(2), word(3), 0x7632));
+          }
         }
       }
       __syncthreads();       // the probabilities have been used
@@ -700,13 +708,17 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
     }
   }
   __syncthreads();            // the ring is idle: it holds the warps' sums from here on
-  float* fp_o = reinterpret_cast<float*>(smem) + NW * kMaxRep * RED_STRIDE;      // [token half][head][channel]
+  float* fp_o = reinterpret_cast<float*>(smem) + NW * kMaxRep * RED_STRIDE;      // [token half (one at 4 bits)][head][channel]
   {
     float* mine = reinterpret_cast<float*>(smem) + warp * kMaxRep * RED_STRIDE;
-    if (g < a.n_rep) {                       // fragment columns 2c, 2c+1 of n-tile j = channels 32 (w / 2) + 8c + j, + 4
-      float4* dst = reinterpret_cast<float4*>(fp_o + ((warp & 1) * kMaxRep + g) * kHeadDim + 32 * (warp >> 1) + 8 * c);
-      dst[0] = make_float4(fo[0][0], fo[1][0], fo[2][0], fo[3][0]);
-      dst[1] = make_float4(fo[0][1], fo[1][1], fo[2][1], fo[3][1]);
+    if (g < a.n_rep) {                       // fragment columns 2c, 2c+1 of n-tile j = channels 32 (w / 2) + 8c + j, + 4 (4 bits: 16w + 4c + j, + 2)
+      if constexpr (VW == 2) {
+        float4* dst = reinterpret_cast<float4*>(fp_o + ((warp & 1) * kMaxRep + g) * kHeadDim + 32 * (warp >> 1) + 8 * c);
+        dst[0] = make_float4(fo[0][0], fo[1][0], fo[2][0], fo[3][0]);
+        dst[1] = make_float4(fo[0][1], fo[1][1], fo[2][1], fo[3][1]);
+      } else {
+        *reinterpret_cast<float4*>(fp_o + g * kHeadDim + 16 * warp + 4 * c) = make_float4(fo[0][0], fo[1][0], fo[0][1], fo[1][1]);
+      }
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -743,7 +755,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_code, const __grid_constant__
     // this CTA's visual and full-precision parts under one reference
     const float m_v = n_u > 0 ? __uint_as_float(cal_s[h][5]) : -INFINITY, m_f = fp_m[h], m = fmaxf(m_v, m_f);
     const float wv = m_v == -INFINITY ? 0.f : exp2f((m_v - m) * LOG2E), wf = m_f == -INFINITY ? 0.f : exp2f((m_f - m) * LOG2E);
-    o = o * wv + (fp_o[e] + fp_o[kMaxRep * kHeadDim + e]) * wf;
+    o = o * wv + (VW == 2 ? fp_o[e] + fp_o[kMaxRep * kHeadDim + e] : fp_o[e]) * wf;
     const int peer = e / slice;
     st_peer(map_peer(smem_u32(&recv_o[rank * slice + e % slice]), peer), o);
     if (d < S) st_peer2(map_peer(smem_u32(&recv_ml[rank][h]), d), m, l * wv + fp_l[h] * wf);
