@@ -155,8 +155,15 @@ quant_encode_kernel(const T* __restrict__ x, int heads, int t_len, int64_t sb, i
       for (int u = 0; u < KEEP; ++u)
         if (t_begin + u * QE_LANES < t_end) encode(t_begin + tl + u * QE_LANES, kept[KEPT ? u : 0]);
     } else {
-      for (int t = t_begin + tl; t < t_last; t += QE_LANES)
-        encode(t, ptx::ld_global16(base + (int64_t)min(t, t_end - 1) * st));
+      // two rows requested together (one after the other 1 x 8 x 4096 tokens at 4 bits took 16.0 us, so 14.5; 16 x 3328 82.1, 78.8; four:
+      // 14.0, 82.0)
+      for (int t0 = t_begin + tl; t0 < t_last; t0 += 2 * QE_LANES) {
+        uint4 v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) v[u] = ptx::ld_global16(base + (int64_t)min(t0 + u * QE_LANES, t_end - 1) * st);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) encode(t0 + u * QE_LANES, v[u]);
+      }
     }
     return;
   }
