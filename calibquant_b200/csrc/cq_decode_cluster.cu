@@ -789,7 +789,9 @@ constexpr int STATIC_SMEM = 9 * 1024;           // upper bound of the kernel's s
 constexpr int SMEM_TWO = 113 * 1024 - STATIC_SMEM;
 
 // Estimates in microseconds, fitted to steps timed both ways and with every cluster size (7376 shapes: batch 1-64, 32 to 32768
-// visual and up to 1000 full-precision tokens, 1 to 8 query heads, all bit widths; they hold to about a tenth).
+// visual and up to 1000 full-precision tokens, 1 to 8 query heads, all bit widths; they held to about a tenth).  The single launch has
+// become 2 to 6 % faster since and the constants were not fitted anew: of 400 drawn shapes timed in both forms, one step after the other,
+// 79 took more than 3 % longer than the other form would, 27 % at most (2 x 8 x 8192 at 4 bits 19.4 us against 15.2).
 struct Cost {
   double unit, unit_ragged;      // a CTA's time per 256 visual tokens
   double split, split_ragged;    // the separate launches', per 256 tokens of a KV head and SM
@@ -808,7 +810,7 @@ inline Cost cost_of(int bits) {
 //   * More pairs than that, 1 and 2 bits, clusters of one or two with up to 16 units and three chunks a CTA: several rounds,
 //     where the last one is at least 0.85 full and there are at most four, or where the second of two is a quarter to a half
 //     full, when its CTAs have an SM each (294 shapes timed: 0.95 of the separate launches' time, 26 of them slower by more than
-//     3 %; 64 x 8 x 6656 at 2 bits and six heads 169 against 179; 80 x 8 x 3328, 2.16 rounds, would take 111 against 107).
+//     3 %; 64 x 8 x 6656 at 2 bits and six heads 169 against 179, 161 now; 80 x 8 x 3328, 2.16 rounds, would take 111 against 107).
 inline bool make_plan(const cq_decode_args* a, Plan* p) {
   const int n_rep = a->n_q_heads / a->n_kv_heads, n_units = (a->t_vis + UNIT_TOK - 1) / UNIT_TOK;
   const int fp_chunks = (a->t_fp + FPC - 1) / FPC, most = n_units > (a->t_fp + 63) / 64 ? n_units : (a->t_fp + 63) / 64;

@@ -786,7 +786,8 @@ extern "C" int cq_qjl_gqa_score(const uint8_t* key_quant, const uint8_t* key_out
   // sketch rows that are whole 16-byte words: the persistent tensor-core kernel, one CTA per SM
   const bool use_mma = sketch_dim % 128 == 0 && outlier_sketch_dim % 128 == 0 && qjl::mma_ptrs_ok(key_quant, key_outlier_quant) && aligned16(proj_score);
   if (!query_sketch && !use_mma) return CQ_ERR_UNSUPPORTED;
-  // 8 x 8 x 16384 keys, four heads: 129 us on the warp MMA, 87 here; 1 x 8 x 512 15.1 and 10.2, 1 x 8 x 8192 16.2 and 15.9
+  // 8 x 8 x 16384 keys, four heads: 133 us on the warp MMA, 87 here; 1 x 8 x 512 15.2 and 10.0, 1 x 8 x 8192 15.9 and 14.9, a single
+  // group 10.5 and 10.0; eight outlier channels 1 x 8 x 8192 15.5 and 15.0
   if (use_mma && qjl_score::eligible(key_quant, key_outlier_quant, group_size, sketch_dim, outlier_sketch_dim, n_rep))
     return qjl_score::run(key_quant, key_outlier_quant, key_norm, key_outlier_norm, outlier_indices, query_sketch, query, proj_score, proj_dtype,
                           batch * n_kv_heads, n_rep, n_groups, outlier_sketch_dim, outlier_count, dtype, scores, st);

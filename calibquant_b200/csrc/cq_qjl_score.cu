@@ -11,14 +11,19 @@
 //      the warps.  A KV head's first tile carries the unmasked queries as well: q S.
 //   2. sums over set sign bits of a unit of 128 keys (4 groups): A = the bits, written by the warps into tensor memory as fp16
 //      powers of two; B = [projection][q_out S hi | lo of 4 groups x 4 heads, q S hi | lo of 4 heads] as read back from (1).
-//      Only a key's own group's columns count (3/4 of the work is idle; the pipe has room for it).
+//      Only a key's own group's columns count (3/4 of the work is idle).
 //      sum_p sgn_p x_p = 2 sum_{bit p} x_p - sum_p x_p, the latter from channel sums of S: sum_p (q_out S)_p = q_out (S 1).
 // A bit stays where it is in its word: one AND makes two operand elements, of weight 2^(i-24) for bit i.  The rows of B carry the
 // inverse.  Bits 4-11 of each half word are used in place, the others after one rotation by eight, so the weights span 2^7.
-// Six roles of warps (below) hand these steps on through mbarriers.  What bounds it now: a tcgen05.mma of 128 rows takes ~70 cycles of
-// the pipe however few columns it has, 32 of them a unit and 32 a tile: 2600 of the 2900 cycles that a unit takes.  8 x 8 x 16384 keys,
-// 32 query heads: 129 -> 87 us; 1 x 8 x 512 keys 15.1 -> 10.2 us; error against 64-bit sums 4.6e-6 -> 7e-7 (the product truncates less
-// often than the warp MMA).  Every wait is bounded; on a timeout the CTA writes the status word and NaN for its scores, frees its tensor memory and returns.
+// Six roles of warps (below) hand these steps on through mbarriers.  What bounds it now is that chain and no unit by itself: a unit
+// of 8 x 8 x 16384 keys takes about 2700 cycles, and without 16 of its 40 products the call takes 84.0 us instead of 87.2, with half
+// of the first product 81.5, without the sums of the masked queries 84.1 (an outlier sketch of 128 bits, whose second half is
+// multiplied although it is zero, would gain 1 % without it).
+// 8 x 8 x 16384 keys, 32 query heads: 129 -> 87 us on the way from the warp MMA; 1 x 8 x 512 keys 15.3 -> 10.0 us; error against 64-bit sums
+// 4.6e-6 -> 3.5e-7 (the product truncates less often than the warp MMA).  The inlier part by itself, of a query that lies 300 to 1 in
+// the outlier channels, is off by 6.4e-5, on the warp MMA by 4.2e-5: q S and q_out S are summed apart and subtracted after the signs,
+// and an fp32 difference ahead of them cost 5 us for 5.9e-5; the whole score of such a query 2.2e-6 and 5.0e-6.
+// Every wait is bounded; on a timeout the CTA writes the status word and NaN for its scores, frees its tensor memory and returns.
 #include <type_traits>
 
 #include "cq_common.cuh"
@@ -33,6 +38,7 @@ using namespace tc;
 
 constexpr int G = 32, SKETCH = 256, R = 4;                 // keys of a group, projections, query heads per KV head (at most)
 constexpr int UNIT_G = 4, MAX_TG = 16;                     // groups of a unit, of a tile (at most)
+constexpr int SLOTS = 8;                                   // tiles whose totals are kept
 // warps by role: sign bits, sketches of the query, scores, masked queries, and one issuer for either product.  (Where one warp did
 // several of these, each waited for the slowest of its own steps: 118 us with two roles and one issuer, 8 x 8 x 16384 keys.)
 constexpr int N_SIGN = 8, N_SKETCH = 8, N_SCORE = 4, N_QUERY = 4;
@@ -120,9 +126,12 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
   __shared__ __align__(8) uint64_t bar_q, bar_out, bar_out_free, bar_x[2], bar_x_free[2], bar_sign[2], bar_done[2], bar_sum_free;
   __shared__ uint32_t tmem_s;
   __shared__ __align__(16) float sum_in_s[kHeadDim], sum_out_s[kHeadDim];      // per channel: sums of S over all / the outlier sketch's projections
-  // per tile; the scores of a tile may be behind the queries of the fourth tile after it
-  __shared__ float tot_in_s[8][MAX_TG][R], tot_out_s[8][MAX_TG][R];            // sums of q_out S
-  __shared__ float tot_q_s[8][R], down_s[8][R], up_s[8][R];                    // sums of q S; powers of two of the queries' scaling
+  // A slot per tile.  With tiles of one unit the queries of tile t are built while the scores of t - 5 may still be read: they follow
+  // the first product of t - 1, that one the sketches of t - 2, these (two operand buffers) the sums of t - 4, and these the
+  // arrival of the scores of t - 5, which comes before their reading of the slot.
+  static_assert(SLOTS > 5 && (SLOTS & (SLOTS - 1)) == 0, "a ring of more tiles than the queries are ahead of the scores");
+  __shared__ float tot_in_s[SLOTS][MAX_TG][R], tot_out_s[SLOTS][MAX_TG][R];    // sums of q_out S
+  __shared__ float tot_q_s[SLOTS][R], down_s[SLOTS][R], up_s[SLOTS][R];        // sums of q S; powers of two of the queries' scaling
   __shared__ float smax_s[N_WARPS];
   __shared__ int again_s;                                                      // does a group of the CTA name a channel more than once?
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -315,7 +324,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
         }
       };
       auto build_queries = [&](const Tile& t) {
-        const int slot = t.i & 7;
+        const int slot = t.i & (SLOTS - 1);
         if (t.fresh) {
           // scaled so that the elements, their sums with 128 channels and a given q S stay below 2^15: fp16 operands keep what they
           // can of the remainders
@@ -360,7 +369,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
             if (qc == 0) { tot_q_s[slot][qh] = tq; down_s[slot][qh] = down; up_s[slot][qh] = up; }
           }
         } else if (wq == 0 && qc == 0) {
-          tot_q_s[slot][qh] = tot_q_s[(slot + 7) & 7][qh]; down_s[slot][qh] = down_s[(slot + 7) & 7][qh];
+          tot_q_s[slot][qh] = tot_q_s[(slot + SLOTS - 1) & (SLOTS - 1)][qh]; down_s[slot][qh] = down_s[(slot + SLOTS - 1) & (SLOTS - 1)][qh];
         }
         int missing = 0;                       // mentions less channels
 #pragma unroll 1
@@ -426,7 +435,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
           if (query_sketch) {
             const float* qs = query_sketch + (int64_t)t.kbh * a.n_rep * SKETCH + 128 * mt + 32 * quad + lane;
 #pragma unroll
-            for (int h = 0; h < R; ++h) r[h] = h < a.n_rep ? __float_as_uint(qs[h * SKETCH] * up_s[t.i & 7][h]) : 0u;
+            for (int h = 0; h < R; ++h) r[h] = h < a.n_rep ? __float_as_uint(qs[h * SKETCH] * up_s[t.i & (SLOTS - 1)][h]) : 0u;
           }
           split2(__uint_as_float(r[0]) * weight, __uint_as_float(r[1]) * weight, sq.x, sq.z);
           split2(__uint_as_float(r[2]) * weight, __uint_as_float(r[3]) * weight, sq.y, sq.w);
@@ -521,7 +530,7 @@ score_kernel(const Args a, const uint8_t* __restrict__ key_quant, const uint8_t*
       fetch(t, 0);
       while (t.i < n_tiles) {
         const Tile next = after(t);
-        const int slot = t.i & 7;
+        const int slot = t.i & (SLOTS - 1);
         for (int u = 0; u < t.units; ++u, ++v) {
           const float nk = Elem<T>::to_f(norm_k), no = Elem<T>::to_f(norm_o);
           const bool more = u + 1 < t.units;
@@ -603,8 +612,8 @@ int run(const uint8_t* kq, const uint8_t* koq, const void* kn, const void* kon, 
   Args a;
   a.n_kbh = n_kbh; a.n_groups = n_groups; a.n_rep = n_rep; a.o_sketch = o_sketch; a.oc = oc;
   // groups per tile: the first product costs a tile about as much as two thirds of a unit, whatever its width; smaller tiles where
-  // they fill the SMs better or
-  // hold the same groups (1 x 4 groups: 11.2 us with a tile of 16, 10.0 with one of 4; on the warp MMA 10.8)
+  // they fill the SMs better, or where they hold the same groups (four heads of 4 groups: 11.2 us with tiles of 16, 10.0 with tiles of
+  // 4; on the warp MMA 10.8)
   a.n_tiles = 0;
   double best = 1e30;
   for (int tg = MAX_TG; tg >= UNIT_G; tg /= 2) {
